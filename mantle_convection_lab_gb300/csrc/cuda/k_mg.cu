@@ -17,14 +17,7 @@
 //                      re-discretised coarse operators with injected
 //                      viscosity, dense inverse on the coarsest grid.
 //
-// The operator is matrix-free.  A tile of 8 x 32 nodes stages its patch of
-// nodal velocity and viscosity (10 x 34 nodes) in shared memory, computes the
-// three stress components at the 4 Gauss points of each of its 9 x 33
-// elements into shared memory, then every thread gathers the two rows of its
-// own node from its 4 elements in a fixed order (deterministic, no atomics).
-// With D = diag(2 eta, 2 eta, eta) and unit-Jacobian derivatives
-// Dx = dN/dxi * sqrt(r), Dz = dN/deta / sqrt(r), r = dz/dx, this is exactly
-// the element matrix of get_element_K (Build_matrix.c:192-271).
+// The operator is matrix-free (k_march.cuh).
 #include <math.h>
 #include "k_mg.cuh"
 
@@ -36,6 +29,9 @@ MCLG_SHAPE_UPLOAD(upload_shape_tables_mg)
 template <class T>
 struct OpTab {
 	T N[4][4], Dx[4][4], Dz[4][4];
+	// the two magnitudes of Dx and Dz over the Gauss points, and of the linear
+	// interpolation along an edge to a Gauss point (k_march.cuh)
+	T axp, axm, azp, azm, p, q;
 };
 __constant__ OpTab<float> cTf;
 __constant__ OpTab<double> cTd;
@@ -58,6 +54,24 @@ void upload_op_tables(const ShapeTables &S, double r, cudaStream_t st)
 			f.Dx[a][g] = (float)d.Dx[a][g];
 			f.Dz[a][g] = (float)d.Dz[a][g];
 		}
+	// corner 2 (xi = eta = 1): dN/dxi = (1 + eta_g)/4
+	double ap = S.dNdxi[2][0], am = S.dNdxi[2][0];
+	for (int g = 1; g < 4; g++) {
+		ap = fmax(ap, S.dNdxi[2][g]);
+		am = fmin(am, S.dNdxi[2][g]);
+	}
+	d.axp = ap * sr;
+	d.axm = am * sr;
+	d.azp = ap / sr;
+	d.azm = am / sr;
+	d.p = 2.0 * ap;
+	d.q = 2.0 * am;
+	f.axp = (float)d.axp;
+	f.axm = (float)d.axm;
+	f.azp = (float)d.azp;
+	f.azm = (float)d.azm;
+	f.p = (float)d.p;
+	f.q = (float)d.q;
 	cudaMemcpyToSymbolAsync(cTd, &d, sizeof d, 0, cudaMemcpyHostToDevice, st);
 	cudaMemcpyToSymbolAsync(cTf, &f, sizeof f, 0, cudaMemcpyHostToDevice, st);
 }
@@ -89,8 +103,8 @@ __device__ __forceinline__ int morton(int ex, int ez)
 	return (int)((spread_bits((unsigned)ex) << 1) | spread_bits((unsigned)ez));
 }
 
-// ---- the tiled matrix-free operator ----------------------------------------
-#include "k_tile.cuh"
+// ---- the matrix-free operator -----------------------------------------------
+#include "k_march.cuh"
 
 // Inverse diagonal of the level operator (the element diagonals summed).
 template <class T, class V>
@@ -157,25 +171,6 @@ __device__ void restrict_res(Part pt, const MGLevel<T> &F, const MGLevel<T> &C)
 		o.x = (m & 1u) ? T(0) : su;
 		o.y = (m & 2u) ? T(0) : sw;
 		C.b[A] = o;
-	}
-}
-
-// out = x_f + P x_c (bilinear).
-template <class T, class V>
-__device__ void prolong_add(Part pt, const MGLevel<T> &F, const V *xf, V *out, const MGLevel<T> &C, const V *xc)
-{
-	int i0, st;
-	span(pt, i0, st);
-	for (int A = i0; A < F.n * F.n; A += st) {
-		const int fx = A / F.n, fz = A - fx * F.n;
-		const int x0 = fx >> 1, z0 = fz >> 1, x1 = (fx + 1) >> 1, z1 = (fz + 1) >> 1;
-		const V a = xc[z0 + x0 * C.n], b = xc[z1 + x0 * C.n], c = xc[z0 + x1 * C.n], d = xc[z1 + x1 * C.n];
-		const T cu = T(0.25) * ((a.x + b.x) + (c.x + d.x)), cw = T(0.25) * ((a.y + b.y) + (c.y + d.y));
-		const unsigned m = F.mask[A];
-		V o = xf[A];
-		o.x = (m & 1u) ? T(0) : o.x + cu;
-		o.y = (m & 2u) ? T(0) : o.y + cw;
-		out[A] = o;
 	}
 }
 
@@ -271,30 +266,55 @@ __device__ void coarse_solve(const MGHier<T> &H, V *x)
 }
 
 // ---- one V(nu,nu) cycle: out0 = B rhs0 -----------------------------------------
-// Levels below nblk run on the whole grid (grid barriers); the small levels
+// Levels below nblk run on the whole team (team barriers); the small levels
 // from nblk down run inside block 0 alone (block barriers).  Every block walks
 // the same buffer bookkeeping so that all of them know where each level's
 // result lies; only the active blocks do the work.
 template <class T>
-__device__ void level_down(Sync &sy, unsigned char *sm, const MGHier<T> &H, int l,
-                           const typename V2T<T>::t *rhs0, bool grid, bool active, typename V2T<T>::t **xcur)
+__device__ __forceinline__ Pass<T> level_pass(const MGLevel<T> &L, const typename V2T<T>::t *b)
+{
+	Pass<T> P;
+	P.N = L.N;
+	P.mask = L.mask;
+	P.eta = L.eta;
+	P.invD = L.invD;
+	P.b = b;
+	P.x = P.xc = P.x0 = nullptr;
+	P.out = P.xout = P.bout = nullptr;
+	P.nc = 0;
+	P.omega = P.wload = P.c0 = T(0);
+	P.cx = T(1);
+	P.dotv = nullptr;
+	return P;
+}
+
+template <class T>
+__device__ void level_down(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, bool grid, bool active,
+                           typename V2T<T>::t **xcur)
 {
 	typedef typename V2T<T>::t V;
 	const MGLevel<T> &L = H.lv[l];
-	const V *b = (l == 0) ? rhs0 : L.b;
 	const int nu = l < H.lfine ? H.nu : H.nu_c;
+	V *x = L.xa, *xt = L.xb;
 	// below the finest level the right-hand side P^T r of the finer level is
 	// formed in this level's first pass (and stored for its later passes)
-	const int xs0 = l >= 1 ? XS_ZERO_R : XS_ZERO;
-	const V *rf = l >= 1 ? H.lv[l - 1].r : nullptr;
-	const int nf = l >= 1 ? H.lv[l - 1].n : 0;
-	V *bo = l >= 1 ? L.b : nullptr;
-	V *x = L.xa, *xt = L.xb;
+	Pass<T> P = level_pass<T>(L, l == 0 ? rhs0 : L.b);
+	if (l >= 1) {
+		P.xc = H.lv[l - 1].r;
+		P.nc = H.lv[l - 1].n;
+		P.bout = L.b;
+	}
+	const Part pt = sy.part(grid);
 	if (nu == 1) {
 		// one sweep from zero, x = omega D^-1 b, formed inside the residual pass
 		if (active) {
-			tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, xt, b, L.invD, L.r, PASS_RESID, H.omega, nullptr,
-			                xs0, rf, nf, nullptr, nullptr, nullptr, nullptr, bo, x);
+			P.wload = H.omega;
+			P.out = L.r;
+			P.xout = x;
+			if (l >= 1)
+				march<T, PASS_RESID, XS_ZERO_R, false>(P, pt, nullptr);
+			else
+				march<T, PASS_RESID, XS_ZERO, false>(P, pt, nullptr);
 			barrier(sy, grid);
 		}
 	} else {
@@ -302,14 +322,23 @@ __device__ void level_down(Sync &sy, unsigned char *sm, const MGHier<T> &H, int 
 		// x1 = w1 D^-1 b, x2 = c1 x1 + w2 D^-1 (b - A x1)
 		const bool ch = H.cheb && nu == 2;
 		if (active) {
-			tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, xt, b, L.invD, x, PASS_SMOOTH,
-			                ch ? H.w2 : H.omega, nullptr, xs0, rf, nf, nullptr, nullptr, nullptr, nullptr, bo, nullptr,
-			                ch ? H.w1 : T(-1), ch ? H.c1 : T(1));
+			P.wload = ch ? H.w1 : H.omega;
+			P.omega = ch ? H.w2 : H.omega;
+			P.cx = ch ? H.c1 : T(1);
+			P.out = x;
+			if (l >= 1)
+				march<T, PASS_SMOOTH, XS_ZERO_R, false>(P, pt, nullptr);
+			else
+				march<T, PASS_SMOOTH, XS_ZERO, false>(P, pt, nullptr);
 			barrier(sy, grid);
 		}
+		P.cx = T(1);
+		P.omega = H.omega;
 		for (int s = 2; s < nu; s++) {
 			if (active) {
-				tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, x, b, L.invD, xt, PASS_SMOOTH, H.omega, nullptr);
+				P.x = x;
+				P.out = xt;
+				march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, nullptr);
 				barrier(sy, grid);
 			}
 			V *tmp = x;
@@ -317,14 +346,16 @@ __device__ void level_down(Sync &sy, unsigned char *sm, const MGHier<T> &H, int 
 			xt = tmp;
 		}
 		if (active) {
-			tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, x, b, L.invD, L.r, PASS_RESID, H.omega, nullptr);
+			P.x = x;
+			P.out = L.r;
+			march<T, PASS_RESID, XS_PLAIN, false>(P, pt, nullptr);
 			barrier(sy, grid);
 		}
 	}
 	// the next level forms its right-hand side from L.r in its first pass,
 	// except the coarsest (a dense solve)
 	if (active && l + 1 == H.nlev - 1) {
-		restrict_res<T, V>(sy.part(grid), L, H.lv[l + 1]);
+		restrict_res<T, V>(pt, L, H.lv[l + 1]);
 		barrier(sy, grid);
 	}
 	xcur[l] = x;
@@ -334,17 +365,20 @@ __device__ void level_down(Sync &sy, unsigned char *sm, const MGHier<T> &H, int 
 // share of out0.dotv into *dot and is not followed by a barrier: the caller's
 // reduction provides it.
 template <class T>
-__device__ void level_up(Sync &sy, unsigned char *sm, const MGHier<T> &H, int l,
-                         const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0, bool grid, bool active,
-                         typename V2T<T>::t **xcur, const double2 *dotv = nullptr, double *dot = nullptr)
+__device__ void level_up(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
+                         bool grid, bool active, typename V2T<T>::t **xcur, const double2 *dotv = nullptr,
+                         double *dot = nullptr)
 {
 	typedef typename V2T<T>::t V;
 	const MGLevel<T> &L = H.lv[l];
-	const V *b = (l == 0) ? rhs0 : L.b;
 	V *x = xcur[l];
 	V *xt = (x == L.xa) ? L.xb : L.xa;
 	const MGLevel<T> &C = H.lv[l + 1];
 	const int nu = l < H.lfine ? H.nu : H.nu_c;
+	const Part pt = sy.part(grid);
+	Pass<T> P = level_pass<T>(L, l == 0 ? rhs0 : L.b);
+	P.xc = xcur[l + 1];
+	P.nc = C.n;
 	// the coarse-grid correction x + P xc is formed inside the first post-smoothing
 	// sweep; the Chebyshev pair keeps that iterate (x0) in L.r, free on the way up,
 	// for x2 = c1 x1 - c0 x0 + w2 D^-1 (b - A x1)
@@ -354,17 +388,24 @@ __device__ void level_up(Sync &sy, unsigned char *sm, const MGHier<T> &H, int l,
 		V *dst = last ? out0 : xt;
 		double *dp = (last && dotv) ? dot : nullptr;
 		if (active) {
-			if (s == 0)
-				tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, x, b, L.invD, dst, PASS_SMOOTH,
-				                ch ? H.w1 : H.omega, dp, XS_PROLONG, xcur[l + 1], C.n, dotv, nullptr, nullptr, nullptr,
-				                nullptr, ch ? L.r : nullptr);
-			else if (ch)
-				tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, x, b, L.invD, dst, PASS_SMOOTH, H.w2, dp,
-				                XS_PLAIN, nullptr, 0, dotv, nullptr, nullptr, nullptr, nullptr, nullptr, T(-1), H.c1,
-				                L.r, H.c0);
-			else
-				tile_pass<T, V>(sm, sy.part(grid), L.N, L.mask, L.eta, x, b, L.invD, dst, PASS_SMOOTH, H.omega, dp,
-				                XS_PLAIN, nullptr, 0, dotv);
+			P.x = x;
+			P.out = dst;
+			P.dotv = dp ? dotv : nullptr;
+			if (s == 0) {
+				P.omega = ch ? H.w1 : H.omega;
+				P.xout = ch ? L.r : nullptr;
+				march<T, PASS_SMOOTH, XS_PROLONG, false>(P, pt, dp);
+			} else if (ch) {
+				P.omega = H.w2;
+				P.cx = H.c1;
+				P.c0 = H.c0;
+				P.x0 = L.r;
+				P.xout = nullptr;
+				march<T, PASS_SMOOTH, XS_PLAIN, true>(P, pt, dp);
+			} else {
+				P.omega = H.omega;
+				march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, dp);
+			}
 			if (!dp)
 				barrier(sy, grid);
 		}
@@ -378,8 +419,8 @@ __device__ void level_up(Sync &sy, unsigned char *sm, const MGHier<T> &H, int l,
 // and the cycle ends without a barrier (the caller reduces *dot, which
 // synchronises the team); without it the cycle ends with a barrier.
 template <class T>
-__device__ void vcycle(Sync &sy, unsigned char *sm, const MGHier<T> &H, const typename V2T<T>::t *rhs0,
-                       typename V2T<T>::t *out0, const double2 *dotv = nullptr, double *dot = nullptr)
+__device__ void vcycle(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
+                       const double2 *dotv = nullptr, double *dot = nullptr)
 {
 	typedef typename V2T<T>::t V;
 	V *xcur[kMaxLev];
@@ -390,25 +431,29 @@ __device__ void vcycle(Sync &sy, unsigned char *sm, const MGHier<T> &H, const ty
 	if (dot)
 		*dot = 0.0;
 	for (int l = 0; l < lc; l++)
-		level_down<T>(sy, sm, H, l, rhs0, l < nb, l < nb || b0, xcur);
+		level_down<T>(sy, H, l, rhs0, l < nb, l < nb || b0, xcur);
 	if (b0)
 		coarse_solve<T, V>(H, H.lv[lc].xa);
 	xcur[lc] = H.lv[lc].xa;
 	for (int l = lc - 1; l >= 0; l--) {
 		if (l == nb - 1)
 			sy.sync();   // block 0's coarse-level results become visible to every block
-		level_up<T>(sy, sm, H, l, rhs0, out0, l < nb, l < nb || b0, xcur, dotv, dot);
+		level_up<T>(sy, H, l, rhs0, out0, l < nb, l < nb || b0, xcur, dotv, dot);
 	}
 	if (nb == 0 && !dotv)
 		sy.sync();
 }
 
 // ---- inner solve: CG preconditioned by one V-cycle, all in T -----------------
+// The recurrences' scalars are formed by one thread of each block while the
+// others wait for its broadcast: a division or a square root on every thread
+// costs the FP64 pipe (2 lanes per clock and SM) about a microsecond each.
 template <class T>
-__device__ int pcg_inner(Sync &sy, unsigned char *sm, const MGHier<T> &H, const typename V2T<T>::t *b,
-                         typename V2T<T>::t *x, double rtol, int maxit)
+__device__ int pcg_inner(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
+                         int maxit)
 {
 	typedef typename V2T<T>::t V;
+	__shared__ double rho, bb0, co;
 	const MGLevel<T> &L = H.lv[0];
 	const int nn = L.n * L.n;
 	const int tid = sy.tid, nth = sy.nth;
@@ -421,56 +466,63 @@ __device__ int pcg_inner(Sync &sy, unsigned char *sm, const MGHier<T> &H, const 
 		zero.x = T(0);
 		zero.y = T(0);
 		x[A] = zero;
-		bb[0] += (double)bv.x * bv.x + (double)bv.y * bv.y;
+		const double b0 = widen(bv.x), b1 = widen(bv.y);
+		bb[0] += b0 * b0 + b1 * b1;
 	}
-	sy.reduce<1>(bb);
-	if (!(bb[0] > 0.0))
+	sy.reduce_then<1>(bb, [&](const double (&v)[1]) { bb0 = v[0]; });
+	if (!(bb0 > 0.0))
 		return 0;
-	vcycle<T>(sy, sm, H, r, z);
+	vcycle<T>(sy, H, r, z);
 	double rz[1] = {0.0};
 	for (int A = tid; A < nn; A += nth) {
 		const V rv = r[A], zv = z[A];
-		rz[0] += (double)rv.x * zv.x + (double)rv.y * zv.y;
+		rz[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
 		p[A] = zv;
 	}
-	sy.reduce<1>(rz);
-	double rho = rz[0];
+	sy.reduce_then<1>(rz, [&](const double (&v)[1]) { rho = v[0]; });
+	Pass<T> P = level_pass<T>(L, nullptr);
+	P.x = p;
+	P.out = q;
 	int it = 0;
 	while (it < maxit) {
 		double pq[1];
-		tile_pass<T, V>(sm, sy.part(true), L.N, L.mask, L.eta, p, nullptr, nullptr, q, PASS_MATVEC, T(0), pq);
-		sy.reduce<1>(pq);
-		const double alpha = rho / pq[0];
+		march<T, PASS_MATVEC, XS_PLAIN, false>(P, sy.part(true), pq);
+		sy.reduce_then<1>(pq, [&](const double (&v)[1]) { co = rho / v[0]; });
+		const double alpha = co;
+		const T al = (T)alpha;
 		double rr[1] = {0.0};
 		for (int A = tid; A < nn; A += nth) {
 			V xv = x[A], rv = r[A];
 			const V pv = p[A], qv = q[A];
-			xv.x += (T)alpha * pv.x;
-			xv.y += (T)alpha * pv.y;
-			rv.x -= (T)alpha * qv.x;
-			rv.y -= (T)alpha * qv.y;
+			xv.x += al * pv.x;
+			xv.y += al * pv.y;
+			rv.x -= al * qv.x;
+			rv.y -= al * qv.y;
 			x[A] = xv;
 			r[A] = rv;
-			rr[0] += (double)rv.x * rv.x + (double)rv.y * rv.y;
+			const double r0 = widen(rv.x), r1 = widen(rv.y);
+			rr[0] += r0 * r0 + r1 * r1;
 		}
 		sy.reduce<1>(rr);
 		it++;
-		if (!(rr[0] > rtol * rtol * bb[0]) || !isfinite(alpha))
+		if (!(rr[0] > rtol * rtol * bb0) || !isfinite(alpha))
 			break;
-		vcycle<T>(sy, sm, H, r, z);
+		vcycle<T>(sy, H, r, z);
 		double rz2[1] = {0.0};
 		for (int A = tid; A < nn; A += nth) {
 			const V rv = r[A], zv = z[A];
-			rz2[0] += (double)rv.x * zv.x + (double)rv.y * zv.y;
+			rz2[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
 		}
-		sy.reduce<1>(rz2);
-		const double beta = rz2[0] / rho;
-		rho = rz2[0];
+		sy.reduce_then<1>(rz2, [&](const double (&v)[1]) {
+			co = v[0] / rho;
+			rho = v[0];
+		});
+		const T be = (T)co;
 		for (int A = tid; A < nn; A += nth) {
 			const V zv = z[A];
 			V pv = p[A];
-			pv.x = zv.x + (T)beta * pv.x;
-			pv.y = zv.y + (T)beta * pv.y;
+			pv.x = zv.x + be * pv.x;
+			pv.y = zv.y + be * pv.y;
 			p[A] = pv;
 		}
 		sy.sync();
@@ -485,7 +537,12 @@ __device__ __forceinline__ void g_entries(double hx, double hz, int a, double &g
 	element_g(cS, hz, hx, a, g0, g1);
 }
 
-// y = G s at every node (masked); s in Morton order.
+// Element vectors of the solve (residual, Lanczos, preconditioner, direction)
+// are x-major, e = ez + ex*N0, so that a warp's elements along z are adjacent;
+// only the pressure itself (a.p and its candidates and history) is in the
+// mesh's Morton order.
+
+// y = G s at every node (masked); s x-major, free dofs only.
 __device__ void gmul64(int N0, const unsigned char *mask, const GTab &gt, const double *s, double2 *y, int tid,
                        int nth)
 {
@@ -499,10 +556,9 @@ __device__ void gmul64(int N0, const unsigned char *mask, const GTab &gt, const 
 			const int ex = eox[q], ez = eoz[q];
 			if (ex < 0 || ex >= N0 || ez < 0 || ez >= N0)
 				continue;
-			const double g0 = gt.g0[ea[q]], g1 = gt.g1[ea[q]];
-			const double se = s[morton(ex, ez)];
-			s0 += g0 * se;
-			s1 += g1 * se;
+			const double se = s[ez + ex * N0];
+			s0 += gt.g0[ea[q]] * se;
+			s1 += gt.g1[ea[q]] * se;
 		}
 		const unsigned m = mask[A];
 		y[A] = make_double2((m & 1u) ? 0.0 : s0, (m & 2u) ? 0.0 : s1);
@@ -530,144 +586,58 @@ __device__ __forceinline__ double gtmul64_elem(int N0, const unsigned char *mask
 	return s;
 }
 
-// FP64 residual R = [F - K d - G p ; G^T d] into a.R, a.Rc; rs = {|R_m|^2, |R_c|^2, |F|^2}
-// summed over the grid (every block holds the same values on return).
 template <class TI>
-__device__ void stokes_residual(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, const double2 *d, const double *p,
-                                double (&rs)[3])
+__device__ __forceinline__ Pass<double> fine_pass64(const MGArgs<TI> &a, const double2 *d, const double *p)
 {
-	const int tid = sy.tid, nth = sy.nth;
-	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
-	const GTab &gt = a.gt;
-	tile_pass<double, double2>(sm, sy.part(true), N0, a.mask0, a.vis, d, nullptr, nullptr, a.Kd, PASS_MATVEC, 0.0, nullptr);
-	gmul64(N0, a.mask0, gt, p, a.R, tid, nth);
-	sy.sync();
-	rs[0] = rs[1] = rs[2] = 0.0;
-	for (int A = tid; A < nn; A += nth) {
-		const double2 f = a.F[A], kd = a.Kd[A], gp = a.R[A];
-		const double2 r = make_double2(f.x - kd.x - gp.x, f.y - kd.y - gp.y);
-		a.R[A] = r;
-		rs[0] += r.x * r.x + r.y * r.y;
-		rs[2] += f.x * f.x + f.y * f.y;
-	}
-	for (int e = tid; e < ne; e += nth) {
-		const int ex = e / N0, ez = e - ex * N0;
-		const double c = gtmul64_elem(N0, a.mask0, gt, d, ex, ez);
-		a.Rc[morton(ex, ez)] = c;
-		rs[1] += c * c;
-	}
+	Pass<double> P;
+	P.N = a.N0;
+	P.mask = a.mask0;
+	P.eta = a.vis;
+	P.x = d;
+	P.b = P.invD = P.xc = P.x0 = nullptr;
+	P.out = P.xout = P.bout = nullptr;
+	P.nc = 0;
+	P.omega = P.wload = P.c0 = 0.0;
+	P.cx = 1.0;
+	P.dotv = nullptr;
+	P.gp = p;
+	P.gp_morton = 1;
+	P.g0 = a.gt.g0[0];
+	P.g1 = a.gt.g1[0];
+	return P;
+}
+
+// FP64 residual R = [F - K d - G p ; G^T d] into a.R, a.Rc; rs = {|R_m|^2, |R_c|^2, |F|^2}
+// summed over the team (every block holds the same values on return).  One
+// pass: as three loops with two team barriers between them it took 0.61 ms at
+// 1024^2.
+template <class TI>
+__device__ void stokes_residual(const MGArgs<TI> &a, Sync &sy, const double2 *d, const double *p, double (&rs)[3])
+{
+	Pass<double> P = fine_pass64(a, d, p);
+	P.F = a.F;
+	P.out64 = a.R;
+	P.gt_out = a.Rc;
+	march<double, PASS_RES64, XS_PLAIN, false>(P, sy.part(true), rs);
 	sy.reduce<3>(rs);
-}
-
-// (G^T u)_e for a TI velocity field (free dofs only).
-template <class V>
-__device__ __forceinline__ double gtmul_elem_t(int N0, const unsigned char *mask, const GTab &gt, const V *u, int ex,
-                                               int ez)
-{
-	const int n = N0 + 1;
-	const int cn[4] = {ez + ex * n, ez + 1 + ex * n, ez + 1 + (ex + 1) * n, ez + (ex + 1) * n};
-	double s = 0.0;
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		const int a = kSortedCorner[c];
-		const double g0 = gt.g0[a], g1 = gt.g1[a];
-		const V ua = u[cn[a]];
-		const unsigned m = mask[cn[a]];
-		if (!(m & 1u))
-			s += g0 * (double)ua.x;
-		if (!(m & 2u))
-			s += g1 * (double)ua.y;
-	}
-	return s;
-}
-
-// a + b = s + e exactly (Knuth's TwoSum, six FP32 additions)
-__device__ __forceinline__ void two_sum_f(float a, float b, float &s, float &e)
-{
-	s = __fadd_rn(a, b);
-	const float bb = __fsub_rn(s, a);
-	e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-
-// (sh, sl) += (gh + gl) x in double-float arithmetic: the product gh x and its
-// rounding error (by FMA), gl x, and a TwoSum into the running pair.
-__device__ __forceinline__ void df_axpy(float &sh, float &sl, float gh, float gl, float x)
-{
-	const float p = __fmul_rn(gh, x);
-	float pe = __fmaf_rn(gh, x, -p);
-	pe = __fmaf_rn(gl, x, pe);
-	float t;
-	two_sum_f(sh, p, sh, t);
-	sl = __fadd_rn(sl, __fadd_rn(t, pe));
-}
-
-// (G^T u)_e for an FP32 velocity field: the eight products and their sum in
-// double-float arithmetic on the FP32 pipe (about 48 bits, in the same corner
-// order as the FP64 form), so that the FP64 pipe -- 1/64 of FP32 on GB300 --
-// only converts and adds the final pair.
-__device__ __forceinline__ double gtmul_elem_t(int N0, const unsigned char *mask, const GTab &gt, const float2 *u,
-                                               int ex, int ez)
-{
-	const int n = N0 + 1;
-	const int cn[4] = {ez + ex * n, ez + 1 + ex * n, ez + 1 + (ex + 1) * n, ez + (ex + 1) * n};
-	float sh = 0.0f, sl = 0.0f;
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		const int a = kSortedCorner[c];
-		const float2 ua = u[cn[a]];
-		const unsigned m = mask[cn[a]];
-		if (!(m & 1u))
-			df_axpy(sh, sl, gt.g0h[a], gt.g0l[a], ua.x);
-		if (!(m & 2u))
-			df_axpy(sh, sl, gt.g1h[a], gt.g1l[a], ua.y);
-	}
-	return (double)sh + (double)sl;
 }
 
 // ---- MINRES vector kernels (FP64), kVecU elements per thread and trip ---------
 // Separate functions so that their registers do not compete with the solver's
-// state; every load of a trip is issued before its arithmetic.
-
-// Ahp = G^T z_u per element (Morton order), in FP64; returns this thread's
-// share of Ahp.z_p.
-template <class VI>
-__device__ __noinline__ double minres_gt_dot(int N0, const unsigned char *__restrict__ mask, const GTab &gt,
-                                             const VI *__restrict__ zu, const double *__restrict__ zp,
-                                             double *__restrict__ Ahp, int tid, int nth)
-{
-	const int ne = N0 * N0;
-	double acc = 0.0;
-	for (int e0 = tid; e0 < ne; e0 += kVecU * nth) {
-		double t[kVecU], zpe[kVecU];
-		int me[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				const int ex = e / N0, ez = e - ex * N0;
-				me[u] = morton(ex, ez);
-				t[u] = gtmul_elem_t(N0, mask, gt, zu, ex, ez);
-				zpe[u] = zp[me[u]];
-			}
-		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++)
-			if (e0 + u * nth < ne) {
-				Ahp[me[u]] = t[u];
-				acc += t[u] * zpe[u];
-			}
-	}
-	return acc;
-}
+// state; every load of a trip is issued before its arithmetic.  Bound by the
+// FP64 pipe and HBM together at 1024^2 (12 and 12 FP64 operations per node and
+// element); conversions to and from TI go through widen / narrow.
 
 // v_old <- az ig - dg v - gg v_old (velocity, with its TI copy into bI) and the
-// same for the pressure part with Ahp.
+// same for the pressure part with Ahp, whose preconditioned vector z_p = v_p / BAB
+// is formed with it; returns this thread's share of z_p.v_p.
 template <class VI>
-__device__ __noinline__ void minres_v_update(int nn, int ne, int tid, int nth, const double2 *__restrict__ az_,
-                                             const double2 *__restrict__ v_, double2 *__restrict__ vo_,
-                                             VI *__restrict__ bI, const double *__restrict__ ah_,
-                                             const double *__restrict__ p0_, double *__restrict__ p1_, double ig,
-                                             double dg, double gg)
+__device__ __noinline__ double minres_v_update(int nn, int ne, int tid, int nth, const double2 *__restrict__ az_,
+                                               const double2 *__restrict__ v_, double2 *__restrict__ vo_,
+                                               VI *__restrict__ bI, const double *__restrict__ ah_,
+                                               const double *__restrict__ p0_, double *__restrict__ p1_,
+                                               const double *__restrict__ ibab, double *__restrict__ zp1_, double ig,
+                                               double dg, double gg)
 {
 	typedef decltype(VI().x) TI;
 	for (int A0 = tid; A0 < nn; A0 += kVecU * nth) {
@@ -689,14 +659,15 @@ __device__ __noinline__ void minres_v_update(int nn, int ne, int tid, int nth, c
 				                                az[u].y * ig - dg * v[u].y - gg * vo[u].y);
 				vo_[A] = vn;
 				VI w;
-				w.x = (TI)vn.x;
-				w.y = (TI)vn.y;
+				w.x = narrow_to<TI>(vn.x);
+				w.y = narrow_to<TI>(vn.y);
 				bI[A] = w;
 			}
 		}
 	}
+	double acc = 0.0;
 	for (int e0 = tid; e0 < ne; e0 += kVecU * nth) {
-		double ah[kVecU], p0[kVecU], p1[kVecU];
+		double ah[kVecU], p0[kVecU], p1[kVecU], ib[kVecU];
 #pragma unroll
 		for (int u = 0; u < kVecU; u++) {
 			const int e = e0 + u * nth;
@@ -704,26 +675,31 @@ __device__ __noinline__ void minres_v_update(int nn, int ne, int tid, int nth, c
 				ah[u] = ah_[e];
 				p0[u] = p0_[e];
 				p1[u] = p1_[e];
+				ib[u] = ibab[e];
 			}
 		}
 #pragma unroll
 		for (int u = 0; u < kVecU; u++) {
 			const int e = e0 + u * nth;
-			if (e < ne)
-				p1_[e] = ah[u] * ig - dg * p0[u] - gg * p1[u];
+			if (e < ne) {
+				const double vn = ah[u] * ig - dg * p0[u] - gg * p1[u], z = vn * ib[u];
+				p1_[e] = vn;
+				zp1_[e] = z;
+				acc += z * vn;
+			}
 		}
 	}
+	return acc;
 }
 
-// w_old <- (z ig - a3 w_old - a2 w) ia1 and x += step w_old, for the velocity
-// (z in TI) and the pressure parts.
+// w_old <- k1 z - k3 w_old - k2 w and x += step w_old, for the velocity (z in
+// TI) and the pressure parts.
 template <class VI>
 __device__ __noinline__ void minres_w_update(int nn, int ne, int tid, int nth, const VI *__restrict__ z_,
                                              double2 *__restrict__ wo_, const double2 *__restrict__ w_,
                                              double2 *__restrict__ x_, const double *__restrict__ zp_,
                                              double *__restrict__ wpo_, const double *__restrict__ wp_,
-                                             double *__restrict__ xp_, double ig, double a3, double a2, double ia1,
-                                             double step)
+                                             double *__restrict__ xp_, double k1, double k3, double k2, double step)
 {
 	for (int A0 = tid; A0 < nn; A0 += kVecU * nth) {
 		VI z[kVecU];
@@ -742,8 +718,8 @@ __device__ __noinline__ void minres_w_update(int nn, int ne, int tid, int nth, c
 		for (int u = 0; u < kVecU; u++) {
 			const int A = A0 + u * nth;
 			if (A < nn) {
-				const double2 wn = make_double2(((double)z[u].x * ig - a3 * wo[u].x - a2 * w[u].x) * ia1,
-				                                ((double)z[u].y * ig - a3 * wo[u].y - a2 * w[u].y) * ia1);
+				const double2 wn = make_double2(widen(z[u].x) * k1 - k3 * wo[u].x - k2 * w[u].x,
+				                                widen(z[u].y) * k1 - k3 * wo[u].y - k2 * w[u].y);
 				wo_[A] = wn;
 				x_[A] = make_double2(x[u].x + step * wn.x, x[u].y + step * wn.y);
 			}
@@ -765,7 +741,7 @@ __device__ __noinline__ void minres_w_update(int nn, int ne, int tid, int nth, c
 		for (int u = 0; u < kVecU; u++) {
 			const int e = e0 + u * nth;
 			if (e < ne) {
-				const double wn = (zz[u] * ig - a3 * wo[u] - a2 * w[u]) * ia1;
+				const double wn = zz[u] * k1 - k3 * wo[u] - k2 * w[u];
 				wpo_[e] = wn;
 				xp_[e] = x[u] + step * wn;
 			}
@@ -773,85 +749,46 @@ __device__ __noinline__ void minres_w_update(int nn, int ne, int tid, int nth, c
 	}
 }
 
-// z_p = v_p / BAB (ibab = 1/BAB); returns this thread's share of z_p.v_p.
-__device__ __noinline__ double precond_pressure(int ne, int tid, int nth, const double *__restrict__ vp,
-                                                const double *__restrict__ ibab, double *__restrict__ zp)
-{
-	double acc = 0.0;
-	for (int e0 = tid; e0 < ne; e0 += kVecU * nth) {
-		double v[kVecU], ib[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				v[u] = vp[e];
-				ib[u] = ibab[e];
-			}
-		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				const double z = v[u] * ib[u];
-				zp[e] = z;
-				acc += z * v[u];
-			}
-		}
-	}
-	return acc;
-}
-
 // z = M^-1 v for M = diag(one V-cycle of K, BAB): the velocity part goes
 // through the TI hierarchy (z_u stays in TI), the pressure part is multiplied
-// by 1/BAB (a.bab holds the reciprocal).  Returns <z, v> over the team.  With
-// converted, the caller has already written v_u in TI to the finest level's
-// right-hand side (H.lv[0].b) and synchronised.
+// by 1/BAB (a.bab holds the reciprocal).  Returns <z, v> over the team.
 template <class TI>
-__device__ double block_precond(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, const double2 *vu, const double *vp,
-                                typename V2T<TI>::t *zu, double *zp, bool converted = false)
+__device__ double block_precond(const MGArgs<TI> &a, Sync &sy, const double2 *vu, const double *vp,
+                                typename V2T<TI>::t *zu, double *zp)
 {
 	typedef typename V2T<TI>::t VI;
 	const MGHier<TI> &H = a.H;
 	const int tid = sy.tid, nth = sy.nth;
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
 	VI *bI = H.lv[0].b;
-	if (!converted) {
-		for (int A = tid; A < nn; A += nth) {
-			const double2 v = vu[A];
-			VI w;
-			w.x = (TI)v.x;
-			w.y = (TI)v.y;
-			bI[A] = w;
-		}
-		sy.sync();
+	for (int A = tid; A < nn; A += nth) {
+		const double2 v = vu[A];
+		VI w;
+		w.x = narrow_to<TI>(v.x);
+		w.y = narrow_to<TI>(v.y);
+		bI[A] = w;
 	}
+	sy.sync();
 	double dot[1] = {0.0};
-	vcycle<TI>(sy, sm, H, bI, zu, vu, &dot[0]);   // the last sweep forms <z_u, v_u>
-	dot[0] += precond_pressure(ne, tid, nth, vp, a.bab, zp);
+	vcycle<TI>(sy, H, bI, zu, vu, &dot[0]);   // the last sweep forms <z_u, v_u>
+	for (int e = tid; e < ne; e += nth) {
+		const double z = vp[e] * a.bab[e];
+		zp[e] = z;
+		dot[0] += z * vp[e];
+	}
 	sy.reduce<1>(dot);
 	return dot[0];
 }
 
-// Y = K u + G p and Yc = G^T u in FP64 (the Stokes operator applied to (u, p));
-// a.Kd is scratch.  Ends with a team barrier: Yc is written at Morton indices,
-// which other threads read.
+// Y = K u + G p and Yc = G^T u in FP64 (the Stokes operator applied to (u, p);
+// p in Morton order).  Ends with a team barrier.
 template <class TI>
-__device__ void stokes_apply(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, const double2 *u, const double *p,
-                             double2 *Y, double *Yc)
+__device__ void stokes_apply(const MGArgs<TI> &a, Sync &sy, const double2 *u, const double *p, double2 *Y, double *Yc)
 {
-	const int tid = sy.tid, nth = sy.nth;
-	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
-	tile_pass<double, double2>(sm, sy.part(true), N0, a.mask0, a.vis, u, nullptr, nullptr, Y, PASS_MATVEC, 0.0, nullptr);
-	gmul64(N0, a.mask0, a.gt, p, a.Kd, tid, nth);
-	sy.sync();
-	for (int A = tid; A < nn; A += nth) {
-		const double2 y = Y[A], g = a.Kd[A];
-		Y[A] = make_double2(y.x + g.x, y.y + g.y);
-	}
-	for (int e = tid; e < ne; e += nth) {
-		const int ex = e / N0, ez = e - ex * N0;
-		Yc[morton(ex, ez)] = gtmul64_elem(N0, a.mask0, a.gt, u, ex, ez);
-	}
+	Pass<double> P = fine_pass64(a, u, p);
+	P.out64 = Y;
+	P.gt_out = Yc;
+	march<double, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), nullptr);
 	sy.sync();
 }
 
@@ -875,7 +812,7 @@ __device__ void stokes_apply(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, c
 // carried on and amplified from step to step), 111 against 100 per step over
 // 30 steps; warm_start=3 stays the default there.
 template <class TI>
-__device__ void warm_guess(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, int ndir)
+__device__ void warm_guess(const MGArgs<TI> &a, Sync &sy, int ndir)
 {
 	typedef typename V2T<TI>::t VI;
 	const int tid = sy.tid, nth = sy.nth;
@@ -885,7 +822,7 @@ __device__ void warm_guess(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, int
 	VI *Z1 = a.H.px, *Z2 = a.H.pr;
 	double *Zp1 = a.mzp[0], *Zp2 = a.mzp[1];
 	double rs[3];
-	stokes_residual(a, sm, sy, a.h1d, a.h1p, rs);   // a.R = F - K h1 - G p1, a.Rc = G^T h1
+	stokes_residual(a, sy, a.h1d, a.h1p, rs);   // a.R = F - K h1 - G p1, a.Rc = G^T h1
 	for (int A = tid; A < nn; A += nth) {
 		const double2 x1 = a.h1d[A], x2 = a.h2d[A];
 		U1[A] = make_double2(x1.x - x2.x, x1.y - x2.y);
@@ -900,14 +837,14 @@ __device__ void warm_guess(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, int
 			P2[e] = a.h1p[e] - 2.0 * a.h2p[e] + a.h3p[e];
 	}
 	sy.sync();
-	stokes_apply(a, sm, sy, U1, P1, Y1, Yc1);
+	stokes_apply(a, sy, U1, P1, Y1, Yc1);
 	if (ndir == 2)
-		stokes_apply(a, sm, sy, U2, P2, Y2, Yc2);
+		stokes_apply(a, sy, U2, P2, Y2, Yc2);
 	// M^-1 a_k (the preconditioner's pressure part divides by BAB); the signs of
 	// the continuity parts follow r = [F - K d - G p ; -G^T d]
 	double q[5];   // <a1, M^-1 a1>, <a2, M^-1 a1>, <a2, M^-1 a2>, <r0, M^-1 a1>, <r0, M^-1 a2>
-	q[0] = block_precond(a, sm, sy, Y1, Yc1, Z1, Zp1);
-	q[2] = ndir == 2 ? block_precond(a, sm, sy, Y2, Yc2, Z2, Zp2) : 0.0;
+	q[0] = block_precond(a, sy, Y1, Yc1, Z1, Zp1);
+	q[2] = ndir == 2 ? block_precond(a, sy, Y2, Yc2, Z2, Zp2) : 0.0;
 	double c[3] = {0.0, 0.0, 0.0};
 	for (int A = tid; A < nn; A += nth) {
 		const double2 r = a.R[A];
@@ -964,104 +901,167 @@ __device__ void warm_guess(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, int
 	sy.sync();
 }
 
+// The scalars of the MINRES recurrences, formed by one thread of each block
+// (all blocks hold the same sums, so all form the same values).
+struct MinresScal {
+	double gam, gam_prev, eta, eta0, delta, c_prev, c_cur, s_prev, s_cur;
+	double ig, dg, gg, k1, k2, k3, step;
+	int stop;   // 1: last iteration; 2: breakdown before the update; 4: a non-finite value
+};
+
 // Correction solve by preconditioned MINRES (the Lanczos-based algorithm of
 // Elman, Silvester and Wathen, "Finite Elements and Fast Iterative Solvers",
 // Alg. 4.1) on [K G; G^T 0][x_u; x_p] = [R_m; -R_c] from a zero start, with
 // the block-diagonal SPD preconditioner diag(V-cycle, BAB).  K is applied in
-// TI by the tiled operator, G and G^T in FP64; Lanczos and direction vectors
-// are FP64 and x_u, x_p accumulate in a.dd, a.dpv.  The FP64 refinement
-// around this solve restores full accuracy.  Stops when the M^-1-norm of the
-// residual has dropped by rtol.  Returns the iterations.
+// TI, G and G^T to FP64 accuracy, in one pass over the mesh; Lanczos and
+// direction vectors are FP64 and x_u, x_p accumulate in a.dd, a.dpv.  The FP64
+// refinement around this solve restores full accuracy.  Stops when the
+// M^-1-norm of the residual has dropped by rtol.  Returns the iterations.
 template <class TI>
-__device__ int minres_correction(const MGArgs<TI> &a, unsigned char *sm, Sync &sy, double rtol, int maxit,
-                                 int *status)
+__device__ int minres_correction(const MGArgs<TI> &a, Sync &sy, double rtol, int maxit, int *status)
 {
 	typedef typename V2T<TI>::t VI;
+	__shared__ MinresScal ms;
 	const MGHier<TI> &H = a.H;
 	const MGLevel<TI> &L0 = H.lv[0];
 	const int tid = sy.tid, nth = sy.nth;
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
 	double2 *vu[2] = {a.mv[0], a.mv[1]}, *wu[2] = {a.mw[0], a.mw[1]};
 	double *vp[2] = {a.mvp[0], a.mvp[1]}, *zp[2] = {a.mzp[0], a.mzp[1]}, *wp[2] = {a.mwp[0], a.mwp[1]};
-	VI *zu[2] = {H.pz, H.pp}, *kz = H.pq;   // inner-CG vectors, free while MINRES runs
-	const GTab &gt = a.gt;
+	VI *zu[2] = {H.pz, H.pp};   // inner-CG vectors, free while MINRES runs
+	VI *bI = L0.b;
 	const double2 zero2 = make_double2(0.0, 0.0);
 	for (int A = tid; A < nn; A += nth) {
-		vu[0][A] = a.R[A];
+		const double2 r = a.R[A];
+		vu[0][A] = r;
+		VI w;
+		w.x = narrow_to<TI>(r.x);
+		w.y = narrow_to<TI>(r.y);
+		bI[A] = w;
 		vu[1][A] = zero2;
 		wu[0][A] = zero2;
 		wu[1][A] = zero2;
 		a.dd[A] = zero2;
 	}
+	double pdot = 0.0;
 	for (int e = tid; e < ne; e += nth) {
-		vp[0][e] = -a.Rc[e];
+		const double v = -a.Rc[e], z = v * a.bab[e];
+		vp[0][e] = v;
+		zp[0][e] = z;
+		pdot += z * v;
 		vp[1][e] = 0.0;
 		wp[0][e] = 0.0;
 		wp[1][e] = 0.0;
 		a.dpv[e] = 0.0;
 	}
 	sy.sync();
-	double gam2 = block_precond(a, sm, sy, vu[0], vp[0], zu[0], zp[0]);
-	if (!(gam2 > 0.0))
+	double dot[1];
+	vcycle<TI>(sy, H, bI, zu[0], vu[0], &dot[0]);
+	dot[0] += pdot;
+	sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
+		const double g = sqrt(fmax(v[0], 0.0));
+		ms.gam = g;
+		ms.gam_prev = 1.0;
+		ms.eta = ms.eta0 = g;
+		ms.c_prev = ms.c_cur = 1.0;
+		ms.s_prev = ms.s_cur = 0.0;
+		ms.ig = 1.0 / g;
+		ms.gg = g;
+		ms.stop = v[0] > 0.0 ? 0 : 2;
+	});
+	if (ms.stop)
 		return 0;
-	double gam = sqrt(gam2), gam_prev = 1.0;
-	const double eta0 = gam;
-	double eta = gam, c_prev = 1.0, c_cur = 1.0, s_prev = 0.0, s_cur = 0.0;
+	Pass<TI> P = level_pass<TI>(L0, nullptr);
+	P.out64 = a.Kd;
+	P.gt_out = a.Ahp;
+	P.g0 = a.gt.g0[0];
+	P.g1 = a.gt.g1[0];
+	P.gp_morton = 0;
 	int cv = 0, cw = 0, it = 0;   // index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1)
 	while (it < maxit) {
-		// A z(j), unscaled (z~ = z / gam): K z_u + G z_p into a.Kd with its
-		// product with z_u formed in the same pass, and G^T z_u per element
-		double dl[1] = {0.0};
-		tile_pass<TI, VI>(sm, sy.part(true), L0.N, L0.mask, L0.eta, zu[cv], nullptr, nullptr, kz, PASS_STOKES, TI(0),
-		                  &dl[0], XS_PLAIN, nullptr, 0, nullptr, zp[cv], &gt, a.Kd);
-		dl[0] += minres_gt_dot<VI>(N0, a.mask0, gt, zu[cv], zp[cv], a.Ahp, tid, nth);
-		sy.reduce<1>(dl);
-		const double delta = dl[0] / (gam * gam);
+		// A z(j), unscaled (z~ = z / gam): K z_u + G z_p into a.Kd, G^T z_u into
+		// a.Ahp, and their product with (z_u, z_p)
+		double dl[1];
+		P.x = zu[cv];
+		P.gp = zp[cv];
+		march<TI, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), dl);
+		sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
+			ms.delta = v[0] * ms.ig * ms.ig;
+			ms.dg = ms.delta * ms.ig;
+		});
 		// v(j+1) = A z~ - (delta/gam) v(j) - (gam/gam_prev) v(j-1), into v(j-1)'s
-		// buffer, and its TI copy as the V-cycle's right-hand side
-		const double ig = 1.0 / gam, dg = delta / gam, gg = gam / gam_prev;
-		minres_v_update<VI>(nn, ne, tid, nth, a.Kd, vu[cv], vu[1 - cv], H.lv[0].b, a.Ahp, vp[cv], vp[1 - cv], ig, dg, gg);
+		// buffer, its TI copy as the V-cycle's right-hand side, and z_p(j+1)
+		const double pd = minres_v_update<VI>(nn, ne, tid, nth, a.Kd, vu[cv], vu[1 - cv], bI, a.Ahp, vp[cv], vp[1 - cv],
+		                                      a.bab, zp[1 - cv], ms.ig, ms.dg, ms.gg);
 		sy.sync();
-		const double gn2 = block_precond(a, sm, sy, vu[1 - cv], vp[1 - cv], zu[1 - cv], zp[1 - cv], true);
-		const double gam_next = sqrt(fmax(gn2, 0.0));
-		// Givens rotations
-		const double a0 = c_cur * delta - c_prev * s_cur * gam;
-		const double a1 = sqrt(a0 * a0 + gam_next * gam_next);
-		const double a2 = s_cur * delta + c_prev * c_cur * gam;
-		const double a3 = s_prev * gam;
-		if (!(a1 > 0.0) || !isfinite(a1)) {
-			if (!isfinite(a1) && tid == 0)
-				atomicOr(status, 2);
+		vcycle<TI>(sy, H, bI, zu[1 - cv], vu[1 - cv], &dot[0]);
+		dot[0] += pd;
+		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
+			// Givens rotations
+			const double gn2 = fmax(v[0], 0.0);
+			const double a0 = ms.c_cur * ms.delta - ms.c_prev * ms.s_cur * ms.gam;
+			const double a1s = a0 * a0 + gn2;
+			const double a2 = ms.s_cur * ms.delta + ms.c_prev * ms.c_cur * ms.gam;
+			const double a3 = ms.s_prev * ms.gam;
+			const double ia1 = rsqrt(a1s);
+			const double gam_next = sqrt(gn2);
+			ms.stop = 0;
+			if (!(a1s > 0.0) || !isfinite(a1s)) {
+				ms.stop = isfinite(a1s) ? 2 : 6;
+				return;
+			}
+			const double c_next = a0 * ia1, s_next = gam_next * ia1;
+			// w(j+1) = (z~(j) - a3 w(j-1) - a2 w(j)) / a1; x += c_next eta w(j+1)
+			ms.k1 = ms.ig * ia1;
+			ms.k2 = a2 * ia1;
+			ms.k3 = a3 * ia1;
+			ms.step = c_next * ms.eta;
+			ms.eta = -s_next * ms.eta;
+			ms.gam_prev = ms.gam;
+			ms.gam = gam_next;
+			ms.c_prev = ms.c_cur;
+			ms.c_cur = c_next;
+			ms.s_prev = ms.s_cur;
+			ms.s_cur = s_next;
+			if (!isfinite(ms.eta))
+				ms.stop = 5;
+			else if (!(fabs(ms.eta) > rtol * ms.eta0) || !(gam_next > 0.0))
+				ms.stop = 1;
+		});
+		const int stop = ms.stop;
+		if ((stop & 4) && tid == 0)
+			atomicOr(status, 2);
+		if (stop & 2)
 			break;
-		}
-		const double c_next = a0 / a1, s_next = gam_next / a1;
-		// w(j+1) = (z~(j) - a3 w(j-1) - a2 w(j)) / a1 into w(j-1)'s buffer; x += c_next eta w(j+1)
-		const double ia1 = 1.0 / a1, step = c_next * eta;
-		minres_w_update<VI>(nn, ne, tid, nth, zu[cv], wu[1 - cw], wu[cw], a.dd, zp[cv], wp[1 - cw], wp[cw], a.dpv, ig,
-		                    a3, a2, ia1, step);
-		eta = -s_next * eta;
+		// into w(j-1)'s buffer
+		minres_w_update<VI>(nn, ne, tid, nth, zu[cv], wu[1 - cw], wu[cw], a.dd, zp[cv], wp[1 - cw], wp[cw], a.dpv, ms.k1,
+		                    ms.k3, ms.k2, ms.step);
 		it++;
 		cv = 1 - cv;
 		cw = 1 - cw;
-		gam_prev = gam;
-		gam = gam_next;
-		c_prev = c_cur;
-		c_cur = c_next;
-		s_prev = s_cur;
-		s_cur = s_next;
-		if (!isfinite(eta)) {
-			if (tid == 0)
-				atomicOr(status, 2);
+		if (stop)
 			break;
+		// the next step's 1/gam and gam/gam_prev, off the other threads' path; they are
+		// read after the next reduction's broadcast
+		if (threadIdx.x == 0) {
+			ms.ig = 1.0 / ms.gam;
+			ms.gg = ms.gam / ms.gam_prev;
 		}
-		if (!(fabs(eta) > rtol * eta0) || !(gam > 0.0))
-			break;
 		// no barrier here: the next operator pass reads z(j+1) and z_p(j+1),
-		// complete since the reduction in block_precond, and touches none of
-		// the vectors the updates above wrote
+		// complete since the reduction, and touches none of the vectors the
+		// updates above wrote
 	}
 	sy.sync();
 	return it;
+}
+
+// p += dp, dp x-major and p in the mesh's Morton order
+__device__ void add_pressure(int N0, const double *dp, double *p, int tid, int nth)
+{
+	for (int e = tid; e < N0 * N0; e += nth) {
+		const int ex = e / N0, ez = e - ex * N0;
+		p[morton(ex, ez)] += dp[e];
+	}
 }
 
 // ---- one converged Stokes solve ----------------------------------------------------
@@ -1069,7 +1069,7 @@ __device__ int minres_correction(const MGArgs<TI> &a, unsigned char *sm, Sync &s
 // refinement, correction solves.  Runs on the cooperative grid (one model) or
 // inside one block (one model of a batch), as `sy` says.
 template <class TI>
-__device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
+__device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 {
 	typedef typename V2T<TI>::t VI;
 	const MGHier<TI> &H = a.H;
@@ -1126,7 +1126,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 			if (!(m & 2u))
 				s += g1 * g1 / kd.y;
 		}
-		a.bab[morton(ex, ez)] = 1.0 / s;   // the solvers multiply by 1/BAB
+		a.bab[e] = 1.0 / s;   // the solvers multiply by 1/BAB
 	}
 	if (sy.leader())
 		coarse_build<TI>(H);
@@ -1137,15 +1137,15 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 	if (a.method == 1 && a.h1d != nullptr) {
 		const int nh = a.sc->nsolved < 3 ? a.sc->nsolved : 3;   // solutions in the history
 		if (nh >= 2)
-			warm_guess<TI>(a, sm, sy, nh - 1);
+			warm_guess<TI>(a, sy, nh - 1);
 	}
 	if (a.d_alt != nullptr) {
 		// Two candidate guesses: (d, p) from the network and (d_alt, p_alt),
 		// the previous step's solution.  Keep the one with the smaller FP64
 		// residual; a non-finite network guess always loses.
 		double rl[3], rp[3];
-		stokes_residual(a, sm, sy, a.d, a.p, rl);
-		stokes_residual(a, sm, sy, a.d_alt, a.p_alt, rp);
+		stokes_residual(a, sy, a.d, a.p, rl);
+		stokes_residual(a, sy, a.d_alt, a.p_alt, rp);
 		const double el = rl[0] + rl[1], ep = rp[0] + rp[1];
 		const bool learned = isfinite(el) && (a.guess_force || el < ep);
 		if (!learned) {
@@ -1164,7 +1164,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 	while (true) {
 		// -- FP64 residual R = [F - K d - G p ; G^T d]
 		double rs[3];
-		stokes_residual(a, sm, sy, a.d, a.p, rs);
+		stokes_residual(a, sy, a.d, a.p, rs);
 		// a zero load (|F| = 0): the residual is measured absolutely
 		fnorm = rs[2] > 0.0 ? sqrt(rs[2]) : 1.0;
 		res_m = sqrt(rs[0]) / fnorm;
@@ -1189,7 +1189,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 			// where MINRES converges fastest; close to it, by what is left to
 			// reach rtol (with a factor 2 margin), but not below outer_rtol.
 			const double prt = res > 1e4 * a.rtol ? 1e-2 : fmax(a.outer_rtol, 0.5 * a.rtol / res);
-			const int it = minres_correction<TI>(a, sm, sy, prt, a.max_outer, status);
+			const int it = minres_correction<TI>(a, sy, prt, a.max_outer, status);
 			outer_total += it;
 			inner_total += it + 1;
 			for (int A = tid; A < nn; A += nth) {
@@ -1199,8 +1199,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 				v.y += c.y;
 				a.d[A] = v;
 			}
-			for (int e = tid; e < ne; e += nth)
-				a.p[e] += a.dpv[e];
+			add_pressure(N0, a.dpv, a.p, tid, nth);
 			sy.sync();
 			continue;
 		}
@@ -1210,25 +1209,24 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 		for (int A = tid; A < nn; A += nth) {
 			const double2 r = a.R[A];
 			VI v;
-			v.x = (TI)r.x;
-			v.y = (TI)r.y;
+			v.x = narrow_to<TI>(r.x);
+			v.y = narrow_to<TI>(r.y);
 			bI[A] = v;
 		}
 		sy.sync();
-		inner_total += pcg_inner<TI>(sy, sm, H, bI, xI, a.inner_rtol, a.max_inner);
+		inner_total += pcg_inner<TI>(sy, H, bI, xI, a.inner_rtol, a.max_inner);
 		for (int A = tid; A < nn; A += nth) {
 			const VI v = xI[A];
-			a.dd[A] = make_double2((double)v.x, (double)v.y);
+			a.dd[A] = make_double2(widen(v.x), widen(v.y));
 		}
 		sy.sync();
 		double *r0 = a.r0, *r1 = a.r1, *r2 = a.r2, *z0 = a.z0, *z1 = a.z1, *s1 = a.s1, *s2 = a.s2;
 		double c0[1] = {0.0};
 		for (int e = tid; e < ne; e += nth) {
 			const int ex = e / N0, ez = e - ex * N0;
-			const int me = morton(ex, ez);
-			const double v = a.Rc[me] + gtmul64_elem(N0, a.mask0, gt, a.dd, ex, ez);
-			r1[me] = v;
-			a.dpv[me] = 0.0;
+			const double v = a.Rc[e] + gtmul64_elem(N0, a.mask0, gt, a.dd, ex, ez);
+			r1[e] = v;
+			a.dpv[e] = 0.0;
 			c0[0] += v * v;
 		}
 		sy.reduce<1>(c0);
@@ -1253,24 +1251,23 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 			for (int A = tid; A < nn; A += nth) {
 				const double2 v = a.u1[A];
 				VI w;
-				w.x = (TI)v.x;
-				w.y = (TI)v.y;
+				w.x = narrow_to<TI>(v.x);
+				w.y = narrow_to<TI>(v.y);
 				bI[A] = w;
 			}
 			sy.sync();
-			inner_total += pcg_inner<TI>(sy, sm, H, bI, xI, a.inner_rtol, a.max_inner);
+			inner_total += pcg_inner<TI>(sy, H, bI, xI, a.inner_rtol, a.max_inner);
 			for (int A = tid; A < nn; A += nth) {
 				const VI v = xI[A];
-				a.u1[A] = make_double2((double)v.x, (double)v.y);
+				a.u1[A] = make_double2(widen(v.x), widen(v.y));
 			}
 			sy.sync();
 			double sa[1] = {0.0};
 			for (int e = tid; e < ne; e += nth) {
 				const int ex = e / N0, ez = e - ex * N0;
-				const int me = morton(ex, ez);
 				const double t = gtmul64_elem(N0, a.mask0, gt, a.u1, ex, ez);
-				a.Ahp[me] = t;
-				sa[0] += s2[me] * t;
+				a.Ahp[e] = t;
+				sa[0] += s2[e] * t;
 			}
 			sy.reduce<1>(sa);
 			const double alpha = rz[0] / sa[0];
@@ -1309,8 +1306,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 			v.y += c.y;
 			a.d[A] = v;
 		}
-		for (int e = tid; e < ne; e += nth)
-			a.p[e] += a.dpv[e];
+		add_pressure(N0, a.dpv, a.p, tid, nth);
 		sy.sync();
 	}
 	if (capped && tid == 0)
@@ -1334,23 +1330,41 @@ __device__ void stokes_solve(const MGArgs<TI> &a, unsigned char *sm, Sync &sy)
 	}
 }
 
+// The solver's arguments in shared memory: noinline passes take references into
+// them, which for kernel parameters would copy them to every thread's stack.
+template <class TI>
+__device__ void load_args(MGArgs<TI> &to, const MGArgs<TI> &from)
+{
+	static_assert(sizeof(MGArgs<TI>) % 4 == 0, "copied by words");
+	const unsigned *s = reinterpret_cast<const unsigned *>(&from);
+	unsigned *d = reinterpret_cast<unsigned *>(&to);
+	for (int i = threadIdx.x; i < (int)(sizeof(MGArgs<TI>) / 4); i += blockDim.x)
+		d[i] = s[i];
+	__syncthreads();
+}
+
+// Blocks per SM: two of 256 threads in FP32; the FP64 passes hold twice the
+// registers and are bound by the FP64 pipe, which one block keeps busy.
+template <class TI> constexpr int kSolveBlocks = sizeof(TI) == 4 ? 2 : 1;
+
 // One model on the whole cooperative grid.
 template <class TI>
-__global__ void __launch_bounds__(kBlock, 2) k_stokes_mg(MGArgs<TI> a)
+__global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg(const __grid_constant__ MGArgs<TI> a)
 {
-	__shared__ __align__(16) unsigned char sm[kSmemBytes];
+	__shared__ MGArgs<TI> sa;
+	load_args(sa, a);
 	cg::grid_group g = cg::this_grid();
 	Sync sy;
 	sy.mode = SYNC_GRID;
 	sy.g = &g;
-	sy.red = a.red;
+	sy.red = sa.red;
 	sy.cpart = nullptr;
 	sy.cflip = 0;
 	sy.rank = blockIdx.x;
 	sy.size = gridDim.x;
 	sy.tid = blockIdx.x * blockDim.x + threadIdx.x;
 	sy.nth = gridDim.x * blockDim.x;
-	stokes_solve<TI>(a, sm, sy);
+	stokes_solve<TI>(sa, sy);
 }
 
 // A batch of independent models.  Launched with clusters of `cs` blocks
@@ -1361,9 +1375,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_stokes_mg(MGArgs<TI> a)
 // reads the draw from its shared memory; all blocks of a cluster leave the
 // loop on the same draw.
 template <class TI>
-__global__ void __launch_bounds__(kBlock, 2) k_stokes_mg_batch(const MGArgs<TI> *models, int nmodels, int *queue)
+__global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(const MGArgs<TI> *models, int nmodels,
+                                                                              int *queue)
 {
-	__shared__ __align__(16) unsigned char sm[kSmemBytes];
+	__shared__ MGArgs<TI> sa;
 	__shared__ int next;
 	__shared__ double cpart[2 * kRedWidth];
 	cg::cluster_group cl = cg::this_cluster();
@@ -1371,23 +1386,24 @@ __global__ void __launch_bounds__(kBlock, 2) k_stokes_mg_batch(const MGArgs<TI> 
 	for (;;) {
 		if (rank == 0 && threadIdx.x == 0)
 			next = atomicAdd(queue, 1);
+		Sync sy;
+		sy.g = nullptr;
+		sy.cflip = 0;
 		if (cs > 1) {
 			cl.sync();
 			const int m = *cl.map_shared_rank(&next, 0);
 			cl.sync();   // every block has read the draw before the next one
 			if (m >= nmodels)
 				break;
-			Sync sy;
+			load_args(sa, models[m]);
 			sy.mode = SYNC_CLUSTER;
-			sy.g = nullptr;
-			sy.red = models[m].red;
+			sy.red = sa.red;
 			sy.cpart = cpart;
-			sy.cflip = 0;
 			sy.rank = rank;
 			sy.size = cs;
 			sy.tid = rank * blockDim.x + threadIdx.x;
 			sy.nth = cs * blockDim.x;
-			stokes_solve<TI>(models[m], sm, sy);
+			stokes_solve<TI>(sa, sy);
 			cl.sync();   // no block starts the next model (or leaves) while another reads its partials
 		} else {
 			__syncthreads();
@@ -1395,17 +1411,15 @@ __global__ void __launch_bounds__(kBlock, 2) k_stokes_mg_batch(const MGArgs<TI> 
 			__syncthreads();
 			if (m >= nmodels)
 				break;
-			Sync sy;
+			load_args(sa, models[m]);
 			sy.mode = SYNC_BLOCK;
-			sy.g = nullptr;
-			sy.red = models[m].red;
+			sy.red = sa.red;
 			sy.cpart = nullptr;
-			sy.cflip = 0;
 			sy.rank = 0;
 			sy.size = 1;
 			sy.tid = threadIdx.x;
 			sy.nth = blockDim.x;
-			stokes_solve<TI>(models[m], sm, sy);
+			stokes_solve<TI>(sa, sy);
 			__syncthreads();
 		}
 	}

@@ -40,33 +40,90 @@ struct Sync {
 		else
 			__syncthreads();
 	}
-	template <int NV>
-	__device__ void reduce(double (&v)[NV])
+	// Sums of NV values over the team, formed by warp 0 of every block from the
+	// same partials in the same order; f(sums) runs on thread 0 of each block, and
+	// what it writes to shared memory is visible to the block on return.  Each
+	// value's 256 thread partials go through shared memory to one warp (8 + 5
+	// additions): a butterfly in every warp takes eight times that of the FP64
+	// pipe, which has 2 lanes per clock and SM.
+	template <int NV, class F>
+	__device__ __forceinline__ void reduce_then(const double (&v)[NV], F f)
 	{
+		static_assert(NV <= kRedWidth, "partials per reduction");
+		__shared__ double sh[NV][kBlock];
+		const int lane = threadIdx.x & 31;
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			sh[k][threadIdx.x] = v[k];
+		__syncthreads();
+		double t[NV];
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			t[k] = 0.0;
+		if (threadIdx.x < 32) {
+#pragma unroll
+			for (int k = 0; k < NV; k++) {
+				const double *s = sh[k] + lane;
+				t[k] = warp_sum(((s[0] + s[32]) + (s[64] + s[96])) + ((s[128] + s[160]) + (s[192] + s[224])));
+			}
+		}
 		if (mode == SYNC_GRID) {
-			grid_reduce<NV>(*g, red, v, 0u);
-		} else if (mode == SYNC_CLUSTER) {
-			block_reduce<NV>(v, 0u);
-			double *mine = cpart + cflip * kRedWidth;
-			if (threadIdx.x == 0)
+			double *buf = red.part + (size_t)red.flip * kMaxCoopBlocks * kRedWidth;
+			if (threadIdx.x == 0) {
+#pragma unroll
 				for (int k = 0; k < NV; k++)
-					mine[k] = v[k];
+					buf[k * kMaxCoopBlocks + rank] = t[k];
+			}
+			g->sync();
+			if (threadIdx.x < 32) {
+#pragma unroll
+				for (int k = 0; k < NV; k++) {
+					double a0 = 0.0, a1 = 0.0;
+					int b = lane;
+					for (; b + 32 < size; b += 64) {
+						a0 += buf[k * kMaxCoopBlocks + b];
+						a1 += buf[k * kMaxCoopBlocks + b + 32];
+					}
+					if (b < size)
+						a0 += buf[k * kMaxCoopBlocks + b];
+					t[k] = warp_sum(a0 + a1);
+				}
+			}
+			red.flip ^= 1;   // the next reduction writes the other buffer (see GridRed)
+		} else if (mode == SYNC_CLUSTER) {
+			double *mine = cpart + cflip * kRedWidth;
+			if (threadIdx.x == 0) {
+#pragma unroll
+				for (int k = 0; k < NV; k++)
+					mine[k] = t[k];
+			}
 			cg::cluster_group cl = cg::this_cluster();
 			cl.sync();
-			double acc[NV];
-			for (int k = 0; k < NV; k++)
-				acc[k] = 0.0;
-			for (int r = 0; r < size; r++) {
-				const double *other = cl.map_shared_rank(mine, r);
+			if (threadIdx.x < 32) {
+				const double *other = cl.map_shared_rank(mine, lane < size ? lane : 0);
+#pragma unroll
 				for (int k = 0; k < NV; k++)
-					acc[k] += other[k];
+					t[k] = warp_sum(lane < size ? other[k] : 0.0);
 			}
-			for (int k = 0; k < NV; k++)
-				v[k] = acc[k];
-			cflip ^= 1;   // the next reduction writes the other buffer (see GridRed)
-		} else {
-			block_reduce<NV>(v, 0u);
+			cflip ^= 1;
 		}
+		if (threadIdx.x == 0)
+			f(t);
+		__syncthreads();
+	}
+	// The sums in every thread.
+	template <int NV>
+	__device__ __forceinline__ void reduce(double (&v)[NV])
+	{
+		__shared__ double out[NV];
+		reduce_then<NV>(v, [&](const double (&t)[NV]) {
+#pragma unroll
+			for (int k = 0; k < NV; k++)
+				out[k] = t[k];
+		});
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			v[k] = out[k];
 	}
 	__device__ bool leader() const { return rank == 0; }
 	// the blocks of a pass: the team for team-wide levels, this block alone otherwise
