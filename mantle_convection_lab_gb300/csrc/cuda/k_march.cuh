@@ -145,47 +145,22 @@ __device__ __forceinline__ double gt_elem(double u0, double u1, double u2, doubl
 	return g0 * ((u0 + u1) - (u2 + u3)) + g1 * ((w0 + w3) - (w1 + w2));
 }
 
-// (P^T r_f) at coarse node (cx, cz): full weighting 1, 1/2, 1/4 over the 3 x 3
-// fine nodes around (2 cx, 2 cz).
-template <class T, class V>
-__device__ __forceinline__ V restrict_at(const V *__restrict__ rf, int nf, int cx, int cz)
-{
-	V o;
-	o.x = T(0);
-	o.y = T(0);
-#pragma unroll
-	for (int dx = -1; dx <= 1; dx++) {
-		const int fx = 2 * cx + dx;
-		if (fx < 0 || fx >= nf)
-			continue;
-#pragma unroll
-		for (int dz = -1; dz <= 1; dz++) {
-			const int fz = 2 * cz + dz;
-			if (fz < 0 || fz >= nf)
-				continue;
-			const T wgt = (dx == 0 ? T(1) : T(0.5)) * (dz == 0 ? T(1) : T(0.5));
-			const V r = rf[fz + fx * nf];
-			o.x += wgt * r.x;
-			o.y += wgt * r.y;
-		}
-	}
-	return o;
-}
-
 // What a lane holds of one column: x as the pass forms it (0 at Dirichlet
-// dofs), viscosity, mask and the epilogue's operands.
-template <class T, class V>
+// dofs), viscosity, mask, the epilogue's operands, and (c) the coarse or fine
+// values that x is formed from.
+template <class T, class V, int NC>
 struct Column {
-	V x, b, d, x0, c[4];
+	V x, b, d, x0, c[NC];
 	T e;
 	unsigned m;
 };
 
 template <class T, int MODE, int XS, bool X0>
-__device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
+__device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 {
 	typedef typename V2T<T>::t V;
-	typedef Column<T, V> Col;
+	constexpr int NC = XS == XS_ZERO_R ? 9 : XS == XS_PROLONG ? 4 : 1;
+	typedef Column<T, V, NC> Col;
 	constexpr unsigned kAll = 0xffffffffu;
 	constexpr bool kStokes = MODE == PASS_STOKES || MODE == PASS_RES64;
 	constexpr bool kNeedB = MODE == PASS_RESID || MODE == PASS_SMOOTH;
@@ -210,44 +185,56 @@ __device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
 		const bool own = zin && lane >= 1 && lane <= kOwn;
 		const bool ein = gz >= 0 && gz < N && lane < 31;   // this lane's element lies in the box
 		const T pl = ein ? ip : T(0), ql = ein ? iq : T(0);
+		const int gzc = min(max(gz, 0), n - 1);
 
-		// the loads of column ix, and the operands its rows need later
+		// The loads of column ix, and the operands its rows need later.  No branch:
+		// outside the box a lane loads the nearest node and form() takes its value
+		// out, so that the loads of several columns are in flight together.
 		auto load = [&](int ix, Col &k) {
-			k.m = 3u;
-			k.e = T(0);
-			k.x.x = k.x.y = T(0);
-			k.b = k.d = k.x0 = k.x;
-			if (XS == XS_PROLONG)
-				k.c[0] = k.c[1] = k.c[2] = k.c[3] = k.x;
-			if (ix < 0 || ix >= n || !zin)
-				return;
-			const int A = gz + ix * n;
+			const int ixc = min(max(ix, 0), n - 1);
+			const int A = gzc + ixc * n;
 			k.m = P.mask[A];
 			k.e = P.eta[A];
 			if (XS == XS_PLAIN || XS == XS_PROLONG)
 				k.x = P.x[A];
-			if (XS == XS_ZERO_R)
-				k.b = restrict_at<T, V>(P.xc, P.nc, ix, gz);
-			else if (XS == XS_ZERO || kNeedB)
+			if (XS == XS_ZERO || (kNeedB && XS != XS_ZERO_R))
 				k.b = P.b[A];
 			if (XS == XS_ZERO || XS == XS_ZERO_R || MODE == PASS_SMOOTH)
 				k.d = P.invD[A];
 			if (X0)
 				k.x0 = P.x0[A];
 			if (XS == XS_PROLONG) {
-				const int nc = P.nc, a0 = (gz >> 1) + (ix >> 1) * nc, up = gz & 1;
+				const int a0 = (gzc >> 1) + (ixc >> 1) * P.nc, up = gzc & 1, rt = (ixc & 1) * P.nc;
 				k.c[0] = P.xc[a0];
 				k.c[1] = P.xc[a0 + up];
-				k.c[2] = k.c[0];
-				k.c[3] = k.c[1];
-				if (ix & 1) {
-					k.c[2] = P.xc[a0 + nc];
-					k.c[3] = P.xc[a0 + nc + up];
+				k.c[2] = P.xc[a0 + rt];
+				k.c[3] = P.xc[a0 + rt + up];
+			}
+			if (XS == XS_ZERO_R) {
+				// P^T r_f over the 3 x 3 fine nodes around (2 ix, 2 gz); those outside
+				// the box are read at the box's edge and weighted 0
+				const int nf = P.nc;
+#pragma unroll
+				for (int q = 0; q < 9; q++) {
+					const int fx = min(max(2 * ixc + q / 3 - 1, 0), nf - 1), fz = min(max(2 * gzc + q % 3 - 1, 0), nf - 1);
+					k.c[q % NC] = P.xc[fz + fx * nf];
 				}
 			}
 		};
-		auto form = [&](Col &k) {
+		auto form = [&](int ix, Col &k) {
+			const bool in = zin && ix >= 0 && ix < n;
+			if (!in) {
+				k.m = 3u;
+				k.e = T(0);
+			}
 			if (XS == XS_ZERO_R) {
+				const T wl = ix > 0 ? T(0.5) : T(0), wr = ix < n - 1 ? T(0.5) : T(0);
+				const T wd = gz > 0 ? T(0.5) : T(0), wu = gz < n - 1 ? T(0.5) : T(0);
+				const V *c = k.c;
+				k.b.x = (wl * (wd * c[0 % NC].x + c[1 % NC].x + wu * c[2 % NC].x) + (wd * c[3 % NC].x + c[4 % NC].x + wu * c[5 % NC].x)) +
+				        wr * (wd * c[6 % NC].x + c[7 % NC].x + wu * c[8 % NC].x);
+				k.b.y = (wl * (wd * c[0 % NC].y + c[1 % NC].y + wu * c[2 % NC].y) + (wd * c[3 % NC].y + c[4 % NC].y + wu * c[5 % NC].y)) +
+				        wr * (wd * c[6 % NC].y + c[7 % NC].y + wu * c[8 % NC].y);
 				k.b.x = (k.m & 1u) ? T(0) : k.b.x;
 				k.b.y = (k.m & 2u) ? T(0) : k.b.y;
 			}
@@ -256,8 +243,8 @@ __device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
 				k.x.y = P.wload * k.d.y * k.b.y;
 			}
 			if (XS == XS_PROLONG) {
-				k.x.x += T(0.25) * ((k.c[0].x + k.c[1].x) + (k.c[2].x + k.c[3].x));
-				k.x.y += T(0.25) * ((k.c[0].y + k.c[1].y) + (k.c[2].y + k.c[3].y));
+				k.x.x += T(0.25) * ((k.c[0].x + k.c[1 % NC].x) + (k.c[2 % NC].x + k.c[3 % NC].x));
+				k.x.y += T(0.25) * ((k.c[0].y + k.c[1 % NC].y) + (k.c[2 % NC].y + k.c[3 % NC].y));
 			}
 			k.x.x = (k.m & 1u) ? T(0) : k.x.x;
 			k.x.y = (k.m & 2u) ? T(0) : k.x.y;
@@ -266,7 +253,7 @@ __device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
 		Col cur, nx, prev;
 		load(xs - 1, prev);
 		load(xs, nx);
-		form(prev);
+		form(xs - 1, prev);
 		// left edge of the element column: this lane's and the upper neighbour's
 		// values, the viscosity at the edge's two Gauss points
 		T u0n = __shfl_down_sync(kAll, prev.x.x, 1), w0n = __shfl_down_sync(kAll, prev.x.y, 1);
@@ -278,8 +265,7 @@ __device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
 
 		for (int ix = xs; ix <= xe; ix++) {
 			cur = nx;
-			if (ix < xe)
-				load(ix + 1, nx);
+			load(ix + 1, nx);
 			const int ex = ix - 1;
 			const bool exin = ex >= 0 && ex < N;
 			double pe = 0.0;
@@ -293,7 +279,7 @@ __device__ __noinline__ void march(const Pass<T> &P, Part pt, double *dot)
 				dv = P.dotv[A];
 			if (row && MODE == PASS_RES64)
 				dv = P.F[A];
-			form(cur);
+			form(ix, cur);
 			const T u0 = prev.x.x, w0 = prev.x.y, u1 = cur.x.x, w1 = cur.x.y;
 			const T u1n = __shfl_down_sync(kAll, u1, 1), w1n = __shfl_down_sync(kAll, w1, 1);
 			const T e1n = __shfl_down_sync(kAll, cur.e, 1);

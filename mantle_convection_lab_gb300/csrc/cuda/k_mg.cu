@@ -77,12 +77,9 @@ void upload_op_tables(const ShapeTables &S, double r, cudaStream_t st)
 }
 
 // ---- small helpers ----------------------------------------------------------
-// Elements per thread and trip of the FP64 vector loops: their loads are all
-// issued before the arithmetic, so each thread keeps several in flight.
-constexpr int kVecU = 4;
 __device__ __forceinline__ void span(Part pt, int &start, int &stride)
 {
-	start = pt.rank * blockDim.x + threadIdx.x;
+	start = pt.thread();
 	stride = pt.size * blockDim.x;
 }
 
@@ -175,23 +172,39 @@ __device__ void restrict_res(Part pt, const MGLevel<T> &F, const MGLevel<T> &C)
 }
 
 // ---- coarsest grid: dense inverse -------------------------------------------
-// Assemble the coarsest operator densely (FP64), put identity rows on the
-// Dirichlet dofs and invert it by Gauss-Jordan; block 0 only.
+// The operator's inverse on the coarsest grid lives in the leading block's
+// shared memory for the whole solve where it fits (a 4 x 4 grid has 50 dofs),
+// in global memory otherwise (8 x 8: 162 dofs).  Inverting in place in shared
+// memory takes 50 ranks of 2500 FP64 multiply-adds; as an augmented elimination
+// in global memory the set-up of a solve took 0.57 ms.
+constexpr int kCoarseShared = 50;
+
 template <class T>
-__device__ void coarse_build(const MGHier<T> &H)
+struct CoarseShared {
+	double m[kCoarseShared * kCoarseShared];   // the matrix, then its inverse in T in the same place
+	T b[kCoarseShared];
+	__device__ T *inv() { return reinterpret_cast<T *>(m); }
+};
+
+// Assemble the coarsest operator densely (FP64) into M (rows of nd), identity
+// rows and columns on the Dirichlet dofs, and invert it in place by
+// Gauss-Jordan (SPD: no pivoting); one block.
+template <class T>
+__device__ __noinline__ void coarse_invert(const MGHier<T> &H, double *M)
 {
 	const MGLevel<T> &L = H.lv[H.nlev - 1];
 	const OpTab<double> &O = tab<double>();
-	const int nd = H.cnd, n = L.n, N = L.N, w2 = 2 * nd;
-	double *M = H.cwork;
-	for (int k = threadIdx.x; k < nd * w2; k += blockDim.x)
-		M[k] = ((k % w2) == nd + k / w2) ? 1.0 : 0.0;
+	const int nd = H.cnd, n = L.n, N = L.N;
+	for (int k = threadIdx.x; k < nd * nd; k += blockDim.x)
+		M[k] = 0.0;
 	__syncthreads();
-	for (int e = 0; e < N * N; e++) {
-		const int ex = e / N, ez = e - ex * N;
-		const int cn[4] = {ez + ex * n, ez + 1 + ex * n, ez + 1 + (ex + 1) * n, ez + (ex + 1) * n};
-		if (threadIdx.x < 64) {
-			const int p = threadIdx.x >> 3, q = threadIdx.x & 7;
+	// elements of one colour (parities of ex, ez) share no node
+	for (int col = 0; col < 4; col++) {
+		const int w = (N - (col >> 1) + 1) / 2, h = (N - (col & 1) + 1) / 2;
+		for (int k = threadIdx.x; k < w * h * 64; k += blockDim.x) {
+			const int e = k >> 6, p = (k >> 3) & 7, q = k & 7;
+			const int ex = 2 * (e / h) + (col >> 1), ez = 2 * (e % h) + (col & 1);
+			const int cn[4] = {ez + ex * n, ez + 1 + ex * n, ez + 1 + (ex + 1) * n, ez + (ex + 1) * n};
 			const int a = p >> 1, i = p & 1, b = q >> 1, j = q & 1;
 			double kv = 0.0;
 			for (int g = 0; g < 4; g++) {
@@ -209,58 +222,95 @@ __device__ void coarse_build(const MGHier<T> &H)
 					t = O.Dx[a][g] * O.Dz[b][g];
 				kv += eg * t;
 			}
-			M[(2 * cn[a] + i) * w2 + 2 * cn[b] + j] += kv;
+			const int r = 2 * cn[a] + i, c = 2 * cn[b] + j;
+			const bool dr = (L.mask[cn[a]] >> i) & 1u, dc = (L.mask[cn[b]] >> j) & 1u;
+			if (!dr && !dc)
+				M[r * nd + c] += kv;
 		}
 		__syncthreads();
 	}
-	// Dirichlet rows and columns -> identity
-	for (int k = threadIdx.x; k < nd * nd; k += blockDim.x) {
-		const int r = k / nd, c = k - r * nd;
-		const bool dr = (L.mask[r >> 1] >> (r & 1)) & 1u, dc = (L.mask[c >> 1] >> (c & 1)) & 1u;
-		if (dr || dc)
-			M[r * w2 + c] = (r == c) ? 1.0 : 0.0;
-	}
+	for (int r = threadIdx.x; r < nd; r += blockDim.x)
+		if ((L.mask[r >> 1] >> (r & 1)) & 1u)
+			M[r * nd + r] = 1.0;
 	__syncthreads();
-	// Gauss-Jordan on [M | I]; the operator is SPD, no pivoting needed
+	__shared__ double ipiv;
 	for (int k = 0; k < nd; k++) {
-		__shared__ double piv;
-		if (threadIdx.x == 0)
-			piv = M[k * w2 + k];
-		__syncthreads();
-		for (int c = threadIdx.x; c < w2; c += blockDim.x)
-			M[k * w2 + c] /= piv;
-		__syncthreads();
-		for (int idx = threadIdx.x; idx < nd * w2; idx += blockDim.x) {
-			const int r = idx / w2, c = idx - r * w2;
-			if (r != k) {
-				const double f = M[r * w2 + k];
-				if (c != k)
-					M[r * w2 + c] -= f * M[k * w2 + c];
-			}
+		if (threadIdx.x == 0) {
+			ipiv = 1.0 / M[k * nd + k];
+			M[k * nd + k] = 1.0;
 		}
 		__syncthreads();
-		for (int r = threadIdx.x; r < nd; r += blockDim.x)
-			if (r != k)
-				M[r * w2 + k] = 0.0;
+		const double s = ipiv;
+		for (int c = threadIdx.x; c < nd; c += blockDim.x)
+			M[k * nd + c] *= s;
+		__syncthreads();
+		// a row per warp: its factor is read before any lane clears it
+		const int lane = threadIdx.x & 31;
+		for (int r = threadIdx.x >> 5; r < nd; r += blockDim.x >> 5) {
+			if (r == k)
+				continue;
+			const double f = M[r * nd + k];
+			__syncwarp();
+			for (int c = lane; c < nd; c += 32)
+				M[r * nd + c] = (c == k ? 0.0 : M[r * nd + c]) - f * M[k * nd + c];
+			__syncwarp();
+		}
 		__syncthreads();
 	}
-	for (int k = threadIdx.x; k < nd * nd; k += blockDim.x)
-		H.cinv[k] = (T)M[(k / nd) * w2 + nd + (k % nd)];
+}
+
+template <class T>
+__device__ void coarse_build(const MGHier<T> &H, CoarseShared<T> &cs)
+{
+	const bool sh = H.cnd <= kCoarseShared;
+	double *M = sh ? cs.m : H.cwork;
+	const int n2 = H.cnd * H.cnd;
+	coarse_invert<T>(H, M);
+	if (!sh) {
+		for (int k = threadIdx.x; k < n2; k += blockDim.x)
+			H.cinv[k] = (T)M[k];
+		__syncthreads();
+		return;
+	}
+	constexpr int kPer = (kCoarseShared * kCoarseShared + kBlock - 1) / kBlock;
+	T v[kPer];
+#pragma unroll
+	for (int u = 0; u < kPer; u++)
+		v[u] = threadIdx.x + u * kBlock < n2 ? (T)M[threadIdx.x + u * kBlock] : T(0);
+	__syncthreads();
+#pragma unroll
+	for (int u = 0; u < kPer; u++)
+		if (threadIdx.x + u * kBlock < n2)
+			cs.inv()[threadIdx.x + u * kBlock] = v[u];
 	__syncthreads();
 }
 
+// x = inverse * b, four lanes per row (interleaved columns); one block.
 template <class T, class V>
-__device__ void coarse_solve(const MGHier<T> &H, V *x)
+__device__ void coarse_solve(const MGHier<T> &H, CoarseShared<T> &cs, V *x)
 {
 	const MGLevel<T> &L = H.lv[H.nlev - 1];
 	const int nd = H.cnd;
-	const T *b = reinterpret_cast<const T *>(L.b);
+	const bool sh = nd <= kCoarseShared;
+	const T *b = reinterpret_cast<const T *>(L.b), *inv = sh ? cs.inv() : H.cinv;
 	T *xo = reinterpret_cast<T *>(x);
-	for (int i = threadIdx.x; i < nd; i += blockDim.x) {
+	if (sh) {
+		for (int i = threadIdx.x; i < nd; i += blockDim.x)
+			cs.b[i] = b[i];
+		__syncthreads();
+		b = cs.b;
+	}
+	const int part = threadIdx.x & 3;
+	for (int i0 = 0; i0 < nd; i0 += blockDim.x / 4) {
+		const int i = i0 + (threadIdx.x >> 2);
 		T s = 0;
-		for (int j = 0; j < nd; j++)
-			s += H.cinv[i * nd + j] * b[j];
-		xo[i] = s;
+		if (i < nd)
+			for (int j = part; j < nd; j += 4)
+				s += inv[i * nd + j] * b[j];
+		s += __shfl_xor_sync(0xffffffffu, s, 1);
+		s += __shfl_xor_sync(0xffffffffu, s, 2);
+		if (i < nd && part == 0)
+			xo[i] = s;
 	}
 	__syncthreads();
 }
@@ -289,7 +339,7 @@ __device__ __forceinline__ Pass<T> level_pass(const MGLevel<T> &L, const typenam
 }
 
 template <class T>
-__device__ void level_down(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, bool grid, bool active,
+__device__ __forceinline__ void level_down(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, bool grid, bool active,
                            typename V2T<T>::t **xcur)
 {
 	typedef typename V2T<T>::t V;
@@ -365,7 +415,7 @@ __device__ void level_down(Sync &sy, const MGHier<T> &H, int l, const typename V
 // share of out0.dotv into *dot and is not followed by a barrier: the caller's
 // reduction provides it.
 template <class T>
-__device__ void level_up(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
+__device__ __forceinline__ void level_up(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
                          bool grid, bool active, typename V2T<T>::t **xcur, const double2 *dotv = nullptr,
                          double *dot = nullptr)
 {
@@ -415,11 +465,15 @@ __device__ void level_up(Sync &sy, const MGHier<T> &H, int l, const typename V2T
 	xcur[l] = x;
 }
 
+// Everything below is inlined, once for each correction solve: the passes use
+// most of a thread's registers, and as calls they saved and restored them on
+// the stack on every level (25 of 98 us per MINRES iteration at 64^2), where a
+// barrier's acquire has just emptied L1.
 // out0 = B rhs0.  With dotv, *dot receives this thread's share of out0.dotv
 // and the cycle ends without a barrier (the caller reduces *dot, which
 // synchronises the team); without it the cycle ends with a barrier.
 template <class T>
-__device__ void vcycle(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
+__device__ __forceinline__ void vcycle(Sync &sy, CoarseShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
                        const double2 *dotv = nullptr, double *dot = nullptr)
 {
 	typedef typename V2T<T>::t V;
@@ -430,11 +484,13 @@ __device__ void vcycle(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *r
 	const bool b0 = sy.leader();
 	if (dot)
 		*dot = 0.0;
+#pragma unroll 1
 	for (int l = 0; l < lc; l++)
 		level_down<T>(sy, H, l, rhs0, l < nb, l < nb || b0, xcur);
 	if (b0)
-		coarse_solve<T, V>(H, H.lv[lc].xa);
+		coarse_solve<T, V>(H, cs, H.lv[lc].xa);
 	xcur[lc] = H.lv[lc].xa;
+#pragma unroll 1
 	for (int l = lc - 1; l >= 0; l--) {
 		if (l == nb - 1)
 			sy.sync();   // block 0's coarse-level results become visible to every block
@@ -449,7 +505,7 @@ __device__ void vcycle(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *r
 // others wait for its broadcast: a division or a square root on every thread
 // costs the FP64 pipe (2 lanes per clock and SM) about a microsecond each.
 template <class T>
-__device__ int pcg_inner(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
+__device__ __noinline__ int pcg_inner(Sync &sy, CoarseShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
                          int maxit)
 {
 	typedef typename V2T<T>::t V;
@@ -472,19 +528,32 @@ __device__ int pcg_inner(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t 
 	sy.reduce_then<1>(bb, [&](const double (&v)[1]) { bb0 = v[0]; });
 	if (!(bb0 > 0.0))
 		return 0;
-	vcycle<T>(sy, H, r, z);
-	double rz[1] = {0.0};
-	for (int A = tid; A < nn; A += nth) {
-		const V rv = r[A], zv = z[A];
-		rz[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
-		p[A] = zv;
-	}
-	sy.reduce_then<1>(rz, [&](const double (&v)[1]) { rho = v[0]; });
 	Pass<T> P = level_pass<T>(L, nullptr);
 	P.x = p;
 	P.out = q;
 	int it = 0;
 	while (it < maxit) {
+		vcycle<T>(sy, cs, H, r, z);
+		double rz[1] = {0.0};
+		for (int A = tid; A < nn; A += nth) {
+			const V rv = r[A], zv = z[A];
+			rz[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
+		}
+		sy.reduce_then<1>(rz, [&](const double (&v)[1]) {
+			co = it > 0 ? v[0] / rho : 0.0;
+			rho = v[0];
+		});
+		const T be = (T)co;
+		for (int A = tid; A < nn; A += nth) {
+			V pv = z[A];
+			if (it > 0) {
+				const V po = p[A];
+				pv.x += be * po.x;
+				pv.y += be * po.y;
+			}
+			p[A] = pv;
+		}
+		sy.sync();
 		double pq[1];
 		march<T, PASS_MATVEC, XS_PLAIN, false>(P, sy.part(true), pq);
 		sy.reduce_then<1>(pq, [&](const double (&v)[1]) { co = rho / v[0]; });
@@ -507,25 +576,6 @@ __device__ int pcg_inner(Sync &sy, const MGHier<T> &H, const typename V2T<T>::t 
 		it++;
 		if (!(rr[0] > rtol * rtol * bb0) || !isfinite(alpha))
 			break;
-		vcycle<T>(sy, H, r, z);
-		double rz2[1] = {0.0};
-		for (int A = tid; A < nn; A += nth) {
-			const V rv = r[A], zv = z[A];
-			rz2[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
-		}
-		sy.reduce_then<1>(rz2, [&](const double (&v)[1]) {
-			co = v[0] / rho;
-			rho = v[0];
-		});
-		const T be = (T)co;
-		for (int A = tid; A < nn; A += nth) {
-			const V zv = z[A];
-			V pv = p[A];
-			pv.x = zv.x + be * pv.x;
-			pv.y = zv.y + be * pv.y;
-			p[A] = pv;
-		}
-		sy.sync();
 	}
 	sy.sync();
 	return it;
@@ -622,138 +672,155 @@ __device__ void stokes_residual(const MGArgs<TI> &a, Sync &sy, const double2 *d,
 	sy.reduce<3>(rs);
 }
 
-// ---- MINRES vector kernels (FP64), kVecU elements per thread and trip ---------
+// ---- MINRES vector kernels (FP64) ---------
 // Separate functions so that their registers do not compete with the solver's
-// state; every load of a trip is issued before its arithmetic.  Bound by the
-// FP64 pipe and HBM together at 1024^2 (12 and 12 FP64 operations per node and
-// element); conversions to and from TI go through widen / narrow.
+// state.  Bound by the FP64 pipe and HBM together at 1024^2 (the velocity and
+// direction updates: 11 and 12 FP64 operations, 120 and 112 B per node and
+// element), so each trip's loads are issued before the previous trip's
+// arithmetic; conversions to and from TI go through widen / narrow.
 
 // v_old <- az ig - dg v - gg v_old (velocity, with its TI copy into bI) and the
 // same for the pressure part with Ahp, whose preconditioned vector z_p = v_p / BAB
 // is formed with it; returns this thread's share of z_p.v_p.
 template <class VI>
-__device__ __noinline__ double minres_v_update(int nn, int ne, int tid, int nth, const double2 *__restrict__ az_,
-                                               const double2 *__restrict__ v_, double2 *__restrict__ vo_,
-                                               VI *__restrict__ bI, const double *__restrict__ ah_,
-                                               const double *__restrict__ p0_, double *__restrict__ p1_,
-                                               const double *__restrict__ ibab, double *__restrict__ zp1_, double ig,
-                                               double dg, double gg)
+__device__ __noinline__ void minres_v_nodes(int nn, int tid, int nth, const double2 *__restrict__ az_,
+                                            const double2 *__restrict__ v_, double2 *__restrict__ vo_,
+                                            VI *__restrict__ bI, double ig, double dg, double gg)
 {
 	typedef decltype(VI().x) TI;
-	for (int A0 = tid; A0 < nn; A0 += kVecU * nth) {
-		double2 az[kVecU], v[kVecU], vo[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int A = A0 + u * nth;
-			if (A < nn) {
-				az[u] = az_[A];
-				v[u] = v_[A];
-				vo[u] = vo_[A];
-			}
+	double2 az, v, vo;
+	auto load = [&](int A) {
+		if (A < nn) {
+			az = az_[A];
+			v = v_[A];
+			vo = vo_[A];
 		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int A = A0 + u * nth;
-			if (A < nn) {
-				const double2 vn = make_double2(az[u].x * ig - dg * v[u].x - gg * vo[u].x,
-				                                az[u].y * ig - dg * v[u].y - gg * vo[u].y);
-				vo_[A] = vn;
-				VI w;
-				w.x = narrow_to<TI>(vn.x);
-				w.y = narrow_to<TI>(vn.y);
-				bI[A] = w;
-			}
-		}
+	};
+	load(tid);
+	for (int A = tid; A < nn; A += nth) {
+		const double2 caz = az, cv = v, cvo = vo;
+		load(A + nth);
+		const double2 vn = make_double2(caz.x * ig - dg * cv.x - gg * cvo.x, caz.y * ig - dg * cv.y - gg * cvo.y);
+		vo_[A] = vn;
+		VI w;
+		w.x = narrow_to<TI>(vn.x);
+		w.y = narrow_to<TI>(vn.y);
+		bI[A] = w;
 	}
-	double acc = 0.0;
-	for (int e0 = tid; e0 < ne; e0 += kVecU * nth) {
-		double ah[kVecU], p0[kVecU], p1[kVecU], ib[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				ah[u] = ah_[e];
-				p0[u] = p0_[e];
-				p1[u] = p1_[e];
-				ib[u] = ibab[e];
-			}
+}
+
+__device__ __noinline__ double minres_v_elems(int ne, int tid, int nth, const double *__restrict__ ah_,
+                                              const double *__restrict__ p0_, double *__restrict__ p1_,
+                                              const double *__restrict__ ibab, double *__restrict__ zp1_, double ig,
+                                              double dg, double gg)
+{
+	double ah, p0, p1, ib, acc = 0.0;
+	auto load = [&](int e) {
+		if (e < ne) {
+			ah = ah_[e];
+			p0 = p0_[e];
+			p1 = p1_[e];
+			ib = ibab[e];
 		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				const double vn = ah[u] * ig - dg * p0[u] - gg * p1[u], z = vn * ib[u];
-				p1_[e] = vn;
-				zp1_[e] = z;
-				acc += z * vn;
-			}
-		}
+	};
+	load(tid);
+	for (int e = tid; e < ne; e += nth) {
+		const double cah = ah, c0 = p0, c1 = p1, cib = ib;
+		load(e + nth);
+		const double vn = cah * ig - dg * c0 - gg * c1, z = vn * cib;
+		p1_[e] = vn;
+		zp1_[e] = z;
+		acc += z * vn;
 	}
 	return acc;
 }
 
-// w_old <- k1 z - k3 w_old - k2 w and x += step w_old, for the velocity (z in
-// TI) and the pressure parts.
+// w_old <- k1 z - k3 w_old - k2 w for the velocity (z in TI) and the pressure
+// parts, and the solution's update: steps 0 none, 1 x += s0 w_new, 2
+// x += s1 w + s0 w_new.
 template <class VI>
-__device__ __noinline__ void minres_w_update(int nn, int ne, int tid, int nth, const VI *__restrict__ z_,
-                                             double2 *__restrict__ wo_, const double2 *__restrict__ w_,
-                                             double2 *__restrict__ x_, const double *__restrict__ zp_,
-                                             double *__restrict__ wpo_, const double *__restrict__ wp_,
-                                             double *__restrict__ xp_, double k1, double k3, double k2, double step)
+__device__ __noinline__ void minres_w_nodes(int steps, int nn, int tid, int nth, const VI *__restrict__ z_,
+                                            double2 *__restrict__ wo_, const double2 *__restrict__ w_,
+                                            double2 *__restrict__ x_, double k1, double k3, double k2, double s0,
+                                            double s1)
 {
-	for (int A0 = tid; A0 < nn; A0 += kVecU * nth) {
-		VI z[kVecU];
-		double2 wo[kVecU], w[kVecU], x[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int A = A0 + u * nth;
-			if (A < nn) {
-				z[u] = z_[A];
-				wo[u] = wo_[A];
-				w[u] = w_[A];
-				x[u] = x_[A];
-			}
+	VI z;
+	double2 wo, w, x = make_double2(0.0, 0.0);
+	auto load = [&](int A) {
+		if (A < nn) {
+			z = z_[A];
+			wo = wo_[A];
+			w = w_[A];
+			if (steps > 0)
+				x = x_[A];
 		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int A = A0 + u * nth;
-			if (A < nn) {
-				const double2 wn = make_double2(widen(z[u].x) * k1 - k3 * wo[u].x - k2 * w[u].x,
-				                                widen(z[u].y) * k1 - k3 * wo[u].y - k2 * w[u].y);
-				wo_[A] = wn;
-				x_[A] = make_double2(x[u].x + step * wn.x, x[u].y + step * wn.y);
+	};
+	load(tid);
+	for (int A = tid; A < nn; A += nth) {
+		const VI cz = z;
+		const double2 co = wo, cw = w;
+		double2 cx = x;
+		load(A + nth);
+		const double2 wn = make_double2(widen(cz.x) * k1 - k3 * co.x - k2 * cw.x, widen(cz.y) * k1 - k3 * co.y - k2 * cw.y);
+		wo_[A] = wn;
+		if (steps > 0) {
+			if (steps > 1) {
+				cx.x += s1 * cw.x;
+				cx.y += s1 * cw.y;
 			}
-		}
-	}
-	for (int e0 = tid; e0 < ne; e0 += kVecU * nth) {
-		double zz[kVecU], wo[kVecU], w[kVecU], x[kVecU];
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				zz[u] = zp_[e];
-				wo[u] = wpo_[e];
-				w[u] = wp_[e];
-				x[u] = xp_[e];
-			}
-		}
-#pragma unroll
-		for (int u = 0; u < kVecU; u++) {
-			const int e = e0 + u * nth;
-			if (e < ne) {
-				const double wn = zz[u] * k1 - k3 * wo[u] - k2 * w[u];
-				wpo_[e] = wn;
-				xp_[e] = x[u] + step * wn;
-			}
+			x_[A] = make_double2(cx.x + s0 * wn.x, cx.y + s0 * wn.y);
 		}
 	}
+}
+
+__device__ __noinline__ void minres_w_elems(int steps, int ne, int tid, int nth, const double *__restrict__ z_,
+                                            double *__restrict__ wo_, const double *__restrict__ w_,
+                                            double *__restrict__ x_, double k1, double k3, double k2, double s0,
+                                            double s1)
+{
+	double z, wo, w, x = 0.0;
+	auto load = [&](int e) {
+		if (e < ne) {
+			z = z_[e];
+			wo = wo_[e];
+			w = w_[e];
+			if (steps > 0)
+				x = x_[e];
+		}
+	};
+	load(tid);
+	for (int e = tid; e < ne; e += nth) {
+		const double cz = z, co = wo, cw = w;
+		double cx = x;
+		load(e + nth);
+		const double wn = cz * k1 - k3 * co - k2 * cw;
+		wo_[e] = wn;
+		if (steps > 0) {
+			if (steps > 1)
+				cx += s1 * cw;
+			x_[e] = cx + s0 * wn;
+		}
+	}
+}
+
+// x += s w, the last pending step of a solve that ends before its next update
+__device__ __noinline__ void minres_x_update(int nn, int ne, int tid, int nth, const double2 *__restrict__ w_,
+                                             double2 *__restrict__ x_, const double *__restrict__ wp_,
+                                             double *__restrict__ xp_, double s)
+{
+	for (int A = tid; A < nn; A += nth) {
+		const double2 w = w_[A], x = x_[A];
+		x_[A] = make_double2(x.x + s * w.x, x.y + s * w.y);
+	}
+	for (int e = tid; e < ne; e += nth)
+		xp_[e] += s * wp_[e];
 }
 
 // z = M^-1 v for M = diag(one V-cycle of K, BAB): the velocity part goes
 // through the TI hierarchy (z_u stays in TI), the pressure part is multiplied
 // by 1/BAB (a.bab holds the reciprocal).  Returns <z, v> over the team.
 template <class TI>
-__device__ double block_precond(const MGArgs<TI> &a, Sync &sy, const double2 *vu, const double *vp,
+__device__ double block_precond(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, const double2 *vu, const double *vp,
                                 typename V2T<TI>::t *zu, double *zp)
 {
 	typedef typename V2T<TI>::t VI;
@@ -770,7 +837,7 @@ __device__ double block_precond(const MGArgs<TI> &a, Sync &sy, const double2 *vu
 	}
 	sy.sync();
 	double dot[1] = {0.0};
-	vcycle<TI>(sy, H, bI, zu, vu, &dot[0]);   // the last sweep forms <z_u, v_u>
+	vcycle<TI>(sy, cs, H, bI, zu, vu, &dot[0]);   // the last sweep forms <z_u, v_u>
 	for (int e = tid; e < ne; e += nth) {
 		const double z = vp[e] * a.bab[e];
 		zp[e] = z;
@@ -812,7 +879,7 @@ __device__ void stokes_apply(const MGArgs<TI> &a, Sync &sy, const double2 *u, co
 // carried on and amplified from step to step), 111 against 100 per step over
 // 30 steps; warm_start=3 stays the default there.
 template <class TI>
-__device__ void warm_guess(const MGArgs<TI> &a, Sync &sy, int ndir)
+__device__ __noinline__ void warm_guess(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, int ndir)
 {
 	typedef typename V2T<TI>::t VI;
 	const int tid = sy.tid, nth = sy.nth;
@@ -843,8 +910,8 @@ __device__ void warm_guess(const MGArgs<TI> &a, Sync &sy, int ndir)
 	// M^-1 a_k (the preconditioner's pressure part divides by BAB); the signs of
 	// the continuity parts follow r = [F - K d - G p ; -G^T d]
 	double q[5];   // <a1, M^-1 a1>, <a2, M^-1 a1>, <a2, M^-1 a2>, <r0, M^-1 a1>, <r0, M^-1 a2>
-	q[0] = block_precond(a, sy, Y1, Yc1, Z1, Zp1);
-	q[2] = ndir == 2 ? block_precond(a, sy, Y2, Yc2, Z2, Zp2) : 0.0;
+	q[0] = block_precond(a, sy, cs, Y1, Yc1, Z1, Zp1);
+	q[2] = ndir == 2 ? block_precond(a, sy, cs, Y2, Yc2, Z2, Zp2) : 0.0;
 	double c[3] = {0.0, 0.0, 0.0};
 	for (int A = tid; A < nn; A += nth) {
 		const double2 r = a.R[A];
@@ -918,7 +985,7 @@ struct MinresScal {
 // refinement around this solve restores full accuracy.  Stops when the
 // M^-1-norm of the residual has dropped by rtol.  Returns the iterations.
 template <class TI>
-__device__ int minres_correction(const MGArgs<TI> &a, Sync &sy, double rtol, int maxit, int *status)
+__device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, double rtol, int maxit, int *status)
 {
 	typedef typename V2T<TI>::t VI;
 	__shared__ MinresScal ms;
@@ -955,56 +1022,57 @@ __device__ int minres_correction(const MGArgs<TI> &a, Sync &sy, double rtol, int
 		a.dpv[e] = 0.0;
 	}
 	sy.sync();
-	double dot[1];
-	vcycle<TI>(sy, H, bI, zu[0], vu[0], &dot[0]);
-	dot[0] += pdot;
-	sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
-		const double g = sqrt(fmax(v[0], 0.0));
-		ms.gam = g;
-		ms.gam_prev = 1.0;
-		ms.eta = ms.eta0 = g;
-		ms.c_prev = ms.c_cur = 1.0;
-		ms.s_prev = ms.s_cur = 0.0;
-		ms.ig = 1.0 / g;
-		ms.gg = g;
-		ms.stop = v[0] > 0.0 ? 0 : 2;
-	});
-	if (ms.stop)
-		return 0;
 	Pass<TI> P = level_pass<TI>(L0, nullptr);
 	P.out64 = a.Kd;
 	P.gt_out = a.Ahp;
 	P.g0 = a.gt.g0[0];
 	P.g1 = a.gt.g1[0];
 	P.gp_morton = 0;
-	int cv = 0, cw = 0, it = 0;   // index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1)
+	double step1 = 0.0;           // the step of the iteration before, not yet applied when `it` is odd
+	// index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1).  it = -1: z(0) = M^-1 v(0)
+	int cv = 1, cw = 0, it = -1;
+#pragma unroll 1
 	while (it < maxit) {
-		// A z(j), unscaled (z~ = z / gam): K z_u + G z_p into a.Kd, G^T z_u into
-		// a.Ahp, and their product with (z_u, z_p)
-		double dl[1];
-		P.x = zu[cv];
-		P.gp = zp[cv];
-		march<TI, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), dl);
-		sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
-			ms.delta = v[0] * ms.ig * ms.ig;
-			ms.dg = ms.delta * ms.ig;
-		});
-		// v(j+1) = A z~ - (delta/gam) v(j) - (gam/gam_prev) v(j-1), into v(j-1)'s
-		// buffer, its TI copy as the V-cycle's right-hand side, and z_p(j+1)
-		const double pd = minres_v_update<VI>(nn, ne, tid, nth, a.Kd, vu[cv], vu[1 - cv], bI, a.Ahp, vp[cv], vp[1 - cv],
-		                                      a.bab, zp[1 - cv], ms.ig, ms.dg, ms.gg);
-		sy.sync();
-		vcycle<TI>(sy, H, bI, zu[1 - cv], vu[1 - cv], &dot[0]);
-		dot[0] += pd;
+		if (it >= 0) {
+			// A z(j), unscaled (z~ = z / gam): K z_u + G z_p into a.Kd, G^T z_u into
+			// a.Ahp, and their product with (z_u, z_p)
+			double dl[1];
+			P.x = zu[cv];
+			P.gp = zp[cv];
+			march<TI, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), dl);
+			sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
+				ms.delta = v[0] * ms.ig * ms.ig;
+				ms.dg = ms.delta * ms.ig;
+			});
+			// v(j+1) = A z~ - (delta/gam) v(j) - (gam/gam_prev) v(j-1), into v(j-1)'s
+			// buffer, its TI copy as the V-cycle's right-hand side, and z_p(j+1)
+			minres_v_nodes<VI>(nn, tid, nth, a.Kd, vu[cv], vu[1 - cv], bI, ms.ig, ms.dg, ms.gg);
+			pdot = minres_v_elems(ne, tid, nth, a.Ahp, vp[cv], vp[1 - cv], a.bab, zp[1 - cv], ms.ig, ms.dg, ms.gg);
+			sy.sync();
+		}
+		double dot[1];
+		vcycle<TI>(sy, cs, H, bI, zu[1 - cv], vu[1 - cv], &dot[0]);
+		dot[0] += pdot;
 		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
-			// Givens rotations
 			const double gn2 = fmax(v[0], 0.0);
+			const double gam_next = sqrt(gn2);
+			if (it < 0) {
+				ms.gam = gam_next;
+				ms.gam_prev = 1.0;
+				ms.eta = ms.eta0 = gam_next;
+				ms.c_prev = ms.c_cur = 1.0;
+				ms.s_prev = ms.s_cur = 0.0;
+				ms.ig = 1.0 / gam_next;
+				ms.gg = gam_next;
+				ms.stop = v[0] > 0.0 ? 0 : 3;
+				return;
+			}
+			// Givens rotations
 			const double a0 = ms.c_cur * ms.delta - ms.c_prev * ms.s_cur * ms.gam;
 			const double a1s = a0 * a0 + gn2;
 			const double a2 = ms.s_cur * ms.delta + ms.c_prev * ms.c_cur * ms.gam;
 			const double a3 = ms.s_prev * ms.gam;
 			const double ia1 = rsqrt(a1s);
-			const double gam_next = sqrt(gn2);
 			ms.stop = 0;
 			if (!(a1s > 0.0) || !isfinite(a1s)) {
 				ms.stop = isfinite(a1s) ? 2 : 6;
@@ -1028,14 +1096,28 @@ __device__ int minres_correction(const MGArgs<TI> &a, Sync &sy, double rtol, int
 			else if (!(fabs(ms.eta) > rtol * ms.eta0) || !(gam_next > 0.0))
 				ms.stop = 1;
 		});
+		if (it < 0) {
+			if (ms.stop)
+				return 0;
+			it = 0;
+			cv = 0;
+			continue;
+		}
 		const int stop = ms.stop;
 		if ((stop & 4) && tid == 0)
 			atomicOr(status, 2);
-		if (stop & 2)
+		if (stop & 2) {
+			if (it & 1)   // the pending step along w(j)
+				minres_x_update(nn, ne, tid, nth, wu[cw], a.dd, wp[cw], a.dpv, step1);
 			break;
-		// into w(j-1)'s buffer
-		minres_w_update<VI>(nn, ne, tid, nth, zu[cv], wu[1 - cw], wu[cw], a.dd, zp[cv], wp[1 - cw], wp[cw], a.dpv, ms.k1,
-		                    ms.k3, ms.k2, ms.step);
+		}
+		// into w(j-1)'s buffer; the solution takes the steps of two iterations at a time
+		// (x += step w(j) + step' w(j+1), the same additions in the same order), or what
+		// is pending when the loop ends
+		const int steps = (it & 1) ? 2 : (stop || it + 1 >= maxit) ? 1 : 0;
+		minres_w_nodes<VI>(steps, nn, tid, nth, zu[cv], wu[1 - cw], wu[cw], a.dd, ms.k1, ms.k3, ms.k2, ms.step, step1);
+		minres_w_elems(steps, ne, tid, nth, zp[cv], wp[1 - cw], wp[cw], a.dpv, ms.k1, ms.k3, ms.k2, ms.step, step1);
+		step1 = ms.step;
 		it++;
 		cv = 1 - cv;
 		cw = 1 - cw;
@@ -1072,6 +1154,7 @@ template <class TI>
 __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 {
 	typedef typename V2T<TI>::t VI;
+	__shared__ CoarseShared<TI> cs;
 	const MGHier<TI> &H = a.H;
 	const int tid = sy.tid, nth = sy.nth;
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
@@ -1129,7 +1212,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 		a.bab[e] = 1.0 / s;   // the solvers multiply by 1/BAB
 	}
 	if (sy.leader())
-		coarse_build<TI>(H);
+		coarse_build<TI>(H, cs);
 	sy.sync();
 
 	int refine = 0, outer_total = 0, inner_total = 0, capped = 0;
@@ -1137,7 +1220,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 	if (a.method == 1 && a.h1d != nullptr) {
 		const int nh = a.sc->nsolved < 3 ? a.sc->nsolved : 3;   // solutions in the history
 		if (nh >= 2)
-			warm_guess<TI>(a, sy, nh - 1);
+			warm_guess<TI>(a, sy, cs, nh - 1);
 	}
 	if (a.d_alt != nullptr) {
 		// Two candidate guesses: (d, p) from the network and (d_alt, p_alt),
@@ -1189,7 +1272,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 			// where MINRES converges fastest; close to it, by what is left to
 			// reach rtol (with a factor 2 margin), but not below outer_rtol.
 			const double prt = res > 1e4 * a.rtol ? 1e-2 : fmax(a.outer_rtol, 0.5 * a.rtol / res);
-			const int it = minres_correction<TI>(a, sy, prt, a.max_outer, status);
+			const int it = minres_correction<TI>(a, sy, cs, prt, a.max_outer, status);
 			outer_total += it;
 			inner_total += it + 1;
 			for (int A = tid; A < nn; A += nth) {
@@ -1214,7 +1297,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 			bI[A] = v;
 		}
 		sy.sync();
-		inner_total += pcg_inner<TI>(sy, H, bI, xI, a.inner_rtol, a.max_inner);
+		inner_total += pcg_inner<TI>(sy, cs, H, bI, xI, a.inner_rtol, a.max_inner);
 		for (int A = tid; A < nn; A += nth) {
 			const VI v = xI[A];
 			a.dd[A] = make_double2(widen(v.x), widen(v.y));
@@ -1256,7 +1339,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 				bI[A] = w;
 			}
 			sy.sync();
-			inner_total += pcg_inner<TI>(sy, H, bI, xI, a.inner_rtol, a.max_inner);
+			inner_total += pcg_inner<TI>(sy, cs, H, bI, xI, a.inner_rtol, a.max_inner);
 			for (int A = tid; A < nn; A += nth) {
 				const VI v = xI[A];
 				a.u1[A] = make_double2(widen(v.x), widen(v.y));
@@ -1362,8 +1445,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg(const __
 	sy.cflip = 0;
 	sy.rank = blockIdx.x;
 	sy.size = gridDim.x;
-	sy.tid = blockIdx.x * blockDim.x + threadIdx.x;
-	sy.nth = gridDim.x * blockDim.x;
+	sy.spread();
 	stokes_solve<TI>(sa, sy);
 }
 
@@ -1401,8 +1483,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(co
 			sy.cpart = cpart;
 			sy.rank = rank;
 			sy.size = cs;
-			sy.tid = rank * blockDim.x + threadIdx.x;
-			sy.nth = cs * blockDim.x;
+			sy.spread();
 			stokes_solve<TI>(sa, sy);
 			cl.sync();   // no block starts the next model (or leaves) while another reads its partials
 		} else {
@@ -1417,8 +1498,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(co
 			sy.cpart = nullptr;
 			sy.rank = 0;
 			sy.size = 1;
-			sy.tid = threadIdx.x;
-			sy.nth = blockDim.x;
+			sy.spread();
 			stokes_solve<TI>(sa, sy);
 			__syncthreads();
 		}

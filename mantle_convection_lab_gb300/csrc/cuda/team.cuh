@@ -11,6 +11,9 @@ namespace mclg {
 // whole grid, a thread-block cluster, or one block alone).
 struct Part {
 	int rank, size;
+	// This thread's number in the blocks of the pass: warps are dealt to the
+	// blocks in turn, so that a loop of few trips uses many SMs.
+	__device__ int thread() const { return (((threadIdx.x >> 5) * size + rank) << 5) + (threadIdx.x & 31); }
 };
 
 // ---- where a solve runs ---------------------------------------------------------
@@ -46,15 +49,20 @@ struct Sync {
 	// value's 256 thread partials go through shared memory to one warp (8 + 5
 	// additions): a butterfly in every warp takes eight times that of the FP64
 	// pipe, which has 2 lanes per clock and SM.
+	__device__ static double *scratch()
+	{
+		__shared__ double sh[kRedWidth * kBlock];
+		return sh;
+	}
 	template <int NV, class F>
 	__device__ __forceinline__ void reduce_then(const double (&v)[NV], F f)
 	{
 		static_assert(NV <= kRedWidth, "partials per reduction");
-		__shared__ double sh[NV][kBlock];
+		double *sh = scratch();
 		const int lane = threadIdx.x & 31;
 #pragma unroll
 		for (int k = 0; k < NV; k++)
-			sh[k][threadIdx.x] = v[k];
+			sh[k * kBlock + threadIdx.x] = v[k];
 		__syncthreads();
 		double t[NV];
 #pragma unroll
@@ -63,7 +71,7 @@ struct Sync {
 		if (threadIdx.x < 32) {
 #pragma unroll
 			for (int k = 0; k < NV; k++) {
-				const double *s = sh[k] + lane;
+				const double *s = sh + k * kBlock + lane;
 				t[k] = warp_sum(((s[0] + s[32]) + (s[64] + s[96])) + ((s[128] + s[160]) + (s[192] + s[224])));
 			}
 		}
@@ -124,6 +132,12 @@ struct Sync {
 #pragma unroll
 		for (int k = 0; k < NV; k++)
 			v[k] = out[k];
+	}
+	// tid and nth for loops over nodes and elements (see Part::thread)
+	__device__ void spread()
+	{
+		tid = Part{rank, size}.thread();
+		nth = size * blockDim.x;
 	}
 	__device__ bool leader() const { return rank == 0; }
 	// the blocks of a pass: the team for team-wide levels, this block alone otherwise
