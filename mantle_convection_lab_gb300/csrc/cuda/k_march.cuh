@@ -26,6 +26,22 @@
 
 constexpr int kOwn = 30;   // nodes of a strip that the warp owns (lanes 1..30)
 
+// How a level's strips and columns are cut into tasks for a number of warps;
+// formed once per solve (the divisions took a tenth of a small level's pass).
+struct Split {
+	int strips, Lx, ntasks;
+	float inv;   // 1/strips: t/strips for t < 2^22 as the truncated product with (t + 1/2)
+	__device__ void set(int n, int nwarps)
+	{
+		strips = (n + kOwn - 1) / kOwn;
+		int chunks = nwarps / strips;   // the columns are cut into as many chunks as there are warps for them
+		chunks = chunks < 1 ? 1 : chunks > n ? n : chunks;
+		Lx = (n + chunks - 1) / chunks;
+		ntasks = strips * ((n + Lx - 1) / Lx);
+		inv = 1.0f / (float)strips;
+	}
+};
+
 enum {
 	PASS_MATVEC = 0,   // out = A x; *dot = this thread's share of x.(A x)
 	PASS_RESID = 1,    // out = b - A x (with xout, x as formed is stored there)
@@ -156,7 +172,7 @@ struct Column {
 };
 
 template <class T, int MODE, int XS, bool X0>
-__device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
+__device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp, double *dot)
 {
 	typedef typename V2T<T>::t V;
 	constexpr int NC = XS == XS_ZERO_R ? 9 : XS == XS_PROLONG ? 4 : 1;
@@ -169,17 +185,13 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 	const int N = P.N, n = N + 1;
 	const int lane = threadIdx.x & 31;
 	const int nwarps = pt.size * (kBlock / 32);
-	// the columns are cut into as many chunks as there are warps for them
-	const int strips = (n + kOwn - 1) / kOwn;
-	int chunks = nwarps / strips;
-	chunks = chunks < 1 ? 1 : chunks > n ? n : chunks;
-	const int Lx = (n + chunks - 1) / chunks;
-	const int ntasks = strips * ((n + Lx - 1) / Lx);
+	const int strips = sp.strips, Lx = sp.Lx, ntasks = sp.ntasks;
+	const float inv = sp.inv;
 	double dacc = 0.0, racc = 0.0, facc = 0.0;
 
 	// consecutive tasks go to different blocks, so that a small level uses many SMs
 	for (int t = (threadIdx.x >> 5) * pt.size + pt.rank; t < ntasks; t += nwarps) {
-		const int c = t / strips, s = t - c * strips;
+		const int c = (int)(((float)t + 0.5f) * inv), s = t - c * strips;
 		const int gz = s * kOwn - 1 + lane, xs = c * Lx, xe = min(xs + Lx, n);
 		const bool zin = gz >= 0 && gz < n;
 		const bool own = zin && lane >= 1 && lane <= kOwn;
@@ -251,8 +263,9 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 		};
 
 		Col cur, nx, prev;
-		load(xs - 1, prev);
-		load(xs, nx);
+		load(xs - 1, prev);   // the first three columns are in flight together
+		load(xs, cur);
+		load(xs + 1, nx);
 		form(xs - 1, prev);
 		// left edge of the element column: this lane's and the upper neighbour's
 		// values, the viscosity at the edge's two Gauss points
@@ -263,9 +276,8 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 		T lou = T(0), low = T(0), upu = T(0), upw = T(0);
 		double cL = 0.0, dL = 0.0;
 
-		for (int ix = xs; ix <= xe; ix++) {
-			cur = nx;
-			load(ix + 1, nx);
+#pragma unroll 1
+		for (int ix = xs;;) {
 			const int ex = ix - 1;
 			const bool exin = ex >= 0 && ex < N;
 			double pe = 0.0;
@@ -381,6 +393,8 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 						P.bout[A] = prev.b;
 				}
 			}
+			if (++ix > xe)
+				break;
 			prev = cur;
 			u0n = u1n;
 			w0n = w1n;
@@ -388,6 +402,8 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, double *dot)
 			E0w = E1w;
 			eL0 = eR0;
 			eL1 = eR1;
+			cur = nx;
+			load(ix + 1, nx);
 		}
 	}
 	if (dot) {

@@ -179,8 +179,14 @@ __device__ void restrict_res(Part pt, const MGLevel<T> &F, const MGLevel<T> &C)
 // in global memory the set-up of a solve took 0.57 ms.
 constexpr int kCoarseShared = 50;
 
+// Tasks of each level's passes, on one block (0) and on the whole team (1).
+struct Splits {
+	Split lev[2][kMaxLev];
+};
+
 template <class T>
-struct CoarseShared {
+struct SolveShared {
+	Splits sp;
 	double m[kCoarseShared * kCoarseShared];   // the matrix, then its inverse in T in the same place
 	T b[kCoarseShared];
 	__device__ T *inv() { return reinterpret_cast<T *>(m); }
@@ -260,7 +266,7 @@ __device__ __noinline__ void coarse_invert(const MGHier<T> &H, double *M)
 }
 
 template <class T>
-__device__ void coarse_build(const MGHier<T> &H, CoarseShared<T> &cs)
+__device__ void coarse_build(const MGHier<T> &H, SolveShared<T> &cs)
 {
 	const bool sh = H.cnd <= kCoarseShared;
 	double *M = sh ? cs.m : H.cwork;
@@ -287,7 +293,7 @@ __device__ void coarse_build(const MGHier<T> &H, CoarseShared<T> &cs)
 
 // x = inverse * b, four lanes per row (interleaved columns); one block.
 template <class T, class V>
-__device__ void coarse_solve(const MGHier<T> &H, CoarseShared<T> &cs, V *x)
+__device__ void coarse_solve(const MGHier<T> &H, SolveShared<T> &cs, V *x)
 {
 	const MGLevel<T> &L = H.lv[H.nlev - 1];
 	const int nd = H.cnd;
@@ -339,12 +345,37 @@ __device__ __forceinline__ Pass<T> level_pass(const MGLevel<T> &L, const typenam
 }
 
 template <class T>
-__device__ __forceinline__ void level_down(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, bool grid, bool active,
-                           typename V2T<T>::t **xcur)
+__device__ __forceinline__ int sweeps(const MGHier<T> &H, int l)
+{
+	return l < H.lfine ? H.nu : H.nu_c;
+}
+
+// The buffer that holds level l's iterate after its passes on the way down
+// (sweeps from the second on alternate), and its result on the way up.  Formed
+// from the level's sweep count where it is needed: a table of them would lie
+// on the stack, which misses L1 after every team barrier.
+template <class T>
+__device__ __forceinline__ typename V2T<T>::t *x_down(const MGHier<T> &H, int l)
+{
+	const int nu = sweeps(H, l);
+	return nu > 2 && (nu & 1) ? H.lv[l].xb : H.lv[l].xa;
+}
+template <class T>
+__device__ __forceinline__ typename V2T<T>::t *x_up(const MGHier<T> &H, int l)
+{
+	if (l == H.nlev - 1)
+		return H.lv[l].xa;
+	const bool b = (x_down(H, l) == H.lv[l].xb) != (sweeps(H, l) & 1);
+	return b ? H.lv[l].xb : H.lv[l].xa;
+}
+
+template <class T>
+__device__ __forceinline__ void level_down(Sync &sy, const Splits &sp, const MGHier<T> &H, int l,
+                                           const typename V2T<T>::t *rhs0, bool wide)
 {
 	typedef typename V2T<T>::t V;
 	const MGLevel<T> &L = H.lv[l];
-	const int nu = l < H.lfine ? H.nu : H.nu_c;
+	const int nu = sweeps(H, l);
 	V *x = L.xa, *xt = L.xb;
 	// below the finest level the right-hand side P^T r of the finer level is
 	// formed in this level's first pass (and stored for its later passes)
@@ -354,81 +385,73 @@ __device__ __forceinline__ void level_down(Sync &sy, const MGHier<T> &H, int l, 
 		P.nc = H.lv[l - 1].n;
 		P.bout = L.b;
 	}
-	const Part pt = sy.part(grid);
+	const Part pt = sy.part(wide);
+	const Split &split = sp.lev[wide][l];
 	if (nu == 1) {
 		// one sweep from zero, x = omega D^-1 b, formed inside the residual pass
-		if (active) {
-			P.wload = H.omega;
-			P.out = L.r;
-			P.xout = x;
-			if (l >= 1)
-				march<T, PASS_RESID, XS_ZERO_R, false>(P, pt, nullptr);
-			else
-				march<T, PASS_RESID, XS_ZERO, false>(P, pt, nullptr);
-			barrier(sy, grid);
-		}
+		P.wload = H.omega;
+		P.out = L.r;
+		P.xout = x;
+		if (l >= 1)
+			march<T, PASS_RESID, XS_ZERO_R, false>(P, pt, split, nullptr);
+		else
+			march<T, PASS_RESID, XS_ZERO, false>(P, pt, split, nullptr);
+		sy.sync(wide);
 	} else {
 		// sweep 1 (from zero) fused into sweep 2; the Chebyshev pair from zero is
 		// x1 = w1 D^-1 b, x2 = c1 x1 + w2 D^-1 (b - A x1)
 		const bool ch = H.cheb && nu == 2;
-		if (active) {
-			P.wload = ch ? H.w1 : H.omega;
-			P.omega = ch ? H.w2 : H.omega;
-			P.cx = ch ? H.c1 : T(1);
-			P.out = x;
-			if (l >= 1)
-				march<T, PASS_SMOOTH, XS_ZERO_R, false>(P, pt, nullptr);
-			else
-				march<T, PASS_SMOOTH, XS_ZERO, false>(P, pt, nullptr);
-			barrier(sy, grid);
-		}
+		P.wload = ch ? H.w1 : H.omega;
+		P.omega = ch ? H.w2 : H.omega;
+		P.cx = ch ? H.c1 : T(1);
+		P.out = x;
+		if (l >= 1)
+			march<T, PASS_SMOOTH, XS_ZERO_R, false>(P, pt, split, nullptr);
+		else
+			march<T, PASS_SMOOTH, XS_ZERO, false>(P, pt, split, nullptr);
+		sy.sync(wide);
 		P.cx = T(1);
 		P.omega = H.omega;
 		for (int s = 2; s < nu; s++) {
-			if (active) {
-				P.x = x;
-				P.out = xt;
-				march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, nullptr);
-				barrier(sy, grid);
-			}
+			P.x = x;
+			P.out = xt;
+			march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, split, nullptr);
+			sy.sync(wide);
 			V *tmp = x;
 			x = xt;
 			xt = tmp;
 		}
-		if (active) {
-			P.x = x;
-			P.out = L.r;
-			march<T, PASS_RESID, XS_PLAIN, false>(P, pt, nullptr);
-			barrier(sy, grid);
-		}
+		P.x = x;
+		P.out = L.r;
+		march<T, PASS_RESID, XS_PLAIN, false>(P, pt, split, nullptr);
+		sy.sync(wide);
 	}
 	// the next level forms its right-hand side from L.r in its first pass,
 	// except the coarsest (a dense solve)
-	if (active && l + 1 == H.nlev - 1) {
+	if (l + 1 == H.nlev - 1) {
 		restrict_res<T, V>(pt, L, H.lv[l + 1]);
-		barrier(sy, grid);
+		sy.sync(wide);
 	}
-	xcur[l] = x;
 }
 
 // With dotv (level 0 only), the last sweep also accumulates this thread's
 // share of out0.dotv into *dot and is not followed by a barrier: the caller's
 // reduction provides it.
 template <class T>
-__device__ __forceinline__ void level_up(Sync &sy, const MGHier<T> &H, int l, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
-                         bool grid, bool active, typename V2T<T>::t **xcur, const double2 *dotv = nullptr,
-                         double *dot = nullptr)
+__device__ __forceinline__ void level_up(Sync &sy, const Splits &sp, const MGHier<T> &H, int l,
+                                         const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0, bool wide,
+                                         const double2 *dotv, double *dot)
 {
 	typedef typename V2T<T>::t V;
 	const MGLevel<T> &L = H.lv[l];
-	V *x = xcur[l];
+	V *x = x_down(H, l);
 	V *xt = (x == L.xa) ? L.xb : L.xa;
-	const MGLevel<T> &C = H.lv[l + 1];
-	const int nu = l < H.lfine ? H.nu : H.nu_c;
-	const Part pt = sy.part(grid);
+	const int nu = sweeps(H, l);
+	const Part pt = sy.part(wide);
+	const Split &split = sp.lev[wide][l];
 	Pass<T> P = level_pass<T>(L, l == 0 ? rhs0 : L.b);
-	P.xc = xcur[l + 1];
-	P.nc = C.n;
+	P.xc = x_up(H, l + 1);
+	P.nc = H.lv[l + 1].n;
 	// the coarse-grid correction x + P xc is formed inside the first post-smoothing
 	// sweep; the Chebyshev pair keeps that iterate (x0) in L.r, free on the way up,
 	// for x2 = c1 x1 - c0 x0 + w2 D^-1 (b - A x1)
@@ -437,64 +460,62 @@ __device__ __forceinline__ void level_up(Sync &sy, const MGHier<T> &H, int l, co
 		const bool last = l == 0 && s == nu - 1;
 		V *dst = last ? out0 : xt;
 		double *dp = (last && dotv) ? dot : nullptr;
-		if (active) {
-			P.x = x;
-			P.out = dst;
-			P.dotv = dp ? dotv : nullptr;
-			if (s == 0) {
-				P.omega = ch ? H.w1 : H.omega;
-				P.xout = ch ? L.r : nullptr;
-				march<T, PASS_SMOOTH, XS_PROLONG, false>(P, pt, dp);
-			} else if (ch) {
-				P.omega = H.w2;
-				P.cx = H.c1;
-				P.c0 = H.c0;
-				P.x0 = L.r;
-				P.xout = nullptr;
-				march<T, PASS_SMOOTH, XS_PLAIN, true>(P, pt, dp);
-			} else {
-				P.omega = H.omega;
-				march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, dp);
-			}
-			if (!dp)
-				barrier(sy, grid);
+		P.x = x;
+		P.out = dst;
+		P.dotv = dp ? dotv : nullptr;
+		if (s == 0) {
+			P.omega = ch ? H.w1 : H.omega;
+			P.xout = ch ? L.r : nullptr;
+			march<T, PASS_SMOOTH, XS_PROLONG, false>(P, pt, split, dp);
+		} else if (ch) {
+			P.omega = H.w2;
+			P.cx = H.c1;
+			P.c0 = H.c0;
+			P.x0 = L.r;
+			P.xout = nullptr;
+			march<T, PASS_SMOOTH, XS_PLAIN, true>(P, pt, split, dp);
+		} else {
+			P.omega = H.omega;
+			march<T, PASS_SMOOTH, XS_PLAIN, false>(P, pt, split, dp);
 		}
+		if (!dp)
+			sy.sync(wide);
 		xt = x;
 		x = dst;
 	}
-	xcur[l] = x;
 }
 
 // Everything below is inlined, once for each correction solve: the passes use
 // most of a thread's registers, and as calls they saved and restored them on
-// the stack on every level (25 of 98 us per MINRES iteration at 64^2), where a
-// barrier's acquire has just emptied L1.
+// the stack on every level (25 of 98 us per MINRES iteration at 64^2).
+//
 // out0 = B rhs0.  With dotv, *dot receives this thread's share of out0.dotv
 // and the cycle ends without a barrier (the caller reduces *dot, which
 // synchronises the team); without it the cycle ends with a barrier.
 template <class T>
-__device__ __forceinline__ void vcycle(Sync &sy, CoarseShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
-                       const double2 *dotv = nullptr, double *dot = nullptr)
+__device__ __forceinline__ void vcycle(Sync &sy, SolveShared<T> &cs, const MGHier<T> &H,
+                                       const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
+                                       const double2 *dotv = nullptr, double *dot = nullptr)
 {
 	typedef typename V2T<T>::t V;
-	V *xcur[kMaxLev];
 	const int lc = H.nlev - 1;
-	// first block-local level (the coarsest always is; in a batch all are)
+	// first block-local level (the coarsest always is; in one block all are)
 	const int nb = sy.size > 1 ? (H.nblk < lc ? H.nblk : lc) : 0;
 	const bool b0 = sy.leader();
 	if (dot)
 		*dot = 0.0;
 #pragma unroll 1
 	for (int l = 0; l < lc; l++)
-		level_down<T>(sy, H, l, rhs0, l < nb, l < nb || b0, xcur);
+		if (l < nb || b0)
+			level_down<T>(sy, cs.sp, H, l, rhs0, l < nb);
 	if (b0)
 		coarse_solve<T, V>(H, cs, H.lv[lc].xa);
-	xcur[lc] = H.lv[lc].xa;
 #pragma unroll 1
 	for (int l = lc - 1; l >= 0; l--) {
 		if (l == nb - 1)
 			sy.sync();   // block 0's coarse-level results become visible to every block
-		level_up<T>(sy, H, l, rhs0, out0, l < nb, l < nb || b0, xcur, dotv, dot);
+		if (l < nb || b0)
+			level_up<T>(sy, cs.sp, H, l, rhs0, out0, l < nb, dotv, dot);
 	}
 	if (nb == 0 && !dotv)
 		sy.sync();
@@ -505,14 +526,15 @@ __device__ __forceinline__ void vcycle(Sync &sy, CoarseShared<T> &cs, const MGHi
 // others wait for its broadcast: a division or a square root on every thread
 // costs the FP64 pipe (2 lanes per clock and SM) about a microsecond each.
 template <class T>
-__device__ __noinline__ int pcg_inner(Sync &sy, CoarseShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
+__device__ __noinline__ int pcg_inner(Sync &team, SolveShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
                          int maxit)
 {
+	Sync sy = team;
 	typedef typename V2T<T>::t V;
 	__shared__ double rho, bb0, co;
 	const MGLevel<T> &L = H.lv[0];
 	const int nn = L.n * L.n;
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	V *r = H.pr, *z = H.pz, *p = H.pp, *q = H.pq;
 	double bb[1] = {0.0};
 	for (int A = tid; A < nn; A += nth) {
@@ -526,8 +548,10 @@ __device__ __noinline__ int pcg_inner(Sync &sy, CoarseShared<T> &cs, const MGHie
 		bb[0] += b0 * b0 + b1 * b1;
 	}
 	sy.reduce_then<1>(bb, [&](const double (&v)[1]) { bb0 = v[0]; });
-	if (!(bb0 > 0.0))
+	if (!(bb0 > 0.0)) {
+		team = sy;
 		return 0;
+	}
 	Pass<T> P = level_pass<T>(L, nullptr);
 	P.x = p;
 	P.out = q;
@@ -555,7 +579,7 @@ __device__ __noinline__ int pcg_inner(Sync &sy, CoarseShared<T> &cs, const MGHie
 		}
 		sy.sync();
 		double pq[1];
-		march<T, PASS_MATVEC, XS_PLAIN, false>(P, sy.part(true), pq);
+		march<T, PASS_MATVEC, XS_PLAIN, false>(P, sy.part(true), cs.sp.lev[1][0], pq);
 		sy.reduce_then<1>(pq, [&](const double (&v)[1]) { co = rho / v[0]; });
 		const double alpha = co;
 		const T al = (T)alpha;
@@ -578,6 +602,7 @@ __device__ __noinline__ int pcg_inner(Sync &sy, CoarseShared<T> &cs, const MGHie
 			break;
 	}
 	sy.sync();
+	team = sy;
 	return it;
 }
 
@@ -662,13 +687,13 @@ __device__ __forceinline__ Pass<double> fine_pass64(const MGArgs<TI> &a, const d
 // pass: as three loops with two team barriers between them it took 0.61 ms at
 // 1024^2.
 template <class TI>
-__device__ void stokes_residual(const MGArgs<TI> &a, Sync &sy, const double2 *d, const double *p, double (&rs)[3])
+__device__ void stokes_residual(const MGArgs<TI> &a, Sync &sy, const Split &split0, const double2 *d, const double *p, double (&rs)[3])
 {
 	Pass<double> P = fine_pass64(a, d, p);
 	P.F = a.F;
 	P.out64 = a.R;
 	P.gt_out = a.Rc;
-	march<double, PASS_RES64, XS_PLAIN, false>(P, sy.part(true), rs);
+	march<double, PASS_RES64, XS_PLAIN, false>(P, sy.part(true), split0, rs);
 	sy.reduce<3>(rs);
 }
 
@@ -820,12 +845,12 @@ __device__ __noinline__ void minres_x_update(int nn, int ne, int tid, int nth, c
 // through the TI hierarchy (z_u stays in TI), the pressure part is multiplied
 // by 1/BAB (a.bab holds the reciprocal).  Returns <z, v> over the team.
 template <class TI>
-__device__ double block_precond(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, const double2 *vu, const double *vp,
+__device__ double block_precond(const MGArgs<TI> &a, Sync &sy, SolveShared<TI> &cs, const double2 *vu, const double *vp,
                                 typename V2T<TI>::t *zu, double *zp)
 {
 	typedef typename V2T<TI>::t VI;
 	const MGHier<TI> &H = a.H;
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
 	VI *bI = H.lv[0].b;
 	for (int A = tid; A < nn; A += nth) {
@@ -850,12 +875,12 @@ __device__ double block_precond(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> 
 // Y = K u + G p and Yc = G^T u in FP64 (the Stokes operator applied to (u, p);
 // p in Morton order).  Ends with a team barrier.
 template <class TI>
-__device__ void stokes_apply(const MGArgs<TI> &a, Sync &sy, const double2 *u, const double *p, double2 *Y, double *Yc)
+__device__ void stokes_apply(const MGArgs<TI> &a, Sync &sy, const Split &split0, const double2 *u, const double *p, double2 *Y, double *Yc)
 {
 	Pass<double> P = fine_pass64(a, u, p);
 	P.out64 = Y;
 	P.gt_out = Yc;
-	march<double, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), nullptr);
+	march<double, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), split0, nullptr);
 	sy.sync();
 }
 
@@ -879,17 +904,17 @@ __device__ void stokes_apply(const MGArgs<TI> &a, Sync &sy, const double2 *u, co
 // carried on and amplified from step to step), 111 against 100 per step over
 // 30 steps; warm_start=3 stays the default there.
 template <class TI>
-__device__ __noinline__ void warm_guess(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, int ndir)
+__device__ __noinline__ void warm_guess(const MGArgs<TI> &a, Sync &sy, SolveShared<TI> &cs, int ndir)
 {
 	typedef typename V2T<TI>::t VI;
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
 	double2 *U1 = a.mw[0], *U2 = a.mw[1], *Y1 = a.mv[0], *Y2 = a.mv[1];
 	double *P1 = a.mwp[0], *P2 = a.mwp[1], *Yc1 = a.mvp[0], *Yc2 = a.mvp[1];
 	VI *Z1 = a.H.px, *Z2 = a.H.pr;
 	double *Zp1 = a.mzp[0], *Zp2 = a.mzp[1];
 	double rs[3];
-	stokes_residual(a, sy, a.h1d, a.h1p, rs);   // a.R = F - K h1 - G p1, a.Rc = G^T h1
+	stokes_residual(a, sy, cs.sp.lev[1][0], a.h1d, a.h1p, rs);   // a.R = F - K h1 - G p1, a.Rc = G^T h1
 	for (int A = tid; A < nn; A += nth) {
 		const double2 x1 = a.h1d[A], x2 = a.h2d[A];
 		U1[A] = make_double2(x1.x - x2.x, x1.y - x2.y);
@@ -904,9 +929,9 @@ __device__ __noinline__ void warm_guess(const MGArgs<TI> &a, Sync &sy, CoarseSha
 			P2[e] = a.h1p[e] - 2.0 * a.h2p[e] + a.h3p[e];
 	}
 	sy.sync();
-	stokes_apply(a, sy, U1, P1, Y1, Yc1);
+	stokes_apply(a, sy, cs.sp.lev[1][0], U1, P1, Y1, Yc1);
 	if (ndir == 2)
-		stokes_apply(a, sy, U2, P2, Y2, Yc2);
+		stokes_apply(a, sy, cs.sp.lev[1][0], U2, P2, Y2, Yc2);
 	// M^-1 a_k (the preconditioner's pressure part divides by BAB); the signs of
 	// the continuity parts follow r = [F - K d - G p ; -G^T d]
 	double q[5];   // <a1, M^-1 a1>, <a2, M^-1 a1>, <a2, M^-1 a2>, <r0, M^-1 a1>, <r0, M^-1 a2>
@@ -972,7 +997,7 @@ __device__ __noinline__ void warm_guess(const MGArgs<TI> &a, Sync &sy, CoarseSha
 // (all blocks hold the same sums, so all form the same values).
 struct MinresScal {
 	double gam, gam_prev, eta, eta0, delta, c_prev, c_cur, s_prev, s_cur;
-	double ig, dg, gg, k1, k2, k3, step;
+	double ig, dg, gg, k1, k2, k3, step, step1;   // step1: the step of the iteration before
 	int stop;   // 1: last iteration; 2: breakdown before the update; 4: a non-finite value
 };
 
@@ -985,50 +1010,47 @@ struct MinresScal {
 // refinement around this solve restores full accuracy.  Stops when the
 // M^-1-norm of the residual has dropped by rtol.  Returns the iterations.
 template <class TI>
-__device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, CoarseShared<TI> &cs, double rtol, int maxit, int *status)
+__device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &team, SolveShared<TI> &cs, double rtol,
+                                              int maxit)
 {
 	typedef typename V2T<TI>::t VI;
 	__shared__ MinresScal ms;
+	// Nothing that lives through a barrier is held in a local array, and sizes and
+	// pointers are read from the arguments in shared memory where they are used:
+	// what does not fit the registers goes to the stack, which misses L1 after every
+	// team barrier.
+	Sync sy = team;
 	const MGHier<TI> &H = a.H;
-	const MGLevel<TI> &L0 = H.lv[0];
-	const int tid = sy.tid, nth = sy.nth;
-	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
-	double2 *vu[2] = {a.mv[0], a.mv[1]}, *wu[2] = {a.mw[0], a.mw[1]};
-	double *vp[2] = {a.mvp[0], a.mvp[1]}, *zp[2] = {a.mzp[0], a.mzp[1]}, *wp[2] = {a.mwp[0], a.mwp[1]};
-	VI *zu[2] = {H.pz, H.pp};   // inner-CG vectors, free while MINRES runs
-	VI *bI = L0.b;
-	const double2 zero2 = make_double2(0.0, 0.0);
-	for (int A = tid; A < nn; A += nth) {
-		const double2 r = a.R[A];
-		vu[0][A] = r;
-		VI w;
-		w.x = narrow_to<TI>(r.x);
-		w.y = narrow_to<TI>(r.y);
-		bI[A] = w;
-		vu[1][A] = zero2;
-		wu[0][A] = zero2;
-		wu[1][A] = zero2;
-		a.dd[A] = zero2;
-	}
+	auto nodes = [&] { return (a.N0 + 1) * (a.N0 + 1); };
+	auto elems = [&] { return a.N0 * a.N0; };
 	double pdot = 0.0;
-	for (int e = tid; e < ne; e += nth) {
-		const double v = -a.Rc[e], z = v * a.bab[e];
-		vp[0][e] = v;
-		zp[0][e] = z;
-		pdot += z * v;
-		vp[1][e] = 0.0;
-		wp[0][e] = 0.0;
-		wp[1][e] = 0.0;
-		a.dpv[e] = 0.0;
+	{
+		const double2 zero2 = make_double2(0.0, 0.0);
+		const int tid = sy.tid(), nth = sy.nth(), nn = nodes(), ne = elems();
+		for (int A = tid; A < nn; A += nth) {
+			const double2 r = a.R[A];
+			a.mv[0][A] = r;
+			VI w;
+			w.x = narrow_to<TI>(r.x);
+			w.y = narrow_to<TI>(r.y);
+			H.lv[0].b[A] = w;
+			a.mv[1][A] = zero2;
+			a.mw[0][A] = zero2;
+			a.mw[1][A] = zero2;
+			a.dd[A] = zero2;
+		}
+		for (int e = tid; e < ne; e += nth) {
+			const double v = -a.Rc[e], z = v * a.bab[e];
+			a.mvp[0][e] = v;
+			a.mzp[0][e] = z;
+			pdot += z * v;
+			a.mvp[1][e] = 0.0;
+			a.mwp[0][e] = 0.0;
+			a.mwp[1][e] = 0.0;
+			a.dpv[e] = 0.0;
+		}
 	}
 	sy.sync();
-	Pass<TI> P = level_pass<TI>(L0, nullptr);
-	P.out64 = a.Kd;
-	P.gt_out = a.Ahp;
-	P.g0 = a.gt.g0[0];
-	P.g1 = a.gt.g1[0];
-	P.gp_morton = 0;
-	double step1 = 0.0;           // the step of the iteration before, not yet applied when `it` is odd
 	// index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1).  it = -1: z(0) = M^-1 v(0)
 	int cv = 1, cw = 0, it = -1;
 #pragma unroll 1
@@ -1037,21 +1059,28 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, Coa
 			// A z(j), unscaled (z~ = z / gam): K z_u + G z_p into a.Kd, G^T z_u into
 			// a.Ahp, and their product with (z_u, z_p)
 			double dl[1];
-			P.x = zu[cv];
-			P.gp = zp[cv];
-			march<TI, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), dl);
+			Pass<TI> P = level_pass<TI>(H.lv[0], nullptr);
+			P.out64 = a.Kd;
+			P.gt_out = a.Ahp;
+			P.g0 = a.gt.g0[0];
+			P.g1 = a.gt.g1[0];
+			P.gp_morton = 0;
+			P.x = a.mzu[cv];
+			P.gp = a.mzp[cv];
+			march<TI, PASS_STOKES, XS_PLAIN, false>(P, sy.part(true), cs.sp.lev[1][0], dl);
 			sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
 				ms.delta = v[0] * ms.ig * ms.ig;
 				ms.dg = ms.delta * ms.ig;
 			});
 			// v(j+1) = A z~ - (delta/gam) v(j) - (gam/gam_prev) v(j-1), into v(j-1)'s
 			// buffer, its TI copy as the V-cycle's right-hand side, and z_p(j+1)
-			minres_v_nodes<VI>(nn, tid, nth, a.Kd, vu[cv], vu[1 - cv], bI, ms.ig, ms.dg, ms.gg);
-			pdot = minres_v_elems(ne, tid, nth, a.Ahp, vp[cv], vp[1 - cv], a.bab, zp[1 - cv], ms.ig, ms.dg, ms.gg);
+			minres_v_nodes<VI>(nodes(), sy.tid(), sy.nth(), a.Kd, a.mv[cv], a.mv[1 - cv], H.lv[0].b, ms.ig, ms.dg, ms.gg);
+			pdot = minres_v_elems(elems(), sy.tid(), sy.nth(), a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv],
+			                      ms.ig, ms.dg, ms.gg);
 			sy.sync();
 		}
 		double dot[1];
-		vcycle<TI>(sy, cs, H, bI, zu[1 - cv], vu[1 - cv], &dot[0]);
+		vcycle<TI>(sy, cs, H, H.lv[0].b, a.mzu[1 - cv], a.mv[1 - cv], &dot[0]);
 		dot[0] += pdot;
 		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
 			const double gn2 = fmax(v[0], 0.0);
@@ -1080,6 +1109,7 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, Coa
 			}
 			const double c_next = a0 * ia1, s_next = gam_next * ia1;
 			// w(j+1) = (z~(j) - a3 w(j-1) - a2 w(j)) / a1; x += c_next eta w(j+1)
+			ms.step1 = ms.step;
 			ms.k1 = ms.ig * ia1;
 			ms.k2 = a2 * ia1;
 			ms.k3 = a3 * ia1;
@@ -1097,27 +1127,28 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, Coa
 				ms.stop = 1;
 		});
 		if (it < 0) {
-			if (ms.stop)
-				return 0;
 			it = 0;
+			if (ms.stop)
+				break;
 			cv = 0;
 			continue;
 		}
 		const int stop = ms.stop;
-		if ((stop & 4) && tid == 0)
-			atomicOr(status, 2);
+		if ((stop & 4) && sy.tid() == 0)
+			atomicOr(&a.sc->status, 2);
 		if (stop & 2) {
 			if (it & 1)   // the pending step along w(j)
-				minres_x_update(nn, ne, tid, nth, wu[cw], a.dd, wp[cw], a.dpv, step1);
+				minres_x_update(nodes(), elems(), sy.tid(), sy.nth(), a.mw[cw], a.dd, a.mwp[cw], a.dpv, ms.step);
 			break;
 		}
 		// into w(j-1)'s buffer; the solution takes the steps of two iterations at a time
 		// (x += step w(j) + step' w(j+1), the same additions in the same order), or what
 		// is pending when the loop ends
 		const int steps = (it & 1) ? 2 : (stop || it + 1 >= maxit) ? 1 : 0;
-		minres_w_nodes<VI>(steps, nn, tid, nth, zu[cv], wu[1 - cw], wu[cw], a.dd, ms.k1, ms.k3, ms.k2, ms.step, step1);
-		minres_w_elems(steps, ne, tid, nth, zp[cv], wp[1 - cw], wp[cw], a.dpv, ms.k1, ms.k3, ms.k2, ms.step, step1);
-		step1 = ms.step;
+		minres_w_nodes<VI>(steps, nodes(), sy.tid(), sy.nth(), a.mzu[cv], a.mw[1 - cw], a.mw[cw], a.dd, ms.k1, ms.k3,
+		                   ms.k2, ms.step, ms.step1);
+		minres_w_elems(steps, elems(), sy.tid(), sy.nth(), a.mzp[cv], a.mwp[1 - cw], a.mwp[cw], a.dpv, ms.k1, ms.k3,
+		               ms.k2, ms.step, ms.step1);
 		it++;
 		cv = 1 - cv;
 		cw = 1 - cw;
@@ -1134,6 +1165,7 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &sy, Coa
 		// updates above wrote
 	}
 	sy.sync();
+	team = sy;
 	return it;
 }
 
@@ -1154,13 +1186,17 @@ template <class TI>
 __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 {
 	typedef typename V2T<TI>::t VI;
-	__shared__ CoarseShared<TI> cs;
+	__shared__ SolveShared<TI> cs;   // this block's working data of the solve
 	const MGHier<TI> &H = a.H;
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	const int N0 = a.N0, n0 = N0 + 1, nn = n0 * n0, ne = N0 * N0;
 	int *status = &a.sc->status;
 	const GTab &gt = a.gt;
 
+	for (int l = threadIdx.x; l < a.H.nlev; l += blockDim.x) {
+		cs.sp.lev[0][l].set(a.H.lv[l].n, kBlock / 32);
+		cs.sp.lev[1][l].set(a.H.lv[l].n, sy.size * (kBlock / 32));
+	}
 	// -- per-step setup: viscosity on every level, inverse diagonals, BAB, coarse inverse
 	for (int A = tid; A < nn; A += nth)
 		H.lv[0].eta[A] = (TI)a.vis[A];
@@ -1227,8 +1263,8 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 		// the previous step's solution.  Keep the one with the smaller FP64
 		// residual; a non-finite network guess always loses.
 		double rl[3], rp[3];
-		stokes_residual(a, sy, a.d, a.p, rl);
-		stokes_residual(a, sy, a.d_alt, a.p_alt, rp);
+		stokes_residual(a, sy, cs.sp.lev[1][0], a.d, a.p, rl);
+		stokes_residual(a, sy, cs.sp.lev[1][0], a.d_alt, a.p_alt, rp);
 		const double el = rl[0] + rl[1], ep = rp[0] + rp[1];
 		const bool learned = isfinite(el) && (a.guess_force || el < ep);
 		if (!learned) {
@@ -1247,7 +1283,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 	while (true) {
 		// -- FP64 residual R = [F - K d - G p ; G^T d]
 		double rs[3];
-		stokes_residual(a, sy, a.d, a.p, rs);
+		stokes_residual(a, sy, cs.sp.lev[1][0], a.d, a.p, rs);
 		// a zero load (|F| = 0): the residual is measured absolutely
 		fnorm = rs[2] > 0.0 ? sqrt(rs[2]) : 1.0;
 		res_m = sqrt(rs[0]) / fnorm;
@@ -1272,7 +1308,7 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 			// where MINRES converges fastest; close to it, by what is left to
 			// reach rtol (with a factor 2 margin), but not below outer_rtol.
 			const double prt = res > 1e4 * a.rtol ? 1e-2 : fmax(a.outer_rtol, 0.5 * a.rtol / res);
-			const int it = minres_correction<TI>(a, sy, cs, prt, a.max_outer, status);
+			const int it = minres_correction<TI>(a, sy, cs, prt, a.max_outer);
 			outer_total += it;
 			inner_total += it + 1;
 			for (int A = tid; A < nn; A += nth) {
@@ -1413,40 +1449,23 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 	}
 }
 
-// The solver's arguments in shared memory: noinline passes take references into
-// them, which for kernel parameters would copy them to every thread's stack.
-template <class TI>
-__device__ void load_args(MGArgs<TI> &to, const MGArgs<TI> &from)
-{
-	static_assert(sizeof(MGArgs<TI>) % 4 == 0, "copied by words");
-	const unsigned *s = reinterpret_cast<const unsigned *>(&from);
-	unsigned *d = reinterpret_cast<unsigned *>(&to);
-	for (int i = threadIdx.x; i < (int)(sizeof(MGArgs<TI>) / 4); i += blockDim.x)
-		d[i] = s[i];
-	__syncthreads();
-}
-
 // Blocks per SM: two of 256 threads in FP32; the FP64 passes hold twice the
 // registers and are bound by the FP64 pipe, which one block keeps busy.
 template <class TI> constexpr int kSolveBlocks = sizeof(TI) == 4 ? 2 : 1;
 
-// One model on the whole cooperative grid.
+// One model on the whole cooperative grid, or on one cluster (a.cluster).
 template <class TI>
 __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg(const __grid_constant__ MGArgs<TI> a)
 {
 	__shared__ MGArgs<TI> sa;
+	__shared__ double cpart[2 * kRedWidth];
 	load_args(sa, a);
-	cg::grid_group g = cg::this_grid();
-	Sync sy;
-	sy.mode = SYNC_GRID;
-	sy.g = &g;
-	sy.red = sa.red;
-	sy.cpart = nullptr;
-	sy.cflip = 0;
-	sy.rank = blockIdx.x;
-	sy.size = gridDim.x;
-	sy.spread();
+	cg::cluster_group cl = cg::this_cluster();
+	Sync sy = sa.cluster ? Sync::of(SYNC_CLUSTER, cpart, blockIdx.x, gridDim.x)
+	                     : Sync::of(SYNC_GRID, sa.red.part, blockIdx.x, gridDim.x);
 	stokes_solve<TI>(sa, sy);
+	if (sa.cluster)
+		cl.sync();   // no block leaves while another reads its partials
 }
 
 // A batch of independent models.  Launched with clusters of `cs` blocks
@@ -1468,9 +1487,6 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(co
 	for (;;) {
 		if (rank == 0 && threadIdx.x == 0)
 			next = atomicAdd(queue, 1);
-		Sync sy;
-		sy.g = nullptr;
-		sy.cflip = 0;
 		if (cs > 1) {
 			cl.sync();
 			const int m = *cl.map_shared_rank(&next, 0);
@@ -1478,12 +1494,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(co
 			if (m >= nmodels)
 				break;
 			load_args(sa, models[m]);
-			sy.mode = SYNC_CLUSTER;
-			sy.red = sa.red;
-			sy.cpart = cpart;
-			sy.rank = rank;
-			sy.size = cs;
-			sy.spread();
+			Sync sy = Sync::of(SYNC_CLUSTER, cpart, rank, cs);
 			stokes_solve<TI>(sa, sy);
 			cl.sync();   // no block starts the next model (or leaves) while another reads its partials
 		} else {
@@ -1493,12 +1504,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(co
 			if (m >= nmodels)
 				break;
 			load_args(sa, models[m]);
-			sy.mode = SYNC_BLOCK;
-			sy.red = sa.red;
-			sy.cpart = nullptr;
-			sy.rank = 0;
-			sy.size = 1;
-			sy.spread();
+			Sync sy = Sync::of(SYNC_BLOCK, nullptr, 0, 1);
 			stokes_solve<TI>(sa, sy);
 			__syncthreads();
 		}

@@ -64,7 +64,8 @@ struct MGArgs {
 	double2 *R, *dd, *u1, *Kd, *invD64, *kdiag64;   // FP64 node vectors
 	double *Rc, *r0, *r1, *r2, *z0, *z1, *s1, *s2, *Ahp, *dpv, *bab;  // FP64 element vectors
 	int method;                  // correction solve: 0 Uzawa with inner MG-PCG, 1 MINRES (block-diagonal preconditioner)
-	double2 *mv[2], *mw[2];      // MINRES Lanczos and direction vectors, velocity part (z_u lives in TI)
+	double2 *mv[2], *mw[2];      // MINRES Lanczos and direction vectors, velocity part
+	typename V2T<TI>::t *mzu[2]; // ... and the preconditioned ones, in TI (inner-CG vectors, free while MINRES runs)
 	double *mvp[2], *mzp[2], *mwp[2]; // Lanczos, preconditioned and direction vectors, pressure part (Morton)
 	// warm_start=4: the last three solutions (h1 the most recent), or null
 	const double2 *h1d, *h2d, *h3d;
@@ -76,6 +77,7 @@ struct MGArgs {
 	StepScalars *sc;
 	double rtol, outer_rtol, inner_rtol;
 	int max_refine, max_outer, max_inner;
+	int cluster;                 // the single model runs on one cluster (SYNC_CLUSTER) instead of the whole grid
 };
 
 }  // namespace mclg

@@ -366,7 +366,7 @@ template <class TI>
 __device__ const typename Q2T<TI>::t *qt_vcycle(Sync &sy, const QtHier<TI> &H)
 {
 	const int top = H.nlev - 1, nb = H.nblk < top ? H.nblk : top;   // the finest level always runs on the team
-	QtTeam team{&sy, true, sy.tid, sy.nth};
+	QtTeam team{&sy, true, sy.tid(), sy.nth()};
 	for (int l = top; l >= (nb > 1 ? nb : 1); l--)
 		qt_down(H, l, team);
 	if (nb > 0) {
@@ -446,7 +446,7 @@ __device__ void qt_coarse_build(const QtHier<TI> &H)
 template <class TI>
 __device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, const double *p, double (&rs)[3])
 {
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	const DevLevel &L = a.L;
 	const QtLevel<TI> &Q = a.H.lv[a.H.nlev - 1];
 	const double *df = reinterpret_cast<const double *>(d);
@@ -484,7 +484,7 @@ template <class TI>
 __device__ double qt_precond(Sync &sy, const QtArgs<TI> &a, const double2 *vu, const double *vp,
                              typename Q2T<TI>::t *zu, double *zp)
 {
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	typedef typename Q2T<TI>::t V;
 	const QtHier<TI> &H = a.H;
 	const QtLevel<TI> &Q = H.lv[H.nlev - 1];
@@ -520,7 +520,7 @@ __device__ double qt_precond(Sync &sy, const QtArgs<TI> &a, const double2 *vu, c
 template <class TI>
 __device__ int qt_minres(Sync &sy, const QtArgs<TI> &a, double rtol, int maxit, int *status)
 {
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	typedef typename Q2T<TI>::t V;
 	const DevLevel &L = a.L;
 	const QtLevel<TI> &Q = a.H.lv[a.H.nlev - 1];
@@ -635,7 +635,7 @@ __device__ int qt_minres(Sync &sy, const QtArgs<TI> &a, double rtol, int maxit, 
 template <class TI>
 __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 {
-	const int tid = sy.tid, nth = sy.nth;
+	const int tid = sy.tid(), nth = sy.nth();
 	const QtHier<TI> &H = a.H;
 	const DevLevel &L = a.L;
 	int *status = &a.sc->status;
@@ -744,20 +744,12 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 
 // One refined model on the whole cooperative grid.
 template <class TI>
-__global__ void __launch_bounds__(kBlock) k_stokes_qt(QtArgs<TI> a)
+__global__ void __launch_bounds__(kBlock) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
 {
-	cg::grid_group g = cg::this_grid();
-	Sync sy;
-	sy.mode = SYNC_GRID;
-	sy.g = &g;
-	sy.red = a.red;
-	sy.cpart = nullptr;
-	sy.cflip = 0;
-	sy.rank = blockIdx.x;
-	sy.size = gridDim.x;
-	sy.tid = blockIdx.x * blockDim.x + threadIdx.x;
-	sy.nth = gridDim.x * blockDim.x;
-	qt_solve<TI>(a, sy);
+	__shared__ QtArgs<TI> sa;
+	load_args(sa, a);
+	Sync sy = Sync::of(SYNC_GRID, a.red.part, blockIdx.x, gridDim.x);
+	qt_solve<TI>(sa, sy);
 }
 
 // A batch of independent refined models, launched with clusters of `cs`
@@ -768,6 +760,7 @@ __global__ void __launch_bounds__(kBlock) k_stokes_qt(QtArgs<TI> a)
 template <class TI>
 __global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *models, int nmodels, int *queue)
 {
+	__shared__ QtArgs<TI> sa;
 	__shared__ int next;
 	__shared__ double cpart[2 * kRedWidth];
 	cg::cluster_group cl = cg::this_cluster();
@@ -775,23 +768,15 @@ __global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *mo
 	for (;;) {
 		if (rank == 0 && threadIdx.x == 0)
 			next = atomicAdd(queue, 1);
-		Sync sy;
-		sy.g = nullptr;
-		sy.cflip = 0;
 		if (cs > 1) {
 			cl.sync();
 			const int m = *cl.map_shared_rank(&next, 0);
 			cl.sync();   // every block has read the draw before the next one
 			if (m >= nmodels)
 				break;
-			sy.mode = SYNC_CLUSTER;
-			sy.red = models[m].red;
-			sy.cpart = cpart;
-			sy.rank = rank;
-			sy.size = cs;
-			sy.tid = rank * blockDim.x + threadIdx.x;
-			sy.nth = cs * blockDim.x;
-			qt_solve<TI>(models[m], sy);
+			load_args(sa, models[m]);
+			Sync sy = Sync::of(SYNC_CLUSTER, cpart, rank, cs);
+			qt_solve<TI>(sa, sy);
 			cl.sync();   // no block starts the next model (or leaves) while another reads its partials
 		} else {
 			__syncthreads();
@@ -799,14 +784,9 @@ __global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *mo
 			__syncthreads();
 			if (m >= nmodels)
 				break;
-			sy.mode = SYNC_BLOCK;
-			sy.red = models[m].red;
-			sy.cpart = nullptr;
-			sy.rank = 0;
-			sy.size = 1;
-			sy.tid = threadIdx.x;
-			sy.nth = blockDim.x;
-			qt_solve<TI>(models[m], sy);
+			load_args(sa, models[m]);
+			Sync sy = Sync::of(SYNC_BLOCK, nullptr, 0, 1);
+			qt_solve<TI>(sa, sy);
 			__syncthreads();
 		}
 	}

@@ -101,6 +101,7 @@ struct mclg_ctx {
 	double *tmpA, *tmpB;
 	// converged solvers on uniform meshes (precision 1 and 2)
 	int coop_mg;
+	int mg_one_cluster;          // its blocks are one cluster instead of a cooperative grid
 	double remesh_ms[5];   // the last remesh: numbering, lists, state, wait, carry (host ms)
 	MGArgs<float> mgf;
 	MGArgs<double> mgd;
@@ -311,6 +312,65 @@ static int coop_blocks(void *kernel, int num_sms, int work)
 	return nb < 1 ? 1 : nb;
 }
 
+// Launch one cluster of cs blocks.
+static cudaError_t launch_cluster(void *kern, int cs, void **args, cudaStream_t st)
+{
+	cudaLaunchConfig_t lc;
+	memset(&lc, 0, sizeof lc);
+	lc.gridDim = dim3(cs);
+	lc.blockDim = dim3(kBlock);
+	lc.stream = st;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = cs;
+	at[0].val.clusterDim.y = 1;
+	at[0].val.clusterDim.z = 1;
+	lc.attrs = at;
+	lc.numAttrs = 1;
+	return cudaLaunchKernelExC(&lc, kern, args);
+}
+
+// Clusters of cs blocks of `kern` that can be resident at once (0: none).
+static int max_clusters(void *kern, int cs)
+{
+	if (cs > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+		cudaGetLastError();
+		return 0;
+	}
+	cudaLaunchConfig_t lc;
+	memset(&lc, 0, sizeof lc);
+	lc.gridDim = dim3(cs);
+	lc.blockDim = dim3(kBlock);
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = cs;
+	at[0].val.clusterDim.y = 1;
+	at[0].val.clusterDim.z = 1;
+	lc.attrs = at;
+	lc.numAttrs = 1;
+	int nc = 0;
+	if (cudaOccupancyMaxActiveClusters(&nc, kern, &lc) != cudaSuccess) {
+		cudaGetLastError();
+		return 0;
+	}
+	return nc;
+}
+
+// The blocks that solve one uniform model: a single cluster for small meshes in
+// FP32, whose iteration is a chain of barriers (0.2 us in a cluster, 1.2 in a
+// grid): 42 against 53 us per MINRES iteration at 64^2 and 81 against 90 per
+// inner iteration at 128^2 on 16 blocks (50 and 110 on 8), 145 against 86 at
+// 256^2.  FP64 passes need the whole device's FP64 pipes from 64^2 on (297
+// against 170 us at 128^2).
+static void mg_team(mclg_ctx *c, void *kern)
+{
+	constexpr int kOneCluster = 16, kOneClusterN32 = 128, kOneClusterN64 = 32;
+	const int N0 = c->mesh.max_elx[c->fl];
+	c->mg_one_cluster = N0 <= (c->cfg.precision == 2 ? kOneClusterN64 : kOneClusterN32) &&
+	                    max_clusters(kern, kOneCluster) >= 1;
+	c->coop_mg = c->mg_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, 1 << 30);
+}
+
 // ---- converged solvers: hierarchy of the uniform mesh -------------------------
 template <class T>
 static cudaError_t mg_alloc(mclg_ctx *c, T **p, size_t n)
@@ -353,8 +413,12 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 	}
 	a.H.nlev = nlev;
 	a.H.nblk = nlev;
+	// small grids: one block beats team barriers; FP64 passes are bound by the FP64
+	// pipe of that block's SM, so there the limit is half (8 x 8 in one block took
+	// 57 us of a V-cycle's 150 at 128^2)
+	const int block_n = sizeof(TI) == 8 ? c->cfg.mg_block_n / 2 : c->cfg.mg_block_n;
 	for (int l = 0; l < nlev; l++)
-		if ((N0 >> l) <= c->cfg.mg_block_n) {   // small grids: one block beats grid barriers
+		if ((N0 >> l) <= block_n) {
 			a.H.nblk = l;
 			break;
 		}
@@ -464,6 +528,8 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 			CK(mg_alloc(c, &a.mzp[k], ne));
 			CK(mg_alloc(c, &a.mwp[k], ne));
 		}
+		a.mzu[0] = a.H.pz;
+		a.mzu[1] = a.H.pp;
 	}
 	a.red.part = c->red_part;
 	a.sc = c->sc;
@@ -1187,14 +1253,14 @@ static int launch_stokes_mg(mclg_ctx *c)
 	int rc = stokes_mg_prepare(c);
 	if (rc)
 		return rc;
-	const dim3 grid(solver_grid(c, c->coop_mg));
-	if (c->cfg.precision == 2) {
-		void *args[] = {&c->mgd};
-		CK(cudaLaunchCooperativeKernel(stokes_mg_kernel(1), grid, dim3(kBlock), args, 0, c->st));
-	} else {
-		void *args[] = {&c->mgf};
-		CK(cudaLaunchCooperativeKernel(stokes_mg_kernel(0), grid, dim3(kBlock), args, 0, c->st));
-	}
+	const bool one = c->mg_one_cluster != 0;
+	c->mgd.cluster = c->mgf.cluster = one;
+	void *args[] = {c->cfg.precision == 2 ? (void *)&c->mgd : (void *)&c->mgf};
+	void *kern = stokes_mg_kernel(c->cfg.precision == 2);
+	if (one)
+		CK(launch_cluster(kern, c->coop_mg, args, c->st));
+	else
+		CK(cudaLaunchCooperativeKernel(kern, dim3(solver_grid(c, c->coop_mg)), dim3(kBlock), args, 0, c->st));
 	c->launches++;
 	return stokes_mg_finish(c);
 }
@@ -1470,7 +1536,7 @@ static int create_impl(mclg_ctx **out, const mclg_config *cfg, const int *leaves
 			*out = NULL;
 			return rc;
 		}
-		c->coop_mg = coop_blocks(stokes_mg_kernel(cfg->precision == 2), c->num_sms, 1 << 30);
+		mg_team(c, stokes_mg_kernel(cfg->precision == 2));
 		if ((cfg->warm_start == 3 || cfg->warm_start == 4) && (rc = alloc_history(c)) != MCLG_OK) {
 			mclg_destroy(c);
 			*out = NULL;

@@ -26,18 +26,32 @@ struct Part {
 //   SYNC_BLOCK    one block of a batch (block barriers and reductions).
 enum { SYNC_GRID = 0, SYNC_CLUSTER = 1, SYNC_BLOCK = 2 };
 
+// Few words, so that a solve keeps it in registers: what lies on the stack misses
+// L1 after every team barrier (whose acquire empties it), an L2 access each time.
 struct Sync {
 	int mode;
-	cg::grid_group *g;
-	GridRed red;
-	double *cpart;               // SYNC_CLUSTER: this block's [2][kRedWidth] partials (shared memory)
-	int cflip;
+	double *partials;            // the reductions' partials: SYNC_GRID [2][kRedWidth][kMaxCoopBlocks] in global
+	                             // memory, SYNC_CLUSTER this block's [2][kRedWidth] in shared memory
+	int flip;                    // which of the two partial buffers the next reduction writes (see GridRed)
 	int rank, size;              // this block in the team
-	int tid, nth;
+	// tid and nth for loops over nodes and elements: warps are dealt to the blocks
+	// in turn (Part::thread)
+	static __device__ Sync of(int mode, double *partials, int rank, int size)
+	{
+		Sync s;
+		s.mode = mode;
+		s.partials = partials;
+		s.flip = 0;
+		s.rank = rank;
+		s.size = size;
+		return s;
+	}
+	__device__ int tid() const { return Part{rank, size}.thread(); }
+	__device__ int nth() const { return size * (int)blockDim.x; }
 	__device__ void sync()
 	{
 		if (mode == SYNC_GRID)
-			g->sync();
+			cg::this_grid().sync();
 		else if (mode == SYNC_CLUSTER)
 			cg::this_cluster().sync();
 		else
@@ -76,13 +90,13 @@ struct Sync {
 			}
 		}
 		if (mode == SYNC_GRID) {
-			double *buf = red.part + (size_t)red.flip * kMaxCoopBlocks * kRedWidth;
+			double *buf = partials + (size_t)flip * kMaxCoopBlocks * kRedWidth;
 			if (threadIdx.x == 0) {
 #pragma unroll
 				for (int k = 0; k < NV; k++)
 					buf[k * kMaxCoopBlocks + rank] = t[k];
 			}
-			g->sync();
+			cg::this_grid().sync();
 			if (threadIdx.x < 32) {
 #pragma unroll
 				for (int k = 0; k < NV; k++) {
@@ -97,9 +111,9 @@ struct Sync {
 					t[k] = warp_sum(a0 + a1);
 				}
 			}
-			red.flip ^= 1;   // the next reduction writes the other buffer (see GridRed)
+			flip ^= 1;
 		} else if (mode == SYNC_CLUSTER) {
-			double *mine = cpart + cflip * kRedWidth;
+			double *mine = partials + flip * kRedWidth;
 			if (threadIdx.x == 0) {
 #pragma unroll
 				for (int k = 0; k < NV; k++)
@@ -113,7 +127,7 @@ struct Sync {
 				for (int k = 0; k < NV; k++)
 					t[k] = warp_sum(lane < size ? other[k] : 0.0);
 			}
-			cflip ^= 1;
+			flip ^= 1;
 		}
 		if (threadIdx.x == 0)
 			f(t);
@@ -133,23 +147,30 @@ struct Sync {
 		for (int k = 0; k < NV; k++)
 			v[k] = out[k];
 	}
-	// tid and nth for loops over nodes and elements (see Part::thread)
-	__device__ void spread()
-	{
-		tid = Part{rank, size}.thread();
-		nth = size * blockDim.x;
-	}
 	__device__ bool leader() const { return rank == 0; }
 	// the blocks of a pass: the team for team-wide levels, this block alone otherwise
 	__device__ Part part(bool wide) const { return wide ? Part{rank, size} : Part{0, 1}; }
+	__device__ void sync(bool wide)
+	{
+		if (wide)
+			sync();
+		else
+			__syncthreads();
+	}
 };
 
-__device__ __forceinline__ void barrier(Sync &sy, bool grid)
+// A solver's arguments copied to shared memory: functions take references into
+// them, which for kernel parameters would copy them to every thread's stack and
+// for a batch's arguments would read global memory after every barrier.
+template <class A>
+__device__ void load_args(A &to, const A &from)
 {
-	if (grid)
-		sy.sync();
-	else
-		__syncthreads();
+	static_assert(sizeof(A) % 4 == 0, "copied by words");
+	const unsigned *s = reinterpret_cast<const unsigned *>(&from);
+	unsigned *d = reinterpret_cast<unsigned *>(&to);
+	for (int i = threadIdx.x; i < (int)(sizeof(A) / 4); i += blockDim.x)
+		d[i] = s[i];
+	__syncthreads();
 }
 
 }  // namespace mclg
