@@ -5,6 +5,7 @@
 // on the device; grid barriers replace the reference's MPI_Allreduce calls.
 #include <math.h>
 #include "cg_solve.cuh"
+#include "team.cuh"
 
 namespace mclg {
 
@@ -497,6 +498,399 @@ __global__ void __launch_bounds__(kBlock) k_uzawa(UzawaArgs a)
 	}
 }
 
+// ---- small meshes without hanging nodes: one cluster, rows in registers ----------
+// The same iteration on a 16-block cluster, a node (and an element) per thread:
+// the node's rows of K, its solution, residual and direction stay in registers,
+// an iteration gathers the neighbours' directions, and its three barriers take
+// 0.2 us each instead of a grid barrier's 1.2.  FP64 runs at two operations per
+// clock and SM, so the recurrences' divisions are left to one thread of a block
+// (in k_uzawa every thread forms them) and groups of 32 nodes are dealt over the
+// blocks.  Measured per CG iteration: 15.6 us in k_uzawa at 16^2 (2 blocks) and
+// 15.8 at 64^2 (17 blocks); here 8.0 and 10.2.
+//
+// Sums are formed in k_uzawa's order (butterflies over 32 consecutive nodes, the
+// 8 groups of 256, then the 256s), so that the iterates are k_uzawa's: at a
+// viscosity contrast of 1e5 another order moves the Uzawa count by 3 in 370.
+constexpr int kUzCluster = 16, kUzWarps = 9, kUzBlock = 32 * kUzWarps;
+constexpr int kUzGroups = kUzCluster * kUzWarps;   // groups of 32: 4608 nodes, 64^2 has 4225
+constexpr int kUzRow = 9;                          // blocks per row
+
+struct UzTeam {
+	double *part;   // this block's [2][kRedWidth][kUzWarps] group sums (shared memory)
+	double *mid;    // [kRedWidth][(kUzGroups + 7) / 8] sums of 256 (shared memory)
+	int flip, ngroups;
+	__device__ void sync() { cg::this_cluster().sync(); }
+	// f(sums) on thread 0 of each block; bit k of MAX set: value k is a maximum (of values >= 0)
+	template <int NV, unsigned MAX = 0u, class F>
+	__device__ __forceinline__ void reduce_then(double (&v)[NV], F f)
+	{
+		constexpr int kMid = (kUzGroups + 7) / 8;
+		const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+		cg::cluster_group cl = cg::this_cluster();
+		double *mine = part + flip * kRedWidth * kUzWarps;
+#pragma unroll
+		for (int k = 0; k < NV; k++) {
+			const double t = ((MAX >> k) & 1u) ? warp_max(v[k]) : warp_sum(v[k]);
+			if (lane == 0)
+				mine[k * kUzWarps + w] = t;
+		}
+		cl.sync();
+		const int g = threadIdx.x;   // group g lies in block g % 16, warp g / 16
+		if (w * 32 < ngroups) {
+			const double *other = cl.map_shared_rank(mine, g % kUzCluster);
+#pragma unroll
+			for (int k = 0; k < NV; k++) {
+				double t = g < ngroups ? other[k * kUzWarps + g / kUzCluster] : 0.0;
+#pragma unroll
+				for (int o = 4; o > 0; o >>= 1) {
+					const double u = __shfl_xor_sync(0xffffffffu, t, o);
+					t = ((MAX >> k) & 1u) ? fmax(t, u) : t + u;
+				}
+				if ((lane & 7) == 0 && g < kUzGroups)
+					mid[k * kMid + g / 8] = t;
+			}
+		}
+		__syncthreads();
+		if (w == 0) {
+			double t[NV];
+#pragma unroll
+			for (int k = 0; k < NV; k++) {
+				const double u = lane < (ngroups + 7) / 8 ? mid[k * kMid + lane] : 0.0;
+				t[k] = ((MAX >> k) & 1u) ? warp_max(u) : warp_sum(u);
+			}
+			if (lane == 0)
+				f(t);
+		}
+		__syncthreads();
+		flip ^= 1;   // the next reduction writes the other buffer: this one may still be read
+	}
+	template <int NV>
+	__device__ __forceinline__ void reduce(double (&v)[NV])
+	{
+		__shared__ double out[NV];
+		reduce_then<NV>(v, [&](const double (&t)[NV]) {
+#pragma unroll
+			for (int k = 0; k < NV; k++)
+				out[k] = t[k];
+		});
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			v[k] = out[k];
+	}
+};
+
+// The rows of one node in registers, and their product with a vector in memory.
+struct UzRow {
+	double4 k[kUzRow];
+	int nb[kUzRow];
+	bool f0, f1;   // free components
+	__device__ __forceinline__ void load(const UzawaArgs &a, int A, bool in)
+	{
+		const int nno = a.L.nno;
+		f0 = in && vfree(a.L, A, 0);
+		f1 = in && vfree(a.L, A, 1);
+#pragma unroll
+		for (int u = 0; u < kUzRow; u++) {
+			const bool has = in && u < a.L.nbw;
+			nb[u] = has ? a.L.nb[(size_t)u * nno + A] : 0;
+			k[u] = has ? a.K[(size_t)u * nno + A] : make_double4(0.0, 0.0, 0.0, 0.0);
+		}
+	}
+	// as kmul_node (padding adds zero times x[0])
+	__device__ __forceinline__ void apply(const double2 *__restrict__ x, double &y0, double &y1) const
+	{
+		double2 xb[kUzRow];
+#pragma unroll
+		for (int u = 0; u < kUzRow; u++)
+			xb[u] = x[nb[u]];
+		double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+		for (int u = 0; u < kUzRow; u++) {
+			s0 += k[u].x * xb[u].x;
+			s0 += k[u].y * xb[u].y;
+			s1 += k[u].z * xb[u].x;
+			s1 += k[u].w * xb[u].y;
+		}
+		y0 = f0 ? s0 : 0.0;
+		y1 = f1 ? s1 : 0.0;
+	}
+};
+
+// Conj_Grad (cg_solve.cuh) for this thread's node A (in: it has one).
+__device__ __forceinline__ int uz_cg(UzTeam &tm, const UzawaArgs &a, const UzRow &R, int A, bool in,
+                                     const double2 *__restrict__ b, double2 *__restrict__ x, double accu, int *status)
+{
+	__shared__ double s_alpha, s_beta, s_delta, s_delta0, s_dq;
+	__shared__ int s_stop;
+	// this thread's solution and 1/diagonal, each used once per iteration: in
+	// registers they would push others to the stack (168 for 9 warps)
+	__shared__ double2 sh_x[kUzBlock], sh_id[kUzBlock];
+	double2 &xx = sh_x[threadIdx.x], &id = sh_id[threadIdx.x];
+	const bool precond = a.precond != 0;
+	const int max_cycle = a.max_cg;
+	double2 *d = a.dd;
+	double2 rr = make_double2(0.0, 0.0), dd = rr, ss = rr, qq = rr;
+	xx = rr;
+	id = make_double2(1.0, 1.0);
+	double a0[1] = {0.0};
+	if (in) {
+		double y0, y1;
+		xx = x[A];
+		if (precond)
+			id = a.idiag[A];
+		R.apply(x, y0, y1);
+		const double2 bb = b[A];
+		if (R.f0) {
+			rr.x = bb.x - y0;
+			dd.x = precond ? rr.x * id.x : rr.x;
+			a0[0] += rr.x * dd.x;
+		}
+		if (R.f1) {
+			rr.y = bb.y - y1;
+			dd.y = precond ? rr.y * id.y : rr.y;
+			a0[0] += rr.y * dd.y;
+		}
+		d[A] = dd;
+	}
+	tm.reduce_then<1>(a0, [&](const double (&v)[1]) {
+		s_delta = s_delta0 = v[0];
+		s_stop = !(0 < max_cycle && v[0] > accu * v[0]);
+	});
+	int cycle = 0;
+	while (!s_stop) {
+		double a1[1] = {0.0};
+		if (in) {
+			R.apply(d, qq.x, qq.y);
+			if (R.f0)
+				a1[0] += dd.x * qq.x;
+			if (R.f1)
+				a1[0] += dd.y * qq.y;
+		}
+		tm.reduce_then<1>(a1, [&](const double (&v)[1]) {
+			s_dq = v[0];
+			s_alpha = s_delta / v[0];
+		});
+		const double alpha = s_alpha;
+		const bool refresh = (cycle % 50) == 0;
+		if (R.f0)
+			xx.x += alpha * dd.x;
+		if (R.f1)
+			xx.y += alpha * dd.y;
+		double2 rn = make_double2(rr.x - alpha * qq.x, rr.y - alpha * qq.y);
+		if (refresh) {
+			if (in)
+				x[A] = xx;
+			tm.sync();
+			if (in) {
+				double y0, y1;
+				R.apply(x, y0, y1);
+				const double2 bb = b[A];
+				rn = make_double2(bb.x - y0, bb.y - y1);
+			}
+		}
+		double a2[2] = {0.0, 0.0};
+		if (R.f0) {
+			rr.x = rn.x;
+			ss.x = precond ? rr.x * id.x : rr.x;
+			a2[0] += rr.x * ss.x;
+			a2[1] = fmax(a2[1], fabs(alpha * rr.x));
+		}
+		if (R.f1) {
+			rr.y = rn.y;
+			ss.y = precond ? rr.y * id.y : rr.y;
+			a2[0] += rr.y * ss.y;
+			a2[1] = fmax(a2[1], fabs(alpha * rr.y));
+		}
+		tm.reduce_then<2, 2u>(a2, [&](const double (&v)[2]) {
+			s_beta = v[0] / s_delta;
+			s_delta = v[0];
+			s_stop = 0;
+			if (!isfinite(v[0]) || !isfinite(s_alpha)) {
+				if (blockIdx.x == 0)
+					atomicOr(status, s_dq == 0.0 ? kStatBreakdown : kStatNan);
+				s_stop = 1;
+			} else if (v[1] < accu || !(cycle + 1 < max_cycle && v[0] > accu * s_delta0)) {
+				s_stop = 1;
+			}
+		});
+		const double beta = s_beta;
+		if (R.f0)
+			dd.x = ss.x + beta * dd.x;
+		if (R.f1)
+			dd.y = ss.y + beta * dd.y;
+		if (in)
+			d[A] = dd;
+		cycle++;
+		if (!s_stop)
+			tm.sync();
+	}
+	if (in)
+		x[A] = xx;
+	if (cycle >= max_cycle && blockIdx.x == 0 && threadIdx.x == 0)
+		atomicOr(status, kStatCap);
+	tm.sync();
+	return cycle;
+}
+
+__global__ void __launch_bounds__(kUzBlock, 1) k_uzawa_cluster(const __grid_constant__ UzawaArgs args)
+{
+	__shared__ UzawaArgs a;
+	__shared__ double part[2 * kRedWidth * kUzWarps], mid[kRedWidth * ((kUzGroups + 7) / 8)];
+	load_args(a, args);
+	UzTeam tm;
+	tm.part = part;
+	tm.mid = mid;
+	tm.flip = 0;
+	const DevLevel &L = a.L;
+	tm.ngroups = ((L.nno > L.nel ? L.nno : L.nel) + 31) / 32;
+	// groups of 32 are dealt to the blocks in turn
+	const int i = (((threadIdx.x >> 5) * kUzCluster + blockIdx.x) << 5) + (threadIdx.x & 31);
+	const bool in = i < L.nno, ine = i < L.nel, lead = blockIdx.x == 0 && threadIdx.x == 0;
+	int *status = &a.sc->status;
+	double accu = a.accuracy;
+	UzRow R;
+	R.load(a, i, in);
+
+	if (a.auto_accuracy) {  // Solver.c:40-51
+		double f[1] = {0.0};
+		if (in) {
+			const double2 fa = a.F[i];
+			f[0] += fa.x * fa.x + fa.y * fa.y;
+		}
+		tm.reduce<1>(f);
+		accu = a.citcom_accu * sqrt(f[0] / a.neq);
+	}
+	// u1 = K d;  Ah = F - G p - u1  (Solver.c:67-77)
+	if (in) {
+		double k0, k1, g0, g1;
+		R.apply(a.d, k0, k1);
+		gmul_node(L, a.p, i, g0, g1);
+		const double2 f = a.F[i];
+		a.u1[i] = make_double2(k0, k1);
+		a.Ah[i] = make_double2(R.f0 ? f.x - g0 - k0 : 0.0, R.f1 ? f.y - g1 - k1 : 0.0);
+	}
+	tm.sync();
+	int cg_total = uz_cg(tm, a, R, i, in, a.Ah, a.u1, accu, status);
+	if (in) {
+		double2 dv = a.d[i];
+		const double2 u = a.u1[i];
+		dv.x += u.x;
+		dv.y += u.y;
+		a.d[i] = dv;
+	}
+	tm.sync();
+	// this thread's element: residuals and preconditioned residuals of the last two
+	// cycles, direction, pressure
+	double r0 = 0.0, r1 = ine ? gtmul_elem(L, a.d, i) : 0.0, z0 = 0.0, s1 = 0.0;
+	double pe = ine ? a.p[i] : 0.0;
+	const double bab = ine ? a.bab[i] : 0.0;
+
+	double dvel = 1.0, dpre = 1.0;
+	int cycle = 0;
+	while ((dvel > a.citcom_accu || (dpre > a.citcom_accu && a.check_v_only == 0)) && cycle < a.max_citcom) {
+		double rz[2] = {0.0, 0.0};
+		const double z1 = bab * r1;
+		if (ine) {
+			rz[0] += r1 * z1;
+			if (cycle > 0)
+				rz[1] += r0 * z0;
+		}
+		tm.reduce<2>(rz);
+		const double r1dotz1 = rz[0];
+		if (cycle > 0 && !(rz[1] > 0.0)) {   // assert(r0dotr0 > 0.0), Solver.c:150
+			if (lead)
+				atomicOr(status, kStatBreakdown);
+			break;
+		}
+		const double delta = cycle == 0 ? 0.0 : r1dotz1 / rz[1];
+		const double s2 = cycle == 0 ? z1 : z1 + delta * s1;
+		if (ine)
+			a.s2[i] = s2;
+		tm.sync();
+		if (in) {
+			double g0, g1;
+			gmul_node(L, a.s2, i, g0, g1);
+			a.Ah[i] = make_double2(g0, g1);
+			a.u1[i] = make_double2(0.0, 0.0);
+		}
+		tm.sync();
+		cg_total += uz_cg(tm, a, R, i, in, a.Ah, a.u1, accu, status);
+		double sa[1] = {0.0}, Ahp = 0.0;
+		if (ine) {
+			Ahp = gtmul_elem(L, a.u1, i);
+			sa[0] += s2 * Ahp;
+		}
+		tm.reduce<1>(sa);
+		const double alpha = r1dotz1 / sa[0];
+		double t[4] = {0.0, 0.0, 0.0, 0.0};
+		double r2 = 0.0;
+		if (ine) {
+			r2 = r1 - alpha * Ahp;
+			pe = pe + alpha * s2;
+			t[0] += s2 * s2;
+			t[1] += pe * pe;
+		}
+		if (in) {
+			const double2 u = a.u1[i];
+			double2 dv = a.d[i];
+			dv.x -= alpha * u.x;
+			dv.y -= alpha * u.y;
+			a.d[i] = dv;
+			t[2] += u.x * u.x + u.y * u.y;
+			t[3] += dv.x * dv.x + dv.y * dv.y;
+		}
+		tm.reduce<4>(t);
+		dpre = alpha * sqrt(t[0] / (1.0e-32 + t[1]));
+		dvel = alpha * sqrt(t[2] / (1.0e-32 + t[3]));
+		cycle++;
+		s1 = s2;
+		r0 = r1;
+		r1 = r2;
+		z0 = z1;
+		if (!isfinite(dvel) || !isfinite(dpre)) {
+			if (lead)
+				atomicOr(status, kStatNan);
+			break;
+		}
+	}
+	if (cycle >= a.max_citcom && lead)
+		atomicOr(status, kStatCap);
+	if (ine)
+		a.p[i] = pe;
+	tm.sync();
+
+	// true residual |[F - K d - G p ; G^T d]| / |F|, and v_to_nodes (Solver.c:1319-1343)
+	double rs[3] = {0.0, 0.0, 0.0};
+	if (in) {
+		double k0, k1, g0, g1;
+		R.apply(a.d, k0, k1);
+		gmul_node(L, a.p, i, g0, g1);
+		const double2 f = a.F[i];
+		const double m0 = R.f0 ? f.x - k0 - g0 : 0.0;
+		const double m1 = R.f1 ? f.y - k1 - g1 : 0.0;
+		rs[0] += m0 * m0 + m1 * m1;
+		rs[2] += f.x * f.x + f.y * f.y;
+		const double2 dv = a.d[i];
+		a.V[i] = make_double2(R.f0 ? dv.x : L.vbcval[i], R.f1 ? dv.y : L.vbcval[L.nno + i]);
+	}
+	if (ine) {
+		const double dvg = gtmul_elem(L, a.d, i);
+		rs[1] += dvg * dvg;
+	}
+	tm.reduce<3>(rs);
+	if (lead) {
+		StepScalars *sc = a.sc;
+		sc->uzawa_cycles = cycle;
+		sc->cg_cycles = cg_total;
+		sc->dv = dvel;
+		sc->dp = dpre;
+		sc->res_m = sqrt(rs[0]) / sqrt(rs[2]);
+		sc->res_c = sqrt(rs[1]) / sqrt(rs[2]);
+		sc->accuracy = accu;
+	}
+	tm.sync();   // no block leaves while another reads its partials
+}
+
 // ---- single operators for the parity API --------------------------------
 __global__ void __launch_bounds__(kBlock) k_kmul(DevLevel L, const double4 *__restrict__ K,
                                                  const double2 *__restrict__ x, double2 *__restrict__ y)
@@ -538,6 +932,15 @@ __global__ void __launch_bounds__(kBlock) k_v_to_nodes(DevLevel L, const double2
 }
 
 void *uzawa_kernel_ptr(int ref) { return ref ? (void *)k_uzawa<true> : (void *)k_uzawa<false>; }
+// The one-cluster form: the kernel, its blocks and threads, and the largest mesh.
+void *uzawa_cluster_kernel(int *blocks, int *threads, int *max_nodes, int *max_row)
+{
+	*blocks = kUzCluster;
+	*threads = kUzBlock;
+	*max_nodes = 32 * kUzGroups;
+	*max_row = kUzRow;
+	return (void *)k_uzawa_cluster;
+}
 void *kmul_kernel_ptr() { return (void *)k_kmul; }
 
 }  // namespace mclg

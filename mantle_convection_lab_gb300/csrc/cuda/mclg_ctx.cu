@@ -20,6 +20,7 @@ void upload_shape_tables_elem(const ShapeTables &s, cudaStream_t st);
 void upload_shape_tables_uzawa(const ShapeTables &s, cudaStream_t st);
 void upload_shape_tables_heat(const ShapeTables &s, cudaStream_t st);
 void *uzawa_kernel_ptr(int ref);
+void *uzawa_cluster_kernel(int *blocks, int *threads, int *max_nodes, int *max_row);
 void *heat_cg_kernel_ptr();
 __global__ void k_buoy_rowavg(DevLevel L, const double *T, double Ra, double *avg);
 __global__ void k_buoy_vis(DevLevel L, const double *T, double Ra, const double *avg, double Aexp, double refT,
@@ -101,6 +102,7 @@ struct mclg_ctx {
 	double *tmpA, *tmpB;
 	// converged solvers on uniform meshes (precision 1 and 2)
 	int coop_mg;
+	int uzawa_cluster;           // the replica's solve runs as one cluster
 	int mg_one_cluster;          // its blocks are one cluster instead of a cooperative grid
 	double remesh_ms[5];   // the last remesh: numbering, lists, state, wait, carry (host ms)
 	MGArgs<float> mgf;
@@ -313,12 +315,12 @@ static int coop_blocks(void *kernel, int num_sms, int work)
 }
 
 // Launch one cluster of cs blocks.
-static cudaError_t launch_cluster(void *kern, int cs, void **args, cudaStream_t st)
+static cudaError_t launch_cluster(void *kern, int cs, int threads, void **args, cudaStream_t st)
 {
 	cudaLaunchConfig_t lc;
 	memset(&lc, 0, sizeof lc);
 	lc.gridDim = dim3(cs);
-	lc.blockDim = dim3(kBlock);
+	lc.blockDim = dim3(threads);
 	lc.stream = st;
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
@@ -331,7 +333,7 @@ static cudaError_t launch_cluster(void *kern, int cs, void **args, cudaStream_t 
 }
 
 // Clusters of cs blocks of `kern` that can be resident at once (0: none).
-static int max_clusters(void *kern, int cs)
+static int max_clusters(void *kern, int cs, int threads)
 {
 	if (cs > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
 		cudaGetLastError();
@@ -340,7 +342,7 @@ static int max_clusters(void *kern, int cs)
 	cudaLaunchConfig_t lc;
 	memset(&lc, 0, sizeof lc);
 	lc.gridDim = dim3(cs);
-	lc.blockDim = dim3(kBlock);
+	lc.blockDim = dim3(threads);
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = cs;
@@ -367,7 +369,7 @@ static void mg_team(mclg_ctx *c, void *kern)
 	constexpr int kOneCluster = 16, kOneClusterN32 = 128, kOneClusterN64 = 32;
 	const int N0 = c->mesh.max_elx[c->fl];
 	c->mg_one_cluster = N0 <= (c->cfg.precision == 2 ? kOneClusterN64 : kOneClusterN32) &&
-	                    max_clusters(kern, kOneCluster) >= 1;
+	                    max_clusters(kern, kOneCluster, kBlock) >= 1;
 	c->coop_mg = c->mg_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, 1 << 30);
 }
 
@@ -1258,7 +1260,7 @@ static int launch_stokes_mg(mclg_ctx *c)
 	void *args[] = {c->cfg.precision == 2 ? (void *)&c->mgd : (void *)&c->mgf};
 	void *kern = stokes_mg_kernel(c->cfg.precision == 2);
 	if (one)
-		CK(launch_cluster(kern, c->coop_mg, args, c->st));
+		CK(launch_cluster(kern, c->coop_mg, kBlock, args, c->st));
 	else
 		CK(cudaLaunchCooperativeKernel(kern, dim3(solver_grid(c, c->coop_mg)), dim3(kBlock), args, 0, c->st));
 	c->launches++;
@@ -1508,6 +1510,12 @@ static int create_impl(mclg_ctx **out, const mclg_config *cfg, const int *leaves
 	}
 	const int work = (int)(nn > ne ? nn : ne);
 	c->coop_uzawa = coop_blocks(uzawa_kernel_ptr(c->ref_kind != kRefNone), c->num_sms, work);
+	{
+		int blocks, threads, nodes, row;
+		void *kern = uzawa_cluster_kernel(&blocks, &threads, &nodes, &row);
+		c->uzawa_cluster = c->ref_kind == kRefNone && c->L.nh == 0 && c->L.nbw <= row && work <= nodes &&
+		                   max_clusters(kern, blocks, threads) >= 1;
+	}
 	c->coop_heat = coop_blocks(heat_cg_kernel_ptr(), c->num_sms, (int)nn);
 	if (cfg->precision != 0 && !c->mesh.uniform) {
 		rc = cfg->precision == 2 ? qt_setup<double>(c, c->qtd, pre) : qt_setup<float>(c, c->qtf, pre);
@@ -1720,6 +1728,22 @@ static int read_scalars(mclg_ctx *c)
 	return MCLG_OK;
 }
 
+// The replica's solve.  On one cluster where a thread can own each node and its
+// rows (no hanging nodes, whose overwrite follows every update, and at most 64^2
+// elements), with the CG inner solver; measured per CG iteration against the
+// cooperative grid: 8.0 against 15.6 us at 16^2, 10.2 against 15.8 at 64^2.
+static cudaError_t run_uzawa(mclg_ctx *c, UzawaArgs &a)
+{
+	void *args[] = {&a};
+	if (c->uzawa_cluster && !a.solver_jc) {
+		int blocks, threads, nodes, row;
+		void *kern = uzawa_cluster_kernel(&blocks, &threads, &nodes, &row);
+		return launch_cluster(kern, blocks, threads, args, c->st);
+	}
+	return cudaLaunchCooperativeKernel(uzawa_kernel_ptr(c->ref_kind != kRefNone), dim3(c->coop_uzawa), dim3(kBlock), args,
+	                                   0, c->st);
+}
+
 static int launch_uzawa(mclg_ctx *c)
 {
 	const mclg_config &f = c->cfg;
@@ -1769,9 +1793,7 @@ static int launch_uzawa(mclg_ctx *c)
 	a.accuracy = f.accuracy;
 	a.ref_kind = c->ref_kind;
 	a.ref = c->ref_dev;
-	void *args[] = {&a};
-	CK(cudaLaunchCooperativeKernel(uzawa_kernel_ptr(c->ref_kind != kRefNone), dim3(c->coop_uzawa), dim3(kBlock), args, 0,
-	                               c->st));
+	CK(run_uzawa(c, a));
 	c->launches++;
 	return MCLG_OK;
 }
@@ -2409,9 +2431,7 @@ extern "C" int mclg_solve_velocity_pressure_noalloc(mclg_ctx *c, mclg_step_stats
 	a.accuracy = f.accuracy;
 	a.ref_kind = c->ref_kind;
 	a.ref = c->ref_dev;
-	void *args[] = {&a};
-	CK(cudaLaunchCooperativeKernel(uzawa_kernel_ptr(c->ref_kind != kRefNone), dim3(c->coop_uzawa), dim3(kBlock), args, 0,
-	                               c->st));
+	CK(run_uzawa(c, a));
 	c->launches++;
 	// compute_stress with the element stresses in the same array
 	k_stress_elem<<<blocks_for(ne), kBlock, 0, c->st>>>(c->L, c->vis, c->V, ev[8]);
