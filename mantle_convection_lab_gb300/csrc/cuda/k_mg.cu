@@ -20,6 +20,7 @@
 // The operator is matrix-free (k_march.cuh).
 #include <math.h>
 #include "k_mg.cuh"
+#include "fp64_util.cuh"
 
 namespace mclg {
 

@@ -5,6 +5,7 @@
 // output, residual) is zero outside the reduced dofs.
 #include <math.h>
 #include "k_qt.cuh"
+#include "fp64_util.cuh"
 
 namespace mclg {
 
@@ -121,39 +122,42 @@ struct QtXFirst {
 	TI omega;
 	__device__ __forceinline__ X2 operator()(int B) const
 	{
-		const X2 bv = b[B];
+		const X2 bv = b[B], dv = reinterpret_cast<const X2 *>(invD)[B];
 		X2 o;
-		o.x = omega * invD[2 * B] * bv.x;
-		o.y = omega * invD[2 * B + 1] * bv.y;
+		o.x = omega * dv.x * bv.x;
+		o.y = omega * dv.y * bv.y;
 		return o;
 	}
 };
 
 // (C^T K C x) at both dofs of node A from the assembled reduced operator: a
 // plain node-block ELL row (x's constrained and fixed entries are stored as 0
-// and the reduced columns hold every coupling); x read through src.
+// and the reduced columns hold every coupling); x read through src.  A row's
+// first kChunk columns (all of an interior row between equal elements) are in
+// flight together: after a team barrier every load is an L2 access.
 template <class TI, class XS>
 __device__ __forceinline__ void qt_kr_node_src(const QtLevel<TI> &L, const XS &src, int A, TI &y0, TI &y1)
 {
 	typedef typename Q2T<TI>::t X2;
 	typedef typename V4T<TI>::t K4;
+	constexpr int kChunk = sizeof(TI) == 4 ? 9 : 4;
 	TI s0 = TI(0), s1 = TI(0);
 	const int n = L.rcnt[A];
-	for (int k0 = 0; k0 < n; k0 += 4) {
-		int B[4];
-		K4 kb[4];
+	for (int k0 = 0; k0 == 0 || k0 < n; k0 += kChunk) {   // (the first chunk does not wait for n)
+		int B[kChunk];
+		K4 kb[kChunk];
 #pragma unroll
-		for (int u = 0; u < 4; u++) {
-			const bool in = k0 + u < n;
+		for (int u = 0; u < kChunk; u++) {
+			const bool in = k0 + u < L.rnbw;   // (columns past the row's end are the row node with a zero block)
 			B[u] = in ? L.rnb[(size_t)(k0 + u) * L.nno + A] : A;
 			kb[u] = in ? L.Kr[(size_t)(k0 + u) * L.nno + A] : K4{};
 		}
-		X2 xv[4];
+		X2 xv[kChunk];
 #pragma unroll
-		for (int u = 0; u < 4; u++)
+		for (int u = 0; u < kChunk; u++)
 			xv[u] = src(B[u]);
 #pragma unroll
-		for (int u = 0; u < 4; u++) {
+		for (int u = 0; u < kChunk; u++) {
 			s0 += kb[u].x * xv[u].x + kb[u].y * xv[u].y;
 			s1 += kb[u].z * xv[u].x + kb[u].w * xv[u].y;
 		}
@@ -169,13 +173,84 @@ __device__ __forceinline__ void qt_kr_node(const QtLevel<TI> &L, const TI *__res
 	qt_kr_node_src(L, src, A, y0, y1);
 }
 
+// s = sum of w[i] x[src[i]] over [i0, i1), C entries at a time: their indices,
+// then their gathers in flight together (a list's loop waits for both in turn).
+template <int C, class T>
+__device__ __forceinline__ T qt_gather(const int *__restrict__ src, const T *__restrict__ w, const T *__restrict__ x,
+                                       int i0, int i1)
+{
+	T s = T(0);
+	for (int i = i0; i < i1; i += C) {
+		int j[C];
+		T ww[C], xv[C];
+#pragma unroll
+		for (int u = 0; u < C; u++) {
+			const bool in = i + u < i1;
+			j[u] = src[in ? i + u : i0];
+			ww[u] = in ? w[i + u] : T(0);
+		}
+#pragma unroll
+		for (int u = 0; u < C; u++)
+			xv[u] = x[j[u]];
+#pragma unroll
+		for (int u = 0; u < C; u++)
+			s += i + u < i1 ? ww[u] * xv[u] : T(0);
+	}
+	return s;
+}
+
+// Node B of a primal vector through the constraints, its stored values and kinds
+// in flight together.
+template <class T, class X>
+__device__ __forceinline__ typename Q2T<X>::t qt_node(const QtLevel<T> &L, const X *__restrict__ xf, int B)
+{
+	typename Q2T<X>::t v = reinterpret_cast<const typename Q2T<X>::t *>(xf)[B];
+	const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[B];
+	if (k.x != 1 || k.y != 1) {
+		v.x = k.x == 1 ? v.x : k.x == 2 ? qt_val(L, xf, 2 * B) : X(0);
+		v.y = k.y == 1 ? v.y : k.y == 2 ? qt_val(L, xf, 2 * B + 1) : X(0);
+	}
+	return v;
+}
+
+// G p at node A on the finest level: an element's entries are +-dz_deta and
+// +-dx_dxi by corner (the sums over the Gauss points that element_g forms, 8
+// FP64 operations a corner, come to one of the two half-widths).
+__device__ __forceinline__ void qt_gmul(const DevLevel &L, const double *__restrict__ p, int A, double &y0, double &y1)
+{
+	double s0 = 0.0, s1 = 0.0;
+	const int n = L.p2n_cnt[A];
+	int e[4], a[4];
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		e[k] = L.p2n_el[k * L.nno + A];
+		a[k] = L.p2n_a[k * L.nno + A];
+	}
+	double pe[4], hz[4], hx[4];
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		const int ek = k < n ? e[k] : e[0];
+		pe[k] = p[ek];
+		hz[k] = L.dzh[ek];
+		hx[k] = L.dxh[ek];
+	}
+#pragma unroll
+	for (int k = 0; k < 4; k++)
+		if (k < n) {
+			s0 += (a[k] < 2 ? hz[k] : -hz[k]) * pe[k];
+			s1 += (a[k] == 0 || a[k] == 3 ? hx[k] : -hx[k]) * pe[k];
+		}
+	y0 = s0;
+	y1 = s1;
+}
+
 // (C^T G p) at both dofs of node A (FP64, the finest level)
 template <class T>
 __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L, const double *__restrict__ p, int A,
                                           double &y0, double &y1)
 {
 	double y[2];
-	gmul_node(L, p, A, y[0], y[1]);
+	qt_gmul(L, p, A, y[0], y[1]);
 #pragma unroll
 	for (int c = 0; c < 2; c++) {
 		const int dof = 2 * A + c;
@@ -186,8 +261,9 @@ __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L
 		for (int i = Q.fo_off[dof]; i < Q.fo_off[dof + 1]; i++) {
 			const int h = Q.fo_dof[i];
 			double h0, h1;
-			gmul_node(L, p, h >> 1, h0, h1);
-			y[c] += (double)Q.fo_w[i] * ((h & 1) ? h1 : h0);
+			qt_gmul(L, p, h >> 1, h0, h1);
+			const double hv = (h & 1) ? (vfree(L, h >> 1, 1) ? h1 : 0.0) : (vfree(L, h >> 1, 0) ? h0 : 0.0);
+			y[c] += (double)Q.fo_w[i] * hv;
 		}
 	}
 	y0 = y[0];
@@ -198,36 +274,43 @@ __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L
 template <class T, class X>
 __device__ __forceinline__ double qt_gt_elem(const QtLevel<T> &Q, const DevLevel &L, const X *__restrict__ uf, int e)
 {
-	double s = 0.0;
+	int n[4];
+	X u[4], w[4];
 #pragma unroll
-	for (int c = 0; c < 4; c++) {
-		const int a = kSortedCorner[c];
-		const int A = L.ienl[a * L.nel + e];
-		double g0, g1;
-		element_g(cS, L.dzh[e], L.dxh[e], a, g0, g1);
-		s += g0 * (double)qt_val(Q, uf, 2 * A);
-		s += g1 * (double)qt_val(Q, uf, 2 * A + 1);
+	for (int a = 0; a < 4; a++)
+		n[a] = L.ienl[a * L.nel + e];
+#pragma unroll
+	for (int a = 0; a < 4; a++) {
+		const typename Q2T<X>::t v = qt_node(Q, uf, n[a]);
+		u[a] = v.x;
+		w[a] = v.y;
 	}
-	return s;
+	return gt_elem(u[0], u[1], u[2], u[3], w[0], w[1], w[2], w[3], L.dzh[e], L.dxh[e]);
 }
 
 // ---- the V-cycle (TI) -------------------------------------------------------------
 // One damped Jacobi sweep on the constrained operator: xo = xi + w D^-1 (b - A xi),
 // xi read through src.
 template <class TI, class XS>
+__device__ __forceinline__ typename Q2T<TI>::t qt_sweep_node(const QtLevel<TI> &L, TI omega, const XS &src, int A)
+{
+	typedef typename Q2T<TI>::t V;
+	TI y0, y1;
+	const V x = src(A), b = L.b[A], dg = reinterpret_cast<const V *>(L.invD)[A];   // invD is 0 off the reduced dofs
+	const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[A];
+	qt_kr_node_src(L, src, A, y0, y1);
+	V o;
+	o.x = k.x == 1 ? x.x + omega * dg.x * (b.x - y0) : TI(0);
+	o.y = k.y == 1 ? x.y + omega * dg.y * (b.y - y1) : TI(0);
+	return o;
+}
+
+template <class TI, class XS>
 __device__ __forceinline__ void qt_sweep_src(const QtLevel<TI> &L, TI omega, const XS &src,
                                              typename Q2T<TI>::t *xo, int tid, int nth)
 {
-	typedef typename Q2T<TI>::t V;
-	for (int A = tid; A < L.nno; A += nth) {
-		TI y0, y1;
-		qt_kr_node_src(L, src, A, y0, y1);
-		const V x = src(A), b = L.b[A];
-		V o;
-		o.x = L.kind[2 * A] == 1 ? x.x + omega * L.invD[2 * A] * (b.x - y0) : TI(0);
-		o.y = L.kind[2 * A + 1] == 1 ? x.y + omega * L.invD[2 * A + 1] * (b.y - y1) : TI(0);
-		xo[A] = o;
-	}
+	for (int A = tid; A < L.nno; A += nth)
+		xo[A] = qt_sweep_node(L, omega, src, A);
 }
 
 template <class TI>
@@ -281,9 +364,10 @@ __device__ void qt_down(const QtHier<TI> &H, int l, QtTeam &t)
 			qt_kr_node_src(L, first, A, y0, y1);
 			x0[A] = first(A);
 			const V b = L.b[A];
+			const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[A];
 			V r;
-			r.x = L.kind[2 * A] == 1 ? b.x - y0 : TI(0);
-			r.y = L.kind[2 * A + 1] == 1 ? b.y - y1 : TI(0);
+			r.x = k.x == 1 ? b.x - y0 : TI(0);
+			r.y = k.y == 1 ? b.y - y1 : TI(0);
 			L.r[A] = r;
 		}
 		cur = 0;
@@ -302,9 +386,10 @@ __device__ void qt_down(const QtHier<TI> &H, int l, QtTeam &t)
 			TI y0, y1;
 			qt_kr_node(L, xf, A, y0, y1);
 			const V b = L.b[A];
+			const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[A];
 			V r;
-			r.x = L.kind[2 * A] == 1 ? b.x - y0 : TI(0);
-			r.y = L.kind[2 * A + 1] == 1 ? b.y - y1 : TI(0);
+			r.x = k.x == 1 ? b.x - y0 : TI(0);
+			r.y = k.y == 1 ? b.y - y1 : TI(0);
 			L.r[A] = r;
 		}
 		t.sync();
@@ -313,32 +398,44 @@ __device__ void qt_down(const QtHier<TI> &H, int l, QtTeam &t)
 	const TI *rf = reinterpret_cast<const TI *>(L.r);
 	TI *cb = reinterpret_cast<TI *>(C.b);
 	for (int d = t.tid; d < 2 * C.nno; d += t.nth) {   // restriction: P^T by rows
-		TI s = TI(0);
-		for (int i = C.r_off[d]; i < C.r_off[d + 1]; i++)
-			s += C.r_w[i] * rf[C.r_src[i]];
-		cb[d] = s;
+		cb[d] = qt_gather<9, TI>(C.r_src, C.r_w, rf, C.r_off[d], C.r_off[d + 1]);
 	}
 	t.sync();
 }
 
 // Level l on the way up: prolongation of level l-1's result added, smoothing.
+// With zout (the finest level) the last sweep writes there, adds this thread's
+// share of zout.v to *dot and is not followed by a barrier: the caller's
+// reduction provides it.
 template <class TI>
-__device__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t)
+__device__ __forceinline__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t, typename Q2T<TI>::t *zout = nullptr,
+                                      const double2 *v = nullptr, double *dot = nullptr)
 {
+	typedef typename Q2T<TI>::t V;
 	const QtLevel<TI> &L = H.lv[l];
 	int cur = (H.smooth - 1) & 1;
 	const TI *xc = reinterpret_cast<const TI *>(H.lv[l - 1].x[qt_final(H, l - 1)]);
 	TI *xf = reinterpret_cast<TI *>(L.x[cur]);
 	for (int d = t.tid; d < 2 * L.nno; d += t.nth) {
-		if (L.p_off[d] == L.p_off[d + 1])
-			continue;
-		TI s = TI(0);
-		for (int i = L.p_off[d]; i < L.p_off[d + 1]; i++)
-			s += L.p_w[i] * xc[L.p_src[i]];
-		xf[d] += s;
+		const int i0 = L.p_off[d], i1 = L.p_off[d + 1];
+		const TI x0 = xf[d];
+		if (i0 < i1)
+			xf[d] = x0 + qt_gather<4, TI>(L.p_src, L.p_w, xc, i0, i1);
 	}
 	t.sync();
 	for (int s = 0; s < H.smooth; s++) {
+		if (zout != nullptr && s == H.smooth - 1) {
+			const QtXStored<TI> src{L.x[cur]};
+			double acc = 0.0;
+			for (int A = t.tid; A < L.nno; A += t.nth) {
+				const double2 va = v[A];
+				const V o = qt_sweep_node(L, H.omega, src, A);
+				zout[A] = o;
+				acc += widen(o.x) * va.x + widen(o.y) * va.y;
+			}
+			*dot += acc;
+			return;
+		}
 		qt_sweep(L, H.omega, L.x[cur], L.x[1 - cur], t.tid, t.nth);
 		cur = 1 - cur;
 		t.sync();
@@ -361,20 +458,27 @@ __device__ void qt_coarse_solve(const QtHier<TI> &H, QtTeam &t)
 	t.sync();
 }
 
-// z = V-cycle(b) with b in the finest level's b; returns the buffer holding z.
+// z = V-cycle(b) with b in the finest level's b; *dot receives this thread's
+// share of z.v.  Ends without a barrier (the caller's reduction follows).
 template <class TI>
-__device__ const typename Q2T<TI>::t *qt_vcycle(Sync &sy, const QtHier<TI> &H)
+__device__ __forceinline__ void qt_vcycle(Sync &sy, const QtHier<TI> &H, typename Q2T<TI>::t *z, const double2 *v,
+                                          double *dot)
 {
+	typedef typename Q2T<TI>::t V;
 	const int top = H.nlev - 1, nb = H.nblk < top ? H.nblk : top;   // the finest level always runs on the team
 	QtTeam team{&sy, true, sy.tid(), sy.nth()};
+	*dot = 0.0;
+#pragma unroll 1
 	for (int l = top; l >= (nb > 1 ? nb : 1); l--)
 		qt_down(H, l, team);
 	if (nb > 0) {
 		if (sy.leader()) {
 			QtTeam blk{&sy, false, (int)threadIdx.x, (int)blockDim.x};
+#pragma unroll 1
 			for (int l = nb - 1; l >= 1; l--)
 				qt_down(H, l, blk);
 			qt_coarse_solve(H, blk);
+#pragma unroll 1
 			for (int l = 1; l < nb; l++)
 				qt_up(H, l, blk);
 		}
@@ -382,9 +486,18 @@ __device__ const typename Q2T<TI>::t *qt_vcycle(Sync &sy, const QtHier<TI> &H)
 	} else {
 		qt_coarse_solve(H, team);
 	}
+#pragma unroll 1
 	for (int l = nb > 1 ? nb : 1; l <= top; l++)
-		qt_up(H, l, team);
-	return H.lv[top].x[qt_final(H, top)];
+		qt_up(H, l, team, l == top ? z : nullptr, v, dot);
+	if (top == 0) {   // the dense solve is the whole cycle
+		const QtLevel<TI> &Q = H.lv[0];
+		for (int A = team.tid; A < Q.nno; A += team.nth) {
+			const V o = Q.x[0][A];
+			const double2 va = v[A];
+			z[A] = o;
+			*dot += widen(o.x) * va.x + widen(o.y) * va.y;
+		}
+	}
 }
 
 // Dense inverse of the coarsest level's constrained operator on its reduced
@@ -479,155 +592,235 @@ __device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, con
 	sy.reduce<3>(rs);
 }
 
-// z = M^-1 v, M = diag(V-cycle, BAB); returns <z, v>.
-template <class TI>
-__device__ double qt_precond(Sync &sy, const QtArgs<TI> &a, const double2 *vu, const double *vp,
-                             typename Q2T<TI>::t *zu, double *zp)
-{
-	const int tid = sy.tid(), nth = sy.nth();
-	typedef typename Q2T<TI>::t V;
-	const QtHier<TI> &H = a.H;
-	const QtLevel<TI> &Q = H.lv[H.nlev - 1];
-	for (int A = tid; A < Q.nno; A += nth) {
-		const double2 v = vu[A];
-		V w;
-		w.x = (TI)v.x;
-		w.y = (TI)v.y;
-		Q.b[A] = w;
-	}
-	sy.sync();
-	const V *x = qt_vcycle(sy, H);
-	double dot[1] = {0.0};
-	for (int A = tid; A < Q.nno; A += nth) {
-		const V z = x[A];
-		zu[A] = z;
-		const double2 v = vu[A];
-		dot[0] += (double)z.x * v.x + (double)z.y * v.y;
-	}
-	for (int e = tid; e < a.L.nel; e += nth) {
-		const double z = vp[e] / a.bab[e];
-		zp[e] = z;
-		dot[0] += z * vp[e];
-	}
-	sy.reduce<1>(dot);
-	return dot[0];
-}
+// The scalars of the MINRES recurrences, formed by one thread of each block: a
+// division or a square root on every thread costs the FP64 pipe about a
+// microsecond each.
+struct QtScal {
+	double gam, gam_prev, eta, eta0, delta, c_prev, c_cur, s_prev, s_cur;
+	double ig, dg, gg, k1, k2, k3, step, step1;   // step1: the step of the iteration before
+	int stop;   // 1: last iteration; 2: breakdown before the update; 4: a non-finite value
+};
 
 // Correction solve by preconditioned MINRES (Elman, Silvester and Wathen,
 // "Finite Elements and Fast Iterative Solvers", Alg. 4.1) on the constrained
-// system [C^T K C, C^T G; G^T C, 0][x_u; x_p] = [R_m; -R_c] from zero; K in TI,
-// G in FP64, Lanczos and direction vectors FP64; x into a.dd, a.dpv.
+// system [C^T K C, C^T G; G^T C, 0][x_u; x_p] = [R_m; -R_c] from zero, with the
+// preconditioner diag(V-cycle, BAB); K in TI, G to FP64 accuracy, Lanczos and
+// direction vectors FP64; x into a.dd, a.dpv, two iterations' steps at a time.
 template <class TI>
-__device__ int qt_minres(Sync &sy, const QtArgs<TI> &a, double rtol, int maxit, int *status)
+__device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rtol, int maxit)
 {
-	const int tid = sy.tid(), nth = sy.nth();
 	typedef typename Q2T<TI>::t V;
+	__shared__ QtScal ms;
+	Sync sy = team;
 	const DevLevel &L = a.L;
 	const QtLevel<TI> &Q = a.H.lv[a.H.nlev - 1];
-	const int nn = L.nno, ne = L.nel;
-	double2 *vu[2] = {a.mv[0], a.mv[1]}, *wu[2] = {a.mw[0], a.mw[1]};
-	double *vp[2] = {a.mvp[0], a.mvp[1]}, *zp[2] = {a.mzp[0], a.mzp[1]}, *wp[2] = {a.mwp[0], a.mwp[1]};
-	V *zu[2] = {a.mz[0], a.mz[1]};
-	const double2 zero2 = make_double2(0.0, 0.0);
-	for (int A = tid; A < nn; A += nth) {
-		vu[0][A] = a.R[A];
-		vu[1][A] = zero2;
-		wu[0][A] = zero2;
-		wu[1][A] = zero2;
-		a.dd[A] = zero2;
-	}
-	for (int e = tid; e < ne; e += nth) {
-		vp[0][e] = -a.Rc[e];
-		vp[1][e] = 0.0;
-		wp[0][e] = 0.0;
-		wp[1][e] = 0.0;
-		a.dpv[e] = 0.0;
+	double pdot = 0.0;
+	{
+		const double2 zero2 = make_double2(0.0, 0.0);
+		const int tid = sy.tid(), nth = sy.nth(), nn = L.nno, ne = L.nel;
+		for (int A = tid; A < nn; A += nth) {
+			const double2 r = a.R[A];
+			a.mv[0][A] = r;
+			V w;
+			w.x = narrow_to<TI>(r.x);
+			w.y = narrow_to<TI>(r.y);
+			Q.b[A] = w;
+			a.mv[1][A] = zero2;
+			a.mw[0][A] = zero2;
+			a.mw[1][A] = zero2;
+			a.dd[A] = zero2;
+		}
+		for (int e = tid; e < ne; e += nth) {
+			const double v = -a.Rc[e], z = v * a.ibab[e];
+			a.mvp[0][e] = v;
+			a.mzp[0][e] = z;
+			pdot += z * v;
+			a.mvp[1][e] = 0.0;
+			a.mwp[0][e] = 0.0;
+			a.mwp[1][e] = 0.0;
+			a.dpv[e] = 0.0;
+		}
 	}
 	sy.sync();
-	double gam2 = qt_precond(sy, a, vu[0], vp[0], zu[0], zp[0]);
-	if (!(gam2 > 0.0))
-		return 0;
-	double gam = sqrt(gam2), gam_prev = 1.0;
-	const double eta0 = gam;
-	double eta = gam, c_prev = 1.0, c_cur = 1.0, s_prev = 0.0, s_cur = 0.0;
-	int cv = 0, cw = 0, it = 0;
+	// index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1).  it = -1: z(0) = M^-1 v(0)
+	int cv = 1, cw = 0, it = -1;
+#pragma unroll 1
 	while (it < maxit) {
-		const TI *zf = reinterpret_cast<const TI *>(zu[cv]);
-		double dl[1] = {0.0};
-		for (int A = tid; A < nn; A += nth) {
-			TI k0, k1;
-			double g0, g1;
-			qt_kr_node(Q, zf, A, k0, k1);
-			qt_g_node(Q, L, zp[cv], A, g0, g1);
-			const double2 az = make_double2((double)k0 + g0, (double)k1 + g1);
-			a.Kd[A] = az;
-			const V z = zu[cv][A];
-			dl[0] += az.x * (double)z.x + az.y * (double)z.y;
+		if (it >= 0) {
+			const int tid = sy.tid(), nth = sy.nth();
+			double dl[1] = {0.0};
+			{
+				const V *z = a.mz[cv];
+				const double *zp = a.mzp[cv];
+				const TI *zf = reinterpret_cast<const TI *>(z);
+				for (int A = tid; A < L.nno; A += nth) {
+					TI k0, k1;
+					double g0, g1;
+					const V zz = z[A];
+					qt_kr_node(Q, zf, A, k0, k1);
+					qt_g_node(Q, L, zp, A, g0, g1);
+					const double2 az = make_double2(widen(k0) + g0, widen(k1) + g1);
+					a.Kd[A] = az;
+					dl[0] += az.x * widen(zz.x) + az.y * widen(zz.y);
+				}
+				for (int e = tid; e < L.nel; e += nth) {
+					const double t = qt_gt_elem(Q, L, zf, e);
+					a.Ahp[e] = t;
+					dl[0] += t * zp[e];
+				}
+			}
+			sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
+				ms.delta = v[0] * ms.ig * ms.ig;
+				ms.dg = ms.delta * ms.ig;
+			});
+			// v(j+1) into v(j-1)'s buffer, its TI copy as the V-cycle's right-hand side,
+			// and z_p(j+1) = v_p(j+1) / BAB
+			const double ig = ms.ig, dg = ms.dg, gg = ms.gg;
+			{
+				const double2 *v = a.mv[cv];
+				double2 *vo = a.mv[1 - cv];
+				for (int A = tid; A < L.nno; A += nth) {
+					const double2 az = a.Kd[A], vc = v[A], vp = vo[A];
+					const double2 vn = make_double2(az.x * ig - dg * vc.x - gg * vp.x, az.y * ig - dg * vc.y - gg * vp.y);
+					vo[A] = vn;
+					V w;
+					w.x = narrow_to<TI>(vn.x);
+					w.y = narrow_to<TI>(vn.y);
+					Q.b[A] = w;
+				}
+			}
+			pdot = 0.0;
+			{
+				const double *p0 = a.mvp[cv];
+				double *p1 = a.mvp[1 - cv], *z1 = a.mzp[1 - cv];
+				for (int e = tid; e < L.nel; e += nth) {
+					const double vn = a.Ahp[e] * ig - dg * p0[e] - gg * p1[e], z = vn * a.ibab[e];
+					p1[e] = vn;
+					z1[e] = z;
+					pdot += z * vn;
+				}
+			}
+			sy.sync();
 		}
-		for (int e = tid; e < ne; e += nth) {
-			const double t = qt_gt_elem(Q, L, zf, e);
-			a.Ahp[e] = t;
-			dl[0] += t * zp[cv][e];
+		double dot[1];
+		qt_vcycle(sy, a.H, a.mz[1 - cv], a.mv[1 - cv], &dot[0]);
+		dot[0] += pdot;
+		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
+			const double gn2 = fmax(v[0], 0.0);
+			const double gam_next = sqrt(gn2);
+			if (it < 0) {
+				ms.gam = gam_next;
+				ms.gam_prev = 1.0;
+				ms.eta = ms.eta0 = gam_next;
+				ms.c_prev = ms.c_cur = 1.0;
+				ms.s_prev = ms.s_cur = 0.0;
+				ms.ig = 1.0 / gam_next;
+				ms.gg = gam_next;
+				ms.stop = v[0] > 0.0 ? 0 : 3;
+				return;
+			}
+			const double a0 = ms.c_cur * ms.delta - ms.c_prev * ms.s_cur * ms.gam;
+			const double a1s = a0 * a0 + gn2;
+			const double a2 = ms.s_cur * ms.delta + ms.c_prev * ms.c_cur * ms.gam;
+			const double a3 = ms.s_prev * ms.gam;
+			const double ia1 = rsqrt(a1s);
+			ms.stop = 0;
+			if (!(a1s > 0.0) || !isfinite(a1s)) {
+				ms.stop = isfinite(a1s) ? 2 : 6;
+				return;
+			}
+			const double c_next = a0 * ia1, s_next = gam_next * ia1;
+			ms.step1 = ms.step;
+			ms.k1 = ms.ig * ia1;
+			ms.k2 = a2 * ia1;
+			ms.k3 = a3 * ia1;
+			ms.step = c_next * ms.eta;
+			ms.eta = -s_next * ms.eta;
+			ms.gam_prev = ms.gam;
+			ms.gam = gam_next;
+			ms.c_prev = ms.c_cur;
+			ms.c_cur = c_next;
+			ms.s_prev = ms.s_cur;
+			ms.s_cur = s_next;
+			if (!isfinite(ms.eta))
+				ms.stop = 5;
+			else if (!(fabs(ms.eta) > rtol * ms.eta0) || !(gam_next > 0.0))
+				ms.stop = 1;
+		});
+		if (it < 0) {
+			it = 0;
+			if (ms.stop)
+				break;
+			cv = 0;
+			continue;
 		}
-		sy.reduce<1>(dl);
-		const double delta = dl[0] / (gam * gam);
-		const double ig = 1.0 / gam, dg = delta / gam, gg = gam / gam_prev;
-		for (int A = tid; A < nn; A += nth) {
-			const double2 az = a.Kd[A], v = vu[cv][A], vo = vu[1 - cv][A];
-			vu[1 - cv][A] = make_double2(az.x * ig - dg * v.x - gg * vo.x, az.y * ig - dg * v.y - gg * vo.y);
-		}
-		for (int e = tid; e < ne; e += nth)
-			vp[1 - cv][e] = a.Ahp[e] * ig - dg * vp[cv][e] - gg * vp[1 - cv][e];
-		sy.sync();
-		const double gn2 = qt_precond(sy, a, vu[1 - cv], vp[1 - cv], zu[1 - cv], zp[1 - cv]);
-		const double gam_next = sqrt(fmax(gn2, 0.0));
-		const double a0 = c_cur * delta - c_prev * s_cur * gam;
-		const double a1 = sqrt(a0 * a0 + gam_next * gam_next);
-		const double a2 = s_cur * delta + c_prev * c_cur * gam;
-		const double a3 = s_prev * gam;
-		if (!(a1 > 0.0) || !isfinite(a1)) {
-			if (!isfinite(a1) && tid == 0)
-				atomicOr(status, kStatNan);
+		const int tid = sy.tid(), nth = sy.nth();
+		const int stop = ms.stop;
+		if ((stop & 4) && tid == 0)
+			atomicOr(&a.sc->status, kStatNan);
+		if (stop & 2) {
+			if (it & 1) {   // the pending step along w(j)
+				const double s = ms.step;
+				for (int A = tid; A < L.nno; A += nth) {
+					const double2 w = a.mw[cw][A], x = a.dd[A];
+					a.dd[A] = make_double2(x.x + s * w.x, x.y + s * w.y);
+				}
+				for (int e = tid; e < L.nel; e += nth)
+					a.dpv[e] += s * a.mwp[cw][e];
+			}
 			break;
 		}
-		const double c_next = a0 / a1, s_next = gam_next / a1;
-		const double ia1 = 1.0 / a1, step = c_next * eta;
-		for (int A = tid; A < nn; A += nth) {
-			const V z = zu[cv][A];
-			const double2 wo = wu[1 - cw][A], w = wu[cw][A];
-			const double2 wn = make_double2(((double)z.x * ig - a3 * wo.x - a2 * w.x) * ia1,
-			                                ((double)z.y * ig - a3 * wo.y - a2 * w.y) * ia1);
-			wu[1 - cw][A] = wn;
-			double2 x = a.dd[A];
-			x.x += step * wn.x;
-			x.y += step * wn.y;
-			a.dd[A] = x;
+		// w(j+1) = (z~(j) - a3 w(j-1) - a2 w(j)) / a1 into w(j-1)'s buffer; the solution
+		// takes the steps of two iterations at a time, or what is pending at the end
+		const int steps = (it & 1) ? 2 : (stop || it + 1 >= maxit) ? 1 : 0;
+		{
+			const double k1 = ms.k1, k2 = ms.k2, k3 = ms.k3, s0 = ms.step, s1 = ms.step1;
+			const V *z = a.mz[cv];
+			double2 *wo = a.mw[1 - cw];
+			const double2 *wc = a.mw[cw];
+			for (int A = tid; A < L.nno; A += nth) {
+				const V zz = z[A];
+				const double2 o = wo[A], w = wc[A];
+				double2 x = make_double2(0.0, 0.0);
+				if (steps > 0)
+					x = a.dd[A];
+				const double2 wn = make_double2(widen(zz.x) * k1 - k3 * o.x - k2 * w.x,
+				                                widen(zz.y) * k1 - k3 * o.y - k2 * w.y);
+				wo[A] = wn;
+				if (steps > 1) {
+					x.x += s1 * w.x;
+					x.y += s1 * w.y;
+				}
+				if (steps > 0)
+					a.dd[A] = make_double2(x.x + s0 * wn.x, x.y + s0 * wn.y);
+			}
+			const double *zp = a.mzp[cv], *pc = a.mwp[cw];
+			double *po = a.mwp[1 - cw];
+			for (int e = tid; e < L.nel; e += nth) {
+				const double w = pc[e];
+				double x = steps > 0 ? a.dpv[e] : 0.0;
+				const double wn = zp[e] * k1 - k3 * po[e] - k2 * w;
+				po[e] = wn;
+				if (steps > 1)
+					x += s1 * w;
+				if (steps > 0)
+					a.dpv[e] = x + s0 * wn;
+			}
 		}
-		for (int e = tid; e < ne; e += nth) {
-			const double wn = (zp[cv][e] * ig - a3 * wp[1 - cw][e] - a2 * wp[cw][e]) * ia1;
-			wp[1 - cw][e] = wn;
-			a.dpv[e] += step * wn;
-		}
-		eta = -s_next * eta;
 		it++;
 		cv = 1 - cv;
 		cw = 1 - cw;
-		gam_prev = gam;
-		gam = gam_next;
-		c_prev = c_cur;
-		c_cur = c_next;
-		s_prev = s_cur;
-		s_cur = s_next;
-		if (!isfinite(eta)) {
-			if (tid == 0)
-				atomicOr(status, kStatNan);
+		if (stop)
 			break;
+		if (threadIdx.x == 0) {   // for the next step; read after the next reduction's broadcast
+			ms.ig = 1.0 / ms.gam;
+			ms.gg = ms.gam / ms.gam_prev;
 		}
-		if (!(fabs(eta) > rtol * eta0) || !(gam > 0.0))
-			break;
-		sy.sync();
+		// no barrier here: the next operator pass reads z(j+1) and z_p(j+1), complete
+		// since the reduction, and writes none of the vectors the updates above read
 	}
 	sy.sync();
+	team = sy;
 	return it;
 }
 
@@ -640,6 +833,8 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 	const DevLevel &L = a.L;
 	int *status = &a.sc->status;
 
+	for (int e = tid; e < L.nel; e += nth)
+		a.ibab[e] = 1.0 / a.bab[e];
 	// -- per step: every level's reduced operator C^T K C in TI, and its diagonal
 	for (int l = 0; l < H.nlev; l++) {
 		const QtLevel<TI> &Q = H.lv[l];
@@ -700,7 +895,7 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 		// far from the target a pass reduces by 1e-2, close to it by what is
 		// left (factor 2 margin), not below outer_rtol
 		const double prt = res > 1e4 * a.rtol ? 1e-2 : fmax(a.outer_rtol, 0.5 * a.rtol / res);
-		const int it = qt_minres(sy, a, prt, a.max_outer, status);
+		const int it = qt_minres(sy, a, prt, a.max_outer);
 		minres_total += it;
 		vcycles += it + 1;
 		for (int A = tid; A < L.nno; A += nth) {
@@ -742,14 +937,18 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 	}
 }
 
-// One refined model on the whole cooperative grid.
+// One refined model on the whole cooperative grid, or on one cluster.
 template <class TI>
 __global__ void __launch_bounds__(kBlock) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
 {
 	__shared__ QtArgs<TI> sa;
 	load_args(sa, a);
-	Sync sy = Sync::of(SYNC_GRID, a.red.part, blockIdx.x, gridDim.x);
+	__shared__ double cpart[2 * kRedWidth];
+	Sync sy = sa.cluster ? Sync::of(SYNC_CLUSTER, cpart, blockIdx.x, gridDim.x)
+	                     : Sync::of(SYNC_GRID, sa.red.part, blockIdx.x, gridDim.x);
 	qt_solve<TI>(sa, sy);
+	if (sa.cluster)
+		cg::this_cluster().sync();   // no block leaves while another reads its partials
 }
 
 // A batch of independent refined models, launched with clusters of `cs`

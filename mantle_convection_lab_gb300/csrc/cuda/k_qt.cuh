@@ -69,16 +69,18 @@ struct QtArgs {
 	QtHier<TI> H;
 	const double2 *F;
 	const double *bab;
+	double *ibab;                           // 1/bab, formed once per solve
 	double2 *d, *V;
 	double *p;
 	// FP64 refinement and MINRES vectors
-	double2 *R, *Kd, *dd, *u1, *mv[2], *mw[2];
+	double2 *R, *Kd, *dd, *mv[2], *mw[2];
 	double *Rc, *dpv, *Ahp, *mvp[2], *mzp[2], *mwp[2];
-	typename Q2T<TI>::t *mz[2], *kz;
+	typename Q2T<TI>::t *mz[2];
 	GridRed red;
 	StepScalars *sc;
 	double rtol, outer_rtol;
 	int max_refine, max_outer;
+	int cluster;                            // run on one cluster (SYNC_CLUSTER) instead of a cooperative grid
 };
 
 void *qt_kernel(int fp64);

@@ -102,6 +102,7 @@ struct mclg_ctx {
 	double *tmpA, *tmpB;
 	// converged solvers on uniform meshes (precision 1 and 2)
 	int coop_mg;
+	int qt_one_cluster;          // a refined model's blocks are one cluster instead of a cooperative grid
 	int uzawa_cluster;           // the replica's solve runs as one cluster
 	int mg_one_cluster;          // its blocks are one cluster instead of a cooperative grid
 	double remesh_ms[5];   // the last remesh: numbering, lists, state, wait, carry (host ms)
@@ -371,6 +372,18 @@ static void mg_team(mclg_ctx *c, void *kern)
 	c->mg_one_cluster = N0 <= (c->cfg.precision == 2 ? kOneClusterN64 : kOneClusterN32) &&
 	                    max_clusters(kern, kOneCluster, kBlock) >= 1;
 	c->coop_mg = c->mg_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, 1 << 30);
+}
+
+// The blocks that solve one refined model.  Up to kOneClusterNodes nodes one
+// cluster, whose barriers take 0.2 us instead of a grid's 1.2 (54 against 65 us
+// per MINRES iteration at 1347 nodes, 64 against 79 at 2441, 87 against 77 at
+// 5125); up to kSpreadNodes four times the blocks its nodes fill, so that its
+// FP64 work uses more SMs (89 against 93 us at 8847 nodes, 95 against 89 at 19977).
+static void qt_team(mclg_ctx *c, void *kern, int nn)
+{
+	constexpr int kOneCluster = 16, kOneClusterNodes = 4096, kSpreadNodes = 12288;
+	c->qt_one_cluster = nn <= kOneClusterNodes && max_clusters(kern, kOneCluster, kBlock) >= 1;
+	c->coop_qt = c->qt_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, nn <= kSpreadNodes ? 4 * nn : nn);
 }
 
 // ---- converged solvers: hierarchy of the uniform mesh -------------------------
@@ -996,7 +1009,7 @@ static int qt_setup(mclg_ctx *c, QtArgs<TI> &a, Prebuilt *pre)
 	CK(dev_zeros(c, &a.R, nn));
 	CK(dev_zeros(c, &a.Kd, nn));
 	CK(dev_zeros(c, &a.dd, nn));
-	CK(dev_zeros(c, &a.u1, nn));
+	CK(dev_zeros(c, &a.ibab, ne));
 	CK(dev_zeros(c, &a.Rc, ne));
 	CK(dev_zeros(c, &a.dpv, ne));
 	CK(dev_zeros(c, &a.Ahp, ne));
@@ -1110,14 +1123,14 @@ static int launch_stokes_qt(mclg_ctx *c)
 	int rc = stokes_qt_prepare(c);
 	if (rc)
 		return rc;
-	const dim3 grid(solver_grid(c, c->coop_qt));
-	if (c->cfg.precision == 2) {
-		void *args[] = {&c->qtd};
-		CK(cudaLaunchCooperativeKernel(qt_kernel(1), grid, dim3(kBlock), args, 0, c->st));
-	} else {
-		void *args[] = {&c->qtf};
-		CK(cudaLaunchCooperativeKernel(qt_kernel(0), grid, dim3(kBlock), args, 0, c->st));
-	}
+	const bool one = c->qt_one_cluster != 0;
+	c->qtd.cluster = c->qtf.cluster = one;
+	void *args[] = {c->cfg.precision == 2 ? (void *)&c->qtd : (void *)&c->qtf};
+	void *kern = qt_kernel(c->cfg.precision == 2);
+	if (one)
+		CK(launch_cluster(kern, c->coop_qt, kBlock, args, c->st));
+	else
+		CK(cudaLaunchCooperativeKernel(kern, dim3(solver_grid(c, c->coop_qt)), dim3(kBlock), args, 0, c->st));
 	c->launches++;
 	stokes_qt_finish(c);
 	return MCLG_OK;
@@ -1520,7 +1533,7 @@ static int create_impl(mclg_ctx **out, const mclg_config *cfg, const int *leaves
 	if (cfg->precision != 0 && !c->mesh.uniform) {
 		rc = cfg->precision == 2 ? qt_setup<double>(c, c->qtd, pre) : qt_setup<float>(c, c->qtf, pre);
 		if (rc == MCLG_OK)
-			c->coop_qt = coop_blocks(qt_kernel(cfg->precision == 2), c->num_sms, (int)nn);
+			qt_team(c, qt_kernel(cfg->precision == 2), (int)nn);
 		if (rc == MCLG_OK && c->coop_qt < 1) {
 			mclg_set_error("cooperative occupancy query failed");
 			rc = MCLG_CUDA_ERROR;
