@@ -46,8 +46,7 @@ namespace mclg {
 
 constexpr int kTile = 16;
 constexpr int kHalo = kTile + 2;
-constexpr int kChunk = 16;
-constexpr int kWgradBlocks = 304;
+constexpr int kWgradBlocks = 456;   // three resident per SM at 32 channels (74 KB of shared memory each)
 
 static int pad_channels(int c)
 {
@@ -98,21 +97,32 @@ __global__ void __launch_bounds__(256) k_conv3x3(const float *__restrict__ in, i
 	__shared__ __align__(16) __nv_bfloat16 s_in[kHalo * kHalo * SI];
 	__shared__ __align__(16) __nv_bfloat16 s_w[9 * CO * SI];
 	const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, b = blockIdx.z;
-	for (int i = threadIdx.x; i < CI * kHalo * kHalo; i += blockDim.x) {
-		const int c = i / (kHalo * kHalo), r = i - c * kHalo * kHalo;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	// A warp stages 8 pixels by 8 channels at a time, two channels to a lane: 32-byte
+	// segments from memory and, like the fragment loads, 32 different banks (a
+	// channel at a time over 32 pixels wrote two bytes with 4-way conflicts).
+	constexpr int kPixGroups = (kHalo * kHalo + 7) / 8;
+#pragma unroll 4
+	for (int i = warp; i < kPixGroups * (CI / 8); i += 8) {
+		const int pg = i % kPixGroups, c = (i / kPixGroups) * 8 + 2 * (lane & 3), r = pg * 8 + (lane >> 2);
 		const int yy = r / kHalo, xx = r - yy * kHalo;
 		const int gy = y0 + yy - 1, gx = x0 + xx - 1;
-		float v = 0.f;
-		if (c < Cin && gy >= 0 && gy < H && gx >= 0 && gx < W)
-			v = in[((size_t)(b * Cin + c) * H + gy) * W + gx];
-		s_in[r * SI + c] = __float2bfloat16_rn(v);
+		float v0 = 0.f, v1 = 0.f;
+		if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
+			const float *src = in + ((size_t)(b * Cin + c) * H + gy) * W + gx;
+			if (c < Cin)
+				v0 = src[0];
+			if (c + 1 < Cin)
+				v1 = src[(size_t)H * W];
+		}
+		if (r < kHalo * kHalo)
+			*reinterpret_cast<__nv_bfloat162 *>(s_in + r * SI + c) = __floats2bfloat162_rn(v0, v1);
 	}
-	for (int i = threadIdx.x; i < 9 * CO * CI; i += blockDim.x) {
-		const int kc = i / CI, c = i - kc * CI;
-		s_w[kc * SI + c] = w[i];
+	for (int i = threadIdx.x; i < 9 * CO * CI / 8; i += blockDim.x) {
+		const int kc = i / (CI / 8), c = (i - kc * (CI / 8)) * 8;
+		*reinterpret_cast<uint4 *>(s_w + kc * SI + c) = reinterpret_cast<const uint4 *>(w)[i];
 	}
 	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int g = lane >> 2, t2 = (lane & 3) * 2;
 	float acc[2][NT][4];
 #pragma unroll
@@ -177,39 +187,55 @@ __global__ void __launch_bounds__(256) k_conv3x3(const float *__restrict__ in, i
 // ---- weight gradient: per-block partials ------------------------------------
 // part[blk][(c*9 + k)*CO + o] = sum over the block's pixels of g[b][o][p] * in[b][c][p + k - 1],
 // part[blk][Cin*9*CO + o]    = sum of g[b][o][p].
+// A thread owns one input channel, four output channels and all nine taps: per
+// pixel three new inputs (the window slides along the row) and one float4 of
+// gradients serve 36 multiply-adds, which bound it (FP32; shared memory needs 7
+// of the 9 cycles).  One tap and four output channels per unit needed two loads
+// for four multiply-adds.  Where the channels leave threads over, the tile's
+// rows are split among slices of them.
 template <int CO>
 __global__ void __launch_bounds__(256) k_conv3x3_wgrad(const float *__restrict__ in, int Cin,
                                                        const float *__restrict__ g, int Cout, int H, int W, int B,
                                                        float *__restrict__ part)
 {
 	extern __shared__ __align__(16) float smw[];
-	float *s_in = smw;                              // [Cin][kHalo*kHalo]
-	float *s_g = smw + Cin * kHalo * kHalo;         // [256][CO]
+	float *s_g = smw;                                // [256][CO]
+	float *s_in = smw + kTile * kTile * CO;          // [Cin][kHalo*kHalo]
 	constexpr int G = CO / 4;                        // float4 groups of output channels
-	constexpr int U = (32 * 9 * G + 255) / 256;      // work units per thread (Cin <= 32)
 	const int tilesx = (W + kTile - 1) / kTile, tilesy = (H + kTile - 1) / kTile;
 	const int nitems = tilesx * tilesy * B;
-	const int nunits = Cin * 9 * G;
-	float acc[U][4];
-	float bacc = 0.f;
+	const int nunits = Cin * G;
+	int slices = 1;
+	while (2 * slices * nunits <= 256 && slices < kTile)
+		slices *= 2;
+	const int slice = threadIdx.x / nunits, unit = threadIdx.x - slice * nunits;
+	const bool on = slice < slices;
+	const int ci = unit / G, grp = unit - ci * G, rows = kTile / slices;
+	// the bias: 256/CO threads per output channel, a share of the pixels each
+	const int bo = threadIdx.x % CO, bseg = threadIdx.x / CO;
+	constexpr int BPX = kTile * kTile / (256 / CO);
+	float acc[9][4], bacc = 0.f;
 #pragma unroll
-	for (int u = 0; u < U; u++)
-		acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.f;
+	for (int k = 0; k < 9; k++)
+		acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.f;
 	for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
 		const int b = item / (tilesx * tilesy), t = item - b * tilesx * tilesy;
 		const int y0 = (t / tilesx) * kTile, x0 = (t - (t / tilesx) * tilesx) * kTile;
 		__syncthreads();
-		for (int i = threadIdx.x; i < Cin * kHalo * kHalo; i += blockDim.x) {
-			const int ci = i / (kHalo * kHalo), r = i - ci * kHalo * kHalo;
+#pragma unroll 4
+		for (int i = threadIdx.x; i < Cin * kHalo * kHalo; i += 256) {
+			const int c = i / (kHalo * kHalo), r = i - c * kHalo * kHalo;
 			const int yy = r / kHalo, xx = r - yy * kHalo;
 			const int gy = y0 + yy - 1, gx = x0 + xx - 1;
 			float v = 0.f;
 			if (gy >= 0 && gy < H && gx >= 0 && gx < W)
-				v = in[((size_t)(b * Cin + ci) * H + gy) * W + gx];
+				v = in[((size_t)(b * Cin + c) * H + gy) * W + gx];
 			s_in[i] = v;
 		}
-		for (int i = threadIdx.x; i < kTile * kTile * CO; i += blockDim.x) {
-			const int o = i / (kTile * kTile), px = i - o * kTile * kTile;
+#pragma unroll 4
+		for (int i = threadIdx.x; i < kTile * kTile * CO; i += 256) {
+			// eight pixels by four channels to a warp: 32-byte segments, 16 of 32 banks
+			const int lane = i & 31, q = i >> 5, og = q % G, px = (q / G) * 8 + (lane >> 2), o = og * 4 + (lane & 3);
 			const int y = y0 + px / kTile, x = x0 + (px & (kTile - 1));
 			float v = 0.f;
 			if (o < Cout && y < H && x < W)
@@ -217,68 +243,102 @@ __global__ void __launch_bounds__(256) k_conv3x3_wgrad(const float *__restrict__
 			s_g[px * CO + o] = v;
 		}
 		__syncthreads();
+		if (on) {
+			const float *sx = s_in + ci * kHalo * kHalo;
+			for (int py = slice * rows; py < (slice + 1) * rows; py++) {
+				const float *r0 = sx + py * kHalo;
+				const float4 *sg = reinterpret_cast<const float4 *>(s_g) + (size_t)py * kTile * G + grp;
+				float w[3][3];
 #pragma unroll
-		for (int u = 0; u < U; u++) {
-			const int unit = threadIdx.x + 256 * u;
-			if (unit < nunits) {
-				const int pair = unit / G, grp = unit - pair * G;
-				const int ci = pair / 9, k = pair - ci * 9, ky = k / 3, kx = k - 3 * ky;
-				const float *sx = s_in + ci * kHalo * kHalo + ky * kHalo + kx;
-				const float4 *sg = reinterpret_cast<const float4 *>(s_g) + grp;
-				float a0 = acc[u][0], a1 = acc[u][1], a2 = acc[u][2], a3 = acc[u][3];
-				for (int py = 0; py < kTile; py++)
-#pragma unroll 4
-					for (int px = 0; px < kTile; px++) {
-						const float xv = sx[py * kHalo + px];
-						const float4 gv = sg[(py * kTile + px) * G];
-						a0 = fmaf(gv.x, xv, a0);
-						a1 = fmaf(gv.y, xv, a1);
-						a2 = fmaf(gv.z, xv, a2);
-						a3 = fmaf(gv.w, xv, a3);
+				for (int ky = 0; ky < 3; ky++) {
+					w[ky][0] = r0[ky * kHalo];
+					w[ky][1] = r0[ky * kHalo + 1];
+				}
+#pragma unroll
+				for (int px = 0; px < kTile; px++) {
+					const float4 gv = sg[px * G];
+#pragma unroll
+					for (int ky = 0; ky < 3; ky++) {
+						w[ky][(px + 2) % 3] = r0[ky * kHalo + px + 2];
+#pragma unroll
+						for (int kx = 0; kx < 3; kx++) {
+							const float xv = w[ky][(px + kx) % 3];
+							float *a = acc[ky * 3 + kx];
+							a[0] = fmaf(gv.x, xv, a[0]);
+							a[1] = fmaf(gv.y, xv, a[1]);
+							a[2] = fmaf(gv.z, xv, a[2]);
+							a[3] = fmaf(gv.w, xv, a[3]);
+						}
 					}
-				acc[u][0] = a0;
-				acc[u][1] = a1;
-				acc[u][2] = a2;
-				acc[u][3] = a3;
+				}
 			}
 		}
-		if (threadIdx.x < Cout)
-			for (int px = 0; px < kTile * kTile; px++)
-				bacc += s_g[px * CO + threadIdx.x];
+		for (int px = bseg * BPX; px < (bseg + 1) * BPX; px++)
+			bacc += s_g[px * CO + bo];
 	}
+	// the slices' sums in slice order, through shared memory
 	float *pb = part + (size_t)blockIdx.x * (Cin * 9 * CO + CO);
+	float4 *sh = reinterpret_cast<float4 *>(smw);
+	for (int sl = 1; sl < slices; sl++) {
+		__syncthreads();
+		if (on && slice == sl)
 #pragma unroll
-	for (int u = 0; u < U; u++) {
-		const int unit = threadIdx.x + 256 * u;
-		if (unit < nunits) {
-			const int pair = unit / G, grp = unit - pair * G;
+			for (int k = 0; k < 9; k++)
+				sh[unit * 9 + k] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+		__syncthreads();
+		if (slice == 0)
 #pragma unroll
-			for (int q = 0; q < 4; q++)
-				pb[pair * CO + grp * 4 + q] = acc[u][q];
-		}
+			for (int k = 0; k < 9; k++) {
+				const float4 v = sh[unit * 9 + k];
+				acc[k][0] += v.x;
+				acc[k][1] += v.y;
+				acc[k][2] += v.z;
+				acc[k][3] += v.w;
+			}
 	}
-	if (threadIdx.x < CO)
-		pb[Cin * 9 * CO + threadIdx.x] = threadIdx.x < Cout ? bacc : 0.f;
+	if (slice == 0)
+#pragma unroll
+		for (int k = 0; k < 9; k++)
+			*reinterpret_cast<float4 *>(pb + (ci * 9 + k) * CO + grp * 4) =
+				make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+	__syncthreads();
+	smw[threadIdx.x] = bacc;
+	__syncthreads();
+	if (threadIdx.x < CO) {
+		float v = 0.f;
+		for (int q = 0; q < 256 / CO; q++)
+			v += smw[q * CO + threadIdx.x];
+		pb[Cin * 9 * CO + threadIdx.x] = threadIdx.x < Cout ? v : 0.f;
+	}
 }
 
-// Fixed-order sum of the partials into the flat gradient W[o][c][k], b[o].
-__global__ void k_wgrad_reduce(const float *__restrict__ part, int nblk, int Cin, int Cout, int CO,
-                               float *__restrict__ grad)
+// Fixed-order sum of the partials into the flat gradient W[o][c][k], b[o]: a
+// block sums 32 entries, each warp an eighth of the partials (coalesced), the
+// eighths in order.
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nblk, int Cin, int Cout,
+                                                      int CO, float *__restrict__ grad)
 {
-	const int nw = Cout * Cin * 9, n = nw + Cout, stride = Cin * 9 * CO + CO;
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		int src;
-		if (i < nw) {
-			const int o = i / (Cin * 9), r = i - o * Cin * 9;   // r = c*9 + k
-			src = r * CO + o;
-		} else {
-			src = Cin * 9 * CO + (i - nw);
-		}
-		float s = 0.f;
-		for (int bk = 0; bk < nblk; bk++)
+	__shared__ float sh[8][32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int stride = Cin * 9 * CO + CO, src = blockIdx.x * 32 + lane;
+	float s = 0.f;
+	if (src < stride) {
+		const int per = (nblk + 7) / 8, b1 = min((w + 1) * per, nblk);
+#pragma unroll 8
+		for (int bk = w * per; bk < b1; bk++)
 			s += part[(size_t)bk * stride + src];
-		grad[i] = s;
 	}
+	sh[w][lane] = s;
+	__syncthreads();
+	if (w != 0 || src >= stride)
+		return;
+	s = sh[0][lane];
+#pragma unroll
+	for (int q = 1; q < 8; q++)
+		s += sh[q][lane];
+	const int r = src / CO, o = src - r * CO;   // r = c*9 + k, or the bias
+	if (o < Cout)
+		grad[r < Cin * 9 ? o * Cin * 9 + r : Cout * Cin * 9 + o] = s;
 }
 
 // ---- loss, optimiser, weight packing ------------------------------------------
@@ -477,8 +537,7 @@ static int cnn_backward_dev(mclg_cnn *net, CnnWork &w, const float *gy, float *g
 			net->part_cap = need;
 		}
 		CKC(wgrad_launch(w.act[l], Cin, gz, Cout, CO, w.B, w.H, w.W, net->part, nblk, st));
-		const int n = Cout * Cin * 9 + Cout;
-		k_wgrad_reduce<<<(n + 255) / 256, 256, 0, st>>>(net->part, nblk, Cin, Cout, CO, net->grad + net->off[l]);
+		k_wgrad_reduce<<<(Cin * 9 * CO + CO + 31) / 32, 256, 0, st>>>(net->part, nblk, Cin, Cout, CO, net->grad + net->off[l]);
 		if (l > 0) {
 			// d loss / d z_{l-1} = (W_l^T g_l) masked by ReLU'(z_{l-1}) = (act_l > 0)
 			float *gin = bufs[l & 1];
