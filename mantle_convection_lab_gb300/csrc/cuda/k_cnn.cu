@@ -20,6 +20,7 @@
 // (per-block partials, then a fixed-order sum over blocks).
 #include <cuda_bf16.h>
 #include <math.h>
+#include <pthread.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -40,6 +41,12 @@ struct mclg_cnn {
 	float *part;                            // weight-gradient partials
 	size_t part_cap;
 	cudaStream_t st;
+	// device buffers of mclg_cnn_forward and mclg_cnn_gradient, kept for the next
+	// call at the largest size asked for and freed with the network (allocating
+	// and freeing them took a third of a call); mu: one such call at a time
+	char *pool;
+	size_t pool_cap;
+	pthread_mutex_t mu;
 };
 
 namespace mclg {
@@ -366,14 +373,18 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
 		part[blockIdx.x] = sh[0];
 }
 
+// (one warp: each lane a run of the partials in order, then the lanes)
 __global__ void k_sum_partials(const double *__restrict__ part, int n, double scale, double *__restrict__ out)
 {
-	if (threadIdx.x == 0 && blockIdx.x == 0) {
-		double s = 0.0;
-		for (int i = 0; i < n; i++)
-			s += part[i];
+	const int per = (n + 31) / 32, i1 = min((int)(threadIdx.x + 1) * per, n);
+	double s = 0.0;
+	for (int i = threadIdx.x * per; i < i1; i++)
+		s += part[i];
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		s += __shfl_xor_sync(0xffffffffu, s, o);
+	if (threadIdx.x == 0)
 		out[0] = s * scale;
-	}
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
@@ -813,6 +824,7 @@ int mclg_cnn_create(mclg_cnn **out, int cin, int width, int depth, int cout, uns
 	mclg_cnn *n = (mclg_cnn *)calloc(1, sizeof(mclg_cnn));
 	if (n == NULL)
 		return MCLG_BAD_INPUT;
+	pthread_mutex_init(&n->mu, NULL);
 	n->nl = depth;
 	size_t off = 0;
 	for (int l = 0; l < depth; l++) {
@@ -869,6 +881,8 @@ void mclg_cnn_destroy(mclg_cnn *n)
 	cudaFree(n->m);
 	cudaFree(n->v);
 	cudaFree(n->part);
+	cudaFree(n->pool);
+	pthread_mutex_destroy(&n->mu);
 	for (int l = 0; l < kCnnMaxLayers; l++) {
 		cudaFree(n->wf[l]);
 		cudaFree(n->wb[l]);
@@ -931,6 +945,53 @@ static int check_grid(const mclg_cnn *n, int batch, int h, int w)
 	return MCLG_OK;
 }
 
+}   // extern "C"
+
+// The call's buffers, carved from the network's pool (256-byte aligned).
+namespace {
+struct Pool {
+	mclg_cnn *n;
+	size_t used = 0;
+	bool carve;   // false: count the bytes; true: hand out addresses
+	template <class T>
+	T *get(size_t count)
+	{
+		T *p = carve ? reinterpret_cast<T *>(n->pool + used) : nullptr;
+		used += (count * sizeof(T) + 255) & ~size_t(255);
+		return p;
+	}
+	// the activations of a batch, as cnn_work_ensure makes them
+	void acts(CnnWork &w, int B, int H, int W)
+	{
+		for (int l = 0; l < n->nl; l++)
+			w.act[l + 1] = get<float>((size_t)B * n->cout[l] * H * W);
+		w.B = B;
+		w.H = H;
+		w.W = W;
+	}
+};
+struct Lock {
+	pthread_mutex_t *m;
+	explicit Lock(pthread_mutex_t *mu) : m(mu) { pthread_mutex_lock(m); }
+	~Lock() { pthread_mutex_unlock(m); }
+};
+}  // namespace
+
+static cudaError_t pool_reserve(mclg_cnn *n, size_t bytes)
+{
+	if (bytes <= n->pool_cap)
+		return cudaSuccess;
+	cudaFree(n->pool);
+	n->pool = NULL;
+	n->pool_cap = 0;
+	const cudaError_t e = cudaMalloc((void **)&n->pool, bytes);
+	if (e == cudaSuccess)
+		n->pool_cap = bytes;
+	return e;
+}
+
+extern "C" {
+
 int mclg_cnn_forward(mclg_cnn *n, const float *x, int batch, int h, int w, float *y)
 {
 	int rc = check_grid(n, batch, h, w);
@@ -938,22 +999,24 @@ int mclg_cnn_forward(mclg_cnn *n, const float *x, int batch, int h, int w, float
 		return rc;
 	if (x == NULL || y == NULL)
 		return MCLG_BAD_INPUT;
+	Lock lock(&n->mu);
 	CnnWork wk;
 	memset(&wk, 0, sizeof wk);
 	float *dx = NULL;
 	const size_t nx = (size_t)batch * n->cin[0] * h * w, ny = (size_t)batch * n->cout[n->nl - 1] * h * w;
-	cudaError_t e = cudaMalloc((void **)&dx, nx * sizeof(float));
-	if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, nx * sizeof(float), cudaMemcpyHostToDevice, n->st);
-	if (e == cudaSuccess) rc = cnn_work_ensure(n, wk, batch, h, w);
-	if (e == cudaSuccess && rc == MCLG_OK) rc = cnn_forward_dev(n, wk, dx, n->st);
-	if (e == cudaSuccess && rc == MCLG_OK)
-		e = cudaMemcpyAsync(y, wk.act[n->nl], ny * sizeof(float), cudaMemcpyDeviceToHost, n->st);
-	if (e == cudaSuccess && rc == MCLG_OK) e = cudaStreamSynchronize(n->st);
-	cudaFree(dx);
-	cnn_work_free(wk);
-	if (e != cudaSuccess)
-		return cnn_fail(e, "mclg_cnn_forward");
-	return rc;
+	for (int pass = 0; pass < 2; pass++) {
+		Pool p{n, 0, pass == 1};
+		dx = p.get<float>(nx);
+		p.acts(wk, batch, h, w);
+		if (pass == 0)
+			CKC(pool_reserve(n, p.used));
+	}
+	CKC(cudaMemcpyAsync(dx, x, nx * sizeof(float), cudaMemcpyHostToDevice, n->st));
+	if ((rc = cnn_forward_dev(n, wk, dx, n->st)))
+		return rc;
+	CKC(cudaMemcpyAsync(y, wk.act[n->nl], ny * sizeof(float), cudaMemcpyDeviceToHost, n->st));
+	CKC(cudaStreamSynchronize(n->st));
+	return MCLG_OK;
 }
 
 // Loss and gradient of the mean squared error for one batch (host buffers).
@@ -967,6 +1030,7 @@ int mclg_cnn_gradient(mclg_cnn *n, const float *x, const float *target, int batc
 		mclg_set_error("gradient buffer has %zu entries, the network %zu", count, n->nparam);
 		return MCLG_BAD_INPUT;
 	}
+	Lock lock(&n->mu);
 	CnnWork wk;
 	memset(&wk, 0, sizeof wk);
 	const size_t nx = (size_t)batch * n->cin[0] * h * w, ny = (size_t)batch * n->cout[n->nl - 1] * h * w;
@@ -977,37 +1041,32 @@ int mclg_cnn_gradient(mclg_cnn *n, const float *x, const float *target, int batc
 	float *dx = NULL, *dt = NULL, *gy = NULL, *g0 = NULL, *g1 = NULL;
 	double *part = NULL, *dl = NULL;
 	const int nb = 256;
-	cudaError_t e = cudaMalloc((void **)&dx, nx * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc((void **)&dt, ny * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc((void **)&gy, ny * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc((void **)&g0, ng * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc((void **)&g1, ng * sizeof(float));
-	if (e == cudaSuccess) e = cudaMalloc((void **)&part, (nb + 1) * sizeof(double));
-	dl = part + nb;
-	if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, nx * sizeof(float), cudaMemcpyHostToDevice, n->st);
-	if (e == cudaSuccess) e = cudaMemcpyAsync(dt, target, ny * sizeof(float), cudaMemcpyHostToDevice, n->st);
-	if (e == cudaSuccess) rc = cnn_work_ensure(n, wk, batch, h, w);
-	if (e == cudaSuccess && rc == MCLG_OK) rc = cnn_forward_dev(n, wk, dx, n->st);
-	if (e == cudaSuccess && rc == MCLG_OK) {
-		k_mse<<<nb, 256, 0, n->st>>>(wk.act[n->nl], dt, ny, gy, part);
-		k_sum_partials<<<1, 32, 0, n->st>>>(part, nb, 1.0 / (double)ny, dl);
-		rc = cnn_backward_dev(n, wk, gy, g0, g1, n->st);
+	for (int pass = 0; pass < 2; pass++) {
+		Pool p{n, 0, pass == 1};
+		dx = p.get<float>(nx);
+		dt = p.get<float>(ny);
+		gy = p.get<float>(ny);
+		g0 = p.get<float>(ng);
+		g1 = p.get<float>(ng);
+		part = p.get<double>(nb);
+		dl = p.get<double>(1);
+		p.acts(wk, batch, h, w);
+		if (pass == 0)
+			CKC(pool_reserve(n, p.used));
 	}
-	if (e == cudaSuccess && rc == MCLG_OK)
-		e = cudaMemcpyAsync(grad, n->grad, count * sizeof(float), cudaMemcpyDeviceToHost, n->st);
-	if (e == cudaSuccess && rc == MCLG_OK && loss)
-		e = cudaMemcpyAsync(loss, dl, sizeof(double), cudaMemcpyDeviceToHost, n->st);
-	if (e == cudaSuccess && rc == MCLG_OK) e = cudaStreamSynchronize(n->st);
-	cudaFree(dx);
-	cudaFree(dt);
-	cudaFree(gy);
-	cudaFree(g0);
-	cudaFree(g1);
-	cudaFree(part);
-	cnn_work_free(wk);
-	if (e != cudaSuccess)
-		return cnn_fail(e, "mclg_cnn_gradient");
-	return rc;
+	CKC(cudaMemcpyAsync(dx, x, nx * sizeof(float), cudaMemcpyHostToDevice, n->st));
+	CKC(cudaMemcpyAsync(dt, target, ny * sizeof(float), cudaMemcpyHostToDevice, n->st));
+	if ((rc = cnn_forward_dev(n, wk, dx, n->st)))
+		return rc;
+	k_mse<<<nb, 256, 0, n->st>>>(wk.act[n->nl], dt, ny, gy, part);
+	k_sum_partials<<<1, 32, 0, n->st>>>(part, nb, 1.0 / (double)ny, dl);
+	if ((rc = cnn_backward_dev(n, wk, gy, g0, g1, n->st)))
+		return rc;
+	CKC(cudaMemcpyAsync(grad, n->grad, count * sizeof(float), cudaMemcpyDeviceToHost, n->st));
+	if (loss)
+		CKC(cudaMemcpyAsync(loss, dl, sizeof(double), cudaMemcpyDeviceToHost, n->st));
+	CKC(cudaStreamSynchronize(n->st));
+	return MCLG_OK;
 }
 
 // Adam on the mean squared error over a device-resident data set: samples
