@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kBlock) k_uzawa(UzawaArgs a)
 // clock and SM, so the recurrences' divisions are left to one thread of a block
 // (in k_uzawa every thread forms them) and groups of 32 nodes are dealt over the
 // blocks.  Measured per CG iteration: 15.6 us in k_uzawa at 16^2 (2 blocks) and
-// 15.8 at 64^2 (17 blocks); here 8.0 and 10.2.
+// 15.8 at 64^2 (17 blocks); here 7.5 and 9.3.
 //
 // Sums are formed in k_uzawa's order (butterflies over 32 consecutive nodes, the
 // 8 groups of 256, then the 256s), so that the iterates are k_uzawa's: at a
@@ -514,6 +514,12 @@ __global__ void __launch_bounds__(kBlock) k_uzawa(UzawaArgs a)
 constexpr int kUzCluster = 16, kUzWarps = 9, kUzBlock = 32 * kUzWarps;
 constexpr int kUzGroups = kUzCluster * kUzWarps;   // groups of 32: 4608 nodes, 64^2 has 4225
 constexpr int kUzRow = 9;                          // blocks per row
+
+// The larger of two values >= 0 (NaN: either) off the FP64 pipe: their bits order as they do.
+__device__ __forceinline__ double larger(double a, double b)
+{
+	return __double_as_longlong(a) < __double_as_longlong(b) ? b : a;
+}
 
 struct UzTeam {
 	double *part;   // this block's [2][kRedWidth][kUzWarps] group sums (shared memory)
@@ -530,7 +536,13 @@ struct UzTeam {
 		double *mine = part + flip * kRedWidth * kUzWarps;
 #pragma unroll
 		for (int k = 0; k < NV; k++) {
-			const double t = ((MAX >> k) & 1u) ? warp_max(v[k]) : warp_sum(v[k]);
+			double t = v[k];
+			if ((MAX >> k) & 1u)
+#pragma unroll
+				for (int o = 16; o > 0; o >>= 1)
+					t = larger(t, __shfl_xor_sync(0xffffffffu, t, o));
+			else
+				t = warp_sum(t);
 			if (lane == 0)
 				mine[k * kUzWarps + w] = t;
 		}
@@ -544,7 +556,7 @@ struct UzTeam {
 #pragma unroll
 				for (int o = 4; o > 0; o >>= 1) {
 					const double u = __shfl_xor_sync(0xffffffffu, t, o);
-					t = ((MAX >> k) & 1u) ? fmax(t, u) : t + u;
+					t = ((MAX >> k) & 1u) ? larger(t, u) : t + u;
 				}
 				if ((lane & 7) == 0 && g < kUzGroups)
 					mid[k * kMid + g / 8] = t;
@@ -556,7 +568,13 @@ struct UzTeam {
 #pragma unroll
 			for (int k = 0; k < NV; k++) {
 				const double u = lane < (ngroups + 7) / 8 ? mid[k * kMid + lane] : 0.0;
-				t[k] = ((MAX >> k) & 1u) ? warp_max(u) : warp_sum(u);
+				t[k] = u;
+				if ((MAX >> k) & 1u)
+#pragma unroll
+					for (int o = 16; o > 0; o >>= 1)
+						t[k] = larger(t[k], __shfl_xor_sync(0xffffffffu, t[k], o));
+				else
+					t[k] = warp_sum(u);
 			}
 			if (lane == 0)
 				f(t);
@@ -693,13 +711,13 @@ __device__ __forceinline__ int uz_cg(UzTeam &tm, const UzawaArgs &a, const UzRow
 			rr.x = rn.x;
 			ss.x = precond ? rr.x * id.x : rr.x;
 			a2[0] += rr.x * ss.x;
-			a2[1] = fmax(a2[1], fabs(alpha * rr.x));
+			a2[1] = larger(a2[1], fabs(rr.x));
 		}
 		if (R.f1) {
 			rr.y = rn.y;
 			ss.y = precond ? rr.y * id.y : rr.y;
 			a2[0] += rr.y * ss.y;
-			a2[1] = fmax(a2[1], fabs(alpha * rr.y));
+			a2[1] = larger(a2[1], fabs(rr.y));
 		}
 		tm.reduce_then<2, 2u>(a2, [&](const double (&v)[2]) {
 			s_beta = v[0] / s_delta;
@@ -709,7 +727,8 @@ __device__ __forceinline__ int uz_cg(UzTeam &tm, const UzawaArgs &a, const UzRow
 				if (blockIdx.x == 0)
 					atomicOr(status, s_dq == 0.0 ? kStatBreakdown : kStatNan);
 				s_stop = 1;
-			} else if (v[1] < accu || !(cycle + 1 < max_cycle && v[0] > accu * s_delta0)) {
+			} else if (fabs(s_alpha * v[1]) < accu || !(   // the largest |alpha r|: rounding is monotone
+			           cycle + 1 < max_cycle && v[0] > accu * s_delta0)) {
 				s_stop = 1;
 			}
 		});
