@@ -108,7 +108,7 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 	const T axp = O.axp, axm = O.axm, azp = O.azp, azm = O.azm, ip = O.p, iq = O.q;
 	const int N = P.N, n = N + 1;
 	const int lane = threadIdx.x & 31;
-	const int nwarps = pt.size * (kBlock / 32);
+	const int nwarps = pt.size * (int)(blockDim.x >> 5);
 	const int strips = sp.strips, Lx = sp.Lx, ntasks = sp.ntasks;
 	const float inv = sp.inv;
 	double dacc = 0.0, racc = 0.0, facc = 0.0;

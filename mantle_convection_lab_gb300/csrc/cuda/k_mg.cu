@@ -280,15 +280,16 @@ __device__ void coarse_build(const MGHier<T> &H, SolveShared<T> &cs)
 		return;
 	}
 	constexpr int kPer = (kCoarseShared * kCoarseShared + kBlock - 1) / kBlock;
+	const int nt = blockDim.x;
 	T v[kPer];
 #pragma unroll
 	for (int u = 0; u < kPer; u++)
-		v[u] = threadIdx.x + u * kBlock < n2 ? (T)M[threadIdx.x + u * kBlock] : T(0);
+		v[u] = (int)threadIdx.x + u * nt < n2 ? (T)M[threadIdx.x + u * nt] : T(0);
 	__syncthreads();
 #pragma unroll
 	for (int u = 0; u < kPer; u++)
-		if (threadIdx.x + u * kBlock < n2)
-			cs.inv()[threadIdx.x + u * kBlock] = v[u];
+		if ((int)threadIdx.x + u * nt < n2)
+			cs.inv()[threadIdx.x + u * nt] = v[u];
 	__syncthreads();
 }
 
@@ -1195,8 +1196,8 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 	const GTab &gt = a.gt;
 
 	for (int l = threadIdx.x; l < a.H.nlev; l += blockDim.x) {
-		cs.sp.lev[0][l].set(a.H.lv[l].n, kBlock / 32);
-		cs.sp.lev[1][l].set(a.H.lv[l].n, sy.size * (kBlock / 32));
+		cs.sp.lev[0][l].set(a.H.lv[l].n, blockDim.x / 32);
+		cs.sp.lev[1][l].set(a.H.lv[l].n, sy.size * (blockDim.x / 32));
 	}
 	// -- per-step setup: viscosity on every level, inverse diagonals, BAB, coarse inverse
 	for (int A = tid; A < nn; A += nth)
@@ -1450,13 +1451,14 @@ __device__ void stokes_solve(const MGArgs<TI> &a, Sync &sy)
 	}
 }
 
-// Blocks per SM: two of 256 threads in FP32; the FP64 passes hold twice the
-// registers and are bound by the FP64 pipe, which one block keeps busy.
-template <class TI> constexpr int kSolveBlocks = sizeof(TI) == 4 ? 2 : 1;
+// Most threads per block: 512 in FP32 (two blocks of 256 per SM on a grid, one of
+// 512 in a single model's cluster); the FP64 passes hold twice the registers and
+// are bound by the FP64 pipe, which 256 threads keep busy.
+template <class TI> constexpr int kSolveThreads = sizeof(TI) == 4 ? 512 : 256;
 
 // One model on the whole cooperative grid, or on one cluster (a.cluster).
 template <class TI>
-__global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg(const __grid_constant__ MGArgs<TI> a)
+__global__ void __launch_bounds__(kSolveThreads<TI>, 1) k_stokes_mg(const __grid_constant__ MGArgs<TI> a)
 {
 	__shared__ MGArgs<TI> sa;
 	__shared__ double cpart[2 * kRedWidth];
@@ -1477,7 +1479,7 @@ __global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg(const __
 // reads the draw from its shared memory; all blocks of a cluster leave the
 // loop on the same draw.
 template <class TI>
-__global__ void __launch_bounds__(kBlock, kSolveBlocks<TI>) k_stokes_mg_batch(const MGArgs<TI> *models, int nmodels,
+__global__ void __launch_bounds__(kSolveThreads<TI>, 1) k_stokes_mg_batch(const MGArgs<TI> *models, int nmodels,
                                                                               int *queue)
 {
 	__shared__ MGArgs<TI> sa;

@@ -939,7 +939,7 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 
 // One refined model on the whole cooperative grid, or on one cluster.
 template <class TI>
-__global__ void __launch_bounds__(kBlock) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
+__global__ void __launch_bounds__(kTeamThreads) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
 {
 	__shared__ QtArgs<TI> sa;
 	load_args(sa, a);

@@ -361,28 +361,34 @@ static int max_clusters(void *kern, int cs, int threads)
 
 // The blocks that solve one uniform model: a single cluster for small meshes in
 // FP32, whose iteration is a chain of barriers (0.2 us in a cluster, 1.2 in a
-// grid): 42 against 53 us per MINRES iteration at 64^2 and 81 against 90 per
-// inner iteration at 128^2 on 16 blocks (50 and 110 on 8), 145 against 86 at
-// 256^2.  FP64 passes need the whole device's FP64 pipes from 64^2 on (297
-// against 170 us at 128^2).
+// grid): per iteration 38 against 53 us at 64^2 (MINRES) and 75 against 90 at
+// 128^2 (inner CG) on 16 blocks of 512 threads, 125 against 77 at 256^2; blocks
+// of 256 threads take 38.5 and 80, 8 of them 50 and 110.  FP64 passes need the
+// whole device's FP64 pipes from 64^2 on (297 against 170 us at 128^2).
+static int mg_cluster_threads(const mclg_ctx *c)
+{
+	return c->cfg.precision == 2 ? kBlock : kTeamThreads;
+}
+
 static void mg_team(mclg_ctx *c, void *kern)
 {
 	constexpr int kOneCluster = 16, kOneClusterN32 = 128, kOneClusterN64 = 32;
 	const int N0 = c->mesh.max_elx[c->fl];
 	c->mg_one_cluster = N0 <= (c->cfg.precision == 2 ? kOneClusterN64 : kOneClusterN32) &&
-	                    max_clusters(kern, kOneCluster, kBlock) >= 1;
+	                    max_clusters(kern, kOneCluster, mg_cluster_threads(c)) >= 1;
 	c->coop_mg = c->mg_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, 1 << 30);
 }
 
 // The blocks that solve one refined model.  Up to kOneClusterNodes nodes one
-// cluster, whose barriers take 0.2 us instead of a grid's 1.2 (54 against 65 us
-// per MINRES iteration at 1347 nodes, 64 against 79 at 2441, 87 against 77 at
-// 5125); up to kSpreadNodes four times the blocks its nodes fill, so that its
-// FP64 work uses more SMs (89 against 93 us at 8847 nodes, 95 against 89 at 19977).
+// cluster, whose barriers take 0.2 us instead of a grid's 1.2, with 512 threads a
+// block (60 against 69 us per MINRES iteration at 5125 nodes, 91 against 81 at
+// 8847); up to kSpreadNodes four times the blocks its nodes fill, so that its
+// FP64 work uses more SMs (89 against 93 us at 8847 nodes, 95 against 89 at
+// 19977, both before the gathers were chunked).
 static void qt_team(mclg_ctx *c, void *kern, int nn)
 {
-	constexpr int kOneCluster = 16, kOneClusterNodes = 4096, kSpreadNodes = 12288;
-	c->qt_one_cluster = nn <= kOneClusterNodes && max_clusters(kern, kOneCluster, kBlock) >= 1;
+	constexpr int kOneCluster = 16, kOneClusterNodes = 6144, kSpreadNodes = 12288;
+	c->qt_one_cluster = nn <= kOneClusterNodes && max_clusters(kern, kOneCluster, kTeamThreads) >= 1;
 	c->coop_qt = c->qt_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, nn <= kSpreadNodes ? 4 * nn : nn);
 }
 
@@ -1128,7 +1134,7 @@ static int launch_stokes_qt(mclg_ctx *c)
 	void *args[] = {c->cfg.precision == 2 ? (void *)&c->qtd : (void *)&c->qtf};
 	void *kern = qt_kernel(c->cfg.precision == 2);
 	if (one)
-		CK(launch_cluster(kern, c->coop_qt, kBlock, args, c->st));
+		CK(launch_cluster(kern, c->coop_qt, kTeamThreads, args, c->st));
 	else
 		CK(cudaLaunchCooperativeKernel(kern, dim3(solver_grid(c, c->coop_qt)), dim3(kBlock), args, 0, c->st));
 	c->launches++;
@@ -1273,7 +1279,7 @@ static int launch_stokes_mg(mclg_ctx *c)
 	void *args[] = {c->cfg.precision == 2 ? (void *)&c->mgd : (void *)&c->mgf};
 	void *kern = stokes_mg_kernel(c->cfg.precision == 2);
 	if (one)
-		CK(launch_cluster(kern, c->coop_mg, kBlock, args, c->st));
+		CK(launch_cluster(kern, c->coop_mg, mg_cluster_threads(c), args, c->st));
 	else
 		CK(cudaLaunchCooperativeKernel(kern, dim3(solver_grid(c, c->coop_mg)), dim3(kBlock), args, 0, c->st));
 	c->launches++;
@@ -1744,7 +1750,7 @@ static int read_scalars(mclg_ctx *c)
 // The replica's solve.  On one cluster where a thread can own each node and its
 // rows (no hanging nodes, whose overwrite follows every update, and at most 64^2
 // elements), with the CG inner solver; measured per CG iteration against the
-// cooperative grid: 8.0 against 15.6 us at 16^2, 10.2 against 15.8 at 64^2.
+// cooperative grid: 7.5 against 15.6 us at 16^2, 9.3 against 15.8 at 64^2.
 static cudaError_t run_uzawa(mclg_ctx *c, UzawaArgs &a)
 {
 	void *args[] = {&a};

@@ -9,6 +9,8 @@ namespace mclg {
 
 // The blocks that share a pass over a level: block `rank` of `size` (the
 // whole grid, a thread-block cluster, or one block alone).
+constexpr int kTeamThreads = 512;   // most threads of a team's block
+
 struct Part {
 	int rank, size;
 	// This thread's number in the blocks of the pass: warps are dealt to the
@@ -60,12 +62,12 @@ struct Sync {
 	// Sums of NV values over the team, formed by warp 0 of every block from the
 	// same partials in the same order; f(sums) runs on thread 0 of each block, and
 	// what it writes to shared memory is visible to the block on return.  Each
-	// value's 256 thread partials go through shared memory to one warp (8 + 5
-	// additions): a butterfly in every warp takes eight times that of the FP64
+	// value's thread partials go through shared memory to one warp (8 or 16, then 5
+	// additions; blocks of 256 or 512 threads): a butterfly in every warp takes eight times that of the FP64
 	// pipe, which has 2 lanes per clock and SM.
 	__device__ static double *scratch()
 	{
-		__shared__ double sh[kRedWidth * kBlock];
+		__shared__ double sh[kRedWidth * kTeamThreads];
 		return sh;
 	}
 	template <int NV, class F>
@@ -76,7 +78,7 @@ struct Sync {
 		const int lane = threadIdx.x & 31;
 #pragma unroll
 		for (int k = 0; k < NV; k++)
-			sh[k * kBlock + threadIdx.x] = v[k];
+			sh[k * kTeamThreads + threadIdx.x] = v[k];
 		__syncthreads();
 		double t[NV];
 #pragma unroll
@@ -85,8 +87,13 @@ struct Sync {
 		if (threadIdx.x < 32) {
 #pragma unroll
 			for (int k = 0; k < NV; k++) {
-				const double *s = sh + k * kBlock + lane;
-				t[k] = warp_sum(((s[0] + s[32]) + (s[64] + s[96])) + ((s[128] + s[160]) + (s[192] + s[224])));
+				const double *s = sh + k * kTeamThreads + lane;
+				t[k] = ((s[0] + s[32]) + (s[64] + s[96])) + ((s[128] + s[160]) + (s[192] + s[224]));
+				if (blockDim.x > 256) {
+					s += 256;
+					t[k] += ((s[0] + s[32]) + (s[64] + s[96])) + ((s[128] + s[160]) + (s[192] + s[224]));
+				}
+				t[k] = warp_sum(t[k]);
 			}
 		}
 		if (mode == SYNC_GRID) {
