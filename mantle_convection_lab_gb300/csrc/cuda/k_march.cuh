@@ -43,11 +43,13 @@ struct Split {
 };
 
 enum {
-	PASS_MATVEC = 0,   // out = A x; *dot = this thread's share of x.(A x)
+	PASS_MATVEC = 0,   // out = A x; *dot = this thread's share of x.(A x) (with xout, x as formed is
+	                   // stored there)
 	PASS_RESID = 1,    // out = b - A x (with xout, x as formed is stored there)
 	PASS_SMOOTH = 2,   // out = cx x - c0 x0 + omega D^-1 (b - A x) (cx = 1, no x0: damped
 	                   // Jacobi; the Chebyshev recurrence otherwise; with xout, x as formed is
-	                   // stored there; with dot, *dot = this thread's share of out.dotv)
+	                   // stored there; *dot = this thread's share of out.dotv, or of out.b
+	                   // with dotb)
 	PASS_STOKES = 3,   // out64 = A x + G gp, gt_out = G^T x per element (x-major);
 	                   // *dot = this thread's share of x.out64 + gp.gt_out
 	PASS_RES64 = 4     // out64 = F - A x - G gp, gt_out = G^T x; dot[0..2] = this thread's
@@ -61,9 +63,10 @@ enum {
 //   XS_ZERO_R   wload D^-1 b with b = P^T r_f formed from the finer level's
 //               residual (xc = r_f, nc = its nodes per side); the pass also
 //               writes b for its own nodes (bout), for the level's later passes
+//   XS_AXPY     x + wload xc         (CG's direction; xc is not read into it when wload is 0)
 // Forming them where the pass reads them saves a barrier and a pass over memory
 // on every multigrid level.
-enum { XS_PLAIN = 0, XS_ZERO = 1, XS_PROLONG = 2, XS_ZERO_R = 3 };
+enum { XS_PLAIN = 0, XS_ZERO = 1, XS_PROLONG = 2, XS_ZERO_R = 3, XS_AXPY = 4 };
 
 template <class T>
 struct Pass {
@@ -76,6 +79,7 @@ struct Pass {
 	int nc;
 	T omega, wload, cx, c0;
 	const double2 *dotv;
+	bool dotb;
 	// PASS_STOKES, PASS_RES64
 	const double *gp;
 	double2 *out64;
@@ -131,8 +135,10 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 			const int A = gzc + ixc * n;
 			k.m = P.mask[A];
 			k.e = P.eta[A];
-			if (XS == XS_PLAIN || XS == XS_PROLONG)
+			if (XS == XS_PLAIN || XS == XS_PROLONG || XS == XS_AXPY)
 				k.x = P.x[A];
+			if (XS == XS_AXPY)
+				k.c[0] = P.xc[A];
 			if (XS == XS_ZERO || (kNeedB && XS != XS_ZERO_R))
 				k.b = P.b[A];
 			if (XS == XS_ZERO || XS == XS_ZERO_R || MODE == PASS_SMOOTH)
@@ -177,6 +183,10 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 			if (XS == XS_ZERO || XS == XS_ZERO_R) {
 				k.x.x = P.wload * k.d.x * k.b.x;
 				k.x.y = P.wload * k.d.y * k.b.y;
+			}
+			if (XS == XS_AXPY && P.wload != T(0)) {
+				k.x.x += P.wload * k.c[0].x;
+				k.x.y += P.wload * k.c[0].y;
 			}
 			if (XS == XS_PROLONG) {
 				k.x.x += T(0.25) * ((k.c[0].x + k.c[1 % NC].x) + (k.c[2 % NC].x + k.c[3 % NC].x));
@@ -309,9 +319,11 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 						o.y = (m & 2u) ? T(0) : py + P.omega * prev.d.y * (prev.b.y - fw);
 						if (P.dotv)
 							dacc += widen(o.x) * dv.x + widen(o.y) * dv.y;
+						else if (P.dotb)
+							dacc += widen(o.x) * widen(prev.b.x) + widen(o.y) * widen(prev.b.y);
 					}
 					P.out[A] = o;
-					if (MODE != PASS_MATVEC && P.xout)
+					if (P.xout)
 						P.xout[A] = prev.x;
 					if (XS == XS_ZERO_R)
 						P.bout[A] = prev.b;

@@ -343,6 +343,7 @@ __device__ __forceinline__ Pass<T> level_pass(const MGLevel<T> &L, const typenam
 	P.omega = P.wload = P.c0 = T(0);
 	P.cx = T(1);
 	P.dotv = nullptr;
+	P.dotb = false;
 	return P;
 }
 
@@ -436,9 +437,9 @@ __device__ __forceinline__ void level_down(Sync &sy, const Splits &sp, const MGH
 	}
 }
 
-// With dotv (level 0 only), the last sweep also accumulates this thread's
-// share of out0.dotv into *dot and is not followed by a barrier: the caller's
-// reduction provides it.
+// With dot (level 0 only), the last sweep also accumulates this thread's
+// share of out0.dotv (out0.rhs0 without dotv) into *dot and is not followed by
+// a barrier: the caller's reduction provides it.
 template <class T>
 __device__ __forceinline__ void level_up(Sync &sy, const Splits &sp, const MGHier<T> &H, int l,
                                          const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0, bool wide,
@@ -461,10 +462,11 @@ __device__ __forceinline__ void level_up(Sync &sy, const Splits &sp, const MGHie
 	for (int s = 0; s < nu; s++) {
 		const bool last = l == 0 && s == nu - 1;
 		V *dst = last ? out0 : xt;
-		double *dp = (last && dotv) ? dot : nullptr;
+		double *dp = last ? dot : nullptr;
 		P.x = x;
 		P.out = dst;
 		P.dotv = dp ? dotv : nullptr;
+		P.dotb = dp && !dotv;
 		if (s == 0) {
 			P.omega = ch ? H.w1 : H.omega;
 			P.xout = ch ? L.r : nullptr;
@@ -491,21 +493,20 @@ __device__ __forceinline__ void level_up(Sync &sy, const Splits &sp, const MGHie
 // most of a thread's registers, and as calls they saved and restored them on
 // the stack on every level (25 of 98 us per MINRES iteration at 64^2).
 //
-// out0 = B rhs0.  With dotv, *dot receives this thread's share of out0.dotv
-// and the cycle ends without a barrier (the caller reduces *dot, which
-// synchronises the team); without it the cycle ends with a barrier.
+// out0 = B rhs0.  *dot receives this thread's share of out0.dotv (of out0.rhs0
+// without dotv) and the cycle ends without a barrier: the caller reduces *dot,
+// which synchronises the team.
 template <class T>
 __device__ __forceinline__ void vcycle(Sync &sy, SolveShared<T> &cs, const MGHier<T> &H,
-                                       const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0,
-                                       const double2 *dotv = nullptr, double *dot = nullptr)
+                                       const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0, const double2 *dotv,
+                                       double *dot)
 {
 	typedef typename V2T<T>::t V;
 	const int lc = H.nlev - 1;
 	// first block-local level (the coarsest always is; in one block all are)
 	const int nb = sy.size > 1 ? (H.nblk < lc ? H.nblk : lc) : 0;
 	const bool b0 = sy.leader();
-	if (dot)
-		*dot = 0.0;
+	*dot = 0.0;
 #pragma unroll 1
 	for (int l = 0; l < lc; l++)
 		if (l < nb || b0)
@@ -519,73 +520,66 @@ __device__ __forceinline__ void vcycle(Sync &sy, SolveShared<T> &cs, const MGHie
 		if (l < nb || b0)
 			level_up<T>(sy, cs.sp, H, l, rhs0, out0, l < nb, dotv, dot);
 	}
-	if (nb == 0 && !dotv)
-		sy.sync();
 }
 
 // ---- inner solve: CG preconditioned by one V-cycle, all in T -----------------
-// The recurrences' scalars are formed by one thread of each block while the
-// others wait for its broadcast: a division or a square root on every thread
-// costs the FP64 pipe (2 lanes per clock and SM) about a microsecond each.
+// x = K^-1 b to rtol; b is overwritten.  The recurrences' scalars are formed by
+// one thread of each block while the others wait for its broadcast: a division
+// or a square root on every thread costs the FP64 pipe (2 lanes per clock and
+// SM) about a microsecond each.  The V-cycle's last sweep forms <z, r>, and the
+// operator pass the new direction p = z + beta p (into the other of two buffers:
+// its neighbours still read the old one).
 template <class T>
-__device__ __noinline__ int pcg_inner(Sync &team, SolveShared<T> &cs, const MGHier<T> &H, const typename V2T<T>::t *b, typename V2T<T>::t *x, double rtol,
-                         int maxit)
+__device__ __noinline__ int pcg_inner(Sync &team, SolveShared<T> &cs, const MGHier<T> &H, typename V2T<T>::t *b,
+                                      typename V2T<T>::t *x, double rtol, int maxit)
 {
-	Sync sy = team;
 	typedef typename V2T<T>::t V;
+	Sync sy = team;
 	__shared__ double rho, bb0, co;
 	const MGLevel<T> &L = H.lv[0];
-	const int nn = L.n * L.n;
-	const int tid = sy.tid(), nth = sy.nth();
-	V *r = H.pr, *z = H.pz, *p = H.pp, *q = H.pq;
-	double bb[1] = {0.0};
-	for (int A = tid; A < nn; A += nth) {
-		const V bv = b[A];
-		r[A] = bv;
-		V zero;
-		zero.x = T(0);
-		zero.y = T(0);
-		x[A] = zero;
-		const double b0 = widen(bv.x), b1 = widen(bv.y);
-		bb[0] += b0 * b0 + b1 * b1;
+	auto nodes = [&] { return H.lv[0].n * H.lv[0].n; };
+	{
+		const int tid = sy.tid(), nth = sy.nth(), nn = nodes();
+		double bb[1] = {0.0};
+		for (int A = tid; A < nn; A += nth) {
+			const V bv = b[A];
+			H.pr[A] = bv;
+			V zero;
+			zero.x = T(0);
+			zero.y = T(0);
+			x[A] = zero;
+			const double b0 = widen(bv.x), b1 = widen(bv.y);
+			bb[0] += b0 * b0 + b1 * b1;
+		}
+		sy.reduce_then<1>(bb, [&](const double (&v)[1]) { bb0 = v[0]; });
 	}
-	sy.reduce_then<1>(bb, [&](const double (&v)[1]) { bb0 = v[0]; });
 	if (!(bb0 > 0.0)) {
 		team = sy;
 		return 0;
 	}
-	Pass<T> P = level_pass<T>(L, nullptr);
-	P.x = p;
-	P.out = q;
+	V *p = H.pp, *po = b;
 	int it = 0;
 	while (it < maxit) {
-		vcycle<T>(sy, cs, H, r, z);
-		double rz[1] = {0.0};
-		for (int A = tid; A < nn; A += nth) {
-			const V rv = r[A], zv = z[A];
-			rz[0] += widen(rv.x) * widen(zv.x) + widen(rv.y) * widen(zv.y);
-		}
+		double rz[1], pq[1];
+		vcycle<T>(sy, cs, H, H.pr, H.pz, nullptr, rz);
 		sy.reduce_then<1>(rz, [&](const double (&v)[1]) {
 			co = it > 0 ? v[0] / rho : 0.0;
 			rho = v[0];
 		});
-		const T be = (T)co;
-		for (int A = tid; A < nn; A += nth) {
-			V pv = z[A];
-			if (it > 0) {
-				const V po = p[A];
-				pv.x += be * po.x;
-				pv.y += be * po.y;
-			}
-			p[A] = pv;
-		}
-		sy.sync();
-		double pq[1];
-		march<T, PASS_MATVEC, XS_PLAIN, false>(P, sy.part(true), cs.sp.lev[1][0], pq);
+		Pass<T> P = level_pass<T>(L, nullptr);
+		P.x = H.pz;
+		P.xc = po;
+		P.wload = (T)co;
+		P.xout = p;
+		P.out = H.pq;
+		march<T, PASS_MATVEC, XS_AXPY, false>(P, sy.part(true), cs.sp.lev[1][0], pq);
 		sy.reduce_then<1>(pq, [&](const double (&v)[1]) { co = rho / v[0]; });
 		const double alpha = co;
 		const T al = (T)alpha;
 		double rr[1] = {0.0};
+		const int tid = sy.tid(), nth = sy.nth(), nn = nodes();
+		V *r = H.pr;
+		const V *q = H.pq;
 		for (int A = tid; A < nn; A += nth) {
 			V xv = x[A], rv = r[A];
 			const V pv = p[A], qv = q[A];
@@ -600,6 +594,9 @@ __device__ __noinline__ int pcg_inner(Sync &team, SolveShared<T> &cs, const MGHi
 		}
 		sy.reduce<1>(rr);
 		it++;
+		V *t = p;
+		p = po;
+		po = t;
 		if (!(rr[0] > rtol * rtol * bb0) || !isfinite(alpha))
 			break;
 	}
@@ -677,6 +674,7 @@ __device__ __forceinline__ Pass<double> fine_pass64(const MGArgs<TI> &a, const d
 	P.omega = P.wload = P.c0 = 0.0;
 	P.cx = 1.0;
 	P.dotv = nullptr;
+	P.dotb = false;
 	P.gp = p;
 	P.gp_morton = 1;
 	P.g0 = a.gt.g0[0];
