@@ -442,18 +442,39 @@ __device__ __forceinline__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t, typ
 	}
 }
 
-// coarsest level: the dense inverse on its reduced dofs
+// coarsest level: the dense inverse on its reduced dofs, a warp per four rows
+// with its lanes along them (a thread per row read the matrix in columns 4*nc
+// bytes apart: 8.3 us of a 128 us iteration for 126 unknowns)
 template <class TI>
-__device__ void qt_coarse_solve(const QtHier<TI> &H, QtTeam &t)
+__device__ __forceinline__ void qt_coarse_solve(const QtHier<TI> &H, QtTeam &t)
 {
+	__shared__ TI sb[kQtMaxCoarse];
 	const QtLevel<TI> &C = H.lv[0];
 	const TI *bf = reinterpret_cast<const TI *>(C.b);
 	TI *xf = reinterpret_cast<TI *>(C.x[0]);
-	for (int i = t.tid; i < H.nc; i += t.nth) {
-		TI s = TI(0);
-		for (int j = 0; j < H.nc; j++)
-			s += H.cinv[(size_t)i * H.nc + j] * bf[H.cdof[j]];
-		xf[H.cdof[i]] = s;
+	const int nc = H.nc, lane = threadIdx.x & 31;
+	for (int j = threadIdx.x; j < nc; j += blockDim.x)
+		sb[j] = bf[H.cdof[j]];
+	__syncthreads();
+	for (int i0 = 4 * (t.tid >> 5); i0 < nc; i0 += 4 * (t.nth >> 5)) {
+		TI s[4] = {TI(0), TI(0), TI(0), TI(0)};
+		const TI *row = H.cinv + (size_t)i0 * nc;
+#pragma unroll 4
+		for (int j = lane; j < nc; j += 32) {
+			const TI b = sb[j];
+#pragma unroll
+			for (int u = 0; u < 4; u++)
+				if (i0 + u < nc)
+					s[u] += row[(size_t)u * nc + j] * b;
+		}
+#pragma unroll
+		for (int u = 0; u < 4; u++) {
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1)
+				s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+			if (lane == u && i0 + u < nc)
+				xf[H.cdof[i0 + u]] = s[u];
+		}
 	}
 	t.sync();
 }
@@ -501,57 +522,60 @@ __device__ __forceinline__ void qt_vcycle(Sync &sy, const QtHier<TI> &H, typenam
 }
 
 // Dense inverse of the coarsest level's constrained operator on its reduced
-// dofs, columns from the operator applied to unit vectors (FP64), inverted
-// by Gauss-Jordan (the operator is SPD: no pivoting).  Block 0 only.
+// dofs (FP64): the rows of C^T K C from their contribution lists, inverted by
+// Gauss-Jordan (SPD: no pivoting) by the whole team, a warp per row.  The matrix
+// alternates between two buffers, so that a pivot takes one team barrier.  One
+// block alone took 1.1 ms per solve at 126 unknowns: an FP64 inversion of that
+// size is 2 million multiply-adds on one SM's two FP64 lanes.
 template <class TI>
-__device__ void qt_coarse_build(const QtHier<TI> &H)
+__device__ __noinline__ void qt_coarse_build(Sync &sy, const QtHier<TI> &H)
 {
 	const QtLevel<TI> &C = H.lv[0];
-	const int nc = H.nc, w2 = 2 * nc;
-	double *M = H.cwork, *e = H.cvec;
-	for (int k = threadIdx.x; k < nc * w2; k += blockDim.x)
-		M[k] = ((k % w2) == nc + k / w2) ? 1.0 : 0.0;
-	for (int k = threadIdx.x; k < 2 * C.nno; k += blockDim.x)
-		e[k] = 0.0;
-	__syncthreads();
-	for (int j = 0; j < nc; j++) {
-		if (threadIdx.x == 0)
-			e[H.cdof[j]] = 1.0;
-		__syncthreads();
-		for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-			const int d = H.cdof[i];
-			double y0, y1;
-			qt_op_node(C, C.K64, (const double *)e, d >> 1, y0, y1);
-			M[(size_t)i * w2 + j] = (d & 1) ? y1 : y0;
+	const int nc = H.nc, tid = sy.tid(), nth = sy.nth(), lane = threadIdx.x & 31;
+	double *M = H.cwork, *N = H.cwork + (size_t)nc * nc, *at = H.cvec;   // at: a dof's row, -1 off the reduced dofs
+	const double *K64f = reinterpret_cast<const double *>(C.K64);
+	for (int k = tid; k < nc * nc; k += nth)
+		M[k] = 0.0;
+	for (int k = tid; k < 2 * C.nno; k += nth)
+		at[k] = -1.0;
+	sy.sync();
+	for (int j = tid; j < nc; j += nth)
+		at[H.cdof[j]] = (double)j;
+	sy.sync();
+	for (int A = tid; A < C.nno; A += nth) {
+		const int i1 = C.rc_off[A + 1];
+		for (int i = C.rc_off[A]; i < i1;) {
+			const int t = C.rc_tgt[i], slot = t >> 2, cc = t & 3;
+			double v = 0.0;
+			for (; i < i1 && C.rc_tgt[i] == t; i++)
+				v += (double)C.rc_w[i] * K64f[C.rc_src[i]];
+			const int r = (int)at[2 * A + (cc >> 1)], c = (int)at[2 * C.rnb[(size_t)slot * C.nno + A] + (cc & 1)];
+			if (r >= 0 && c >= 0)
+				M[(size_t)r * nc + c] = v;
 		}
-		__syncthreads();
-		if (threadIdx.x == 0)
-			e[H.cdof[j]] = 0.0;
-		__syncthreads();
 	}
-	__shared__ double piv;
+	sy.sync();
 	for (int k = 0; k < nc; k++) {
-		if (threadIdx.x == 0)
-			piv = M[(size_t)k * w2 + k];
-		__syncthreads();
-		for (int c = threadIdx.x; c < w2; c += blockDim.x)
-			M[(size_t)k * w2 + c] /= piv;
-		__syncthreads();
-		for (int r = threadIdx.x; r < nc; r += blockDim.x) {
-			if (r == k)
-				continue;
-			const double f = M[(size_t)r * w2 + k];
-			if (f != 0.0)
-				for (int c = 0; c < w2; c++)
-					M[(size_t)r * w2 + c] -= f * M[(size_t)k * w2 + c];
+		const double *pk = M + (size_t)k * nc;
+		const double ip = (tid >> 5) < nc ? 1.0 / pk[k] : 0.0;   // (warps with rows only: see QtScal)
+		for (int r = tid >> 5; r < nc; r += nth >> 5) {
+			const double *row = M + (size_t)r * nc;
+			double *out = N + (size_t)r * nc;
+			const double f = row[k] * ip;
+#pragma unroll 4
+			for (int c = lane; c < nc; c += 32) {
+				const double p = pk[c], m = row[c];
+				out[c] = r == k ? (c == k ? ip : p * ip) : (c == k ? -f : m - f * p);
+			}
 		}
-		__syncthreads();
+		sy.sync();
+		double *t = M;
+		M = N;
+		N = t;
 	}
-	for (int k = threadIdx.x; k < nc * nc; k += blockDim.x) {
-		const int r = k / nc, c = k - r * nc;
-		H.cinv[k] = (TI)M[(size_t)r * w2 + nc + c];
-	}
-	__syncthreads();
+	for (int k = tid; k < nc * nc; k += nth)
+		H.cinv[k] = (TI)M[k];
+	sy.sync();
 }
 
 // ---- FP64 residual and the preconditioner ------------------------------------------
@@ -653,7 +677,17 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 				const V *z = a.mz[cv];
 				const double *zp = a.mzp[cv];
 				const TI *zf = reinterpret_cast<const TI *>(z);
-				for (int A = tid; A < L.nno; A += nth) {
+				// nodes and elements in one range: with two loops each would end in a
+				// trip for the few left over
+				const int nn = L.nno, ni = nn + L.nel;
+				for (int A = tid; A < ni; A += nth) {
+					if (A >= nn) {
+						const int e = A - nn;
+						const double t = qt_gt_elem(Q, L, zf, e);
+						a.Ahp[e] = t;
+						dl[0] += t * zp[e];
+						continue;
+					}
 					TI k0, k1;
 					double g0, g1;
 					const V zz = z[A];
@@ -662,11 +696,6 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 					const double2 az = make_double2(widen(k0) + g0, widen(k1) + g1);
 					a.Kd[A] = az;
 					dl[0] += az.x * widen(zz.x) + az.y * widen(zz.y);
-				}
-				for (int e = tid; e < L.nel; e += nth) {
-					const double t = qt_gt_elem(Q, L, zf, e);
-					a.Ahp[e] = t;
-					dl[0] += t * zp[e];
 				}
 			}
 			sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
@@ -866,9 +895,7 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 		}
 	}
 	sy.sync();
-	if (sy.leader())
-		qt_coarse_build(H);
-	sy.sync();
+	qt_coarse_build(sy, H);
 
 	int refine = 0, minres_total = 0, vcycles = 0, capped = 0;
 	double res_m = 0.0, res_c = 0.0;

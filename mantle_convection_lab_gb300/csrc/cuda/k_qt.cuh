@@ -24,6 +24,8 @@ template <> struct Q2T<double> { typedef double2 t; };
 // as stored, fixed entries being kept at 0).
 constexpr int kQtCon = 1 << 30;
 
+constexpr int kQtMaxCoarse = 1024;   // unknowns of the coarsest level
+
 template <class T>
 struct QtLevel {
 	int nno, nbw;
@@ -58,9 +60,9 @@ struct QtHier {
 	int nblk;                               // levels lv[0..nblk-1] are small: block 0 alone runs them
 	int nc;                                 // reduced dofs of the coarsest level
 	const int *cdof;                        // [nc] their dof numbers
-	double *cwork;                          // [nc * 2nc] Gauss-Jordan workspace
+	double *cwork;                          // [2 * nc * nc] the inversion's two buffers
 	T *cinv;                                // [nc * nc] inverse of the coarsest constrained operator
-	double *cvec;                           // [2 * nno_coarsest] unit-vector scratch (FP64)
+	double *cvec;                           // [2 * nno_coarsest] a dof's row
 };
 
 template <class TI>
