@@ -9,7 +9,29 @@
 
 namespace mclg {
 
-MCLG_SHAPE_UPLOAD(upload_shape_tables_elem)
+// Per pair of corners and Gauss point, the products of the parent derivatives,
+// and the shape functions' mass matrix (sums over the Gauss points).
+struct ElemTables {
+	double xx[4][4][4], zz[4][4][4], zx[4][4][4], M[4][4];   // zx: dN_a/deta dN_b/dxi
+};
+static __constant__ ElemTables cE;
+
+void upload_shape_tables_elem(const ShapeTables &s, cudaStream_t st)
+{
+	ElemTables t;
+	for (int a = 0; a < 4; a++)
+		for (int b = 0; b < 4; b++) {
+			t.M[a][b] = 0.0;
+			for (int g = 0; g < 4; g++) {
+				t.xx[a][b][g] = s.dNdxi[a][g] * s.dNdxi[b][g];
+				t.zz[a][b][g] = s.dNdeta[a][g] * s.dNdeta[b][g];
+				t.zx[a][b][g] = s.dNdeta[a][g] * s.dNdxi[b][g];
+				t.M[a][b] += s.N[a][g] * s.N[b][g];
+			}
+		}
+	cudaMemcpyToSymbolAsync(cS, &s, sizeof s, 0, cudaMemcpyHostToDevice, st);
+	cudaMemcpyToSymbolAsync(cE, &t, sizeof t, 0, cudaMemcpyHostToDevice, st);
+}
 
 // ---- buoyancy: Ra*T minus its horizontal average (Buoyancy.c:3-22) -------
 // get_node_horiz_avg (Parallel.c:354-437) interpolates Ra*T at every fine-grid
@@ -124,48 +146,14 @@ __device__ __forceinline__ void gauss_eta(const DevLevel &L, const double *__res
 	}
 }
 
-// One thread per node: block row of K, F and Kdiag.  With withK == 0 only F
-// is formed (the matrix-free solvers never need the assembled K).
-__global__ void __launch_bounds__(kBlock) k_assemble_stokes(DevLevel L, const double *__restrict__ vis,
-                                                            const double *__restrict__ buoy,
-                                                            double4 *__restrict__ K, double2 *__restrict__ F,
-                                                            double2 *__restrict__ Kdiag, int withK)
+// The element loads of node A (F_matrix / get_element_F, Build_matrix.c:117-140,
+// 273-344) on top of f; with fast, the buoyancy through the mass matrix (4 FP64
+// operations an element instead of 24).
+template <bool FAST>
+__device__ __forceinline__ void stokes_load(const DevLevel &L, const double *__restrict__ buoy, int A, const bool (&fr)[2],
+                                            double (&f)[2])
 {
-	const int A = blockIdx.x * blockDim.x + threadIdx.x;
-	if (A >= L.nno)
-		return;
 	const int nno = L.nno, nel = L.nel, cnt = L.p2n_cnt[A];
-	const bool fr[2] = {vfree(L, A, 0), vfree(L, A, 1)};
-	if (withK)
-		for (int k = 0; k < L.nbw; k++)
-			K[(size_t)k * nno + A] = make_double4(0.0, 0.0, 0.0, 0.0);
-	double f[2] = {0.0, 0.0};
-	// pass 1: K entries and Dirichlet lifting (K_matrix, Build_matrix.c:42-115)
-	for (int s = 0; s < cnt; s++) {
-		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
-		double etag[4];
-		gauss_eta(L, vis, e, etag);
-		const double dxh = L.dxh[e], dzh = L.dzh[e], jac = L.jac[e];
-		for (int i = 0; i < 2; i++) {
-			if (!fr[i])
-				continue;
-			for (int j = 0; j < 2; j++)
-				for (int b = 0; b < 4; b++) {
-					const int B = L.ienl[b * nel + e];
-					if (!withK && vfree(L, B, j))
-						continue;
-					const double kv = ke_entry(etag, dxh, dzh, jac, a, i, b, j);
-					if (vfree(L, B, j)) {
-						const int slot = L.kslot[(a * 4 + b) * nel + e];
-						double *blk = reinterpret_cast<double *>(&K[(size_t)slot * nno + A]);
-						blk[i * 2 + j] += kv;
-					} else {
-						f[i] -= kv * L.vbcval[j * nno + B];
-					}
-				}
-		}
-	}
-	// pass 2: element loads (F_matrix / get_element_F, Build_matrix.c:117-140, 273-344)
 	for (int s = 0; s < cnt; s++) {
 		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
 		int idx[4];
@@ -173,22 +161,26 @@ __global__ void __launch_bounds__(kBlock) k_assemble_stokes(DevLevel L, const do
 		for (int d = 0; d < 4; d++)
 			idx[d] = L.ienl[d * nel + e];
 		double fe[2] = {0.0, 0.0};
-		{
+		double t = 0.0;
+		if (FAST) {
+#pragma unroll
+			for (int d = 0; d < 4; d++)
+				t += cE.M[a][d] * buoy[idx[d]];
+		} else {
 			double force[4];
 #pragma unroll
 			for (int g = 0; g < 4; g++) {
-				double t = 0.0;
+				double u = 0.0;
 #pragma unroll
 				for (int d = 0; d < 4; d++)
-					t += cS.N[d][g] * buoy[idx[d]];
-				force[g] = t;
+					u += cS.N[d][g] * buoy[idx[d]];
+				force[g] = u;
 			}
-			double t = 0.0;
 #pragma unroll
 			for (int g = 0; g < 4; g++)
 				t += cS.N[a][g] * force[g];
-			fe[1] = t * L.jac[e];
 		}
+		fe[1] = t * L.jac[e];
 		for (int i = 0; i < 2; i++) {
 			int nat = 0;
 #pragma unroll
@@ -209,19 +201,133 @@ __global__ void __launch_bounds__(kBlock) k_assemble_stokes(DevLevel L, const do
 				f[i] += fe[i];
 		}
 	}
-	F[A] = make_double2(fr[0] ? f[0] : 0.0, fr[1] ? f[1] : 0.0);
-	if (!withK)
-		return;
-	// Kdiag (Build_matrix.c:740-744): the self slot of the block row
+}
+
+// Kdiag (Build_matrix.c:740-744): the self slot of the block row
+__device__ __forceinline__ void stokes_diag(const DevLevel &L, const double4 *__restrict__ K, double2 *__restrict__ Kdiag,
+                                            int A, const bool (&fr)[2])
+{
 	double2 dg = make_double2(1.0, 1.0);
-	{
-		const double4 blk = K[(size_t)L.self_slot[A] * nno + A];
-		if (fr[0])
-			dg.x = blk.x;
-		if (fr[1])
-			dg.y = blk.w;
-	}
+	const double4 blk = K[(size_t)L.self_slot[A] * L.nno + A];
+	if (fr[0])
+		dg.x = blk.x;
+	if (fr[1])
+		dg.y = blk.w;
 	Kdiag[A] = dg;
+}
+
+// One thread per node: block row of K, F and Kdiag in the reference's order of operations.
+__global__ void __launch_bounds__(kBlock) k_assemble_stokes(DevLevel L, const double *__restrict__ vis,
+                                                            const double *__restrict__ buoy,
+                                                            double4 *__restrict__ K, double2 *__restrict__ F,
+                                                            double2 *__restrict__ Kdiag)
+{
+	const int A = blockIdx.x * blockDim.x + threadIdx.x;
+	if (A >= L.nno)
+		return;
+	const int nno = L.nno, nel = L.nel, cnt = L.p2n_cnt[A];
+	const bool fr[2] = {vfree(L, A, 0), vfree(L, A, 1)};
+	for (int k = 0; k < L.nbw; k++)
+		K[(size_t)k * nno + A] = make_double4(0.0, 0.0, 0.0, 0.0);
+	double f[2] = {0.0, 0.0};
+	// pass 1: K entries and Dirichlet lifting (K_matrix, Build_matrix.c:42-115)
+	for (int s = 0; s < cnt; s++) {
+		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
+		double etag[4];
+		gauss_eta(L, vis, e, etag);
+		const double dxh = L.dxh[e], dzh = L.dzh[e], jac = L.jac[e];
+		for (int i = 0; i < 2; i++) {
+			if (!fr[i])
+				continue;
+			for (int j = 0; j < 2; j++)
+				for (int b = 0; b < 4; b++) {
+					const int B = L.ienl[b * nel + e];
+					const double kv = ke_entry(etag, dxh, dzh, jac, a, i, b, j);
+					if (vfree(L, B, j)) {
+						const int slot = L.kslot[(a * 4 + b) * nel + e];
+						double *blk = reinterpret_cast<double *>(&K[(size_t)slot * nno + A]);
+						blk[i * 2 + j] += kv;
+					} else {
+						f[i] -= kv * L.vbcval[j * nno + B];
+					}
+				}
+		}
+	}
+	stokes_load<false>(L, buoy, A, fr, f);
+	F[A] = make_double2(fr[0] ? f[0] : 0.0, fr[1] ? f[1] : 0.0);
+	stokes_diag(L, K, Kdiag, A, fr);
+}
+
+// The same for the converged solvers (K null: F alone): an element's 2 x 2 block
+// of a corner pair from four sums of eta over the Gauss points with tabulated
+// products of derivatives, about 20 FP64 operations a pair instead of 130; equal
+// to the reference's to the last bits.
+__global__ void __launch_bounds__(kBlock) k_assemble_stokes_fast(DevLevel L, const double *__restrict__ vis,
+                                                                 const double *__restrict__ buoy,
+                                                                 double4 *__restrict__ K, double2 *__restrict__ F,
+                                                                 double2 *__restrict__ Kdiag)
+{
+	const int A = blockIdx.x * blockDim.x + threadIdx.x;
+	if (A >= L.nno)
+		return;
+	const int nno = L.nno, nel = L.nel, cnt = L.p2n_cnt[A];
+	const bool fr[2] = {vfree(L, A, 0), vfree(L, A, 1)};
+	if (K)
+		for (int k = 0; k < L.nbw; k++)
+			K[(size_t)k * nno + A] = make_double4(0.0, 0.0, 0.0, 0.0);
+	double f[2] = {0.0, 0.0};
+	for (int s = 0; s < cnt; s++) {
+		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
+		int B[4];
+		bool fx[4][2], lift = false;
+#pragma unroll
+		for (int b = 0; b < 4; b++) {
+			B[b] = L.ienl[b * nel + e];
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				fx[b][j] = !vfree(L, B[b], j);
+				lift |= fx[b][j] && L.vbcval[j * nno + B[b]] != 0.0;
+			}
+		}
+		if (!K && !lift)   // a zero boundary value lifts nothing
+			continue;
+		double eg[4];
+		gauss_eta(L, vis, e, eg);
+		const double rx = L.dzh[e] / L.dxh[e], rz = L.dxh[e] / L.dzh[e];   // dzh^2/jac, dxh^2/jac
+#pragma unroll
+		for (int b = 0; b < 4; b++) {
+			double xx = 0.0, zz = 0.0, zx = 0.0, xz = 0.0;
+#pragma unroll
+			for (int g = 0; g < 4; g++) {
+				xx += eg[g] * cE.xx[a][b][g];
+				zz += eg[g] * cE.zz[a][b][g];
+				zx += eg[g] * cE.zx[a][b][g];
+				xz += eg[g] * cE.zx[b][a][g];
+			}
+			xx *= rx;
+			zz *= rz;
+			const double kv[2][2] = {{2.0 * xx + zz, zx}, {xz, 2.0 * zz + xx}};
+			const int slot = K ? L.kslot[(a * 4 + b) * nel + e] : 0;
+			double *blk = reinterpret_cast<double *>(K + ((size_t)slot * nno + A));
+#pragma unroll
+			for (int i = 0; i < 2; i++)
+#pragma unroll
+				for (int j = 0; j < 2; j++) {
+					if (!fr[i])
+						continue;
+					if (!fx[b][j]) {
+						if (K)
+							blk[i * 2 + j] += kv[i][j];
+					} else {
+						f[i] -= kv[i][j] * L.vbcval[j * nno + B[b]];
+					}
+				}
+		}
+	}
+	stokes_load<true>(L, buoy, A, fr, f);
+	F[A] = make_double2(fr[0] ? f[0] : 0.0, fr[1] ? f[1] : 0.0);
+	if (K)
+		stokes_diag(L, K, Kdiag, A, fr);
 }
 
 // BAB[e] = sum over the element's free dofs of G^2/Kdiag (Solver.c:54-64),

@@ -26,7 +26,9 @@ __global__ void k_buoy_rowavg(DevLevel L, const double *T, double Ra, double *av
 __global__ void k_buoy_vis(DevLevel L, const double *T, double Ra, const double *avg, double Aexp, double refT,
                            double lm_jump, double vmin, double vmax, double *buoy, double *vis);
 __global__ void k_assemble_stokes(DevLevel L, const double *vis, const double *buoy, double4 *K, double2 *F,
-                                  double2 *Kdiag, int withK);
+                                  double2 *Kdiag);
+__global__ void k_assemble_stokes_fast(DevLevel L, const double *vis, const double *buoy, double4 *K, double2 *F,
+                                       double2 *Kdiag);
 void upload_shape_tables_mg(const ShapeTables &s, cudaStream_t st);
 void upload_shape_tables_qt(const ShapeTables &s, cudaStream_t st);
 __global__ void k_qt_extrapolate(int n2, int ne, const double *d1, const double *d2, const double *p1, const double *p2,
@@ -568,6 +570,15 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 // History buffers of the converged solvers: the last two solutions (for
 // warm_start=3 and the learned guess) and a second candidate guess.
 // ---- the reference's own inner solvers: solver="gs" and solver="mg" ---------
+// FP64 work per node or element dominates these kernels: blocks of 64, so that a
+// small mesh's work reaches more SMs (64^2: 17 blocks of 256 threads took 77 us
+// for the load, 81 for the heat rows).
+constexpr int kSmallBlock = 64;
+static int small_blocks(size_t n)
+{
+	return (int)((n + kSmallBlock - 1) / kSmallBlock);
+}
+
 static int blocks_for(size_t n)
 {
 	return (int)((n + kBlock - 1) / kBlock);
@@ -692,7 +703,7 @@ static int ref_setup(mclg_ctx *c)
 			                                                 c->lvl_vis[k]);
 			if ((rc = check_launch(c, "k_buoy_vis")))
 				return rc;
-			k_assemble_stokes<<<blocks_for(nn), kBlock, 0, c->st>>>(L, c->lvl_vis[k], buoy, c->lvl_K[k], F, Kd, 1);
+			k_assemble_stokes<<<small_blocks(nn), kSmallBlock, 0, c->st>>>(L, c->lvl_vis[k], buoy, c->lvl_K[k], F, Kd);
 			if ((rc = check_launch(c, "k_assemble_stokes")))
 				return rc;
 			R.K = c->lvl_K[k];
@@ -1000,7 +1011,7 @@ static int qt_setup(mclg_ctx *c, QtArgs<TI> &a, Prebuilt *pre)
 		for (int d = 0; d < 2 * S.nno; d++)
 			if (S.kind[d] == 1)
 				cd.push_back(d);
-		if (cd.empty() || cd.size() > 1024) {
+		if (cd.empty() || cd.size() > (size_t)kQtMaxCoarse) {
 			mclg_set_error("the coarsest level (%d) has %zu unknowns; it needs 1..1024 (lower mg_min_level)", lo,
 			               cd.size());
 			return MCLG_BAD_INPUT;
@@ -1097,8 +1108,8 @@ static int stokes_qt_prepare(mclg_ctx *c)
 		                                                      c->cfg.mg_eta_avg, U.nno, nbu, cntu, U.X);
 		if ((rc = check_launch(c, "k_qt_inject")))
 			return rc;
-		k_assemble_stokes<<<blocks_for(L.nno), kBlock, 0, c->st>>>(L, c->lvl_vis[k], c->lvl_buoy[k], c->lvl_K[k],
-		                                                           c->lvl_F[k], c->lvl_Kd[k], 1);
+		k_assemble_stokes_fast<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->lvl_vis[k], c->lvl_buoy[k],
+		                                                                       c->lvl_K[k], c->lvl_F[k], c->lvl_Kd[k]);
 		if ((rc = check_launch(c, "k_assemble_stokes")))
 			return rc;
 	}
@@ -1717,8 +1728,11 @@ int mclg_velocity_pressure_KGF_matrix(mclg_ctx *c)
 	if (c == NULL)
 		return MCLG_BAD_INPUT;
 	const int withK = c->cfg.precision == 0 || c->qt_on;
-	k_assemble_stokes<<<blocks_for(c->L.nno), kBlock, 0, c->st>>>(c->L, c->vis, c->buoy, c->K, c->F, c->Kdiag,
-	                                                               withK);
+	if (c->cfg.precision == 0)   // the replica: the reference's operation order
+		k_assemble_stokes<<<small_blocks(c->L.nno), kSmallBlock, 0, c->st>>>(c->L, c->vis, c->buoy, c->K, c->F, c->Kdiag);
+	else                         // K for the refined-mesh solver only, the load for all
+		k_assemble_stokes_fast<<<small_blocks(c->L.nno), kSmallBlock, 0, c->st>>>(
+			c->L, c->vis, c->buoy, withK ? c->K : nullptr, c->F, c->Kdiag);
 	int rc = check_launch(c, "k_assemble_stokes");
 	if (rc || !withK)
 		return rc;
@@ -1819,7 +1833,7 @@ static int launch_uzawa(mclg_ctx *c)
 
 static int launch_stress(mclg_ctx *c)
 {
-	k_stress_elem<<<blocks_for(c->L.nel), kBlock, 0, c->st>>>(c->L, c->vis, c->V, c->stress_e);
+	k_stress_elem<<<small_blocks(c->L.nel), kSmallBlock, 0, c->st>>>(c->L, c->vis, c->V, c->stress_e);
 	int rc = check_launch(c, "k_stress_elem");
 	if (rc)
 		return rc;
@@ -1871,23 +1885,23 @@ static int launch_heat(mclg_ctx *c)
 	const mclg_config &f = c->cfg;
 	const DevLevel &L = c->L;
 	int rc;
-	k_tau<<<blocks_for(L.nel), kBlock, 0, c->st>>>(L, c->V, f.accuracy, c->tau0, c->tau1, c->mins,
+	k_tau<<<small_blocks(L.nel), kSmallBlock, 0, c->st>>>(L, c->V, f.accuracy, c->tau0, c->tau1, c->mins,
 	                                                f.precision != 0);
 	if ((rc = check_launch(c, "k_tau")))
 		return rc;
 	// the converged solvers take the heat rows with fewer FP64 operations (equal to
 	// the reference's to the last bits); the FP64 replica keeps its operation order
 	if (c->cfg.precision != 0)
-		k_assemble_heat_fast<<<blocks_for(L.nno), kBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC,
+		k_assemble_heat_fast<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC,
 		                                                              c->HF);
 	else
-		k_assemble_heat<<<blocks_for(L.nno), kBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC, c->HF);
+		k_assemble_heat<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC, c->HF);
 	if ((rc = check_launch(c, "k_assemble_heat")))
 		return rc;
 	k_heat_dt<<<blocks_for(L.nel), kBlock, 0, c->st>>>(L, c->V, c->mins);
 	if ((rc = check_launch(c, "k_heat_dt")))
 		return rc;
-	k_heat_system<<<blocks_for(L.nno), kBlock, 0, c->st>>>(L, c->mins, f.theta, c->T, c->HK, c->HC, c->HF, c->HA,
+	k_heat_system<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->mins, f.theta, c->T, c->HK, c->HC, c->HF, c->HA,
 	                                                        c->HB, c->hx, c->hidiag, c->sc);
 	if ((rc = check_launch(c, "k_heat_system")))
 		return rc;
