@@ -495,11 +495,12 @@ __device__ __forceinline__ void level_up(Sync &sy, const Splits &sp, const MGHie
 //
 // out0 = B rhs0.  *dot receives this thread's share of out0.dotv (of out0.rhs0
 // without dotv) and the cycle ends without a barrier: the caller reduces *dot,
-// which synchronises the team.
-template <class T>
+// which synchronises the team.  While the leading block works on the smallest
+// levels, the others run aside().
+template <class T, class Aside>
 __device__ __forceinline__ void vcycle(Sync &sy, SolveShared<T> &cs, const MGHier<T> &H,
                                        const typename V2T<T>::t *rhs0, typename V2T<T>::t *out0, const double2 *dotv,
-                                       double *dot)
+                                       double *dot, Aside aside)
 {
 	typedef typename V2T<T>::t V;
 	const int lc = H.nlev - 1;
@@ -513,6 +514,8 @@ __device__ __forceinline__ void vcycle(Sync &sy, SolveShared<T> &cs, const MGHie
 			level_down<T>(sy, cs.sp, H, l, rhs0, l < nb);
 	if (b0)
 		coarse_solve<T, V>(H, cs, H.lv[lc].xa);
+	else
+		aside();
 #pragma unroll 1
 	for (int l = lc - 1; l >= 0; l--) {
 		if (l == nb - 1)
@@ -561,7 +564,7 @@ __device__ __noinline__ int pcg_inner(Sync &team, SolveShared<T> &cs, const MGHi
 	int it = 0;
 	while (it < maxit) {
 		double rz[1], pq[1];
-		vcycle<T>(sy, cs, H, H.pr, H.pz, nullptr, rz);
+		vcycle<T>(sy, cs, H, H.pr, H.pz, nullptr, rz, [] {});
 		sy.reduce_then<1>(rz, [&](const double (&v)[1]) {
 			co = it > 0 ? v[0] / rho : 0.0;
 			rho = v[0];
@@ -862,7 +865,7 @@ __device__ double block_precond(const MGArgs<TI> &a, Sync &sy, SolveShared<TI> &
 	}
 	sy.sync();
 	double dot[1] = {0.0};
-	vcycle<TI>(sy, cs, H, bI, zu, vu, &dot[0]);   // the last sweep forms <z_u, v_u>
+	vcycle<TI>(sy, cs, H, bI, zu, vu, &dot[0], [] {});   // the last sweep forms <z_u, v_u>
 	for (int e = tid; e < ne; e += nth) {
 		const double z = vp[e] * a.bab[e];
 		zp[e] = z;
@@ -1053,6 +1056,14 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &team, S
 	sy.sync();
 	// index cv: z(j), v(j); 1-cv: v(j-1).  cw: w(j); 1-cw: w(j-1).  it = -1: z(0) = M^-1 v(0)
 	int cv = 1, cw = 0, it = -1;
+	// The direction update is needed only by the next one, and the pressure part of
+	// the Lanczos update by the reduction after the V-cycle: on a team they run in
+	// the V-cycle, on the blocks that would wait for the leading block's small
+	// levels (8 us of an iteration at 64^2, 17 at 1024^2).  Not where that block runs
+	// the whole cycle: its last sweep would overwrite the z that is still read.
+	// steps: the pending direction update's (-1: none).
+	const bool defer = sy.size >= 4 && H.nblk > 0;
+	int steps = -1;
 #pragma unroll 1
 	while (it < maxit) {
 		if (it >= 0) {
@@ -1075,13 +1086,31 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &team, S
 			// v(j+1) = A z~ - (delta/gam) v(j) - (gam/gam_prev) v(j-1), into v(j-1)'s
 			// buffer, its TI copy as the V-cycle's right-hand side, and z_p(j+1)
 			minres_v_nodes<VI>(nodes(), sy.tid(), sy.nth(), a.Kd, a.mv[cv], a.mv[1 - cv], H.lv[0].b, ms.ig, ms.dg, ms.gg);
-			pdot = minres_v_elems(elems(), sy.tid(), sy.nth(), a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv],
-			                      ms.ig, ms.dg, ms.gg);
+			if (!defer)
+				pdot = minres_v_elems(elems(), sy.tid(), sy.nth(), a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv],
+				                      ms.ig, ms.dg, ms.gg);
 			sy.sync();
 		}
 		double dot[1];
-		vcycle<TI>(sy, cs, H, H.lv[0].b, a.mzu[1 - cv], a.mv[1 - cv], &dot[0]);
+		vcycle<TI>(sy, cs, H, H.lv[0].b, a.mzu[1 - cv], a.mv[1 - cv], &dot[0], [&] {
+			if (!defer || it < 0)
+				return;
+			// the previous iteration's direction update (its z(j-1) and z_p(j-1) lie in
+			// the buffers that this iteration's z(j+1) overwrites: z_u after this point,
+			// z_p below by the same thread), and the pressure part of the Lanczos update
+			const Part pt{sy.rank - 1, sy.size - 1};
+			const int tid = pt.thread(), nth = pt.size * (int)blockDim.x;
+			if (steps >= 0) {
+				minres_w_nodes<VI>(steps, nodes(), tid, nth, a.mzu[1 - cv], a.mw[cw], a.mw[1 - cw], a.dd, ms.k1, ms.k3,
+				                   ms.k2, ms.step, ms.step1);
+				minres_w_elems(steps, elems(), tid, nth, a.mzp[1 - cv], a.mwp[cw], a.mwp[1 - cw], a.dpv, ms.k1, ms.k3,
+				               ms.k2, ms.step, ms.step1);
+			}
+			pdot = minres_v_elems(elems(), tid, nth, a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv], ms.ig, ms.dg,
+			                      ms.gg);
+		});
 		dot[0] += pdot;
+		pdot = 0.0;
 		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
 			const double gn2 = fmax(v[0], 0.0);
 			const double gam_next = sqrt(gn2);
@@ -1144,11 +1173,14 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &team, S
 		// into w(j-1)'s buffer; the solution takes the steps of two iterations at a time
 		// (x += step w(j) + step' w(j+1), the same additions in the same order), or what
 		// is pending when the loop ends
-		const int steps = (it & 1) ? 2 : (stop || it + 1 >= maxit) ? 1 : 0;
-		minres_w_nodes<VI>(steps, nodes(), sy.tid(), sy.nth(), a.mzu[cv], a.mw[1 - cw], a.mw[cw], a.dd, ms.k1, ms.k3,
-		                   ms.k2, ms.step, ms.step1);
-		minres_w_elems(steps, elems(), sy.tid(), sy.nth(), a.mzp[cv], a.mwp[1 - cw], a.mwp[cw], a.dpv, ms.k1, ms.k3,
-		               ms.k2, ms.step, ms.step1);
+		const bool last = stop || it + 1 >= maxit;
+		steps = (it & 1) ? 2 : last ? 1 : 0;
+		if (!defer || last) {
+			minres_w_nodes<VI>(steps, nodes(), sy.tid(), sy.nth(), a.mzu[cv], a.mw[1 - cw], a.mw[cw], a.dd, ms.k1, ms.k3,
+			                   ms.k2, ms.step, ms.step1);
+			minres_w_elems(steps, elems(), sy.tid(), sy.nth(), a.mzp[cv], a.mwp[1 - cw], a.mwp[cw], a.dpv, ms.k1, ms.k3,
+			               ms.k2, ms.step, ms.step1);
+		}
 		it++;
 		cv = 1 - cv;
 		cw = 1 - cw;
@@ -1161,8 +1193,8 @@ __device__ __noinline__ int minres_correction(const MGArgs<TI> &a, Sync &team, S
 			ms.gg = ms.gam / ms.gam_prev;
 		}
 		// no barrier here: the next operator pass reads z(j+1) and z_p(j+1),
-		// complete since the reduction, and touches none of the vectors the
-		// updates above wrote
+		// complete since the reduction, and touches none of the vectors that the
+		// updates write
 	}
 	sy.sync();
 	team = sy;
