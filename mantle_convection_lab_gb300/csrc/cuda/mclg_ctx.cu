@@ -39,9 +39,10 @@ __global__ void k_qt_inject(int n, const int *map, const double *src, double *ds
                             const int *nb_f, const unsigned char *cnt_f, const double *X_f);
 void upload_op_tables(const ShapeTables &S, double r, cudaStream_t st);
 // refined meshes: levels of at most this many nodes run in one block of the
-// solver kernel (block barriers instead of grid barriers); from a sweep on
-// configuration 2 (2048: 25.8, 512: 27.5, 128: 27.8, 0: 27.4 steps/s)
-constexpr int kQtBlockNodes = 256;
+// solver kernel (block barriers instead of team barriers); measured per MINRES
+// iteration with 64, 256, 320 and 1100 on meshes of 1347 nodes: 44.6, 42.7, 40.9
+// and 47.2 us; 8847 nodes: 81, 76, 74 and 84; 85k nodes: 130, -, 126 and 139
+constexpr int kQtBlockNodes = 320;
 void *stokes_mg_kernel(int fp64);
 void *stokes_mg_batch_kernel(int fp64);
 __global__ void k_bab(DevLevel L, const double2 *Kdiag, double *bab);
