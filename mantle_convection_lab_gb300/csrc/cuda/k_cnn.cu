@@ -42,8 +42,8 @@ struct mclg_cnn {
 	size_t part_cap;
 	cudaStream_t st;
 	// device buffers of mclg_cnn_forward and mclg_cnn_gradient, kept for the next
-	// call at the largest size asked for and freed with the network (allocating
-	// and freeing them took a third of a call); mu: one such call at a time
+	// call up to kPoolKeep bytes and freed with the network (allocating and freeing
+	// them took a third of a call); mu: one such call at a time
 	char *pool;
 	size_t pool_cap;
 	pthread_mutex_t mu;
@@ -544,6 +544,7 @@ static int cnn_backward_dev(mclg_cnn *net, CnnWork &w, const float *gy, float *g
 		if (need > net->part_cap) {
 			cudaFree(net->part);
 			net->part = nullptr;
+			net->part_cap = 0;
 			CKC(cudaMalloc((void **)&net->part, need * sizeof(float)));
 			net->part_cap = need;
 		}
@@ -970,10 +971,21 @@ struct Pool {
 		w.W = W;
 	}
 };
+// One call on a network at a time; what it needed beyond kPoolKeep is given back
+// at its end (a call that large takes longer than an allocation).
+constexpr size_t kPoolKeep = size_t(1) << 30;
 struct Lock {
-	pthread_mutex_t *m;
-	explicit Lock(pthread_mutex_t *mu) : m(mu) { pthread_mutex_lock(m); }
-	~Lock() { pthread_mutex_unlock(m); }
+	mclg_cnn *n;
+	explicit Lock(mclg_cnn *net) : n(net) { pthread_mutex_lock(&n->mu); }
+	~Lock()
+	{
+		if (n->pool_cap > kPoolKeep) {
+			cudaFree(n->pool);
+			n->pool = nullptr;
+			n->pool_cap = 0;
+		}
+		pthread_mutex_unlock(&n->mu);
+	}
 };
 }  // namespace
 
@@ -999,7 +1011,7 @@ int mclg_cnn_forward(mclg_cnn *n, const float *x, int batch, int h, int w, float
 		return rc;
 	if (x == NULL || y == NULL)
 		return MCLG_BAD_INPUT;
-	Lock lock(&n->mu);
+	Lock lock(n);
 	CnnWork wk;
 	memset(&wk, 0, sizeof wk);
 	float *dx = NULL;
@@ -1030,7 +1042,7 @@ int mclg_cnn_gradient(mclg_cnn *n, const float *x, const float *target, int batc
 		mclg_set_error("gradient buffer has %zu entries, the network %zu", count, n->nparam);
 		return MCLG_BAD_INPUT;
 	}
-	Lock lock(&n->mu);
+	Lock lock(n);
 	CnnWork wk;
 	memset(&wk, 0, sizeof wk);
 	const size_t nx = (size_t)batch * n->cin[0] * h * w, ny = (size_t)batch * n->cout[n->nl - 1] * h * w;
