@@ -3,8 +3,8 @@
 //
 // A task is a strip of 30 nodes along z (the contiguous direction of the node
 // numbering A = iz + ix*n) by a few columns along x.  A warp holds 32 nodes of
-// a column, one per lane (the 30 owned ones and one halo node at each end),
-// and walks along x: at each column every lane forms its element's corner
+// a column, one per lane (the 30 owned ones and one halo node at each end; 16 in
+// a paired task, see Split), and walks along x: at each column every lane forms its element's corner
 // forces from its own and its upper neighbour's nodal values (shuffles), adds
 // them to the two columns' accumulators, and finishes the left column's rows.
 // No shared memory, no block barrier, no atomics; every sum has a fixed order.
@@ -24,18 +24,31 @@
 // is 1.2.  The column walk issues about 120 instructions per column of 30 nodes.
 #pragma once
 
-constexpr int kOwn = 30;   // nodes of a strip that the warp owns (lanes 1..30)
+constexpr int kOwn = 30;       // nodes of a strip that the warp owns (lanes 1..30)
+constexpr int kOwnPair = 14;   // ... of a paired task (lanes 17..30)
 
 // How a level's strips and columns are cut into tasks for a number of warps;
 // formed once per solve (the divisions took a tenth of a small level's pass).
+//
+// Where every node column of 14-node strips has a warp of its own, tasks are
+// paired: the half-warps form the element columns left and right of one node
+// column at the same time and the left one's forces are handed over by shuffles,
+// in place of two steps one after the other (the same sums).  Such a level's pass
+// is a chain of dependent operations, not throughput: per iteration 129 against
+// 169 us at 128^2 in FP64, 34.3 against 37.1 at 64^2, 70.8 against 75.0 at 256^2
+// and 248 against 255 at 1024^2 in FP32.  With two paired tasks a warp the work
+// counts again (137, 36.7, 70.9 and 247 us), with four it loses everywhere.
 struct Split {
-	int strips, Lx, ntasks;
+	int strips, Lx, ntasks, pair;
 	float inv;   // 1/strips: t/strips for t < 2^22 as the truncated product with (t + 1/2)
 	__device__ void set(int n, int nwarps)
 	{
-		strips = (n + kOwn - 1) / kOwn;
+		strips = (n + kOwnPair - 1) / kOwnPair;
+		pair = strips * n <= nwarps;
+		if (!pair)
+			strips = (n + kOwn - 1) / kOwn;
 		int chunks = nwarps / strips;   // the columns are cut into as many chunks as there are warps for them
-		chunks = chunks < 1 ? 1 : chunks > n ? n : chunks;
+		chunks = chunks < 1 ? 1 : chunks > n ? n : chunks;   // (n: one column a task, when paired)
 		Lx = (n + chunks - 1) / chunks;
 		ntasks = strips * ((n + Lx - 1) / Lx);
 		inv = 1.0f / (float)strips;
@@ -115,15 +128,17 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 	const int nwarps = pt.size * (int)(blockDim.x >> 5);
 	const int strips = sp.strips, Lx = sp.Lx, ntasks = sp.ntasks;
 	const float inv = sp.inv;
+	const bool pair = sp.pair != 0;
+	const int zlane = pair ? lane & 15 : lane, zlast = pair ? 15 : 31, half = pair ? lane >> 4 : 0;
 	double dacc = 0.0, racc = 0.0, facc = 0.0;
 
 	// consecutive tasks go to different blocks, so that a small level uses many SMs
 	for (int t = (threadIdx.x >> 5) * pt.size + pt.rank; t < ntasks; t += nwarps) {
 		const int c = (int)(((float)t + 0.5f) * inv), s = t - c * strips;
-		const int gz = s * kOwn - 1 + lane, xs = c * Lx, xe = min(xs + Lx, n);
+		const int gz = s * (zlast - 1) - 1 + zlane, xs = c * Lx, xe = pair ? xs + half : min(xs + Lx, n);
 		const bool zin = gz >= 0 && gz < n;
-		const bool own = zin && lane >= 1 && lane <= kOwn;
-		const bool ein = gz >= 0 && gz < N && lane < 31;   // this lane's element lies in the box
+		const bool own = zin && zlane >= 1 && zlane < zlast;
+		const bool ein = gz >= 0 && gz < N && zlane < zlast;   // this lane's element lies in the box
 		const T pl = ein ? ip : T(0), ql = ein ? iq : T(0);
 		const int gzc = min(max(gz, 0), n - 1);
 
@@ -197,10 +212,10 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 		};
 
 		Col cur, nx, prev;
-		load(xs - 1, prev);   // the first three columns are in flight together
-		load(xs, cur);
-		load(xs + 1, nx);
-		form(xs - 1, prev);
+		load(xs - 1 + half, prev);   // the first columns are in flight together
+		load(xs + half, cur);
+		load(xs + 1 + half, nx);
+		form(xs - 1 + half, prev);
 		// left edge of the element column: this lane's and the upper neighbour's
 		// values, the viscosity at the edge's two Gauss points
 		T u0n = __shfl_down_sync(kAll, prev.x.x, 1), w0n = __shfl_down_sync(kAll, prev.x.y, 1);
@@ -211,7 +226,7 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 		double cL = 0.0, dL = 0.0;
 
 #pragma unroll 1
-		for (int ix = xs;;) {
+		for (int ix = xs + half;;) {
 			const int ex = ix - 1;
 			const bool exin = ex >= 0 && ex < N;
 			double pe = 0.0;
@@ -259,6 +274,12 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 				f2w = Rp + Hp;
 				f3w = Hm - Rp;
 			}
+			if (pair) {   // the left element column's forces on the node column, from the other half
+				lou = __shfl_xor_sync(kAll, f3u, 16);
+				low = __shfl_xor_sync(kAll, f3w, 16);
+				upu = __shfl_xor_sync(kAll, f2u, 16);
+				upw = __shfl_xor_sync(kAll, f2w, 16);
+			}
 			// the left column's rows: lower corner of this element, upper corner of the one below
 			const T su = upu + f1u, sw = upw + f1w;
 			const T fu_ = (lou + f0u) + __shfl_up_sync(kAll, su, 1), fw_ = (low + f0w) + __shfl_up_sync(kAll, sw, 1);
@@ -273,6 +294,10 @@ __device__ __forceinline__ void march(const Pass<T> &P, Part pt, const Split &sp
 				const double pd = __shfl_up_sync(kAll, pe, 1);
 				c1 = pe + pd;
 				d1 = pe - pd;
+				if (pair) {
+					cL = __shfl_xor_sync(kAll, c1, 16);
+					dL = __shfl_xor_sync(kAll, d1, 16);
+				}
 				s0 = c1 - cL;
 				s1 = d1 + dL;
 				cL = c1;
