@@ -199,20 +199,6 @@ __device__ __forceinline__ T qt_gather(const int *__restrict__ src, const T *__r
 	return s;
 }
 
-// Node B of a primal vector through the constraints, its stored values and kinds
-// in flight together.
-template <class T, class X>
-__device__ __forceinline__ typename Q2T<X>::t qt_node(const QtLevel<T> &L, const X *__restrict__ xf, int B)
-{
-	typename Q2T<X>::t v = reinterpret_cast<const typename Q2T<X>::t *>(xf)[B];
-	const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[B];
-	if (k.x != 1 || k.y != 1) {
-		v.x = k.x == 1 ? v.x : k.x == 2 ? qt_val(L, xf, 2 * B) : X(0);
-		v.y = k.y == 1 ? v.y : k.y == 2 ? qt_val(L, xf, 2 * B + 1) : X(0);
-	}
-	return v;
-}
-
 // G p at node A on the finest level: an element's entries are +-dz_deta and
 // +-dx_dxi by corner (the sums over the Gauss points that element_g forms, 8
 // FP64 operations a corner, come to one of the two half-widths).
@@ -249,25 +235,104 @@ template <class T>
 __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L, const double *__restrict__ p, int A,
                                           double &y0, double &y1)
 {
-	double y[2];
-	qt_gmul(L, p, A, y[0], y[1]);
+	const uchar2 k = reinterpret_cast<const uchar2 *>(Q.kind)[A];
+	const int f0 = Q.fo_off[2 * A], f1 = Q.fo_off[2 * A + 1], f2 = Q.fo_off[2 * A + 2];
+	qt_gmul(L, p, A, y0, y1);
+	y0 = k.x == 1 ? y0 : 0.0;
+	y1 = k.y == 1 ? y1 : 0.0;
+	// the rows of the constrained dofs that hold this node, both components' lists
+	// in one, two entries at a time with their loads in flight together
+	const int ie = k.y == 1 ? f2 : f1;
+	for (int i = k.x == 1 ? f0 : f1; i < ie; i += 2) {
+		int h[2], e[2][4], a[2][4], n[2];
+		double w[2], pe[2][4], g[2][4];
 #pragma unroll
-	for (int c = 0; c < 2; c++) {
-		const int dof = 2 * A + c;
-		if (Q.kind[dof] != 1) {
-			y[c] = 0.0;
-			continue;
+		for (int u = 0; u < 2; u++) {
+			const bool in = i + u < ie;
+			h[u] = Q.fo_dof[in ? i + u : i];
+			w[u] = in ? (double)Q.fo_w[i + u] : 0.0;
 		}
-		for (int i = Q.fo_off[dof]; i < Q.fo_off[dof + 1]; i++) {
-			const int h = Q.fo_dof[i];
-			double h0, h1;
-			qt_gmul(L, p, h >> 1, h0, h1);
-			const double hv = (h & 1) ? (vfree(L, h >> 1, 1) ? h1 : 0.0) : (vfree(L, h >> 1, 0) ? h0 : 0.0);
-			y[c] += (double)Q.fo_w[i] * hv;
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			const int B = h[u] >> 1;
+			n[u] = vfree(L, B, h[u] & 1) ? L.p2n_cnt[B] : 0;
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				e[u][q] = L.p2n_el[q * L.nno + B];
+				a[u][q] = L.p2n_a[q * L.nno + B];
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			const double *hh = (h[u] & 1) ? L.dxh : L.dzh;
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				const int eq = q < n[u] ? e[u][q] : e[u][0];
+				pe[u][q] = p[eq];
+				g[u][q] = hh[eq];
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			double s = 0.0;
+#pragma unroll
+			for (int q = 0; q < 4; q++)
+				if (q < n[u]) {
+					const bool pos = (h[u] & 1) ? (a[u][q] == 0 || a[u][q] == 3) : a[u][q] < 2;
+					s += (pos ? g[u][q] : -g[u][q]) * pe[u][q];
+				}
+			if (i + u < ie)
+				(i + u < f1 ? y0 : y1) += w[u] * s;
 		}
 	}
-	y0 = y[0];
-	y1 = y[1];
+}
+
+// Component c of an element's four corners through the constraints, x as stored
+// on entry (k: the corners' kinds).  A few elements along the edges of refinement
+// have constrained corners and would hold up the whole pass: the corners' lists go
+// two entries at a time with every corner's loads in flight together, instead of a
+// chain of three accesses for each corner and component in turn.
+template <int c, class T, class X>
+__device__ __forceinline__ void qt_constrained(const QtLevel<T> &Q, const X *__restrict__ xf, const int (&n)[4],
+                                               const uchar2 (&k)[4], X (&x)[4])
+{
+	int i0[4], i1[4];
+	bool any = false;
+#pragma unroll
+	for (int a = 0; a < 4; a++) {
+		const unsigned char ka = c ? k[a].y : k[a].x;
+		x[a] = ka == 1 ? x[a] : X(0);
+		i0[a] = i1[a] = 0;
+		if (ka == 2) {
+			i0[a] = Q.ex_off[2 * n[a] + c];
+			i1[a] = Q.ex_off[2 * n[a] + c + 1];
+			any = true;
+		}
+	}
+	while (any) {
+		int s[8];
+		X w[8], v[8];
+#pragma unroll
+		for (int q = 0; q < 8; q++) {
+			const int i = i0[q >> 1] + (q & 1);
+			const bool in = i < i1[q >> 1];
+			s[q] = in ? Q.ex_src[i] : -1;
+			w[q] = in ? (X)Q.ex_w[i] : X(0);
+		}
+#pragma unroll
+		for (int q = 0; q < 8; q++)
+			v[q] = s[q] >= 0 ? xf[s[q]] : X(0);
+		any = false;
+#pragma unroll
+		for (int a = 0; a < 4; a++) {
+			if (s[2 * a] >= 0)
+				x[a] += w[2 * a] * v[2 * a];
+			if (s[2 * a + 1] >= 0)
+				x[a] += w[2 * a + 1] * v[2 * a + 1];
+			i0[a] += 2;
+			any |= i0[a] < i1[a];
+		}
+	}
 }
 
 // (G^T C u)_e of a primal vector u (flat, X) on the finest level
@@ -276,15 +341,19 @@ __device__ __forceinline__ double qt_gt_elem(const QtLevel<T> &Q, const DevLevel
 {
 	int n[4];
 	X u[4], w[4];
+	uchar2 k[4];
 #pragma unroll
 	for (int a = 0; a < 4; a++)
 		n[a] = L.ienl[a * L.nel + e];
 #pragma unroll
 	for (int a = 0; a < 4; a++) {
-		const typename Q2T<X>::t v = qt_node(Q, uf, n[a]);
+		const typename Q2T<X>::t v = reinterpret_cast<const typename Q2T<X>::t *>(uf)[n[a]];
+		k[a] = reinterpret_cast<const uchar2 *>(Q.kind)[n[a]];
 		u[a] = v.x;
 		w[a] = v.y;
 	}
+	qt_constrained<0>(Q, uf, n, k, u);
+	qt_constrained<1>(Q, uf, n, k, w);
 	return gt_elem(u[0], u[1], u[2], u[3], w[0], w[1], w[2], w[3], L.dzh[e], L.dxh[e]);
 }
 
