@@ -92,7 +92,7 @@ WORKLOADS["cfg2_amr_128"] = {
 ENSEMBLE_METRIC = "aggregate model-steps/s at Stokes residual 1e-8"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one steady launch
 # of the workload's solver kernel, from the ncu capture summarised in profiles/
-TRAFFIC = {"cfg3_mg_1024": (45.78e9, "profiles/k_stokes_mg_f32_1024.md (one steady launch, ncu --set full)")}
+TRAFFIC = {"cfg3_mg_1024": (31.04e9, "profiles/k_stokes_mg_f32_1024.md (one steady launch, ncu)")}
 DEFAULT_WORKLOAD = "cfg3_mg_1024"
 GUESS_NET = os.path.join(ROOT, "mantle_convection_lab_gb300", "weights", "guess_cfg3.bin")
 GUESS_GRID = 128
@@ -155,7 +155,7 @@ def replica_bytes(st, neq, nno, nel, w=8):
 
 
 def converged_bytes(st, N, method=0, w=4, cheb=False, nu=2, nu_c=2, lfine=2):
-    """Mixed solver, per launch.  V-cycle: 2 nu tile passes per level (nu sweeps
+    """Mixed solver, per launch.  V-cycle: 2 nu passes per level (nu sweeps
     per side: nu on the lfine finest levels, nu_c below; read x, b, D^-1 as 2w
     each, eta w, mask 1; write 2w: 9w+1 B/node) and the transfer (restriction
     reads 9 fine residuals per coarse node, prolongation 4 coarse values per fine
@@ -166,8 +166,11 @@ def converged_bytes(st, N, method=0, w=4, cheb=False, nu=2, nu_c=2, lfine=2):
     nn plus a V-cycle; per Uzawa iteration: FP64 G s, G^T u and the pressure
     updates, 8*(4 n_v + 8 ne).
     MINRES (method 1), per iteration: a V-cycle, the TI operator (5w+1 B/node),
-    and the FP64 Lanczos, direction and solution updates with G and G^T:
-    (225 + 10w) B per node and 136 B per element.
+    and the FP64 vectors: A z written and read (32), v and v_old read, v written
+    (48) with its TI copy (2w), v read by the V-cycle's last sweep (16), the
+    direction update (48 and z in TI, 2w) and the solution's, read and written
+    every second iteration (16): 160 + 4w B per node; of the pressure 104 B per
+    element (G z_p and G^T z_u 16, Lanczos update 48, direction and solution 40).
     Per refinement pass: FP64 K d + G p residual, 8*(3 n_v + nn) + 8*3 ne."""
     nn = (N + 1) ** 2
     nv = 2 * nn
@@ -181,7 +184,7 @@ def converged_bytes(st, N, method=0, w=4, cheb=False, nu=2, nu_c=2, lfine=2):
         lev += 1
     refine = 8 * (3 * nv + nn) + 8 * 3 * ne
     if method == 1:
-        it = vcyc + (5 * w + 1) * nn + (225 + 10 * w) * nn + 136 * ne
+        it = vcyc + (5 * w + 1) * nn + (160 + 4 * w) * nn + 104 * ne
         extra_vcycles = max(st.cg_cycles - st.uzawa_cycles, 0)
         return st.uzawa_cycles * it + extra_vcycles * (vcyc + 24 * nn) + max(st.refine_passes, 1) * refine
     inner = w * (10 * nv + nn) + nn + vcyc
@@ -793,7 +796,7 @@ def run_gpu(args, wl):
         dtype = "f32 inner / f64 outer"
     else:
         alg = sum(replica_bytes(s, model.neq, nno, nel) for s in acc["stats"]) / n_launch
-        kname = "k_uzawa (persistent FP64 Uzawa/CG)"
+        kname = "k_uzawa_cluster / k_uzawa (persistent FP64 Uzawa/CG)"
         dtype = "f64"
     ms_launch = acc["ms_solver"] / n_launch
     achieved = alg / (ms_launch / 1e3) / 1e9 if ms_launch > 0 else 0.0

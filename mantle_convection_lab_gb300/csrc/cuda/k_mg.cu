@@ -1,8 +1,8 @@
 // Converged Stokes solve for uniform meshes: FP64 iterative refinement around
 // the reference's Uzawa iteration, whose inner velocity solves run as
 // multigrid-preconditioned CG in TI (float for the mixed-precision solver,
-// double for the plain FP64 one).  One persistent cooperative kernel per
-// time step; every loop has a cap.
+// double for the plain FP64 one), or preconditioned MINRES.  One persistent
+// kernel per time step (a cooperative grid or one cluster); every loop has a cap.
 //
 //   refinement (FP64):  R = [F - K d - G p ; G^T d],  stop when |R|/|F| < rtol
 //   correction:        the Uzawa loop of citcom_solver (Solver.c:14-249) on

@@ -66,7 +66,7 @@ struct MGArgs {
 	int method;                  // correction solve: 0 Uzawa with inner MG-PCG, 1 MINRES (block-diagonal preconditioner)
 	double2 *mv[2], *mw[2];      // MINRES Lanczos and direction vectors, velocity part
 	typename V2T<TI>::t *mzu[2]; // ... and the preconditioned ones, in TI (inner-CG vectors, free while MINRES runs)
-	double *mvp[2], *mzp[2], *mwp[2]; // Lanczos, preconditioned and direction vectors, pressure part (Morton)
+	double *mvp[2], *mzp[2], *mwp[2]; // Lanczos, preconditioned and direction vectors, pressure part
 	// warm_start=4: the last three solutions (h1 the most recent), or null
 	const double2 *h1d, *h2d, *h3d;
 	const double *h1p, *h2p, *h3p;

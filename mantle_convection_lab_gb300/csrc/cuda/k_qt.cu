@@ -1,5 +1,5 @@
 // Converged Stokes solve on quadtree meshes with hanging nodes; see k_qt.cuh.
-// One persistent cooperative kernel per time step.  Vectors are node layout
+// One persistent kernel per time step.  Vectors are node layout
 // (both components of a node together); a primal vector stores its reduced
 // dofs and is read through the constraints (qt_val), a dual vector (operator
 // output, residual) is zero outside the reduced dofs.

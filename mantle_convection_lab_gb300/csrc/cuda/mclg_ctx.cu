@@ -364,10 +364,11 @@ static int max_clusters(void *kern, int cs, int threads)
 
 // The blocks that solve one uniform model: a single cluster for small meshes in
 // FP32, whose iteration is a chain of barriers (0.2 us in a cluster, 1.2 in a
-// grid): per iteration 38 against 53 us at 64^2 (MINRES) and 75 against 90 at
-// 128^2 (inner CG) on 16 blocks of 512 threads, 125 against 77 at 256^2; blocks
-// of 256 threads take 38.5 and 80, 8 of them 50 and 110.  FP64 passes need the
-// whole device's FP64 pipes from 64^2 on (297 against 170 us at 128^2).
+// grid): on 16 blocks of 512 threads 34 against 44 us per MINRES iteration at 64^2
+// and 55 against 55 at 128^2, 46 against 69 and 69 against 79 per inner CG; at
+// 256^2 the grid wins (125 against 77 us when the passes took longer).  FP64 passes
+// need the whole device's FP64 pipes from 64^2 on (122 against 84 us; 59 against
+// 62 at 32^2).
 static int mg_cluster_threads(const mclg_ctx *c)
 {
 	return c->cfg.precision == 2 ? kBlock : kTeamThreads;
@@ -384,10 +385,10 @@ static void mg_team(mclg_ctx *c, void *kern)
 
 // The blocks that solve one refined model.  Up to kOneClusterNodes nodes one
 // cluster, whose barriers take 0.2 us instead of a grid's 1.2, with 512 threads a
-// block (60 against 69 us per MINRES iteration at 5125 nodes, 91 against 81 at
-// 8847); up to kSpreadNodes four times the blocks its nodes fill, so that its
-// FP64 work uses more SMs (89 against 93 us at 8847 nodes, 95 against 89 at
-// 19977, both before the gathers were chunked).
+// block (52.6 us per MINRES iteration at 5125 nodes; 76.9 at 8847, where a grid
+// takes 71.1); up to kSpreadNodes four times the blocks its nodes fill, so that its
+// work uses more SMs (71.1 against 74.7 us at 8847 nodes, 74.0 with eight times;
+// 85.3 against 82.7 at 22433).
 static void qt_team(mclg_ctx *c, void *kern, int nn)
 {
 	constexpr int kOneCluster = 16, kOneClusterNodes = 6144, kSpreadNodes = 12288;
