@@ -258,10 +258,12 @@ __global__ void __launch_bounds__(kBlock) k_assemble_stokes(DevLevel L, const do
 	stokes_diag(L, K, Kdiag, A, fr);
 }
 
-// The same for the converged solvers (K null: F alone): an element's 2 x 2 block
-// of a corner pair from four sums of eta over the Gauss points with tabulated
-// products of derivatives, about 20 FP64 operations a pair instead of 130; equal
-// to the reference's to the last bits.
+// The same for the converged solvers whose result does not follow the last bits:
+// the load of uniform meshes (K null), and K of the refined members of a batch.  An
+// element's 2 x 2 block of a corner pair from four sums of eta over the Gauss points
+// with tabulated products of derivatives, about 20 FP64 operations a pair instead of
+// 130; equal to the reference's to the last bits.  (A step of a batch of seven refined
+// members assembles 47 levels one after another: 134 us each in the reference's order.)
 __global__ void __launch_bounds__(kBlock) k_assemble_stokes_fast(DevLevel L, const double *__restrict__ vis,
                                                                  const double *__restrict__ buoy,
                                                                  double4 *__restrict__ K, double2 *__restrict__ F,

@@ -124,12 +124,52 @@ __device__ __forceinline__ void heat_rows(const DevLevel &L, const double2 *__re
 	}
 }
 
+// The same rows with the common factors taken out of the Gauss-point loop:
+// u.grad N_b per (b, g) once, one reciprocal of the Jacobian instead of a
+// division per term, and the terms multiplied by the reference's zero
+// off-diagonal conductivity dropped.  About a third of the FP64 operations of
+// heat_rows; the rows differ from the reference's in the last bits, so the FP64
+// replica keeps heat_rows.  For a single refined model, whose pressure follows the
+// last bits of the temperature that the next step starts from (see k_qt.cu).
+__device__ __forceinline__ void heat_rows_gauss(const DevLevel &L, const double2 *__restrict__ V, double t0,
+                                                double t1, int e, int a, double (&kr)[4], double (&cr)[4])
+{
+	double u1 = 0.0, u2 = 0.0;
+#pragma unroll
+	for (int b = 0; b < 4; b++) {
+		const double2 v = V[L.ienl[b * L.nel + e]];
+		u1 += v.x * 0.25;
+		u2 += v.y * 0.25;
+	}
+	const double dzh = L.dzh[e], dxh = L.dxh[e], jac = L.jac[e], ijac = 1.0 / jac;
+	double ax[4], az[4], ah[4], an[4];
+#pragma unroll
+	for (int g = 0; g < 4; g++) {
+		ax[g] = cS.dNdxi[a][g] * dzh;
+		az[g] = cS.dNdeta[a][g] * dxh;
+		ah[g] = t0 * ax[g] + t1 * az[g];
+		an[g] = cS.N[a][g];
+	}
+#pragma unroll
+	for (int b = 0; b < 4; b++) {
+		double k = 0.0, c = 0.0;
+#pragma unroll
+		for (int g = 0; g < 4; g++) {
+			const double bx = cS.dNdxi[b][g] * dzh, bz = cS.dNdeta[b][g] * dxh;
+			const double ub = u1 * bx + u2 * bz;
+			k += an[g] * ub + (ah[g] * ub + ax[g] * bx + az[g] * bz) * ijac;
+			c += (an[g] + ah[g]) * cS.N[b][g];
+		}
+		kr[b] = k;
+		cr[b] = c * jac;
+	}
+}
+
 // The same rows from the sums over the Gauss points (HeatTables): with the
 // element's velocity, artificial diffusivity and half-widths constant over it, a
 // pair of corners takes 9 FP64 operations instead of about 40 at its Gauss points
-// (FP64 runs at 1/56 of FP32 on GB300: 1.97 ms of a step at 1024^2 before).  The
-// rows differ from the reference's in the last bits, so the converged solvers use
-// them and the FP64 replica keeps heat_rows.
+// (FP64 runs at 1/56 of FP32 on GB300: 1.97 ms of a step at 1024^2 before).  For
+// the converged solvers' uniform meshes and the members of a batch.
 __device__ __forceinline__ void heat_rows_fast(const DevLevel &L, const double2 *__restrict__ V, double t0,
                                                double t1, int e, int a, double (&kr)[4], double (&cr)[4])
 {
@@ -155,7 +195,8 @@ __device__ __forceinline__ void heat_rows_fast(const DevLevel &L, const double2 
 }
 
 // One thread per node: rows of heat K, C (same slots as the Stokes blocks) and F.
-template <bool FAST>
+enum { HEAT_REFERENCE, HEAT_GAUSS, HEAT_TABLES };
+template <int ROWS>
 __device__ __forceinline__ void assemble_heat_node(DevLevel L, const double2 *__restrict__ V,
                                                    const double *__restrict__ tau0, const double *__restrict__ tau1,
                                                    double Q, double *__restrict__ HK, double *__restrict__ HC,
@@ -178,8 +219,10 @@ __device__ __forceinline__ void assemble_heat_node(DevLevel L, const double2 *__
 	for (int s = 0; s < cnt; s++) {
 		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
 		double kr[4], cr[4];
-		if (FAST)
+		if (ROWS == HEAT_TABLES)
 			heat_rows_fast(L, V, tau0[e], tau1[e], e, a, kr, cr);
+		else if (ROWS == HEAT_GAUSS)
+			heat_rows_gauss(L, V, tau0[e], tau1[e], e, a, kr, cr);
 		else
 			heat_rows(L, V, tau0[e], tau1[e], e, a, kr, cr);
 #pragma unroll
@@ -199,7 +242,7 @@ __device__ __forceinline__ void assemble_heat_node(DevLevel L, const double2 *__
 		const int e = L.p2n_el[s * nno + A], a = L.p2n_a[s * nno + A];
 		const double t0 = tau0[e], t1 = tau1[e];
 		double fa = 0.0;
-		if (FAST)   // (the shape functions sum to 1 over the Gauss points)
+		if (ROWS == HEAT_TABLES)   // (the shape functions sum to 1 over the Gauss points)
 			fa = (1.0 + t0 * L.dzh[e] * cH.sx[a] + t1 * L.dxh[e] * cH.sz[a]) * Q;
 		else
 #pragma unroll
@@ -233,7 +276,16 @@ __global__ void __launch_bounds__(kBlock) k_assemble_heat(DevLevel L, const doub
                                                           double *__restrict__ HK, double *__restrict__ HC,
                                                           double *__restrict__ HF)
 {
-	assemble_heat_node<false>(L, V, tau0, tau1, Q, HK, HC, HF);
+	assemble_heat_node<HEAT_REFERENCE>(L, V, tau0, tau1, Q, HK, HC, HF);
+}
+
+__global__ void __launch_bounds__(kBlock) k_assemble_heat_gauss(DevLevel L, const double2 *__restrict__ V,
+                                                                const double *__restrict__ tau0,
+                                                                const double *__restrict__ tau1, double Q,
+                                                                double *__restrict__ HK, double *__restrict__ HC,
+                                                                double *__restrict__ HF)
+{
+	assemble_heat_node<HEAT_GAUSS>(L, V, tau0, tau1, Q, HK, HC, HF);
 }
 
 __global__ void __launch_bounds__(kBlock) k_assemble_heat_fast(DevLevel L, const double2 *__restrict__ V,
@@ -242,7 +294,7 @@ __global__ void __launch_bounds__(kBlock) k_assemble_heat_fast(DevLevel L, const
                                                                double *__restrict__ HK, double *__restrict__ HC,
                                                                double *__restrict__ HF)
 {
-	assemble_heat_node<true>(L, V, tau0, tau1, Q, HK, HC, HF);
+	assemble_heat_node<HEAT_TABLES>(L, V, tau0, tau1, Q, HK, HC, HF);
 }
 
 // advection_dt (:135-177): min over elements of L^2 and of 0.5/(|u|/L0 + |w|/L1),

@@ -3,6 +3,15 @@
 // (both components of a node together); a primal vector stores its reduced
 // dofs and is read through the constraints (qt_val), a dual vector (operator
 // output, residual) is zero outside the reduced dofs.
+//
+// Order of operations.  The pressure's least determined modes on a mesh of many
+// refinement levels follow the rounding of the iterates: on a mesh of 85k nodes
+// half an ulp on the temperature moves P by 3e-10 .. 1.2e-8, whatever the stop that
+// FP64 allows.  So every value that reaches the iterates is formed by one fixed
+// sequence of operations, and every sum in one fixed order (QtSync), whichever team
+// runs the solve and however a pass cuts its work.  What a pass is free to choose is
+// which thread does a node's work, what is in flight together, and when a vector
+// update runs.
 #include <math.h>
 #include "k_qt.cuh"
 #include "fp64_util.cuh"
@@ -173,8 +182,24 @@ __device__ __forceinline__ void qt_kr_node(const QtLevel<TI> &L, const TI *__res
 	qt_kr_node_src(L, src, A, y0, y1);
 }
 
-// s = sum of w[i] x[src[i]] over [i0, i1), C entries at a time: their indices,
-// then their gathers in flight together (a list's loop waits for both in turn).
+__device__ __forceinline__ float madd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double madd(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// a b - c d - e f, as every recurrence of vectors here rounds it
+__device__ __forceinline__ double lin3(double a, double b, double c, double d, double e, double f)
+{
+	return __fma_rn(-e, f, __fma_rn(a, b, -__dmul_rn(c, d)));
+}
+
+// acc + (a b + c d), as every sum of products over nodes rounds it
+__device__ __forceinline__ double add2(double acc, double a, double b, double c, double d)
+{
+	return __dadd_rn(acc, __fma_rn(a, b, __dmul_rn(c, d)));
+}
+
+// s = sum of w[i] x[src[i]] over [i0, i1) in the list's order, C entries at a time:
+// their indices, then their gathers in flight together (a list's loop waits for
+// both in turn).
 template <int C, class T>
 __device__ __forceinline__ T qt_gather(const int *__restrict__ src, const T *__restrict__ w, const T *__restrict__ x,
                                        int i0, int i1)
@@ -194,15 +219,42 @@ __device__ __forceinline__ T qt_gather(const int *__restrict__ src, const T *__r
 			xv[u] = x[j[u]];
 #pragma unroll
 		for (int u = 0; u < C; u++)
-			s += i + u < i1 ? ww[u] * xv[u] : T(0);
+			s = i + u < i1 ? madd(ww[u], xv[u], s) : s;
 	}
 	return s;
 }
 
-// G p at node A on the finest level: an element's entries are +-dz_deta and
-// +-dx_dxi by corner (the sums over the Gauss points that element_g forms, 8
-// FP64 operations a corner, come to one of the two half-widths).
-__device__ __forceinline__ void qt_gmul(const DevLevel &L, const double *__restrict__ p, int A, double &y0, double &y1)
+// G's entries of an element (element_g) by corner: the magnitudes of component 0 are
+// those of corners 0 (0 and 3) and 1 (1 and 2), of component 1 those of corners 0
+// (0 and 1) and 2 (2 and 3); the sums over the Gauss points that give them run
+// through the same products in the same order.  8 FP64 operations a corner, formed
+// once per solve (a.ge[4 e ..]) instead of at every corner that an iteration visits.
+// They are the half-widths to within their last bit.
+__device__ __forceinline__ void qt_g_table(const DevLevel &L, int e, double *ge)
+{
+	double g0, g1, h0, h1, k0, k1;
+	element_g(cS, L.dzh[e], L.dxh[e], 0, g0, g1);
+	element_g(cS, L.dzh[e], L.dxh[e], 1, h0, h1);
+	element_g(cS, L.dzh[e], L.dxh[e], 2, k0, k1);
+	ge[4 * (size_t)e] = g0;
+	ge[4 * (size_t)e + 1] = h0;
+	ge[4 * (size_t)e + 2] = g1;
+	ge[4 * (size_t)e + 3] = -k1;
+}
+template <int c>
+__device__ __forceinline__ int qt_g_slot(int a)
+{
+	return c ? 2 + (a >> 1) : (a == 1 || a == 2);
+}
+template <int c>
+__device__ __forceinline__ bool qt_g_pos(int a)
+{
+	return c ? a == 0 || a == 3 : a < 2;
+}
+
+// G p at node A on the finest level, its elements in order (gmul_node).
+__device__ __forceinline__ void qt_gmul(const DevLevel &L, const double *__restrict__ ge, const double *__restrict__ p,
+                                        int A, double &y0, double &y1)
 {
 	double s0 = 0.0, s1 = 0.0;
 	const int n = L.p2n_cnt[A];
@@ -212,19 +264,20 @@ __device__ __forceinline__ void qt_gmul(const DevLevel &L, const double *__restr
 		e[k] = L.p2n_el[k * L.nno + A];
 		a[k] = L.p2n_a[k * L.nno + A];
 	}
-	double pe[4], hz[4], hx[4];
+	double pe[4], h0[4], h1[4];
 #pragma unroll
 	for (int k = 0; k < 4; k++) {
-		const int ek = k < n ? e[k] : e[0];
+		const int ek = k < n ? e[k] : e[0], ak = k < n ? a[k] : 0;
+		const double *g = ge + 4 * (size_t)ek;
 		pe[k] = p[ek];
-		hz[k] = L.dzh[ek];
-		hx[k] = L.dxh[ek];
+		h0[k] = g[qt_g_slot<0>(ak)];
+		h1[k] = g[qt_g_slot<1>(ak)];
 	}
 #pragma unroll
 	for (int k = 0; k < 4; k++)
 		if (k < n) {
-			s0 += (a[k] < 2 ? hz[k] : -hz[k]) * pe[k];
-			s1 += (a[k] == 0 || a[k] == 3 ? hx[k] : -hx[k]) * pe[k];
+			s0 = madd(qt_g_pos<0>(a[k]) ? h0[k] : -h0[k], pe[k], s0);
+			s1 = madd(qt_g_pos<1>(a[k]) ? h1[k] : -h1[k], pe[k], s1);
 		}
 	y0 = s0;
 	y1 = s1;
@@ -232,12 +285,12 @@ __device__ __forceinline__ void qt_gmul(const DevLevel &L, const double *__restr
 
 // (C^T G p) at both dofs of node A (FP64, the finest level)
 template <class T>
-__device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L, const double *__restrict__ p, int A,
-                                          double &y0, double &y1)
+__device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L, const double *__restrict__ ge,
+                                          const double *__restrict__ p, int A, double &y0, double &y1)
 {
 	const uchar2 k = reinterpret_cast<const uchar2 *>(Q.kind)[A];
 	const int f0 = Q.fo_off[2 * A], f1 = Q.fo_off[2 * A + 1], f2 = Q.fo_off[2 * A + 2];
-	qt_gmul(L, p, A, y0, y1);
+	qt_gmul(L, ge, p, A, y0, y1);
 	y0 = k.x == 1 ? y0 : 0.0;
 	y1 = k.y == 1 ? y1 : 0.0;
 	// the rows of the constrained dofs that hold this node, both components' lists
@@ -264,12 +317,13 @@ __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L
 		}
 #pragma unroll
 		for (int u = 0; u < 2; u++) {
-			const double *hh = (h[u] & 1) ? L.dxh : L.dzh;
+			const int c = h[u] & 1;
 #pragma unroll
 			for (int q = 0; q < 4; q++) {
-				const int eq = q < n[u] ? e[u][q] : e[u][0];
+				const bool in = q < n[u];
+				const int eq = in ? e[u][q] : e[u][0], aq = in ? a[u][q] : 0;
 				pe[u][q] = p[eq];
-				g[u][q] = hh[eq];
+				g[u][q] = ge[4 * (size_t)eq + (c ? qt_g_slot<1>(aq) : qt_g_slot<0>(aq))];
 			}
 		}
 #pragma unroll
@@ -278,11 +332,15 @@ __device__ __forceinline__ void qt_g_node(const QtLevel<T> &Q, const DevLevel &L
 #pragma unroll
 			for (int q = 0; q < 4; q++)
 				if (q < n[u]) {
-					const bool pos = (h[u] & 1) ? (a[u][q] == 0 || a[u][q] == 3) : a[u][q] < 2;
-					s += (pos ? g[u][q] : -g[u][q]) * pe[u][q];
+					const bool pos = (h[u] & 1) ? qt_g_pos<1>(a[u][q]) : qt_g_pos<0>(a[u][q]);
+					s = madd(pos ? g[u][q] : -g[u][q], pe[u][q], s);
 				}
-			if (i + u < ie)
-				(i + u < f1 ? y0 : y1) += w[u] * s;
+			if (i + u < ie) {
+				if (i + u < f1)
+					y0 = madd(w[u], s, y0);
+				else
+					y1 = madd(w[u], s, y1);
+			}
 		}
 	}
 }
@@ -326,22 +384,25 @@ __device__ __forceinline__ void qt_constrained(const QtLevel<T> &Q, const X *__r
 #pragma unroll
 		for (int a = 0; a < 4; a++) {
 			if (s[2 * a] >= 0)
-				x[a] += w[2 * a] * v[2 * a];
+				x[a] = madd(w[2 * a], v[2 * a], x[a]);
 			if (s[2 * a + 1] >= 0)
-				x[a] += w[2 * a + 1] * v[2 * a + 1];
+				x[a] = madd(w[2 * a + 1], v[2 * a + 1], x[a]);
 			i0[a] += 2;
 			any |= i0[a] < i1[a];
 		}
 	}
 }
 
-// (G^T C u)_e of a primal vector u (flat, X) on the finest level
+// (G^T C u)_e of a primal vector u (flat, X) on the finest level, in FP64: the
+// corners in ascending order of their equations.
 template <class T, class X>
-__device__ __forceinline__ double qt_gt_elem(const QtLevel<T> &Q, const DevLevel &L, const X *__restrict__ uf, int e)
+__device__ __forceinline__ double qt_gt_elem(const QtLevel<T> &Q, const DevLevel &L, const double *__restrict__ ge,
+                                             const X *__restrict__ uf, int e)
 {
 	int n[4];
 	X u[4], w[4];
 	uchar2 k[4];
+	double g[4];
 #pragma unroll
 	for (int a = 0; a < 4; a++)
 		n[a] = L.ienl[a * L.nel + e];
@@ -352,10 +413,182 @@ __device__ __forceinline__ double qt_gt_elem(const QtLevel<T> &Q, const DevLevel
 		u[a] = v.x;
 		w[a] = v.y;
 	}
+	{
+		const double2 *g2 = reinterpret_cast<const double2 *>(ge) + 2 * (size_t)e;
+		const double2 ga = g2[0], gb = g2[1];
+		g[0] = ga.x;
+		g[1] = ga.y;
+		g[2] = gb.x;
+		g[3] = gb.y;
+	}
 	qt_constrained<0>(Q, uf, n, k, u);
 	qt_constrained<1>(Q, uf, n, k, w);
-	return gt_elem(u[0], u[1], u[2], u[3], w[0], w[1], w[2], w[3], L.dzh[e], L.dxh[e]);
+	double s = 0.0;
+#pragma unroll
+	for (int q = 0; q < 4; q++) {
+		const int a = q < 2 ? q : 5 - q;   // kSortedCorner: 0, 1, 3, 2
+		const double g0 = g[qt_g_slot<0>(a)], g1 = g[qt_g_slot<1>(a)];
+		s = madd(qt_g_pos<0>(a) ? g0 : -g0, widen(u[a]), s);
+		s = madd(qt_g_pos<1>(a) ? g1 : -g1, widen(w[a]), s);
+	}
+	return s;
 }
+
+// ---- sums over the team -----------------------------------------------------------
+// The order of a single model's sums is that of blocks of 256 threads that take the
+// nodes, then the elements, in their own order: butterflies over 32 threads (distances
+// 16 .. 1), over a block's eight warps (4, 2, 1), and over the blocks (the same tree
+// over blocks 0 .. 255, those from 256 on added to them first).  A grid runs just so:
+// id() numbers its threads.  A cluster deals its warps over 16 blocks of 512 threads,
+// each node having a thread of its own, and runs its sums through the same tree.
+// A batch's teams, whose size is chosen by timing them, sum in the order of their own.
+constexpr int kQtPartials = 3 * (kTeamThreads / 32);   // a block's partials of one reduction
+struct QtSync : Sync {
+	static constexpr int kWarps = kTeamThreads / 32, kPad = 36;   // (stride 36: warps 0 .. 3 in different banks)
+	bool single;   // a single model (else a batch)
+	__device__ static double *scratch()
+	{
+		__shared__ double sh[3 * kWarps * kPad];
+		return sh;
+	}
+	__device__ int id() const { return mode == SYNC_GRID ? rank * (int)blockDim.x + (int)threadIdx.x : tid(); }
+	// f(sums) on thread 0 of each block; what it writes to shared memory is visible
+	// to the block on return.  A warp takes eight warps' values through shared memory,
+	// so that the halves that a butterfly would drop cost nothing: 12 FP64 additions
+	// of one warp for a block of 256 instead of 40 (the FP64 pipe has two lanes per
+	// clock and SM).
+	template <int NV, class F>
+	__device__ __forceinline__ void reduce_then(const double (&v)[NV], F f)
+	{
+		static_assert(NV <= 3, "scratch");
+		double *sh = scratch();
+		const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			sh[(k * kWarps + w) * kPad + lane] = v[k];
+		__syncthreads();
+		double t[NV];
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			t[k] = 0.0;
+		if (w < (int)(blockDim.x >> 8)) {   // warp w: the sums of warps 8 w .. 8 w + 7, four lanes each
+#pragma unroll
+			for (int k = 0; k < NV; k++) {
+				const double *s = sh + (k * kWarps + 8 * w + (lane >> 2)) * kPad + (lane & 3);
+				t[k] = ((s[0] + s[16]) + (s[8] + s[24])) + ((s[4] + s[20]) + (s[12] + s[28]));
+				t[k] += __shfl_xor_sync(0xffffffffu, t[k], 2);
+				t[k] += __shfl_xor_sync(0xffffffffu, t[k], 1);
+			}
+		}
+		if (single && mode == SYNC_CLUSTER) {
+			// partials[flip][k][warp]; group g of 32 threads is warp g / 16 of block g % 16
+			double *mine = partials + flip * kQtPartials;
+			if (w < 2 && (lane & 3) == 0)
+#pragma unroll
+				for (int k = 0; k < NV; k++)
+					mine[k * kWarps + 8 * w + (lane >> 2)] = t[k];
+			cg::cluster_group cl = cg::this_cluster();
+			cl.sync();
+			if (w == 0) {   // lane b: groups 8 b .. 8 b + 7
+#pragma unroll
+				for (int k = 0; k < NV; k++) {
+					double x[8];
+#pragma unroll
+					for (int q = 0; q < 8; q++)
+						x[q] = cl.map_shared_rank(mine, (lane & 1) * 8 + q)[k * kWarps + (lane >> 1)];
+					t[k] = warp_sum(((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7])));
+				}
+			}
+			flip ^= 1;
+		} else {
+			if (w == 0)
+#pragma unroll
+				for (int k = 0; k < NV; k++)
+					t[k] = eight(t[k]);
+			if (mode == SYNC_GRID) {
+				double *buf = partials + (size_t)flip * kMaxCoopBlocks * kRedWidth;
+				if (threadIdx.x == 0)
+#pragma unroll
+					for (int k = 0; k < NV; k++)
+						buf[k * kMaxCoopBlocks + rank] = t[k];
+				cg::this_grid().sync();
+				if (w == 0) {
+#pragma unroll
+					for (int k = 0; k < NV; k++) {
+						const double *src = buf + k * kMaxCoopBlocks;
+						const int b0 = (lane >> 2) * 32 + (lane & 3);
+						double x[8];
+#pragma unroll
+						for (int m = 0; m < 8; m++)
+							x[m] = b0 + 4 * m < size ? src[b0 + 4 * m] : 0.0;
+						for (int o = 256; o < size; o += 256) {
+							double y[8];
+#pragma unroll
+							for (int m = 0; m < 8; m++)
+								y[m] = o + b0 + 4 * m < size ? src[o + b0 + 4 * m] : 0.0;
+#pragma unroll
+							for (int m = 0; m < 8; m++)
+								x[m] += y[m];
+						}
+						double s = ((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7]));
+						s += __shfl_xor_sync(0xffffffffu, s, 2);
+						s += __shfl_xor_sync(0xffffffffu, s, 1);
+						t[k] = eight(s);
+					}
+				}
+				flip ^= 1;
+			} else if (mode == SYNC_CLUSTER) {
+				double *mine = partials + flip * kQtPartials;
+				if (threadIdx.x == 0)
+#pragma unroll
+					for (int k = 0; k < NV; k++)
+						mine[k] = t[k];
+				cg::cluster_group cl = cg::this_cluster();
+				cl.sync();
+				if (w == 0) {
+					const double *other = cl.map_shared_rank(mine, lane < size ? lane : 0);
+#pragma unroll
+					for (int k = 0; k < NV; k++) {
+						t[k] = warp_sum(lane < size ? other[k] : 0.0);
+					}
+				}
+				flip ^= 1;   // the next reduction writes the other buffer (see GridRed)
+			}
+		}
+		if (threadIdx.x == 0)
+			f(t);
+		__syncthreads();
+	}
+	// The sums in every thread.
+	template <int NV>
+	__device__ __forceinline__ void reduce(double (&v)[NV])
+	{
+		__shared__ double out[NV];
+		reduce_then<NV>(v, [&](const double (&t)[NV]) {
+#pragma unroll
+			for (int k = 0; k < NV; k++)
+				out[k] = t[k];
+		});
+#pragma unroll
+		for (int k = 0; k < NV; k++)
+			v[k] = out[k];
+	}
+	// the sum over eight warps from lanes of four each
+	static __device__ double eight(double v)
+	{
+		v += __shfl_xor_sync(0xffffffffu, v, 16);
+		v += __shfl_xor_sync(0xffffffffu, v, 8);
+		v += __shfl_xor_sync(0xffffffffu, v, 4);
+		return v;
+	}
+	static __device__ QtSync of(int mode, double *partials, int rank, int size, bool single)
+	{
+		QtSync s;
+		static_cast<Sync &>(s) = Sync::of(mode, partials, rank, size);
+		s.single = single;
+		return s;
+	}
+};
 
 // ---- the V-cycle (TI) -------------------------------------------------------------
 // One damped Jacobi sweep on the constrained operator: xo = xi + w D^-1 (b - A xi),
@@ -394,7 +627,7 @@ __device__ __forceinline__ void qt_sweep(const QtLevel<TI> &L, TI omega, const t
 // or its leading block alone for the smallest levels (block barriers instead
 // of team barriers).
 struct QtTeam {
-	Sync *sy;
+	QtSync *sy;
 	bool wide;
 	int tid, nth;
 	__device__ void sync()
@@ -473,9 +706,9 @@ __device__ __forceinline__ void qt_down(const QtHier<TI> &H, int l, QtTeam &t)
 }
 
 // Level l on the way up: prolongation of level l-1's result added, smoothing.
-// With zout (the finest level) the last sweep writes there, adds this thread's
-// share of zout.v to *dot and is not followed by a barrier: the caller's
-// reduction provides it.
+// With zout (the finest level) the last sweep writes there and leaves this thread's
+// share of zout.v in *dot (nodes by QtSync::id), and is not followed by a barrier:
+// the caller's reduction provides it.
 template <class TI>
 __device__ __forceinline__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t, typename Q2T<TI>::t *zout = nullptr,
                                       const double2 *v = nullptr, double *dot = nullptr)
@@ -496,13 +729,13 @@ __device__ __forceinline__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t, typ
 		if (zout != nullptr && s == H.smooth - 1) {
 			const QtXStored<TI> src{L.x[cur]};
 			double acc = 0.0;
-			for (int A = t.tid; A < L.nno; A += t.nth) {
+			for (int A = t.sy->id(); A < L.nno; A += t.nth) {
 				const double2 va = v[A];
 				const V o = qt_sweep_node(L, H.omega, src, A);
 				zout[A] = o;
-				acc += widen(o.x) * va.x + widen(o.y) * va.y;
+				acc = add2(acc, widen(o.x), va.x, widen(o.y), va.y);
 			}
-			*dot += acc;
+			*dot = acc;
 			return;
 		}
 		qt_sweep(L, H.omega, L.x[cur], L.x[1 - cur], t.tid, t.nth);
@@ -511,9 +744,11 @@ __device__ __forceinline__ void qt_up(const QtHier<TI> &H, int l, QtTeam &t, typ
 	}
 }
 
-// coarsest level: the dense inverse on its reduced dofs, a warp per four rows
-// with its lanes along them (a thread per row read the matrix in columns 4*nc
-// bytes apart: 8.3 us of a 128 us iteration for 126 unknowns)
+// coarsest level: the dense inverse on its reduced dofs, a thread per row, each row's
+// products in order.  The inverse is stored by columns, so that a warp's rows are
+// adjacent (by rows, 4*nc bytes apart, it took 8.3 us of a 128 us iteration for 126
+// unknowns, now 3 .. 4), and sixteen columns are in flight together; more of them, or
+// the next sixteen ahead, cost the solver its registers (133 .. 160 against 124 us).
 template <class TI>
 __device__ __forceinline__ void qt_coarse_solve(const QtHier<TI> &H, QtTeam &t)
 {
@@ -521,38 +756,33 @@ __device__ __forceinline__ void qt_coarse_solve(const QtHier<TI> &H, QtTeam &t)
 	const QtLevel<TI> &C = H.lv[0];
 	const TI *bf = reinterpret_cast<const TI *>(C.b);
 	TI *xf = reinterpret_cast<TI *>(C.x[0]);
-	const int nc = H.nc, lane = threadIdx.x & 31;
+	const int nc = H.nc;
 	for (int j = threadIdx.x; j < nc; j += blockDim.x)
 		sb[j] = bf[H.cdof[j]];
 	__syncthreads();
-	for (int i0 = 4 * (t.tid >> 5); i0 < nc; i0 += 4 * (t.nth >> 5)) {
-		TI s[4] = {TI(0), TI(0), TI(0), TI(0)};
-		const TI *row = H.cinv + (size_t)i0 * nc;
-#pragma unroll 4
-		for (int j = lane; j < nc; j += 32) {
-			const TI b = sb[j];
+	constexpr int kCols = 16;
+	for (int i = t.tid; i < nc; i += t.nth) {
+		TI s = TI(0);
+		for (int j0 = 0; j0 < nc; j0 += kCols) {
+			TI m[kCols];
 #pragma unroll
-			for (int u = 0; u < 4; u++)
-				if (i0 + u < nc)
-					s[u] += row[(size_t)u * nc + j] * b;
+			for (int u = 0; u < kCols; u++)
+				m[u] = j0 + u < nc ? H.cinv[(size_t)(j0 + u) * nc + i] : TI(0);
+#pragma unroll
+			for (int u = 0; u < kCols; u++)
+				if (j0 + u < nc)
+					s = madd(m[u], sb[j0 + u], s);
 		}
-#pragma unroll
-		for (int u = 0; u < 4; u++) {
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-			if (lane == u && i0 + u < nc)
-				xf[H.cdof[i0 + u]] = s[u];
-		}
+		xf[H.cdof[i]] = s;
 	}
 	t.sync();
 }
 
 // z = V-cycle(b) with b in the finest level's b; *dot receives this thread's
-// share of z.v.  Ends without a barrier (the caller's reduction follows).  While
+// share of z.v (nodes by QtSync::id).  Ends without a barrier (the caller's reduction follows).  While
 // the leading block works on the smallest levels, the others run aside().
 template <class TI, class Aside>
-__device__ __forceinline__ void qt_vcycle(Sync &sy, const QtHier<TI> &H, typename Q2T<TI>::t *z, const double2 *v,
+__device__ __forceinline__ void qt_vcycle(QtSync &sy, const QtHier<TI> &H, typename Q2T<TI>::t *z, const double2 *v,
                                           double *dot, Aside aside)
 {
 	typedef typename Q2T<TI>::t V;
@@ -584,78 +814,112 @@ __device__ __forceinline__ void qt_vcycle(Sync &sy, const QtHier<TI> &H, typenam
 		qt_up(H, l, team, l == top ? z : nullptr, v, dot);
 	if (top == 0) {   // the dense solve is the whole cycle
 		const QtLevel<TI> &Q = H.lv[0];
-		for (int A = team.tid; A < Q.nno; A += team.nth) {
+		for (int A = sy.id(); A < Q.nno; A += team.nth) {
 			const V o = Q.x[0][A];
 			const double2 va = v[A];
 			z[A] = o;
-			*dot += widen(o.x) * va.x + widen(o.y) * va.y;
+			*dot = add2(*dot, widen(o.x), va.x, widen(o.y), va.y);
 		}
 	}
 }
 
+// Entry (row dof d, column dof j) of C^T K C on a level: qt_op_node applied to the
+// unit vector of j.
+template <class T>
+__device__ double qt_unit_val(const QtLevel<T> &L, int dof, int j)
+{
+	const unsigned char k = L.kind[dof];
+	if (k == 1)
+		return dof == j ? 1.0 : 0.0;
+	double s = 0.0;
+	if (k == 2)
+		for (int i = L.ex_off[dof]; i < L.ex_off[dof + 1]; i++)
+			if (L.ex_src[i] == j)
+				s += (double)L.ex_w[i];
+	return s;
+}
+template <class T>
+__device__ double qt_unit_row(const QtLevel<T> &L, int d, int j)
+{
+	const int A = d >> 1, n = L.cnt[A];
+	double s = 0.0;
+	for (int k = 0; k < n; k++) {
+		const int B = L.nb[(size_t)k * L.nno + A] & ~kQtCon;
+		const double4 kb = L.K64[(size_t)k * L.nno + A];
+		const double x = qt_unit_val(L, 2 * B, j), y = qt_unit_val(L, 2 * B + 1, j);
+		s += (d & 1) ? kb.z * x + kb.w * y : kb.x * x + kb.y * y;
+	}
+	return s;
+}
+template <class T>
+__device__ __noinline__ double qt_unit_entry(const QtLevel<T> &L, int d, int j)
+{
+	double y = qt_unit_row(L, d, j);
+	for (int i = L.fo_off[d]; i < L.fo_off[d + 1]; i++)
+		y = madd((double)L.fo_w[i], qt_unit_row(L, L.fo_dof[i], j), y);
+	return y;
+}
+
 // Dense inverse of the coarsest level's constrained operator on its reduced
-// dofs (FP64): the rows of C^T K C from their contribution lists, inverted by
-// Gauss-Jordan (SPD: no pivoting) by the whole team, a warp per row.  The matrix
-// alternates between two buffers, so that a pivot takes one team barrier.  One
-// block alone took 1.1 ms per solve at 126 unknowns: an FP64 inversion of that
-// size is 2 million multiply-adds on one SM's two FP64 lanes.
+// dofs (FP64), by Gauss-Jordan (SPD: no pivoting) by the whole team, a warp per
+// row: the pivot's row divided by the pivot, then taken from the others.  The
+// matrix alternates between two buffers, so that a pivot takes one team barrier;
+// the warp that forms the next pivot's row divides it as well (every warp dividing
+// it for itself cost a batch's cluster 6 us of its FP64 pipes a pivot).  One block
+// alone took 1.1 ms per solve at 126 unknowns: an FP64 inversion of that size is 2
+// million multiply-adds on one SM's two FP64 lanes.
 template <class TI>
-__device__ __noinline__ void qt_coarse_build(Sync &sy, const QtHier<TI> &H)
+__device__ __noinline__ void qt_coarse_build(QtSync &sy, const QtHier<TI> &H)
 {
 	const QtLevel<TI> &C = H.lv[0];
 	const int nc = H.nc, tid = sy.tid(), nth = sy.nth(), lane = threadIdx.x & 31;
-	double *M = H.cwork, *N = H.cwork + (size_t)nc * nc, *at = H.cvec;   // at: a dof's row, -1 off the reduced dofs
-	const double *K64f = reinterpret_cast<const double *>(C.K64);
+	const size_t n2 = (size_t)nc * nc;
+	double *M = H.cwork, *N = M + n2, *pk = N + n2, *pn = pk + nc;   // pk, pn: this pivot's row divided, the next one's
 	for (int k = tid; k < nc * nc; k += nth)
-		M[k] = 0.0;
-	for (int k = tid; k < 2 * C.nno; k += nth)
-		at[k] = -1.0;
+		M[k] = qt_unit_entry(C, H.cdof[k / nc], H.cdof[k % nc]);
 	sy.sync();
-	for (int j = tid; j < nc; j += nth)
-		at[H.cdof[j]] = (double)j;
-	sy.sync();
-	for (int A = tid; A < C.nno; A += nth) {
-		const int i1 = C.rc_off[A + 1];
-		for (int i = C.rc_off[A]; i < i1;) {
-			const int t = C.rc_tgt[i], slot = t >> 2, cc = t & 3;
-			double v = 0.0;
-			for (; i < i1 && C.rc_tgt[i] == t; i++)
-				v += (double)C.rc_w[i] * K64f[C.rc_src[i]];
-			const int r = (int)at[2 * A + (cc >> 1)], c = (int)at[2 * C.rnb[(size_t)slot * C.nno + A] + (cc & 1)];
-			if (r >= 0 && c >= 0)
-				M[(size_t)r * nc + c] = v;
-		}
-	}
+	if (tid >> 5 == 0)
+		for (int c = lane; c < nc; c += 32)
+			pk[c] = (c == 0 ? 1.0 : M[c]) / M[0];
 	sy.sync();
 	for (int k = 0; k < nc; k++) {
-		const double *pk = M + (size_t)k * nc;
-		const double ip = (tid >> 5) < nc ? 1.0 / pk[k] : 0.0;   // (warps with rows only: see QtScal)
 		for (int r = tid >> 5; r < nc; r += nth >> 5) {
 			const double *row = M + (size_t)r * nc;
 			double *out = N + (size_t)r * nc;
-			const double f = row[k] * ip;
+			const double f = row[k];
+			auto entry = [&](int c) {
+				const double p = pk[c], m = c == k ? 0.0 : row[c];
+				return r == k ? p : f != 0.0 ? madd(-f, p, m) : m;
+			};
+			const bool next = r == k + 1;
+			const double piv = next ? entry(r) : 1.0;
 #pragma unroll 4
 			for (int c = lane; c < nc; c += 32) {
-				const double p = pk[c], m = row[c];
-				out[c] = r == k ? (c == k ? ip : p * ip) : (c == k ? -f : m - f * p);
+				const double v = entry(c);
+				out[c] = v;
+				if (next)
+					pn[c] = (c == r ? 1.0 : v) / piv;
 			}
 		}
 		sy.sync();
 		double *t = M;
 		M = N;
 		N = t;
+		t = pk;
+		pk = pn;
+		pn = t;
 	}
 	for (int k = tid; k < nc * nc; k += nth)
-		H.cinv[k] = (TI)M[k];
+		H.cinv[(size_t)(k % nc) * nc + k / nc] = (TI)M[k];   // by columns
 	sy.sync();
 }
 
 // ---- FP64 residual and the preconditioner ------------------------------------------
 // R = [C^T (F - K d - G p) ; G^T C d] (FP64); rs = |R_m|^2, |R_c|^2, |C^T F|^2.
 template <class TI>
-__device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, const double *p, double (&rs)[3])
+__device__ void qt_residual(QtSync &sy, const QtArgs<TI> &a, const double2 *d, const double *p, double (&rs)[3])
 {
-	const int tid = sy.tid(), nth = sy.nth();
+	const int tid = sy.id(), nth = sy.nth();
 	const DevLevel &L = a.L;
 	const QtLevel<TI> &Q = a.H.lv[a.H.nlev - 1];
 	const double *df = reinterpret_cast<const double *>(d);
@@ -664,7 +928,7 @@ __device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, con
 	for (int A = tid; A < L.nno; A += nth) {
 		double k0, k1, g0, g1;
 		qt_op_node(Q, Q.K64, df, A, k0, k1);
-		qt_g_node(Q, L, p, A, g0, g1);
+		qt_g_node(Q, L, a.ge, p, A, g0, g1);
 		double f[2] = {0.0, 0.0};
 		for (int c = 0; c < 2; c++) {   // C^T F
 			const int dof = 2 * A + c;
@@ -677,13 +941,13 @@ __device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, con
 		const double2 r = make_double2(Q.kind[2 * A] == 1 ? f[0] - k0 - g0 : 0.0,
 		                               Q.kind[2 * A + 1] == 1 ? f[1] - k1 - g1 : 0.0);
 		a.R[A] = r;
-		rs[0] += r.x * r.x + r.y * r.y;
-		rs[2] += f[0] * f[0] + f[1] * f[1];
+		rs[0] = add2(rs[0], r.x, r.x, r.y, r.y);
+		rs[2] = add2(rs[2], f[0], f[0], f[1], f[1]);
 	}
 	for (int e = tid; e < L.nel; e += nth) {
-		const double c = qt_gt_elem(Q, L, df, e);
+		const double c = qt_gt_elem(Q, L, a.ge, df, e);
 		a.Rc[e] = c;
-		rs[1] += c * c;
+		rs[1] = madd(c, c, rs[1]);
 	}
 	sy.reduce<3>(rs);
 }
@@ -693,7 +957,9 @@ __device__ void qt_residual(Sync &sy, const QtArgs<TI> &a, const double2 *d, con
 // microsecond each.
 struct QtScal {
 	double gam, gam_prev, eta, eta0, delta, c_prev, c_cur, s_prev, s_cur;
-	double ig, dg, gg, k1, k2, k3, step, step1;   // step1: the step of the iteration before
+	double ig, dg, gg;               // of the Lanczos step: 1/gam, delta/gam, gam/gam_prev
+	double wig, a2, a3, ia1, step;   // of the direction update: 1/gam, the rotations' entries, 1/a1, the solution's step
+	double step1;                    // the step of the iteration before
 	int stop;   // 1: last iteration; 2: breakdown before the update; 4: a non-finite value
 };
 
@@ -701,70 +967,66 @@ struct QtScal {
 // registers to the loop's state, whose accesses on the stack miss L1 after every
 // team barrier: 157 against 117 us per iteration).
 
-// v_p(j+1) = A z - dg v_p(j) - gg v_p(j-1) into v_p(j-1)'s buffer and z_p = v_p / BAB;
-// returns this thread's share of z_p.v_p
-__device__ __forceinline__ double qt_v_elems(int ne, int tid, int nth, const double *Ahp, const double *p0, double *p1,
-                                             const double *ibab, double *z1, double ig, double dg, double gg)
+// v_p(j+1) = A z - dg v_p(j) - gg v_p(j-1) into v_p(j-1)'s buffer and z_p = v_p / BAB
+__device__ __forceinline__ void qt_v_elems(int ne, int tid, int nth, const double *Ahp, const double *p0, double *p1,
+                                           const double *bab, double *z1, double ig, double dg, double gg)
 {
-	double acc = 0.0;
 	for (int e = tid; e < ne; e += nth) {
-		const double vn = Ahp[e] * ig - dg * p0[e] - gg * p1[e], z = vn * ibab[e];
+		const double vn = lin3(Ahp[e], ig, dg, p0[e], gg, p1[e]);
 		p1[e] = vn;
-		z1[e] = z;
-		acc += z * vn;
+		z1[e] = vn / bab[e];
 	}
-	return acc;
 }
 
-// w(j+1) = (z~(j) - a3 w(j-1) - a2 w(j)) / a1 into w(j-1)'s buffer, and the steps of
-// the solution: 0 none, 1 x += step w(j+1), 2 x += step1 w(j) + step w(j+1)
+// w(j+1) = (z~(j) / gam - a3 w(j-1) - a2 w(j)) / a1 into w(j-1)'s buffer, and the steps
+// of the solution: 0 none, 1 x += step w(j+1), 2 x += step1 w(j) + step w(j+1)
 template <class V>
 __device__ __forceinline__ void qt_w_update(int steps, int nn, int ne, int tid, int nth, const QtScal &ms, const V *z,
                                             double2 *wo, const double2 *wc, double2 *xu, const double *zp, double *po,
                                             const double *pc, double *xp)
 {
-	const double k1 = ms.k1, k2 = ms.k2, k3 = ms.k3, s0 = ms.step, s1 = ms.step1;
+	const double ig = ms.wig, a2 = ms.a2, a3 = ms.a3, ia1 = ms.ia1, s0 = ms.step, s1 = ms.step1;
 	for (int A = tid; A < nn; A += nth) {
 		const V zz = z[A];
 		const double2 o = wo[A], w = wc[A];
 		double2 x = make_double2(0.0, 0.0);
 		if (steps > 0)
 			x = xu[A];
-		const double2 wn = make_double2(widen(zz.x) * k1 - k3 * o.x - k2 * w.x, widen(zz.y) * k1 - k3 * o.y - k2 * w.y);
+		const double2 wn = make_double2(lin3(widen(zz.x), ig, a3, o.x, a2, w.x) * ia1,
+		                                lin3(widen(zz.y), ig, a3, o.y, a2, w.y) * ia1);
 		wo[A] = wn;
 		if (steps > 1) {
-			x.x += s1 * w.x;
-			x.y += s1 * w.y;
+			x.x = madd(s1, w.x, x.x);
+			x.y = madd(s1, w.y, x.y);
 		}
 		if (steps > 0)
-			xu[A] = make_double2(x.x + s0 * wn.x, x.y + s0 * wn.y);
+			xu[A] = make_double2(madd(s0, wn.x, x.x), madd(s0, wn.y, x.y));
 	}
 	for (int e = tid; e < ne; e += nth) {
 		const double w = pc[e];
 		double x = steps > 0 ? xp[e] : 0.0;
-		const double wn = zp[e] * k1 - k3 * po[e] - k2 * w;
+		const double wn = lin3(zp[e], ig, a3, po[e], a2, w) * ia1;
 		po[e] = wn;
 		if (steps > 1)
-			x += s1 * w;
+			x = madd(s1, w, x);
 		if (steps > 0)
-			xp[e] = x + s0 * wn;
+			xp[e] = madd(s0, wn, x);
 	}
 }
 
 // Correction solve by preconditioned MINRES (Elman, Silvester and Wathen,
 // "Finite Elements and Fast Iterative Solvers", Alg. 4.1) on the constrained
 // system [C^T K C, C^T G; G^T C, 0][x_u; x_p] = [R_m; -R_c] from zero, with the
-// preconditioner diag(V-cycle, BAB); K in TI, G to FP64 accuracy, Lanczos and
+// preconditioner diag(V-cycle, BAB); K in TI, G and G^T in FP64, Lanczos and
 // direction vectors FP64; x into a.dd, a.dpv, two iterations' steps at a time.
 template <class TI>
-__device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rtol, int maxit)
+__device__ __noinline__ int qt_minres(QtSync &team, const QtArgs<TI> &a, double rtol, int maxit)
 {
 	typedef typename Q2T<TI>::t V;
 	__shared__ QtScal ms;
-	Sync sy = team;
+	QtSync sy = team;
 	const DevLevel &L = a.L;
 	const QtLevel<TI> &Q = a.H.lv[a.H.nlev - 1];
-	double pdot = 0.0;
 	{
 		const double2 zero2 = make_double2(0.0, 0.0);
 		const int tid = sy.tid(), nth = sy.nth(), nn = L.nno, ne = L.nel;
@@ -781,10 +1043,9 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 			a.dd[A] = zero2;
 		}
 		for (int e = tid; e < ne; e += nth) {
-			const double v = -a.Rc[e], z = v * a.ibab[e];
+			const double v = -a.Rc[e];
 			a.mvp[0][e] = v;
-			a.mzp[0][e] = z;
-			pdot += z * v;
+			a.mzp[0][e] = v / a.bab[e];
 			a.mvp[1][e] = 0.0;
 			a.mwp[0][e] = 0.0;
 			a.mwp[1][e] = 0.0;
@@ -805,36 +1066,31 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 #pragma unroll 1
 	while (it < maxit) {
 		if (it >= 0) {
-			const int tid = sy.tid(), nth = sy.nth();
+			const int tid = sy.id(), nth = sy.nth();
 			double dl[1] = {0.0};
 			{
 				const V *z = a.mz[cv];
 				const double *zp = a.mzp[cv];
 				const TI *zf = reinterpret_cast<const TI *>(z);
-				// nodes and elements in one range: with two loops each would end in a
-				// trip for the few left over
-				const int nn = L.nno, ni = nn + L.nel;
-				for (int A = tid; A < ni; A += nth) {
-					if (A >= nn) {
-						const int e = A - nn;
-						const double t = qt_gt_elem(Q, L, zf, e);
-						a.Ahp[e] = t;
-						dl[0] += t * zp[e];
-						continue;
-					}
+				for (int A = tid; A < L.nno; A += nth) {
 					TI k0, k1;
 					double g0, g1;
 					const V zz = z[A];
 					qt_kr_node(Q, zf, A, k0, k1);
-					qt_g_node(Q, L, zp, A, g0, g1);
+					qt_g_node(Q, L, a.ge, zp, A, g0, g1);
 					const double2 az = make_double2(widen(k0) + g0, widen(k1) + g1);
 					a.Kd[A] = az;
-					dl[0] += az.x * widen(zz.x) + az.y * widen(zz.y);
+					dl[0] = add2(dl[0], az.x, widen(zz.x), az.y, widen(zz.y));
+				}
+				for (int e = tid; e < L.nel; e += nth) {
+					const double t = qt_gt_elem(Q, L, a.ge, zf, e);
+					a.Ahp[e] = t;
+					dl[0] = madd(t, zp[e], dl[0]);
 				}
 			}
 			sy.reduce_then<1>(dl, [&](const double (&v)[1]) {
-				ms.delta = v[0] * ms.ig * ms.ig;
-				ms.dg = ms.delta * ms.ig;
+				ms.delta = v[0] / (ms.gam * ms.gam);
+				ms.dg = ms.delta / ms.gam;
 			});
 			// v(j+1) into v(j-1)'s buffer, its TI copy as the V-cycle's right-hand side,
 			// and z_p(j+1) = v_p(j+1) / BAB
@@ -844,7 +1100,7 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 				double2 *vo = a.mv[1 - cv];
 				for (int A = tid; A < L.nno; A += nth) {
 					const double2 az = a.Kd[A], vc = v[A], vp = vo[A];
-					const double2 vn = make_double2(az.x * ig - dg * vc.x - gg * vp.x, az.y * ig - dg * vc.y - gg * vp.y);
+					const double2 vn = make_double2(lin3(az.x, ig, dg, vc.x, gg, vp.x), lin3(az.y, ig, dg, vc.y, gg, vp.y));
 					vo[A] = vn;
 					V w;
 					w.x = narrow_to<TI>(vn.x);
@@ -852,9 +1108,8 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 					Q.b[A] = w;
 				}
 			}
-			pdot = 0.0;
 			if (!defer)
-				pdot = qt_v_elems(L.nel, tid, nth, a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.ibab, a.mzp[1 - cv], ig, dg, gg);
+				qt_v_elems(L.nel, tid, nth, a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv], ig, dg, gg);
 			sy.sync();
 		}
 		double dot[1];
@@ -869,13 +1124,16 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 			if (steps >= 0)
 				qt_w_update(steps, L.nno, L.nel, tid, nth, ms, a.mz[1 - cv], a.mw[cw], a.mw[1 - cw], a.dd, a.mzp[1 - cv],
 				            a.mwp[cw], a.mwp[1 - cw], a.dpv);
-			pdot = qt_v_elems(L.nel, tid, nth, a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.ibab, a.mzp[1 - cv], ms.ig, ms.dg,
-			                  ms.gg);
+			qt_v_elems(L.nel, tid, nth, a.Ahp, a.mvp[cv], a.mvp[1 - cv], a.bab, a.mzp[1 - cv], ms.ig, ms.dg, ms.gg);
 		});
-		dot[0] += pdot;
+		{
+			const double *zp = a.mzp[1 - cv], *vp = a.mvp[1 - cv];
+			const int nth = sy.nth();
+			for (int e = sy.id(); e < L.nel; e += nth)
+				dot[0] = madd(zp[e], vp[e], dot[0]);
+		}
 		sy.reduce_then<1>(dot, [&](const double (&v)[1]) {
-			const double gn2 = fmax(v[0], 0.0);
-			const double gam_next = sqrt(gn2);
+			const double gam_next = sqrt(fmax(v[0], 0.0));
 			if (it < 0) {
 				ms.gam = gam_next;
 				ms.gam_prev = 1.0;
@@ -883,25 +1141,26 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 				ms.c_prev = ms.c_cur = 1.0;
 				ms.s_prev = ms.s_cur = 0.0;
 				ms.ig = 1.0 / gam_next;
-				ms.gg = gam_next;
+				ms.gg = gam_next;   // (gam_prev = 1)
 				ms.stop = v[0] > 0.0 ? 0 : 3;
 				return;
 			}
-			const double a0 = ms.c_cur * ms.delta - ms.c_prev * ms.s_cur * ms.gam;
-			const double a1s = a0 * a0 + gn2;
-			const double a2 = ms.s_cur * ms.delta + ms.c_prev * ms.c_cur * ms.gam;
+			const double cs = __dmul_rn(ms.c_prev, ms.s_cur), cc = __dmul_rn(ms.c_prev, ms.c_cur);
+			const double a0 = __fma_rn(ms.c_cur, ms.delta, -__dmul_rn(cs, ms.gam));
+			const double a1 = sqrt(__fma_rn(a0, a0, __dmul_rn(gam_next, gam_next)));
+			const double a2 = __fma_rn(cc, ms.gam, __dmul_rn(ms.s_cur, ms.delta));
 			const double a3 = ms.s_prev * ms.gam;
-			const double ia1 = rsqrt(a1s);
 			ms.stop = 0;
-			if (!(a1s > 0.0) || !isfinite(a1s)) {
-				ms.stop = isfinite(a1s) ? 2 : 6;
+			if (!(a1 > 0.0) || !isfinite(a1)) {
+				ms.stop = isfinite(a1) ? 2 : 6;
 				return;
 			}
-			const double c_next = a0 * ia1, s_next = gam_next * ia1;
+			const double c_next = a0 / a1, s_next = gam_next / a1;
 			ms.step1 = ms.step;
-			ms.k1 = ms.ig * ia1;
-			ms.k2 = a2 * ia1;
-			ms.k3 = a3 * ia1;
+			ms.wig = ms.ig;
+			ms.a2 = a2;
+			ms.a3 = a3;
+			ms.ia1 = 1.0 / a1;
 			ms.step = c_next * ms.eta;
 			ms.eta = -s_next * ms.eta;
 			ms.gam_prev = ms.gam;
@@ -931,10 +1190,10 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 				const double s = ms.step;
 				for (int A = tid; A < L.nno; A += nth) {
 					const double2 w = a.mw[cw][A], x = a.dd[A];
-					a.dd[A] = make_double2(x.x + s * w.x, x.y + s * w.y);
+					a.dd[A] = make_double2(madd(s, w.x, x.x), madd(s, w.y, x.y));
 				}
 				for (int e = tid; e < L.nel; e += nth)
-					a.dpv[e] += s * a.mwp[cw][e];
+					a.dpv[e] = madd(s, a.mwp[cw][e], a.dpv[e]);
 			}
 			break;
 		}
@@ -962,7 +1221,7 @@ __device__ __noinline__ int qt_minres(Sync &team, const QtArgs<TI> &a, double rt
 
 // The whole converged solve of one refined model on the team `sy`.
 template <class TI>
-__device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
+__device__ void qt_solve(const QtArgs<TI> &a, QtSync &sy)
 {
 	const int tid = sy.tid(), nth = sy.nth();
 	const QtHier<TI> &H = a.H;
@@ -970,7 +1229,7 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 	int *status = &a.sc->status;
 
 	for (int e = tid; e < L.nel; e += nth)
-		a.ibab[e] = 1.0 / a.bab[e];
+		qt_g_table(L, e, a.ge);
 	// -- per step: every level's reduced operator C^T K C in TI, and its diagonal
 	for (int l = 0; l < H.nlev; l++) {
 		const QtLevel<TI> &Q = H.lv[l];
@@ -1073,13 +1332,13 @@ __device__ void qt_solve(const QtArgs<TI> &a, Sync &sy)
 
 // One refined model on the whole cooperative grid, or on one cluster.
 template <class TI>
-__global__ void __launch_bounds__(kTeamThreads) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
+__global__ void __launch_bounds__(kTeamThreads, 1) k_stokes_qt(const __grid_constant__ QtArgs<TI> a)
 {
 	__shared__ QtArgs<TI> sa;
 	load_args(sa, a);
-	__shared__ double cpart[2 * kRedWidth];
-	Sync sy = sa.cluster ? Sync::of(SYNC_CLUSTER, cpart, blockIdx.x, gridDim.x)
-	                     : Sync::of(SYNC_GRID, sa.red.part, blockIdx.x, gridDim.x);
+	__shared__ double cpart[2 * kQtPartials];
+	QtSync sy = sa.cluster ? QtSync::of(SYNC_CLUSTER, cpart, blockIdx.x, gridDim.x, true)
+	                       : QtSync::of(SYNC_GRID, sa.red.part, blockIdx.x, gridDim.x, true);
 	qt_solve<TI>(sa, sy);
 	if (sa.cluster)
 		cg::this_cluster().sync();   // no block leaves while another reads its partials
@@ -1091,11 +1350,11 @@ __global__ void __launch_bounds__(kTeamThreads) k_stokes_qt(const __grid_constan
 // barriers, so clusters never wait on one another.  The rank-0 block draws and
 // every block reads the draw from its shared memory.
 template <class TI>
-__global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *models, int nmodels, int *queue)
+__global__ void __launch_bounds__(kBlock, 2) k_stokes_qt_batch(const QtArgs<TI> *models, int nmodels, int *queue)
 {
 	__shared__ QtArgs<TI> sa;
 	__shared__ int next;
-	__shared__ double cpart[2 * kRedWidth];
+	__shared__ double cpart[2 * kQtPartials];
 	cg::cluster_group cl = cg::this_cluster();
 	const int cs = (int)cl.num_blocks(), rank = (int)cl.block_rank();
 	for (;;) {
@@ -1108,7 +1367,7 @@ __global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *mo
 			if (m >= nmodels)
 				break;
 			load_args(sa, models[m]);
-			Sync sy = Sync::of(SYNC_CLUSTER, cpart, rank, cs);
+			QtSync sy = QtSync::of(SYNC_CLUSTER, cpart, rank, cs, false);
 			qt_solve<TI>(sa, sy);
 			cl.sync();   // no block starts the next model (or leaves) while another reads its partials
 		} else {
@@ -1118,7 +1377,7 @@ __global__ void __launch_bounds__(kBlock) k_stokes_qt_batch(const QtArgs<TI> *mo
 			if (m >= nmodels)
 				break;
 			load_args(sa, models[m]);
-			Sync sy = Sync::of(SYNC_BLOCK, nullptr, 0, 1);
+			QtSync sy = QtSync::of(SYNC_BLOCK, nullptr, 0, 1, false);
 			qt_solve<TI>(sa, sy);
 			__syncthreads();
 		}

@@ -60,9 +60,8 @@ struct QtHier {
 	int nblk;                               // levels lv[0..nblk-1] are small: block 0 alone runs them
 	int nc;                                 // reduced dofs of the coarsest level
 	const int *cdof;                        // [nc] their dof numbers
-	double *cwork;                          // [2 * nc * nc] the inversion's two buffers
-	T *cinv;                                // [nc * nc] inverse of the coarsest constrained operator
-	double *cvec;                           // [2 * nno_coarsest] a dof's row
+	double *cwork;                          // [2 * nc * (nc + 1)] the inversion's buffers
+	T *cinv;                                // [nc * nc] inverse of the coarsest constrained operator, by columns
 };
 
 template <class TI>
@@ -71,7 +70,7 @@ struct QtArgs {
 	QtHier<TI> H;
 	const double2 *F;
 	const double *bab;
-	double *ibab;                           // 1/bab, formed once per solve
+	double *ge;                             // [4*nel] G's entries by corner, formed once per solve
 	double2 *d, *V;
 	double *p;
 	// FP64 refinement and MINRES vectors

@@ -55,6 +55,8 @@ __global__ void k_tau(DevLevel L, const double2 *V, double accuracy, double *tau
                       unsigned long long *mins, int safe);
 __global__ void k_assemble_heat(DevLevel L, const double2 *V, const double *tau0, const double *tau1, double Q,
                                 double *HK, double *HC, double *HF);
+__global__ void k_assemble_heat_gauss(DevLevel L, const double2 *V, const double *tau0, const double *tau1, double Q,
+                                      double *HK, double *HC, double *HF);
 __global__ void k_assemble_heat_fast(DevLevel L, const double2 *V, const double *tau0, const double *tau1,
                                      double Q, double *HK, double *HC, double *HF);
 __global__ void k_heat_dt(DevLevel L, const double2 *V, unsigned long long *mins);
@@ -386,14 +388,16 @@ static void mg_team(mclg_ctx *c, void *kern)
 // The blocks that solve one refined model.  Up to kOneClusterNodes nodes one
 // cluster, whose barriers take 0.2 us instead of a grid's 1.2, with 512 threads a
 // block (52.6 us per MINRES iteration at 5125 nodes; 76.9 at 8847, where a grid
-// takes 71.1); up to kSpreadNodes four times the blocks its nodes fill, so that its
-// work uses more SMs (71.1 against 74.7 us at 8847 nodes, 74.0 with eight times;
-// 85.3 against 82.7 at 22433).
+// takes 74.7): a thread for each node.  Otherwise a grid of a thread for each node, at
+// most two blocks an SM.  The sums are formed in that grid's order on either team
+// (QtSync), so its size is part of the result's last bits and follows the mesh alone.
 static void qt_team(mclg_ctx *c, void *kern, int nn)
 {
-	constexpr int kOneCluster = 16, kOneClusterNodes = 6144, kSpreadNodes = 12288;
+	constexpr int kOneCluster = 16, kOneClusterNodes = 6144, kPerSm = 2;
+	static_assert(kOneClusterNodes <= kOneCluster * kTeamThreads, "a thread for each node");
 	c->qt_one_cluster = nn <= kOneClusterNodes && max_clusters(kern, kOneCluster, kTeamThreads) >= 1;
-	c->coop_qt = c->qt_one_cluster ? kOneCluster : coop_blocks(kern, c->num_sms, nn <= kSpreadNodes ? 4 * nn : nn);
+	const int room = coop_blocks(kern, c->num_sms, nn), most = kPerSm * c->num_sms;
+	c->coop_qt = c->qt_one_cluster ? kOneCluster : room < most ? room : most;
 }
 
 // ---- converged solvers: hierarchy of the uniform mesh -------------------------
@@ -579,6 +583,14 @@ constexpr int kSmallBlock = 64;
 static int small_blocks(size_t n)
 {
 	return (int)((n + kSmallBlock - 1) / kSmallBlock);
+}
+
+// A single refined model's matrix, load and heat rows keep their order of operations,
+// as its solver does (see k_qt.cu); a batch's members share the ensemble's stream and
+// are solved by teams whose size is timed, with sums in the order of those.
+static bool keeps_order(const mclg_ctx *c)
+{
+	return c->qt_on && !c->st_borrowed;
 }
 
 static int blocks_for(size_t n)
@@ -1020,15 +1032,14 @@ static int qt_setup(mclg_ctx *c, QtArgs<TI> &a, Prebuilt *pre)
 		}
 		H.nc = (int)cd.size();
 		CK(dev_upload(c, (int **)&H.cdof, cd));
-		CK(dev_zeros(c, &H.cwork, (size_t)H.nc * 2 * H.nc));
+		CK(dev_zeros(c, &H.cwork, 2 * (size_t)H.nc * (H.nc + 1)));
 		CK(dev_zeros(c, &H.cinv, (size_t)H.nc * H.nc));
-		CK(dev_zeros(c, &H.cvec, 2 * (size_t)S.nno));
 	}
 	const size_t nn = c->L.nno, ne = c->L.nel;
 	CK(dev_zeros(c, &a.R, nn));
 	CK(dev_zeros(c, &a.Kd, nn));
 	CK(dev_zeros(c, &a.dd, nn));
-	CK(dev_zeros(c, &a.ibab, ne));
+	CK(dev_zeros(c, &a.ge, 4 * ne));
 	CK(dev_zeros(c, &a.Rc, ne));
 	CK(dev_zeros(c, &a.dpv, ne));
 	CK(dev_zeros(c, &a.Ahp, ne));
@@ -1110,8 +1121,9 @@ static int stokes_qt_prepare(mclg_ctx *c)
 		                                                      c->cfg.mg_eta_avg, U.nno, nbu, cntu, U.X);
 		if ((rc = check_launch(c, "k_qt_inject")))
 			return rc;
-		k_assemble_stokes_fast<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->lvl_vis[k], c->lvl_buoy[k],
-		                                                                       c->lvl_K[k], c->lvl_F[k], c->lvl_Kd[k]);
+		auto *assemble = keeps_order(c) ? k_assemble_stokes : k_assemble_stokes_fast;
+		assemble<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->lvl_vis[k], c->lvl_buoy[k], c->lvl_K[k],
+		                                                         c->lvl_F[k], c->lvl_Kd[k]);
 		if ((rc = check_launch(c, "k_assemble_stokes")))
 			return rc;
 	}
@@ -1730,9 +1742,9 @@ int mclg_velocity_pressure_KGF_matrix(mclg_ctx *c)
 	if (c == NULL)
 		return MCLG_BAD_INPUT;
 	const int withK = c->cfg.precision == 0 || c->qt_on;
-	if (c->cfg.precision == 0)   // the replica: the reference's operation order
+	if (c->cfg.precision == 0 || keeps_order(c))
 		k_assemble_stokes<<<small_blocks(c->L.nno), kSmallBlock, 0, c->st>>>(c->L, c->vis, c->buoy, c->K, c->F, c->Kdiag);
-	else                         // K for the refined-mesh solver only, the load for all
+	else   // K for the refined-mesh solver only, the load for all
 		k_assemble_stokes_fast<<<small_blocks(c->L.nno), kSmallBlock, 0, c->st>>>(
 			c->L, c->vis, c->buoy, withK ? c->K : nullptr, c->F, c->Kdiag);
 	int rc = check_launch(c, "k_assemble_stokes");
@@ -1891,13 +1903,13 @@ static int launch_heat(mclg_ctx *c)
 	                                                f.precision != 0);
 	if ((rc = check_launch(c, "k_tau")))
 		return rc;
-	// the converged solvers take the heat rows with fewer FP64 operations (equal to
-	// the reference's to the last bits); the FP64 replica keeps its operation order
-	if (c->cfg.precision != 0)
-		k_assemble_heat_fast<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC,
-		                                                              c->HF);
-	else
-		k_assemble_heat<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC, c->HF);
+	// The converged solvers take the heat rows with fewer FP64 operations (equal to
+	// the reference's to the last bits): summed over the Gauss points beforehand on
+	// uniform meshes and in batches, at the Gauss points for a single refined model,
+	// whose pressure follows the last bits of T.  The FP64 replica keeps the
+	// reference's operation order.
+	auto *assemble = f.precision == 0 ? k_assemble_heat : keeps_order(c) ? k_assemble_heat_gauss : k_assemble_heat_fast;
+	assemble<<<small_blocks(L.nno), kSmallBlock, 0, c->st>>>(L, c->V, c->tau0, c->tau1, f.Q, c->HK, c->HC, c->HF);
 	if ((rc = check_launch(c, "k_assemble_heat")))
 		return rc;
 	k_heat_dt<<<blocks_for(L.nel), kBlock, 0, c->st>>>(L, c->V, c->mins);
