@@ -442,10 +442,8 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 	}
 	a.H.nlev = nlev;
 	a.H.nblk = nlev;
-	// small grids: one block beats team barriers; FP64 passes are bound by the FP64
-	// pipe of that block's SM, so there the limit is half (8 x 8 in one block took
-	// 57 us of a V-cycle's 150 at 128^2)
-	const int block_n = sizeof(TI) == 8 ? c->cfg.mg_block_n / 2 : c->cfg.mg_block_n;
+	// small grids: one block beats team barriers
+	const int block_n = mclg_block_n(&c->cfg);
 	for (int l = 0; l < nlev; l++)
 		if ((N0 >> l) <= block_n) {
 			a.H.nblk = l;

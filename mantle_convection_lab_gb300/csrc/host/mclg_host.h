@@ -62,6 +62,9 @@ typedef struct mclg_mesh {
 	mclg_level lev[MCLG_MAX_LEVEL];
 } mclg_mesh;
 
+/* elements per side up to which a grid of the uniform V-cycle runs in one block (mg_block_n) */
+int mclg_block_n(const mclg_config *cfg);
+
 /* Build the mesh the way Main.c:33-52 does on its first step, for one rank. */
 int mclg_mesh_build(mclg_mesh *m, const mclg_config *cfg);
 /* The same mesh stack from a given leaf set (finest-level Morton start codes). */
