@@ -470,6 +470,8 @@ size_t mclg_cnn_num_params(const mclg_cnn *net);
 int mclg_cnn_shape(const mclg_cnn *net, int *cin, int *width, int *depth, int *cout);
 int mclg_cnn_get_params(const mclg_cnn *net, float *out, size_t n);
 int mclg_cnn_set_params(mclg_cnn *net, const float *in, size_t n);   /* also resets the Adam moments */
+/* forward and gradient keep their device buffers with the network for the next call, 256 MiB at most
+   (larger ones are given back at the call's end); mclg_cnn_destroy frees them */
 int mclg_cnn_forward(mclg_cnn *net, const float *x, int batch, int h, int w, float *y);
 /* Mean squared error against target and its gradient (flat parameter layout). */
 int mclg_cnn_gradient(mclg_cnn *net, const float *x, const float *target, int batch, int h, int w,

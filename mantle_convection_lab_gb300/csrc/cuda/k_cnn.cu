@@ -42,8 +42,8 @@ struct mclg_cnn {
 	size_t part_cap;
 	cudaStream_t st;
 	// device buffers of mclg_cnn_forward and mclg_cnn_gradient, kept for the next
-	// call up to kPoolKeep bytes and freed with the network (allocating and freeing
-	// them took a third of a call); mu: one such call at a time
+	// call up to kPoolKeep bytes and freed with the network; mu: one call of these two
+	// at a time
 	char *pool;
 	size_t pool_cap;
 	pthread_mutex_t mu;
@@ -971,9 +971,11 @@ struct Pool {
 		w.W = W;
 	}
 };
-// One call on a network at a time; what it needed beyond kPoolKeep is given back
-// at its end (a call that large takes longer than an allocation).
-constexpr size_t kPoolKeep = size_t(1) << 30;
+// One call on a network at a time.  A pool of more than kPoolKeep is given back at
+// the call's end, so that several networks of a program leave the device's memory to
+// its models.  200 MB hold a training batch of eight 160 x 160 samples, for which
+// allocating and freeing took a third of a call; larger calls it holds up less.
+constexpr size_t kPoolKeep = size_t(256) << 20;
 struct Lock {
 	mclg_cnn *n;
 	explicit Lock(mclg_cnn *net) : n(net) { pthread_mutex_lock(&n->mu); }
