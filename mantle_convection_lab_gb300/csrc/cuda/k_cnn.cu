@@ -42,11 +42,21 @@ struct mclg_cnn {
 	size_t part_cap;
 	cudaStream_t st;
 	// device buffers of mclg_cnn_forward and mclg_cnn_gradient, kept for the next
-	// call up to kPoolKeep bytes and freed with the network; mu: one call of these two
-	// at a time
+	// call up to kPoolKeep bytes and freed with the network; mu: one of the calls that
+	// use them, grad or part, or change the parameters, at a time (train: one iteration)
 	char *pool;
 	size_t pool_cap;
 	pthread_mutex_t mu;
+};
+
+// The calls of one network that use its buffers or change its parameters, one at a
+// time; their work is ordered by the network's stream.
+struct Hold {
+	mclg_cnn *n;
+	explicit Hold(mclg_cnn *net) : n(net) { pthread_mutex_lock(&n->mu); }
+	~Hold() { pthread_mutex_unlock(&n->mu); }
+	Hold(const Hold &) = delete;
+	Hold &operator=(const Hold &) = delete;
 };
 
 namespace mclg {
@@ -926,6 +936,7 @@ int mclg_cnn_set_params(mclg_cnn *n, const float *in, size_t count)
 		mclg_set_error("parameter buffer has %zu entries, the network %zu", count, n ? n->nparam : 0);
 		return MCLG_BAD_INPUT;
 	}
+	Hold hold(n);
 	CKC(cudaMemcpyAsync(n->master, in, count * sizeof(float), cudaMemcpyHostToDevice, n->st));
 	CKC(cudaMemsetAsync(n->m, 0, count * sizeof(float), n->st));
 	CKC(cudaMemsetAsync(n->v, 0, count * sizeof(float), n->st));
@@ -971,22 +982,22 @@ struct Pool {
 		w.W = W;
 	}
 };
-// One call on a network at a time.  A pool of more than kPoolKeep is given back at
+// A pool of more than kPoolKeep is given back at
 // the call's end, so that several networks of a program leave the device's memory to
 // its models.  200 MB hold a training batch of eight 160 x 160 samples, for which
 // allocating and freeing took a third of a call; larger calls it holds up less.
 constexpr size_t kPoolKeep = size_t(256) << 20;
-struct Lock {
-	mclg_cnn *n;
-	explicit Lock(mclg_cnn *net) : n(net) { pthread_mutex_lock(&n->mu); }
+// Hold, and what the pool needs at the end of a call.
+struct Lock : Hold {
+	explicit Lock(mclg_cnn *net) : Hold(net) {}
 	~Lock()
 	{
+		cudaStreamSynchronize(n->st);   // (a call that failed half way: its copies and kernels end with it)
 		if (n->pool_cap > kPoolKeep) {
 			cudaFree(n->pool);
 			n->pool = nullptr;
 			n->pool_cap = 0;
 		}
-		pthread_mutex_unlock(&n->mu);
 	}
 };
 }  // namespace
@@ -1133,6 +1144,7 @@ int mclg_cnn_train(mclg_cnn *n, const float *x, const float *y, int nsamples, in
 		}
 		if (e != cudaSuccess)
 			break;
+		Hold hold(n);
 		rc = cnn_forward_dev(n, wk, bx, n->st);
 		if (rc)
 			break;
@@ -1179,6 +1191,7 @@ int mclg_cnn_adam_step(mclg_cnn *n, const float *grad, size_t count, float lr)
 	if (n == NULL || grad == NULL || count != n->nparam)
 		return MCLG_BAD_INPUT;
 	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+	Hold hold(n);
 	CKC(cudaMemcpyAsync(n->grad, grad, count * sizeof(float), cudaMemcpyHostToDevice, n->st));
 	n->adam_t++;
 	const float c1 = 1.f - powf(b1, (float)n->adam_t), c2 = 1.f - powf(b2, (float)n->adam_t);
