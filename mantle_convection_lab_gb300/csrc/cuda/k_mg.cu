@@ -178,7 +178,6 @@ __device__ void restrict_res(Part pt, const MGLevel<T> &F, const MGLevel<T> &C)
 // in global memory otherwise (8 x 8: 162 dofs).  Inverting in place in shared
 // memory takes 50 ranks of 2500 FP64 multiply-adds; as an augmented elimination
 // in global memory the set-up of a solve took 0.57 ms.
-constexpr int kCoarseShared = 50;
 
 // Tasks of each level's passes, on one block (0) and on the whole team (1).
 struct Splits {

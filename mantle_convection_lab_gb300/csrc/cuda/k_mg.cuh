@@ -20,13 +20,18 @@ struct MGLevel {
 	typename V2T<T>::t *invD, *xa, *xb, *b, *r;
 };
 
+// Dofs of the coarsest grid whose dense inverse lives in shared memory (4 x 4: 50).
+constexpr int kCoarseShared = 50;
+
 template <class T>
 struct MGHier {
 	int nlev;                    // number of levels
 	int nblk;                    // levels >= nblk run inside block 0 only
 	MGLevel<T> lv[kMaxLev];
-	T *cinv;                     // dense inverse of the coarsest operator [cnd*cnd]
-	double *cwork;               // [cnd * 2*cnd] scratch for the inversion
+	// coarsest grids of more than kCoarseShared dofs (else null): the dense inverse of
+	// the operator and the inversion's matrix, [cnd * cnd] each
+	T *cinv;
+	double *cwork;
 	int cnd;                     // 2 * n_coarsest^2
 	T omega;
 	int nu;                      // smoothing sweeps per side on the lfine finest levels
@@ -44,7 +49,6 @@ struct MGHier {
 // element of the uniform mesh, filled on the host.
 struct GTab {
 	double g0[4], g1[4];
-	float g0h[4], g0l[4], g1h[4], g1l[4];   // the same as float pairs: g = h + l
 };
 
 // The converged Stokes solve of one time step (FP64 state, TI inner solves).

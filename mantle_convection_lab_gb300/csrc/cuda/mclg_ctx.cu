@@ -478,8 +478,10 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 	}
 	const int ncn = a.H.lv[nlev - 1].n;
 	a.H.cnd = 2 * ncn * ncn;
-	CK(mg_alloc(c, &a.H.cinv, (size_t)a.H.cnd * a.H.cnd));
-	CK(mg_alloc(c, &a.H.cwork, (size_t)a.H.cnd * 2 * a.H.cnd));
+	if (a.H.cnd > kCoarseShared) {
+		CK(mg_alloc(c, &a.H.cinv, (size_t)a.H.cnd * a.H.cnd));
+		CK(mg_alloc(c, &a.H.cwork, (size_t)a.H.cnd * a.H.cnd));
+	}
 	a.H.omega = (TI)c->cfg.mg_omega;
 	a.H.nu = c->cfg.mg_smooth < 1 ? 1 : c->cfg.mg_smooth;
 	a.H.nu_c = c->cfg.mg_smooth_coarse < 1 ? a.H.nu : c->cfg.mg_smooth_coarse;
@@ -525,10 +527,6 @@ static int mg_setup(mclg_ctx *c, MGArgs<TI> &a)
 			}
 			a.gt.g0[k] = g0;
 			a.gt.g1[k] = g1;
-			a.gt.g0h[k] = (float)g0;
-			a.gt.g0l[k] = (float)(g0 - (double)a.gt.g0h[k]);
-			a.gt.g1h[k] = (float)g1;
-			a.gt.g1l[k] = (float)(g1 - (double)a.gt.g1h[k]);
 		}
 	}
 	a.vis = c->vis;
