@@ -1008,7 +1008,7 @@ struct MinresScal {
 // Elman, Silvester and Wathen, "Finite Elements and Fast Iterative Solvers",
 // Alg. 4.1) on [K G; G^T 0][x_u; x_p] = [R_m; -R_c] from a zero start, with
 // the block-diagonal SPD preconditioner diag(V-cycle, BAB).  K is applied in
-// TI, G and G^T to FP64 accuracy, in one pass over the mesh; Lanczos and
+// TI, G in FP64 and G^T in float pairs (gt_elem), in one pass over the mesh; Lanczos and
 // direction vectors are FP64 and x_u, x_p accumulate in a.dd, a.dpv.  The FP64
 // refinement around this solve restores full accuracy.  Stops when the
 // M^-1-norm of the residual has dropped by rtol.  Returns the iterations.

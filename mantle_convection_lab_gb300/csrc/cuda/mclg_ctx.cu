@@ -364,13 +364,12 @@ static int max_clusters(void *kern, int cs, int threads)
 	return nc;
 }
 
-// The blocks that solve one uniform model: a single cluster for small meshes in
-// FP32, whose iteration is a chain of barriers (0.2 us in a cluster, 1.2 in a
-// grid): on 16 blocks of 512 threads 34 against 44 us per MINRES iteration at 64^2
-// and 55 against 55 at 128^2, 46 against 69 and 69 against 79 per inner CG; at
-// 256^2 the grid wins (125 against 77 us when the passes took longer).  FP64 passes
-// need the whole device's FP64 pipes from 64^2 on (122 against 84 us; 59 against
-// 62 at 32^2).
+// The blocks that solve one uniform model: a single cluster for small meshes, whose
+// iteration is a chain of barriers (0.2 us in a cluster, 1.2 in a grid).  On 16 blocks
+// of 512 threads against the grid, us per MINRES iteration in mixed precision: 34 / 45
+// at 64^2, 56 / 58 at 128^2, 120 / 73 at 256^2; per inner CG of the Uzawa correction
+// 47 / 70, 69 / 79 and 129 / 95.  FP64 passes need the whole device's FP64 pipes
+// earlier: 38 / 49 at 16^2, 60 / 61 at 32^2, 123 / 85 at 64^2.
 static int mg_cluster_threads(const mclg_ctx *c)
 {
 	return c->cfg.precision == 2 ? kBlock : kTeamThreads;
@@ -387,8 +386,8 @@ static void mg_team(mclg_ctx *c, void *kern)
 
 // The blocks that solve one refined model.  Up to kOneClusterNodes nodes one
 // cluster, whose barriers take 0.2 us instead of a grid's 1.2, with 512 threads a
-// block (52.6 us per MINRES iteration at 5125 nodes; 76.9 at 8847, where a grid
-// takes 74.7): a thread for each node.  Otherwise a grid of a thread for each node, at
+// block (45 against 58 us per MINRES iteration at 1347 nodes, 58 against 72 at 5125;
+// with two nodes a thread, 77 against 75 at 8847): a thread for each node.  Otherwise a grid of a thread for each node, at
 // most two blocks an SM.  The sums are formed in that grid's order on either team
 // (QtSync), so its size is part of the result's last bits and follows the mesh alone.
 static void qt_team(mclg_ctx *c, void *kern, int nn)

@@ -8,7 +8,7 @@
  * composite creep viscosity at the node's stress and new r, clipped to
  * [lowest_vis, highest_vis].  A node's steps depend on one another and each is
  * a chain of FP64 pow/exp: on GB300 one thread per node would need of the
- * order of 10^4 cycles a step (FP64 at 1/64 of the FP32 rate), no faster than
+ * order of 10^4 cycles a step (FP64 at 1/56 of the FP32 rate), no faster than
  * a host core, so this runs on host threads, nodes in chunks.
  *
  * Restructured from the reference's loop order (all nodes per step) into all
