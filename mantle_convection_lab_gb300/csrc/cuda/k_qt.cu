@@ -20,6 +20,13 @@ namespace mclg {
 
 MCLG_SHAPE_UPLOAD(upload_shape_tables_qt)
 
+// ---- rounding -----------------------------------------------------------------------
+// Where a multiply-add could be formed in more than one way, the way is stated.
+__device__ __forceinline__ float madd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double madd(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+
 // ---- values through the constraints ----------------------------------------------
 // dof (2*node + component) of a primal vector: stored if reduced, the weighted
 // sum of its reduced dofs if constrained, 0 if fixed.
@@ -133,8 +140,8 @@ struct QtXFirst {
 	{
 		const X2 bv = b[B], dv = reinterpret_cast<const X2 *>(invD)[B];
 		X2 o;
-		o.x = omega * dv.x * bv.x;
-		o.y = omega * dv.y * bv.y;
+		o.x = mul(mul(omega, dv.x), bv.x);
+		o.y = mul(mul(omega, dv.y), bv.y);
 		return o;
 	}
 };
@@ -181,9 +188,6 @@ __device__ __forceinline__ void qt_kr_node(const QtLevel<TI> &L, const TI *__res
 	const QtXStored<TI> src{reinterpret_cast<const typename Q2T<TI>::t *>(xf)};
 	qt_kr_node_src(L, src, A, y0, y1);
 }
-
-__device__ __forceinline__ float madd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double madd(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // a b - c d - e f, as every recurrence of vectors here rounds it
 __device__ __forceinline__ double lin3(double a, double b, double c, double d, double e, double f)
@@ -602,8 +606,8 @@ __device__ __forceinline__ typename Q2T<TI>::t qt_sweep_node(const QtLevel<TI> &
 	const uchar2 k = reinterpret_cast<const uchar2 *>(L.kind)[A];
 	qt_kr_node_src(L, src, A, y0, y1);
 	V o;
-	o.x = k.x == 1 ? x.x + omega * dg.x * (b.x - y0) : TI(0);
-	o.y = k.y == 1 ? x.y + omega * dg.y * (b.y - y1) : TI(0);
+	o.x = k.x == 1 ? madd(mul(omega, dg.x), b.x - y0, x.x) : TI(0);
+	o.y = k.y == 1 ? madd(mul(omega, dg.y), b.y - y1, x.y) : TI(0);
 	return o;
 }
 

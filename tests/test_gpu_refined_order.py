@@ -30,12 +30,15 @@ from mantle_convection_lab_gb300.amr import CFG2_INPUT, uniform_leaves  # noqa: 
 pytestmark = pytest.mark.gpu
 
 STRIDE = 61
-# base side, refinement levels above it, ln(viscosity contrast), precision
+# base side, refinement levels above it, ln(viscosity contrast), other options
 CASES = {
-    "cluster_mixed": (32, 2, 2.3025850929940456, 1),
-    "cluster_fp64": (32, 2, 2.3025850929940456, 2),
-    "grid_mixed": (64, 2, 6.907755278982137, 1),
-    "grid_two_trips_mixed": (128, 3, 9.210340371976184, 1),
+    "cluster_mixed": (32, 2, 2.3025850929940456, {}),
+    "cluster_fp64": (32, 2, 2.3025850929940456, {"precision": 2}),
+    "cluster_two_sweeps": (32, 2, 2.3025850929940456, {"mg_smooth": 2}),
+    "cluster_long_box": (32, 2, 2.3025850929940456, {"model_length": 1.7}),
+    "grid_mixed": (64, 2, 6.907755278982137, {}),
+    "grid_three_sweeps": (64, 2, 6.907755278982137, {"mg_smooth": 3}),
+    "grid_two_trips_mixed": (128, 3, 9.210340371976184, {}),
 }
 
 
@@ -50,15 +53,17 @@ def temperature(x, z):
     return np.where(z <= 0.0, 1.0, np.where(z >= 1.0, 0.0, T))
 
 
-def fields(base, extra, A, precision):
+def fields(base, extra, A, opts):
     c = Config.from_input(CFG2_INPUT)
     F = base.bit_length() - 1 + extra
     c.level, c.mg_min_level = F + 1, 4
     c.Rayleigh, c.A = 1e7, A
-    c.precision, c.warm_start, c.stokes_method = precision, 3, 1
+    c.precision, c.warm_start, c.stokes_method = 1, 3, 1
     c.stokes_rtol = max(1e-12, 6e-18 * 4.0 ** F)
     c.outer_rtol, c.max_outer, c.max_refine = 1e-2, 2000, 40
     c.mg_smooth, c.mg_eta_avg = 1, 1
+    for k, v in opts.items():
+        setattr(c, k, v)
     out, its = {}, []
     with Model(c, leaves=uniform_leaves(F, F - extra)) as m:
         m.initial_temperature()
