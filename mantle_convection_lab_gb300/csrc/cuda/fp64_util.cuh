@@ -62,9 +62,9 @@ __device__ __forceinline__ void diff4(float a, float b, float c, float d, float 
 // 2 = (ex+1,ez+1), 3 = (ex+1,ez)): g0 [(u0+u1) - (u2+u3)] + g1 [(w0+w3) - (w1+w2)].
 // In FP32 the sums run as float pairs on the FP32 pipe and the FP64 pipe only adds and
 // scales the result: to 2^-52 of the largest product where the corners' values are of
-// one size, to 2^-47 over 12 binades (400000 random elements each; the products summed
-// in float pairs corner by corner, as before, 2^-52 and 2^-46.5, and 2^-43 where the
-// element is not square).  For the uniform meshes' MINRES: the FP64 residual around it
+// one size, to 2^-47 over 12 binades (400000 random elements each; summing the products
+// in float pairs corner by corner gives 2^-52 and 2^-46.5, and 2^-43 where the element
+// is not square).  For the uniform meshes' MINRES: the FP64 residual around it
 // runs on the other overload.
 __device__ __forceinline__ double gt_elem(float u0, float u1, float u2, float u3, float w0, float w1, float w2, float w3,
                                           double g0, double g1)
